@@ -36,10 +36,6 @@ __device__ __forceinline__ double Ffoo(const double *__restrict__ f, const Geo &
   size_t ld = (size_t)g.n * g.n;
   return f[(size_t)(c + (size_t)d * g.nocc) * ld + a + (size_t)b * g.n];
 }
-__device__ __forceinline__ double RV(const double *__restrict__ rv, int nocc, int i, int j, int k,
-                                     int l) {
-  return rv[i + (size_t)nocc * (j + (size_t)nocc * (k + (size_t)nocc * l))];
-}
 // AuxCoeff(g1,g2,g3,g4): g.same if the four orbital groups are equal, else lambda.
 __device__ __forceinline__ double AC(const Geo &g, int a, int b, int c, int d, double lam) {
   return (a == b && b == c && c == d) ? g.same : lam;
@@ -51,352 +47,377 @@ __device__ __forceinline__ int AuxInd(int a, int b) {
   return 0;
 }
 
-// ---------------------------------------------------------------------------
-// One-body matrices (lambda dependent): HNO, AuxI, AuxIO; column-major n x n.
-__global__ void k_onebody(Geo g, const double *__restrict__ h, const double *__restrict__ occ,
-                          const int *__restrict__ grp, const double *__restrict__ fofo,
-                          const double *__restrict__ ffoo, double lam, double *__restrict__ hno,
-                          double *__restrict__ auxi, double *__restrict__ auxio) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  int j = blockIdx.y * blockDim.y + threadIdx.y;
-  if (i >= g.n || j >= g.n) return;
-  int gi = grp[i], gj = grp[j];
-  double hv = h[i + (size_t)j * g.n];
-  double corr = 0.0, ai = 0.0, aio = 0.0;
-  for (int k = 0; k < g.nocc; ++k) {
-    int gk = grp[k];
-    double ok = occ[k];
-    double jv = Ffoo(ffoo, g, i, j, k, k);          // (ij|kk)
-    double kv = Fofo(fofo, g, j, k, i, k);          // (jk|ik)
-    if (gi == gj && gk != gi) corr += ok * (2.0 * jv - kv);
-    double t = ok * (2.0 * AC(g, gi, gj, gk, gk, lam) * jv - AC(g, gi, gi, gj, gk, lam) * kv);
-    ai += t;
-    if (k < g.nin) aio += t;
-  }
-  size_t o = i + (size_t)j * g.n;
-  hno[o] = (gi != gj) ? lam * hv : (g.ab1 ? -corr : hv + (1.0 - lam) * corr);
-  auxi[o] = ai;
-  auxio[o] = aio;
+// RDM2val(i, j, k, l) of active orbitals (abfofo.f90:84-92), indices within the active block.
+__device__ __forceinline__ double RVa(const double *__restrict__ rv, int na, int i, int j, int k,
+                                      int l) {
+  return rv[i + na * (j + na * (k + (size_t)na * l))];
 }
 
-// WMAT(k, r) = sum_{l,i,j < nocc} AuxCoeff(k,l,i,j) (kl|ij) RDM2val(i,j,r,l); zero for r >= nocc.
-// WMAT[k, r] = sum_{i,j,l < nocc} AC(k, l, i, j) (kl|ij) RDM2val(i, j, r, l) for r < nocc
-// is a product Fw RV' with K = nocc^3 (kappa = i + nocc (j + nocc l)):
-//   Fw[k + n kappa] = AC(groups of k, l, i, j) (ij|kl)     (n x K; consecutive k are
-//                                                           consecutive FOFO elements)
-//   RV'[kappa + K r] = RDM2val(i, j, r, l)                  (K x nocc)
-// so it runs as one FP64 DGEMM instead of an nocc^3 loop per element on the CUDA cores.
-__global__ void k_pack_wmat_f(Geo g, const int *__restrict__ grp, const double *__restrict__ fofo,
-                              double lam, double *__restrict__ fw) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= g.n) return;
-  const int K = g.nocc * g.nocc * g.nocc, gk = grp[k];
-  for (int kappa = blockIdx.y; kappa < K; kappa += gridDim.y) {  // i + nocc (j + nocc l)
-    const int i = kappa % g.nocc, j = (kappa / g.nocc) % g.nocc, l = kappa / (g.nocc * g.nocc);
-    fw[k + (size_t)g.n * kappa] = AC(g, gk, grp[l], grp[i], grp[j], lam) * Fofo(fofo, g, i, j, k, l);
-  }
-}
-__global__ void k_pack_wmat_rv(int nocc, const double *__restrict__ rv, double *__restrict__ rvp) {
-  const size_t K = (size_t)nocc * nocc * nocc;
-  const size_t total = K * nocc;
-  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total;
-       t += (size_t)gridDim.x * blockDim.x) {
-    const size_t kappa = t % K;
-    const int r = (int)(t / K);
-    const int i = (int)(kappa % nocc), j = (int)((kappa / nocc) % nocc), l = (int)(kappa / ((size_t)nocc * nocc));
-    rvp[t] = RV(rv, nocc, i, j, r, l);
-  }
-}
-
-// E_CAS two-electron part: sum_{ijkl < nocc} RDM2val(i,j,k,l) (ij|kl); per-block partials.
-__global__ void k_etwo(Geo g, const double *__restrict__ ffoo, const double *__restrict__ rv,
-                       double *__restrict__ part) {
-  __shared__ double red[256];
-  size_t total = (size_t)g.nocc * g.nocc * g.nocc * g.nocc;
-  double s = 0.0;
-  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total;
-       t += (size_t)gridDim.x * blockDim.x) {
-    int i = t % g.nocc;
-    size_t r = t / g.nocc;
-    int j = r % g.nocc;
-    r /= g.nocc;
-    int k = r % g.nocc;
-    int l = (int)(r / g.nocc);
-    s += rv[t] * Ffoo(ffoo, g, i, j, k, l);
-  }
-  red[threadIdx.x] = s;
-  __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) part[blockIdx.x] = red[0];
-}
-
-// ---------------------------------------------------------------------------
-// 2-RDM intermediates (lambda independent). Capital letters are orbital
-// indices T = nin + t of active orbitals; small letters index the active block.
-
-// Z1[a,b,c,d] = sum_tu (ab|TU) RV[T,U,C,D]; a < n, b < nocc, c,d < nact.
-__global__ void k_z1(Geo g, const double *__restrict__ fofo, const double *__restrict__ rv,
-                     double *__restrict__ z) {
-  size_t total = (size_t)g.n * g.nocc * g.nact * g.nact;
-  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total;
-       t += (size_t)gridDim.x * blockDim.x) {
-    int a = t % g.n;
-    size_t r = t / g.n;
-    int b = r % g.nocc;
-    r /= g.nocc;
-    int c = r % g.nact, d = (int)(r / g.nact);
-    double s = 0.0;
-    for (int u = 0; u < g.nact; ++u)
-      for (int tt = 0; tt < g.nact; ++tt)
-        s += Fofo(fofo, g, g.nin + tt, g.nin + u, a, b) *  // (ab|TU) as (TU|ab): coalesced in a
-             RV(rv, g.nocc, g.nin + tt, g.nin + u, g.nin + c, g.nin + d);
-    z[t] = s;
-  }
-}
-
-// Z4[p,r,q,s] = sum_tu (rU|pT) RV[T,Q,S,U];  Z7[p,r,q,s] = sum_tu (rU|pT) RV[T,Q,U,S]
-// (p fastest, so that the element kernel reads them along consecutive p).
-__global__ void k_z47(Geo g, const double *__restrict__ fofo, const double *__restrict__ rv,
-                      double *__restrict__ z4, double *__restrict__ z7) {
-  size_t total = (size_t)g.n * g.n * g.nact * g.nact;
-  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total;
-       t += (size_t)gridDim.x * blockDim.x) {
-    int p = t % g.n;
-    size_t r0 = t / g.n;
-    int r = r0 % g.n;
-    r0 /= g.n;
-    int q = r0 % g.nact, s = (int)(r0 / g.nact);
-    int Q = g.nin + q, S = g.nin + s;
-    double a4 = 0.0, a7 = 0.0;
-    for (int u = 0; u < g.nact; ++u)
-      for (int tt = 0; tt < g.nact; ++tt) {
-        double f = Fofo(fofo, g, r, g.nin + u, p, g.nin + tt);
-        a4 += f * RV(rv, g.nocc, g.nin + tt, Q, S, g.nin + u);
-        a7 += f * RV(rv, g.nocc, g.nin + tt, Q, g.nin + u, S);
-      }
-    size_t o = p + (size_t)g.n * (r + (size_t)g.n * (q + (size_t)g.nact * s));
-    z4[o] = a4;
-    z7[o] = a7;
-  }
-}
-
-// Z5[r,q,p,s] = sum_tu (rU|Tq) RV[T,P,S,U];  Z6[r,q,p,s] = sum_tu (rU|Tq) RV[T,P,U,S].
-__global__ void k_z56(Geo g, const double *__restrict__ fofo, const double *__restrict__ rv,
-                      double *__restrict__ z5, double *__restrict__ z6) {
-  size_t total = (size_t)g.n * g.nocc * g.nact * g.nact;
-  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total;
-       t += (size_t)gridDim.x * blockDim.x) {
-    int r = t % g.n;
-    size_t r0 = t / g.n;
-    int q = r0 % g.nocc;
-    r0 /= g.nocc;
-    int p = r0 % g.nact, s = (int)(r0 / g.nact);
-    int P = g.nin + p, S = g.nin + s;
-    double a5 = 0.0, a6 = 0.0;
-    for (int u = 0; u < g.nact; ++u)
-      for (int tt = 0; tt < g.nact; ++tt) {
-        double f = Fofo(fofo, g, g.nin + tt, q, r, g.nin + u);  // (rU|Tq) as (Tq|rU)
-        a5 += f * RV(rv, g.nocc, g.nin + tt, P, S, g.nin + u);
-        a6 += f * RV(rv, g.nocc, g.nin + tt, P, g.nin + u, S);
-      }
-    z5[t] = a5;
-    z6[t] = a6;
-  }
-}
-
-// Z8[q,s,p,r] = sum_tu (TU|qs) RV[T,U,P,R];  q,s < nocc (read from FOFO record (T,U)).
-__global__ void k_z8(Geo g, const double *__restrict__ fofo, const double *__restrict__ rv,
-                     double *__restrict__ z) {
-  size_t total = (size_t)g.nocc * g.nocc * g.nact * g.nact;
-  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total;
-       t += (size_t)gridDim.x * blockDim.x) {
-    int q = t % g.nocc;
-    size_t r0 = t / g.nocc;
-    int s = r0 % g.nocc;
-    r0 /= g.nocc;
-    int p = r0 % g.nact, r = (int)(r0 / g.nact);
-    double a = 0.0;
-    for (int u = 0; u < g.nact; ++u)
-      for (int tt = 0; tt < g.nact; ++tt)
-        a += Fofo(fofo, g, g.nin + tt, g.nin + u, q, s) *  // (TU|qs) from FOFO: coalesced in q
-             RV(rv, g.nocc, g.nin + tt, g.nin + u, g.nin + p, g.nin + r);
-    z[t] = a;
-  }
-}
-
-// Z9[p,r,q,s] = sum_kl (pr|KL) RV[Q,S,K,L].
-__global__ void k_z9(Geo g, const double *__restrict__ ffoo, const double *__restrict__ rv,
-                     double *__restrict__ z) {
-  size_t total = (size_t)g.n * g.n * g.nact * g.nact;
-  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total;
-       t += (size_t)gridDim.x * blockDim.x) {
-    int p = t % g.n;
-    size_t r0 = t / g.n;
-    int r = r0 % g.n;
-    r0 /= g.n;
-    int q = r0 % g.nact, s = (int)(r0 / g.nact);
-    double a = 0.0;
-    for (int l = 0; l < g.nact; ++l)
-      for (int k = 0; k < g.nact; ++k)
-        a += Ffoo(ffoo, g, p, r, g.nin + k, g.nin + l) *
-             RV(rv, g.nocc, g.nin + q, g.nin + s, g.nin + k, g.nin + l);
-    z[t] = a;
-  }
-}
-
-// Z10[q,s,p,r] = sum_tu (Tq|sU) RV[T,P,R,U];  Z13[q,s,p,r] = sum_tu (Tq|sU) RV[T,P,U,R].
-__global__ void k_z1013(Geo g, const double *__restrict__ ffoo, const double *__restrict__ rv,
-                        double *__restrict__ z10, double *__restrict__ z13) {
-  size_t total = (size_t)g.nocc * g.nocc * g.nact * g.nact;
-  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total;
-       t += (size_t)gridDim.x * blockDim.x) {
-    int q = t % g.nocc;
-    size_t r0 = t / g.nocc;
-    int s = r0 % g.nocc;
-    r0 /= g.nocc;
-    int p = r0 % g.nact, r = (int)(r0 / g.nact);
-    int P = g.nin + p, R = g.nin + r;
-    double a10 = 0.0, a13 = 0.0;
-    for (int u = 0; u < g.nact; ++u)
-      for (int tt = 0; tt < g.nact; ++tt) {
-        double f = Ffoo(ffoo, g, q, g.nin + tt, s, g.nin + u);  // (Tq|sU) as (qT|sU)
-        a10 += f * RV(rv, g.nocc, g.nin + tt, P, R, g.nin + u);
-        a13 += f * RV(rv, g.nocc, g.nin + tt, P, g.nin + u, R);
-      }
-    z10[t] = a10;
-    z13[t] = a13;
-  }
-}
-
-// Z11[p,s,q,r] = sum_tu (Tp|sU) RV[T,Q,R,U];  Z12[p,s,q,r] = sum_tu (Tp|sU) RV[T,Q,U,R].
-__global__ void k_z1112(Geo g, const double *__restrict__ ffoo, const double *__restrict__ rv,
-                        double *__restrict__ z11, double *__restrict__ z12) {
-  size_t total = (size_t)g.n * g.nocc * g.nact * g.nact;
-  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total;
-       t += (size_t)gridDim.x * blockDim.x) {
-    int p = t % g.n;
-    size_t r0 = t / g.n;
-    int s = r0 % g.nocc;
-    r0 /= g.nocc;
-    int q = r0 % g.nact, r = (int)(r0 / g.nact);
-    int Q = g.nin + q, R = g.nin + r;
-    double a11 = 0.0, a12 = 0.0;
-    for (int u = 0; u < g.nact; ++u)
-      for (int tt = 0; tt < g.nact; ++tt) {
-        double f = Ffoo(ffoo, g, p, g.nin + tt, s, g.nin + u);  // (Tp|sU) as (pT|sU)
-        a11 += f * RV(rv, g.nocc, g.nin + tt, Q, R, g.nin + u);
-        a12 += f * RV(rv, g.nocc, g.nin + tt, Q, g.nin + u, R);
-      }
-    z11[t] = a11;
-    z12[t] = a12;
-  }
-}
-
-struct Zs {
-  const double *z1, *z4, *z7, *z5, *z6, *z8, *z9, *z10, *z13, *z11, *z12;
+// The buffers between the two kernels of an assembly. The 2-RDM intermediates hold, per
+// element, the part that enters A+B and A-B with one sign (x) and the part that enters them with
+// opposite signs (y); nv = n - nin.
+//   za[p, s, q, r]  x = -Z12            y = Z1[p,s,q,r] + Z11   (p >= nin, s < nocc; q, r active)
+//   zb[r, q, p, s]  x = -Z6             y = Z1[r,q,p,s] + Z5    (r >= nin, q < nocc; p, s active)
+//   zc[p, r, q, s]  x = Z4 + Z9         y = -Z7                 (p, r >= nin; q, s active)
+//   zd[q, s, p, r]  x = Z8 + Z10        y = -Z13                (q, s < nocc; p, r active)
+// with, over active t, u, k, l (capitals: their orbital indices):
+//   Z1[a,b,c,d] = sum (ab|TU) RV[t,u,c,d]    Z4[p,r,q,s] = sum (rU|pT) RV[t,q,s,u]
+//   Z5[r,q,p,s] = sum (rU|Tq) RV[t,p,s,u]    Z6[r,q,p,s] = sum (rU|Tq) RV[t,p,u,s]
+//   Z7[p,r,q,s] = sum (rU|pT) RV[t,q,u,s]    Z8[q,s,p,r] = sum (TU|qs) RV[t,u,p,r]
+//   Z9[p,r,q,s] = sum (pr|KL) RV[q,s,k,l]    Z10[q,s,p,r] = sum (Tq|sU) RV[t,p,r,u]
+//   Z11[p,s,q,r] = sum (Tp|sU) RV[t,q,r,u]   Z12[p,s,q,r] = sum (Tp|sU) RV[t,q,u,r]
+//   Z13[q,s,p,r] = sum (Tq|sU) RV[t,p,u,r]
+struct Inter {
+  double2 *za, *zb, *zc, *zd;
+  double2 *ct;                        // ct[q + nocc s], see k_ab (nocc x nocc)
+  double *hno, *auxi, *auxio, *wmat;  // n x n, column-major
+  double *part;                       // kEtotWarps partial sums of E_CAS
 };
+
+constexpr int kEtotWarps = 256;
+
+// Everything that the element kernel reads, in one launch: the parts do not depend on one
+// another, and each of them alone is a short kernel that leaves most of the chip idle at
+// small n. The unit of work is one warp: 32 consecutive values of the fastest index
+// (coalesced along FOFO / FFOO records) for one value of the others, which are then uniform
+// over the warp. Bound at large n by the FP64 pipe: 6 nact^2 FMAs per element of zc, and
+// ten per element of za and zb. Measured at n = 249, nocc = 28, nact = 6: 0.53 ms (FP64 pipe
+// 89%), against 1.14 ms for a kernel per part and a DGEMM with K = nocc^3 for WMAT; at n = 64
+// 25 us, against 126 us.
+struct InterWork {  // first warp of each part
+  int wc, wab, wd, wone, wwm, wct, wet, end;
+};
+
+__global__ void __launch_bounds__(256)
+    k_intermediates(Geo g, InterWork W, const double *__restrict__ h, const double *__restrict__ occ,
+                    const int *__restrict__ grp, const double *__restrict__ fofo,
+                    const double *__restrict__ ffoo, const double *__restrict__ rv, double lam,
+                    Inter I) {
+  const int lane = threadIdx.x & 31;
+  const int n = g.n, nin = g.nin, na = g.nact, nocc = g.nocc, nv = n - nin;
+  const size_t ldo = (size_t)n * nocc, ldf = (size_t)n * n;
+  for (int w = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); w < W.end;
+       w += (int)((gridDim.x * blockDim.x) >> 5)) {
+    if (w < W.wab) {  // zc
+      const int ch = (nv + 31) / 32;
+      int t0 = w;
+      const int p = (t0 % ch) * 32 + lane + nin;
+      t0 /= ch;
+      const int r = t0 % nv + nin;
+      t0 /= nv;
+      const int q = t0 % na, s = t0 / na;
+      if (p >= n) continue;
+      double x = 0.0, y = 0.0;
+      for (int u = 0; u < na; ++u) {
+        // (rU|pT): record (r, U), element p + T n;  (pr|KL): record (K, L), element p + r n
+        const double *fr = fofo + ((size_t)r + (size_t)(nin + u) * n) * ldo + p + (size_t)nin * n;
+        const double *ff = ffoo + ((size_t)nin + (size_t)(nin + u) * nocc) * ldf + p + (size_t)r * n;
+#pragma unroll 2
+        for (int t = 0; t < na; ++t) {
+          const double f = fr[(size_t)t * n];
+          x += f * RVa(rv, na, t, q, s, u);
+          y -= f * RVa(rv, na, t, q, u, s);
+          x += ff[(size_t)t * ldf] * RVa(rv, na, q, s, t, u);
+        }
+      }
+      I.zc[(p - nin) + (size_t)nv * ((r - nin) + (size_t)nv * (q + na * s))] = make_double2(x, y);
+    } else if (w < W.wd) {  // za and zb at (a, b, c, d)
+      const int ch = (nv + 31) / 32;
+      int t0 = w - W.wab;
+      const int a = (t0 % ch) * 32 + lane + nin;
+      t0 /= ch;
+      const int b = t0 % nocc;
+      t0 /= nocc;
+      const int c = t0 % na, d = t0 / na;
+      if (a >= n) continue;
+      double z1 = 0.0, z5 = 0.0, z6 = 0.0, z11 = 0.0, z12 = 0.0;
+      for (int u = 0; u < na; ++u) {
+        const int U = nin + u;
+#pragma unroll 2
+        for (int t = 0; t < na; ++t) {
+          const int T = nin + t;
+          const double rx = RVa(rv, na, t, c, d, u), ry = RVa(rv, na, t, c, u, d);
+          z1 += Fofo(fofo, g, T, U, a, b) * RVa(rv, na, t, u, c, d);  // (ab|TU) as (TU|ab)
+          const double f5 = Fofo(fofo, g, T, b, a, U);               // (rU|Tq) as (Tq|rU)
+          z5 += f5 * rx;
+          z6 += f5 * ry;
+          const double f11 = Ffoo(ffoo, g, a, T, b, U);              // (Tp|sU) as (pT|sU)
+          z11 += f11 * rx;
+          z12 += f11 * ry;
+        }
+      }
+      const size_t o = (a - nin) + (size_t)nv * (b + (size_t)nocc * (c + na * d));
+      I.za[o] = make_double2(-z12, z1 + z11);
+      I.zb[o] = make_double2(-z6, z1 + z5);
+    } else if (w < W.wone) {  // zd
+      const int ch = (nocc + 31) / 32;
+      int t0 = w - W.wd;
+      const int q = (t0 % ch) * 32 + lane;
+      t0 /= ch;
+      const int s = t0 % nocc;
+      t0 /= nocc;
+      const int p = t0 % na, r = t0 / na;
+      if (q >= nocc) continue;
+      double x = 0.0, y = 0.0;
+      for (int u = 0; u < na; ++u)
+#pragma unroll 2
+        for (int t = 0; t < na; ++t) {
+          const double f10 = Ffoo(ffoo, g, q, nin + t, s, nin + u);  // (Tq|sU) as (qT|sU)
+          x += Fofo(fofo, g, nin + t, nin + u, q, s) * RVa(rv, na, t, u, p, r);
+          x += f10 * RVa(rv, na, t, p, r, u);
+          y -= f10 * RVa(rv, na, t, p, u, r);
+        }
+      I.zd[q + (size_t)nocc * (s + (size_t)nocc * (p + na * r))] = make_double2(x, y);
+    } else if (w < W.wwm) {  // HNO, AuxI, AuxIO at (i, j)
+      const int ch = (n + 31) / 32;
+      const int t0 = w - W.wone;
+      const int i = (t0 % ch) * 32 + lane, j = t0 / ch;
+      if (i >= n) continue;
+      const int gi = grp[i], gj = grp[j];
+      const double hv = h[i + (size_t)j * n];
+      double corr = 0.0, ai = 0.0, aio = 0.0;
+#pragma unroll 4
+      for (int k = 0; k < nocc; ++k) {
+        const int gk = grp[k];
+        const double ok = occ[k];
+        const double jv = Ffoo(ffoo, g, i, j, k, k);  // (ij|kk)
+        const double kv = Fofo(fofo, g, j, k, i, k);  // (jk|ik)
+        if (gi == gj && gk != gi) corr += ok * (2.0 * jv - kv);
+        const double t = ok * (2.0 * AC(g, gi, gj, gk, gk, lam) * jv - AC(g, gi, gi, gj, gk, lam) * kv);
+        ai += t;
+        if (k < nin) aio += t;
+      }
+      const size_t o = i + (size_t)j * n;
+      I.hno[o] = (gi != gj) ? lam * hv : (g.ab1 ? -corr : hv + (1.0 - lam) * corr);
+      I.auxi[o] = ai;
+      I.auxio[o] = aio;
+    } else if (w < W.wct) {
+      // WMAT(k, r) = sum_{i,j,l < nocc} AuxCoeff(k,l,i,j) (ij|kl) RDM2val(i,j,r,l), 0 for
+      // r >= nocc. RDM2val(i,j,r,l) is 2 n_i n_r delta_ij delta_rl - n_i n_r delta_il delta_rj
+      // unless i and r are both active (and only where one of n_i, n_r is 1), and the active
+      // 2-RDM for four active orbitals: 2 nocc + nact^3 terms instead of nocc^3.
+      const int ch = (n + 31) / 32;
+      const int t0 = w - W.wwm;
+      const int k = (t0 % ch) * 32 + lane, r = t0 / ch;
+      if (k >= n) continue;
+      double v = 0.0;
+      if (r < nocc) {
+        const int gk = grp[k], gr = grp[r];
+        const double nr = occ[r];
+#pragma unroll 4
+        for (int i = 0; i < nocc; ++i) {
+          const double ni = occ[i];
+          const int gi = grp[i];
+          const double c = ((i >= nin && r >= nin) || !(ni == 1.0 || nr == 1.0)) ? 0.0 : ni * nr;
+          v += c * (2.0 * AC(g, gk, gr, gi, gi, lam) * Fofo(fofo, g, i, i, k, r) -
+                    AC(g, gk, gi, gi, gr, lam) * Fofo(fofo, g, i, r, k, i));
+        }
+        if (r >= nin) {
+          const double c = AC(g, gk, 1, 1, 1, lam);
+          double a = 0.0;
+#pragma unroll 8
+          for (int t = 0; t < na * na * na; ++t) {  // flat: eight loads in flight
+            const int i = t % na, j = (t / na) % na, l = t / (na * na);
+            a += Fofo(fofo, g, nin + i, nin + j, k, nin + l) * RVa(rv, na, i, j, r - nin, l);
+          }
+          v += c * a;
+        }
+      }
+      I.wmat[k + (size_t)r * n] = v;
+    } else if (w < W.wet) {
+      const int t = (w - W.wct) * 32 + lane;
+      if (t >= nocc * nocc) continue;
+      const int q = t % nocc, s = t / nocc;
+      // C = sign(n - 1/2) sqrt(n); a sum or difference of 0 is not divided by
+      auto ci = [&](int a) { return occ[a] >= 0.5 ? sqrt(occ[a]) : -sqrt(occ[a]); };
+      const double cv = ci(n - 1), cq = ci(q), cs = ci(s);
+      const double dp = (cv + cq) * (cv + cs), dm = (cv - cq) * (cv - cs);
+      const double x = grp[q] + grp[s] <= 1 ? lam * (occ[q] * occ[s]) : 0.0;
+      I.ct[t] = make_double2(dp != 0.0 ? x / dp : x, dm != 0.0 ? x / dm : x);
+    } else {
+      // E_CAS = 2 sum_i n_i h_ii + sum RDM2val(i,j,k,l) (ij|kl), kEtotWarps partial sums in a
+      // fixed order. Every integral is read, also those with a zero RDM2val, so that a
+      // non-finite one shows in the energy.
+      const int e = w - W.wet;
+      double v = 0.0;
+      for (int i = e * 32 + lane; i < nocc; i += 32 * kEtotWarps)
+        v += 2.0 * occ[i] * h[i + (size_t)i * n];
+      const unsigned o2 = (unsigned)nocc * nocc;
+      for (unsigned rec = e; rec < o2; rec += kEtotWarps) {  // record (k, l), elements (i, j)
+        const int k = rec % nocc, l = rec / nocc;
+        const double *fr = ffoo + (size_t)rec * ldf;
+#pragma unroll 4
+        for (unsigned t = lane; t < o2; t += 32) {
+          const int j = t / nocc, i = t - j * nocc;
+          double c = 0.0;
+          if (i >= nin && j >= nin && k >= nin && l >= nin) {
+            c = RVa(rv, na, i - nin, j - nin, k - nin, l - nin);
+          } else if ((i == j && k == l) || (i == l && k == j)) {
+            const double ni = occ[i], nk = occ[k];
+            if (ni == 1.0 || nk == 1.0)
+              c = ((i == j && k == l) ? 2.0 * ni * nk : 0.0) - ((i == l && k == j) ? ni * nk : 0.0);
+          }
+          v += c * fr[i + (size_t)j * n];
+        }
+      }
+      for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
+      if (lane == 0) I.part[e] = v;
+    }
+  }
+}
 
 // ---------------------------------------------------------------------------
 // A+B and A-B, element (row = pair i, column = pair j), column-major N x N.
-__global__ void k_ab(Geo g, int N, const int *__restrict__ pp, const int *__restrict__ pq,
-                     const double *__restrict__ occ, const int *__restrict__ grp,
-                     const double *__restrict__ fofo, const double *__restrict__ ffoo, Zs Z,
-                     const double *__restrict__ hno, const double *__restrict__ auxi,
-                     const double *__restrict__ auxio, const double *__restrict__ wmat, double lam,
-                     const double *__restrict__ rpl, const double *__restrict__ rmi,
-                     double *__restrict__ abp, double *__restrict__ abm) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  int j = blockIdx.y * blockDim.y + threadIdx.y;
-  if (i >= N || j >= N) return;
-  const int n = g.n, nin = g.nin, nocc = g.nocc, na = g.nact;
-  int p = pp[i], q = pq[i], r = pp[j], s = pq[j];
-  int gp = grp[p], gq = grp[q], gr = grp[r], gs = grp[s];
-  double op = occ[p], oq = occ[q], orr = occ[r], os = occ[s];
-  // Every term enters A+B and A-B either with the same sign (sym, accumulated in S) or
-  // with opposite signs (anti, in A); A+B = S + A, A-B = S - A (+ the Coulomb term, A-B
-  // only). Each Z term is then one FP64 FMA with its coefficient (1, 0 or lambda):
-  // GB300's FP64 pipe, not HBM, bounds this kernel.
-  double S = 0.0, A = 0.0, Mo = 0.0;
-  const double ac = AC(g, gp, gq, gr, gs, lam);
-  auto ai = [](int a, int b) { return AuxInd(a, b) == 1; };
-  const double X1 = (ai(gp, gr) ? op * orr : 0.0) + (ai(gq, gs) ? oq * os : 0.0) -
-                    (ai(gq, gr) ? oq * orr : 0.0) - (ai(gp, gs) ? op * os : 0.0);
-  if (r >= nin && p >= nin) {
-    const double t = ac * X1;
-    // FOFO Coulomb: A- += 4 AC X1 (rs|pq) (its two A+ parts cancel)
-    Mo = 4.0 * t * Fofo(fofo, g, r, s, p, q);
-    // FOFO exchange (anti): AC X1 (ps|rq), read as (rq|ps): record (r, q) is shared by a
-    // warp of consecutive p and its elements p + s n are contiguous
-    A = t * Fofo(fofo, g, r, q, p, s);
-    // FFOO exchange (sym): -AC X1 (pr|qs)
-    S = -t * Ffoo(ffoo, g, p, r, q, s);
-  }
-  const bool pa = gp == 1, qa = gq == 1, ra = gr == 1, sa = gs == 1;
-  const int pA = p - nin, qA = q - nin, rA = r - nin, sA = s - nin;
-  // FOFO T1 (p -> q), anti
-  if (p >= nin && ra && qa)
-    A = fma(AC(g, gp, gs, 1, 1, lam),
-            Z.z1[p + (size_t)n * (s + (size_t)nocc * (qA + (size_t)na * rA))], A);
-  // FOFO T3, anti
-  if (r >= nin && sa && pa)
-    A = fma(AC(g, gq, gr, 1, 1, lam),
-            Z.z1[r + (size_t)n * (q + (size_t)nocc * (pA + (size_t)na * sA))], A);
-  if (r >= nin && sa) {
-    if (qa && p >= nin) {
-      const size_t o = p + (size_t)n * (r + (size_t)n * (qA + (size_t)na * sA));
-      const double c = AC(g, gp, gr, 1, 1, lam);
-      S = fma(c, Z.z4[o], S);   // T4
-      A = fma(-c, Z.z7[o], A);  // T6 (p -> q)
+//
+// Bound by the FP64 pipe (2 FMAs per cycle per SM), then by the three gathers, so whatever is
+// not a product of the element itself is kept off that pipe: groups, zero and NaN tests are
+// integer work, the addresses are a row part (held by the thread over `cols` columns) plus a
+// column part that is uniform over the warp. Nine in ten elements of a large system have p
+// and r virtual and q, s not both active. There the element is
+//   A+B = t (f2 - f3) / ((C_p + C_q)(C_r + C_s)),  A-B = t (4 f1 - f2 - f3) / ((C_p - C_q)(C_r - C_s))
+// with t = lambda n_q n_s (0 beside an active pair), and as long as the virtual occupations
+// are all the same (`vuni`) the factors depend on q and s alone: they come from the table ct,
+// and the element takes 5 FP64 operations instead of 19. Measured at NDimX 6335: 0.73 ms,
+// with the general form for every element 1.46 ms, without the row order and with the same
+// conditional products for every element 2.10 ms.
+// The rows go through `slot`, an order of the pairs in which a warp holds 8 consecutive p
+// times 4 consecutive q of one pair of orbital groups: the branches are then uniform over
+// almost every warp, the gathers use whole sectors (8 consecutive elements of a record) and
+// so do the stores, whichever of p and q is the outer index of the caller's pair list.
+constexpr int kAbWarps = 4;
+
+__device__ __forceinline__ bool nonzero(double x) {
+  return (__double_as_longlong(x) << 1) != 0;  // integer test: the FP64 pipe is the bound
+}
+__device__ __forceinline__ bool nonfinite(double x) {
+  return (__double2hiint(x) & 0x7ff00000) == 0x7ff00000;
+}
+
+__global__ void __launch_bounds__(32 * kAbWarps)
+    k_ab(Geo g, int N, int cols, const int *__restrict__ slot, const int *__restrict__ pp,
+         const int *__restrict__ pq, const double *__restrict__ occ, const int *__restrict__ grp,
+         const double *__restrict__ fofo, const double *__restrict__ ffoo, Inter I, double lam,
+         int vuni, const double *__restrict__ rpl, const double *__restrict__ rmi, double *__restrict__ abp,
+         double *__restrict__ abm) {
+  const int sl = (blockIdx.x * kAbWarps + (threadIdx.x >> 5)) * 32 + (threadIdx.x & 31);
+  if (sl >= N) return;
+  const int i = slot[sl];
+  const int n = g.n, nin = g.nin, nocc = g.nocc, na = g.nact, nv = n - nin;
+  const size_t ldo = (size_t)n * nocc, ldf = (size_t)n * n;
+  const int p = pp[i], q = pq[i], gp = grp[p], gq = grp[q];
+  const double op = occ[p], oq = occ[q];
+  const double ri_p = rpl[i], ri_m = rmi[i];
+  const bool zi_p = nonzero(ri_p), zi_m = nonzero(ri_m);
+  const bool pa = gp == 1, qa = gq == 1;
+  const int pA = p - nin, qA = q - nin;
+  const double *f1 = fofo + p + (size_t)q * n;        // (rs|pq): record (r, s)
+  const double *f2 = fofo + (size_t)q * n * ldo + p;  // (rq|ps): record (r, q)
+  const double *f3 = ffoo + (size_t)q * ldf + p;      // (pr|qs): record (q, s)
+  // The assembly of the reference sums over every (ij|kl) with i, j, l occupied, most of them
+  // with a zero coefficient. A non-finite one must still show in A+-B: each thread looks at its
+  // share of them and adds a NaN to its elements where it finds one.
+  bool bad = false;
+  {
+    const size_t rec = (size_t)n * nocc, cnt = (size_t)nocc * nocc * rec,
+                 nth = (size_t)N * gridDim.y;
+    for (size_t e = (size_t)blockIdx.y * N + sl; e < cnt; e += nth) {
+      const size_t ij = e / rec;
+      bad |= nonfinite(fofo[((ij % nocc) + (ij / nocc) * n) * ldo + (e - ij * rec)]);
     }
-    if (pa) {
-      const size_t o = r + (size_t)n * (q + (size_t)nocc * (pA + (size_t)na * sA));
-      const double c = AC(g, gq, gr, 1, 1, lam);
-      A = fma(c, Z.z5[o], A);   // T4 (p -> q)
-      S = fma(-c, Z.z6[o], S);  // T6
-    }
   }
-  if (ra && pa) {
-    const size_t o = q + (size_t)nocc * (s + (size_t)nocc * (pA + (size_t)na * rA));
-    const double c = AC(g, gq, gs, 1, 1, lam);
-    S = fma(c, Z.z8[o] + Z.z10[o], S);  // FFOO T1 + T2
-    A = fma(-c, Z.z13[o], A);           // T5 (p -> q)
-  }
-  if (sa && r >= nin && qa && p >= nin)  // FFOO T3, sym
-    S = fma(AC(g, gp, gr, 1, 1, lam),
-            Z.z9[p + (size_t)n * (r + (size_t)n * (qA + (size_t)na * sA))], S);
-  if (ra && qa && p >= nin) {
-    const size_t o = p + (size_t)n * (s + (size_t)nocc * (qA + (size_t)na * rA));
-    const double c = AC(g, gp, gs, 1, 1, lam);
-    A = fma(c, Z.z11[o], A);   // T2 (p -> q)
-    S = fma(-c, Z.z12[o], S);  // T5
-  }
-  // one-body part (final loop of AB_CAS_FOFO): sym (p = r, q = s) and anti (q = r, p = s)
   auto aux = [&](int ga, int gb, int x, int y) -> double {
-    int a = AuxInd(ga, gb);
-    if (a == 1) return auxi[x + (size_t)y * n];
-    if (a == 2) return auxio[x + (size_t)y * n];
+    const int a = AuxInd(ga, gb);
+    if (a == 1) return I.auxi[x + (size_t)y * n];
+    if (a == 2) return I.auxio[x + (size_t)y * n];
     return 0.0;
   };
-  if (p == r)
-    S += (op - os) * hno[q + (size_t)s * n] - wmat[q + (size_t)s * n] + op * aux(gp, gr, q, s);
-  if (q == s)
-    S += (oq - orr) * hno[p + (size_t)r * n] - wmat[p + (size_t)r * n] + oq * aux(gq, gs, p, r);
-  if (q == r)
-    A += (oq - os) * hno[p + (size_t)s * n] - wmat[p + (size_t)s * n] + oq * aux(gq, gr, p, s);
-  if (p == s)
-    A += (op - orr) * hno[q + (size_t)r * n] - wmat[q + (size_t)r * n] + op * aux(gp, gs, q, r);
-  double vp = S + A, vm = S - A + Mo;
-  // divide by (C_p + C_q)(C_r + C_s) and (C_p - C_q)(C_r - C_s) where they are not 0,
-  // as products of the pair reciprocals (no FP64 square root or division per element)
-  const double ai_ = rpl[i], aj_ = rpl[j], bi_ = rmi[i], bj_ = rmi[j];
-  if (ai_ != 0.0 && aj_ != 0.0) vp *= ai_ * aj_;
-  if (bi_ != 0.0 && bj_ != 0.0) vm *= bi_ * bj_;
-  size_t o = i + (size_t)j * N;
-  abp[o] = vp;
-  abm[o] = vm;
+  const bool vrow = vuni && gp == 2;
+  const int j1 = min(N, (int)(blockIdx.y + 1) * cols);
+  for (int j = blockIdx.y * cols; j < j1; ++j) {
+    const int r = pp[j], s = pq[j], gr = grp[r], gs = grp[s];
+    const bool ra = gr == 1, sa = gs == 1;
+    const double orr = occ[r], os = occ[s];
+    const double rj_p = rpl[j], rj_m = rmi[j];
+    const size_t o = i + (size_t)j * N;
+    if (vrow && gr == 2 && !(qa && sa)) {
+      const double2 k = I.ct[q + nocc * s];
+      const double v1 = f1[((size_t)r + (size_t)s * n) * ldo], v2 = f2[(size_t)r * ldo + (size_t)s * n],
+                   v3 = f3[(size_t)s * nocc * ldf + (size_t)r * n];
+      double vp = k.x * (v2 - v3), vm = k.y * fma(4.0, v1, -(v2 + v3));
+      if (p == r || q == s) {  // the one-body part (q = r and p = s cannot be)
+        double ob = 0.0;
+        if (p == r)
+          ob = (op - os) * I.hno[q + (size_t)s * n] - I.wmat[q + (size_t)s * n] + op * aux(gp, gr, q, s);
+        if (q == s)
+          ob += (oq - orr) * I.hno[p + (size_t)r * n] - I.wmat[p + (size_t)r * n] + oq * aux(gq, gs, p, r);
+        vp += (zi_p && nonzero(rj_p)) ? ob * (ri_p * rj_p) : ob;
+        vm += (zi_m && nonzero(rj_m)) ? ob * (ri_m * rj_m) : ob;
+      }
+      abp[o] = bad ? __longlong_as_double(0x7ff8000000000000ll) : vp;
+      abm[o] = bad ? __longlong_as_double(0x7ff8000000000000ll) : vm;
+      continue;
+    }
+    // Every term enters A+B and A-B either with the same sign (S) or with opposite signs
+    // (A); A+B = S + A, A-B = S - A + the Coulomb term Mo.
+    double S = bad ? __longlong_as_double(0x7ff8000000000000ll) : 0.0, A = 0.0, Mo = 0.0;
+    if (r >= nin && p >= nin) {
+      // AuxInd = 1: both inactive or active, not both active (a virtual orbital takes no part)
+      double x1 = 0.0;
+      if (gp + gr <= 1) x1 = op * orr;
+      if (gq + gs <= 1) x1 = fma(oq, os, x1);
+      if (gq + gr <= 1) x1 = fma(-oq, orr, x1);
+      if (gp + gs <= 1) x1 = fma(-op, os, x1);
+      const double t = AC(g, gp, gq, gr, gs, lam) * x1;
+      // A- += 4 t (rs|pq); anti: t (ps|rq), read as (rq|ps); sym: -t (pr|qs)
+      Mo = 4.0 * t * f1[((size_t)r + (size_t)s * n) * ldo];
+      A = t * f2[(size_t)r * ldo + (size_t)s * n];
+      S = fma(-t, f3[(size_t)s * nocc * ldf + (size_t)r * n], S);
+    }
+    if (ra && qa && p >= nin) {  // FOFO T1 (p -> q), FFOO T2 (p -> q) and T5
+      const double2 z = I.za[(p - nin) + (size_t)nv * (s + (size_t)nocc * (qA + na * (r - nin)))];
+      const double c = AC(g, gp, gs, 1, 1, lam);
+      S = fma(c, z.x, S);
+      A = fma(c, z.y, A);
+    }
+    if (sa && r >= nin) {
+      if (pa) {  // FOFO T3, T4 (p -> q) and T6
+        const double2 z = I.zb[(r - nin) + (size_t)nv * (q + (size_t)nocc * (pA + na * (s - nin)))];
+        const double c = AC(g, gq, gr, 1, 1, lam);
+        S = fma(c, z.x, S);
+        A = fma(c, z.y, A);
+      }
+      if (qa && p >= nin) {  // FOFO T4 and T6 (p -> q), FFOO T3
+        const double2 z = I.zc[(p - nin) + (size_t)nv * ((r - nin) + (size_t)nv * (qA + na * (s - nin)))];
+        const double c = AC(g, gp, gr, 1, 1, lam);
+        S = fma(c, z.x, S);
+        A = fma(c, z.y, A);
+      }
+    }
+    if (ra && pa) {  // FFOO T1, T2 and T5 (p -> q)
+      const double2 z = I.zd[q + (size_t)nocc * (s + (size_t)nocc * (pA + na * (r - nin)))];
+      const double c = AC(g, gq, gs, 1, 1, lam);
+      S = fma(c, z.x, S);
+      A = fma(c, z.y, A);
+    }
+    // one-body part (final loop of AB_CAS_FOFO): sym (p = r, q = s) and anti (q = r, p = s)
+    if (p == r || q == s || q == r || p == s) {
+      if (p == r)
+        S += (op - os) * I.hno[q + (size_t)s * n] - I.wmat[q + (size_t)s * n] + op * aux(gp, gr, q, s);
+      if (q == s)
+        S += (oq - orr) * I.hno[p + (size_t)r * n] - I.wmat[p + (size_t)r * n] + oq * aux(gq, gs, p, r);
+      if (q == r)
+        A += (oq - os) * I.hno[p + (size_t)s * n] - I.wmat[p + (size_t)s * n] + oq * aux(gq, gr, p, s);
+      if (p == s)
+        A += (op - orr) * I.hno[q + (size_t)r * n] - I.wmat[q + (size_t)r * n] + op * aux(gp, gs, q, r);
+    }
+    double vp = S + A, vm = S - A + Mo;
+    // divide by (C_p + C_q)(C_r + C_s) and (C_p - C_q)(C_r - C_s) where they are not 0,
+    // as products of the pair reciprocals (no FP64 square root or division per element)
+    if (zi_p && nonzero(rj_p)) vp *= ri_p * rj_p;
+    if (zi_m && nonzero(rj_m)) vm *= ri_m * rj_m;
+    abp[o] = vp;
+    abm[o] = vm;
+  }
 }
 
 // sq_symmetrize (tran.f90:1303-1319): a(i,j) = a(j,i) = (a(i,j) + a(j,i)) / 2.
@@ -480,6 +501,9 @@ int sys_upload(gc_context *ctx, SysDev &sd, int nbas, int ninact, int nact, int 
   sd.nact = nact;
   sd.nocc = nocc;
   sd.ndimx = ndimx;
+  sd.vuni = n > nocc;
+  for (int i = nocc; i < n; ++i)
+    if (occ[i] != occ[nocc]) sd.vuni = 0;
   std::vector<int> grp(n), pp(ndimx), pq(ndimx);
   for (int i = 0; i < n; ++i) grp[i] = i < ninact ? 0 : (i < nocc ? 1 : 2);
   for (int i = 0; i < ndimx; ++i) {
@@ -522,68 +546,39 @@ int sys_upload(gc_context *ctx, SysDev &sd, int nbas, int ninact, int nact, int 
       }
     GC_TRY(sd.h.upload(ctx, h.data(), h.size()));
   }
-  // RDM2val(i,j,k,l) = FRDM2(i,k,j,l) (abfofo.f90:84-92, interpa.f:5244-5272)
-  std::vector<double> rv((size_t)nocc * nocc * nocc * nocc, 0.0);
-  auto frdm2 = [&](int ip, int iq, int ir, int is) -> double {
-    double r = 0.0;
-    if (ip == ir && iq == is && (occ[ip] == 1.0 || occ[iq] == 1.0)) r += 2.0 * occ[ip] * occ[iq];
-    if (ip == is && iq == ir && (occ[ip] == 1.0 || occ[iq] == 1.0)) r -= occ[ip] * occ[iq];
-    if (ip >= ninact && iq >= ninact && ir >= ninact && is >= ninact) {
-      long long i12 = (long long)(ip - ninact) * nact + (iq - ninact) + 1;
-      long long i34 = (long long)(ir - ninact) * nact + (is - ninact) + 1;
-      long long mx = i12 > i34 ? i12 : i34, mn = i12 > i34 ? i34 : i12;
-      r = rdm2act[mx * (mx - 1) / 2 + mn - 1];
-    }
-    return r;
-  };
-  for (int l = 0; l < nocc; ++l)
-    for (int k = 0; k < nocc; ++k)
-      for (int j = 0; j < nocc; ++j)
-        for (int i = 0; i < nocc; ++i)
-          rv[i + (size_t)nocc * (j + (size_t)nocc * (k + (size_t)nocc * l))] = frdm2(i, k, j, l);
+  // Active block of RDM2val(i,j,k,l) = FRDM2(i,k,j,l) (abfofo.f90:84-92, interpa.f:5244-5272);
+  // outside it RDM2val is products of occupations, which the kernels form themselves.
+  std::vector<double> rv(std::max<size_t>((size_t)nact * nact * nact * nact, 1), 0.0);
+  {
+    size_t t = 0;
+    for (int l = 0; l < nact; ++l)
+      for (int k = 0; k < nact; ++k)
+        for (int j = 0; j < nact; ++j)
+          for (int i = 0; i < nact; ++i, ++t) {
+            const long long a = (long long)i * nact + k + 1, b = (long long)j * nact + l + 1;
+            const long long mx = std::max(a, b), mn = std::min(a, b);
+            rv[t] = rdm2act[mx * (mx - 1) / 2 + mn - 1];
+          }
+  }
   GC_TRY(sd.rv.upload(ctx, rv.data(), rv.size()));
-  return GC_OK;
-}
-
-// Intermediates that depend only on the system, cached per assembly call set.
-struct ZBufs {
-  DevBuf<double> z1, z4, z7, z5, z6, z8, z9, z10, z13, z11, z12;
-};
-
-static int build_z(gc_context *ctx, const SysDev &sd, const double *ffoo, const double *fofo,
-                   ZBufs &Zb) {
-  Geo g{sd.n, sd.nin, sd.nact, sd.nocc};
-  size_t na2 = (size_t)sd.nact * sd.nact;
-  size_t s1 = (size_t)sd.n * sd.nocc * na2, s4 = (size_t)sd.n * sd.n * na2,
-         s8 = (size_t)sd.nocc * sd.nocc * na2;
-  size_t one = 1;
-  GC_TRY(Zb.z1.alloc(ctx, std::max(s1, one)));
-  GC_TRY(Zb.z4.alloc(ctx, std::max(s4, one)));
-  GC_TRY(Zb.z7.alloc(ctx, std::max(s4, one)));
-  GC_TRY(Zb.z5.alloc(ctx, std::max(s1, one)));
-  GC_TRY(Zb.z6.alloc(ctx, std::max(s1, one)));
-  GC_TRY(Zb.z8.alloc(ctx, std::max(s8, one)));
-  GC_TRY(Zb.z9.alloc(ctx, std::max(s4, one)));
-  GC_TRY(Zb.z10.alloc(ctx, std::max(s8, one)));
-  GC_TRY(Zb.z13.alloc(ctx, std::max(s8, one)));
-  GC_TRY(Zb.z11.alloc(ctx, std::max(s1, one)));
-  GC_TRY(Zb.z12.alloc(ctx, std::max(s1, one)));
-  if (sd.nact == 0) return GC_OK;
-  auto grid = [](size_t total) { return std::min<unsigned>(ceil_div(total, 256), 152u * 64u); };
-  k_z1<<<grid(s1), 256, 0, ctx->stream>>>(g, fofo, sd.rv.p, Zb.z1.p);
-  GC_LAUNCHED(ctx);
-  k_z47<<<grid(s4), 256, 0, ctx->stream>>>(g, fofo, sd.rv.p, Zb.z4.p, Zb.z7.p);
-  GC_LAUNCHED(ctx);
-  k_z56<<<grid(s1), 256, 0, ctx->stream>>>(g, fofo, sd.rv.p, Zb.z5.p, Zb.z6.p);
-  GC_LAUNCHED(ctx);
-  k_z8<<<grid(s8), 256, 0, ctx->stream>>>(g, fofo, sd.rv.p, Zb.z8.p);
-  GC_LAUNCHED(ctx);
-  k_z9<<<grid(s4), 256, 0, ctx->stream>>>(g, ffoo, sd.rv.p, Zb.z9.p);
-  GC_LAUNCHED(ctx);
-  k_z1013<<<grid(s8), 256, 0, ctx->stream>>>(g, ffoo, sd.rv.p, Zb.z10.p, Zb.z13.p);
-  GC_LAUNCHED(ctx);
-  k_z1112<<<grid(s1), 256, 0, ctx->stream>>>(g, ffoo, sd.rv.p, Zb.z11.p, Zb.z12.p);
-  GC_LAUNCHED(ctx);
+  // Row order of the element kernel: pairs by orbital groups, then tiles of 8 p x 4 q. The
+  // pairs are listed per (p, q) cell (head, next) and the cells are walked in that order.
+  std::vector<int> slot, head((size_t)n * nocc, -1), next(ndimx);
+  for (int i = ndimx - 1; i >= 0; --i) {
+    int &c = head[pp[i] + (size_t)pq[i] * n];
+    next[i] = c;
+    c = i;
+  }
+  slot.reserve(ndimx);
+  const int pb[4] = {0, ninact, nocc, n}, qb[3] = {0, ninact, nocc};
+  for (int gq = 0; gq < 2; ++gq)
+    for (int gp = gq; gp < 3; ++gp)
+      for (int p0 = pb[gp]; p0 < pb[gp + 1]; p0 += 8)
+        for (int q0 = qb[gq]; q0 < qb[gq + 1]; q0 += 4)
+          for (int q = q0; q < std::min(q0 + 4, qb[gq + 1]); ++q)
+            for (int p = p0; p < std::min(p0 + 8, pb[gp + 1]); ++p)
+              for (int i = head[p + (size_t)q * n]; i >= 0; i = next[i]) slot.push_back(i);
+  GC_TRY(sd.slot.upload(ctx, slot.data(), ndimx));
   return GC_OK;
 }
 
@@ -591,40 +586,45 @@ int assemble_ab(gc_context *ctx, const SysDev &sd, const double *ffoo, const dou
                 double alpha, double *abplus, double *abmin, double *etot_host, int ab1) {
   PhaseScope ph(ctx, GC_PHASE_ASSEMBLY);
   Geo g{sd.n, sd.nin, sd.nact, sd.nocc, ab1 ? 0.0 : 1.0, ab1 ? 1 : 0};
-  const int n = sd.n, N = sd.ndimx;
-  ZBufs Zb;
-  GC_TRY(build_z(ctx, sd, ffoo, fofo, Zb));
-  DevBuf<double> hno, auxi, auxio, wmat;
-  GC_TRY(hno.alloc(ctx, (size_t)n * n));
-  GC_TRY(auxi.alloc(ctx, (size_t)n * n));
-  GC_TRY(auxio.alloc(ctx, (size_t)n * n));
-  GC_TRY(wmat.alloc(ctx, (size_t)n * n));
-  dim3 b2(16, 16), g2(ceil_div(n, 16), ceil_div(n, 16));
-  k_onebody<<<g2, b2, 0, ctx->stream>>>(g, sd.h.p, sd.occ.p, sd.grp.p, fofo, ffoo, alpha, hno.p,
-                                        auxi.p, auxio.p);
+  const int n = sd.n, N = sd.ndimx, nocc = sd.nocc, nv = n - sd.nin;
+  const size_t na2 = (size_t)sd.nact * sd.nact, n2 = (size_t)n * n;
+  const size_t sab = (size_t)nv * nocc * na2, sc = (size_t)nv * nv * na2,
+               o2 = (size_t)nocc * nocc, sdd = o2 * na2;
+  DevBuf<double> buf;
+  GC_TRY(buf.alloc(ctx, 2 * (2 * sab + sc + sdd + o2) + 4 * n2 + kEtotWarps));
+  Inter I;
+  I.za = reinterpret_cast<double2 *>(buf.p);
+  I.zb = I.za + sab;
+  I.zc = I.zb + sab;
+  I.zd = I.zc + sc;
+  I.ct = I.zd + sdd;
+  I.hno = reinterpret_cast<double *>(I.ct + o2);
+  I.auxi = I.hno + n2;
+  I.auxio = I.auxi + n2;
+  I.wmat = I.auxio + n2;
+  I.part = I.wmat + n2;
+  const long long chv = ceil_div(nv, 32), chn = ceil_div(n, 32), cho = ceil_div(nocc, 32);
+  const long long cnt[7] = {chv * nv * (long long)na2, chv * nocc * (long long)na2,
+                            cho * nocc * (long long)na2, chn * n, chn * n, ceil_div(o2, 32),
+                            etot_host ? kEtotWarps : 0};
+  long long first[8] = {0};
+  for (int k = 0; k < 7; ++k) first[k + 1] = first[k] + cnt[k];
+  if (first[7] > 0x7fffffffll - (1 << 24))
+    return set_error(ctx, GC_EUNSUPPORTED, "assembly: nbas=%d nact=%d too large", n, sd.nact);
+  const InterWork W{(int)first[0], (int)first[1], (int)first[2], (int)first[3],
+                    (int)first[4], (int)first[5], (int)first[6], (int)first[7]};
+  k_intermediates<<<std::min<unsigned>(ceil_div((size_t)W.end, 8), 152u * 64u), 256, 0,
+                    ctx->stream>>>(g, W, sd.h.p, sd.occ.p, sd.grp.p, fofo, ffoo, sd.rv.p, alpha, I);
   GC_LAUNCHED(ctx);
-  GC_CUDA(ctx, cudaMemsetAsync(wmat.p, 0, (size_t)n * n * sizeof(double), ctx->stream));
-  if (sd.nocc > 0) {
-    const int nocc = sd.nocc, K = nocc * nocc * nocc;
-    DevBuf<double> fw, rvp;
-    GC_TRY(fw.alloc(ctx, (size_t)n * K));
-    GC_TRY(rvp.alloc(ctx, (size_t)K * nocc));
-    k_pack_wmat_f<<<dim3(ceil_div(n, 128), std::min(K, 65535)), 128, 0, ctx->stream>>>(
-        g, sd.grp.p, fofo, alpha, fw.p);
-    GC_LAUNCHED(ctx);
-    k_pack_wmat_rv<<<std::min<unsigned>(ceil_div((size_t)K * nocc, 256), 152u * 8u), 256, 0,
-                     ctx->stream>>>(nocc, sd.rv.p, rvp.p);
-    GC_LAUNCHED(ctx);
-    const double one = 1.0, zero = 0.0;
-    GC_CUBLAS(ctx, cublasDgemm(ctx->cublas, CUBLAS_OP_N, CUBLAS_OP_N, n, nocc, K, &one, fw.p, n,
-                               rvp.p, K, &zero, wmat.p, n));
-  }
-  Zs Z{Zb.z1.p, Zb.z4.p, Zb.z7.p, Zb.z5.p, Zb.z6.p, Zb.z8.p, Zb.z9.p, Zb.z10.p, Zb.z13.p,
-       Zb.z11.p, Zb.z12.p};
-  dim3 b3(32, 8), g3(ceil_div(N, 32), ceil_div(N, 8));
-  k_ab<<<g3, b3, 0, ctx->stream>>>(g, N, sd.pair_p.p, sd.pair_q.p, sd.occ.p, sd.grp.p, fofo, ffoo,
-                                   Z, hno.p, auxi.p, auxio.p, wmat.p, alpha, sd.rpl.p, sd.rmi.p,
-                                   abplus, abmin);
+  // Columns per warp: up to 8 share the row part of a warp's work; fewer where 8 would leave
+  // the chip with less than 32 warps per SM (N = 570: 30 us with 8, 20 us with 2).
+  const int cols = (int)std::min<long long>(8, std::max<long long>(1, (long long)ceil_div(N, 32) * N / (152 * 32)));
+  const dim3 g3(ceil_div(N, 32 * kAbWarps), ceil_div(N, cols));
+  if (g3.y > 65535)
+    return set_error(ctx, GC_EUNSUPPORTED, "assembly: ndimx=%d too large", N);
+  k_ab<<<g3, 32 * kAbWarps, 0, ctx->stream>>>(g, N, cols, sd.slot.p, sd.pair_p.p, sd.pair_q.p, sd.occ.p,
+                                              sd.grp.p, fofo, ffoo, I, alpha, sd.vuni, sd.rpl.p, sd.rmi.p,
+                                              abplus, abmin);
   GC_LAUNCHED(ctx);
   if (ab1) {  // AB_CAS_FOFO symmetrises the AB1 matrices (sq_symmetrize, abfofo.f90:260-263)
     dim3 bs(32, 8), gs(ceil_div(N, 32), ceil_div(N, 8));
@@ -634,23 +634,12 @@ int assemble_ab(gc_context *ctx, const SysDev &sd, const double *ffoo, const dou
     GC_LAUNCHED(ctx);
   }
   if (etot_host) {
-    const int nb = 120;
-    DevBuf<double> part;
-    GC_TRY(part.alloc(ctx, nb));
-    k_etwo<<<nb, 256, 0, ctx->stream>>>(g, ffoo, sd.rv.p, part.p);
-    GC_LAUNCHED(ctx);
-    double hpart[nb];
-    std::vector<double> occ(n), h((size_t)n * n);
-    GC_CUDA(ctx, cudaMemcpyAsync(hpart, part.p, sizeof hpart, cudaMemcpyDeviceToHost, ctx->stream));
-    GC_CUDA(ctx, cudaMemcpyAsync(occ.data(), sd.occ.p, n * sizeof(double), cudaMemcpyDeviceToHost,
-                                 ctx->stream));
-    GC_CUDA(ctx, cudaMemcpyAsync(h.data(), sd.h.p, h.size() * sizeof(double),
-                                 cudaMemcpyDeviceToHost, ctx->stream));
+    double hpart[kEtotWarps];
+    GC_CUDA(ctx, cudaMemcpyAsync(hpart, I.part, sizeof hpart, cudaMemcpyDeviceToHost, ctx->stream));
     GC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    double e1 = 0.0, e2 = 0.0;
-    for (int i = 0; i < sd.nocc; ++i) e1 += occ[i] * h[i + (size_t)i * n];
-    for (int b = 0; b < nb; ++b) e2 += hpart[b];
-    *etot_host = 2.0 * e1 + e2;
+    double e = 0.0;
+    for (double v : hpart) e += v;
+    *etot_host = e;
   }
   return GC_OK;
 }

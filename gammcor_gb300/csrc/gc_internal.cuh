@@ -160,12 +160,14 @@ inline bool is_sliced(int precision) {
 // Per-system description resident on the device ------------------------------
 struct SysDev {
   int n = 0, nin = 0, nact = 0, nocc = 0, ndimx = 0;
+  int vuni = 0;            // the virtual occupations are all equal
   DevBuf<double> occ;      // (n)
   DevBuf<int> grp;         // (n) 0 inactive, 1 active, 2 virtual
   DevBuf<int> pair_p;      // (ndimx) 0-based p of pair (p > q)
   DevBuf<int> pair_q;      // (ndimx)
   DevBuf<double> h;        // (n, n) symmetrised one-electron MO matrix
-  DevBuf<double> rv;       // RDM2val (nocc^4), RV[i + nocc*(j + nocc*(k + nocc*l))]
+  DevBuf<double> rv;       // active block of RDM2val, RV[i + nact*(j + nact*(k + nact*l))]
+  DevBuf<int> slot;        // (ndimx) row order of the element kernel of the assembly
   // Per pair i = (p, q), with the CI coefficients C = sign(n - 1/2) sqrt(n) of
   // ACEneERPA_FOFO / AB_CAS_FOFO: C_p + C_q, C_p - C_q and their reciprocals (0 where
   // the sum or difference is 0), and n_p (1 - n_q) + n_q (1 - n_p). Computed once on

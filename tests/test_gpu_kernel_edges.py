@@ -1,0 +1,65 @@
+"""Kernels at the sizes where their tiling can go wrong, against the oracle.
+
+Inputs need no SCF here: random orthogonal orbitals and occupations, so that the sizes
+are free. Tolerances as in the parity tests.
+"""
+import numpy as np
+import pytest
+import torch
+
+from gammcor_gb300 import api, synth
+from oracle import ac_cas_ref as R
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def t(x):
+    return torch.as_tensor(np.ascontiguousarray(x), dtype=torch.float64, device=DEV)
+
+
+def model(n, nin, nact, seed=0):
+    """Integrals, one-electron part, occupations and 2-RDM without an SCF."""
+    rng = np.random.default_rng(seed)
+    lf = synth.make_lfac(n, 3 * n, rng) * 0.1
+    C, _ = np.linalg.qr(rng.standard_normal((n, n)))
+    occ = np.zeros(n)
+    occ[:nin] = 1.0
+    occ[nin:nin + nact] = np.linspace(0.96, 0.05, nact)
+    ffoo, fofo = R.transform_fofo_ffoo(C, lf @ lf.T, nin, nact)
+    return dict(n=n, nin=nin, nact=nact, occ=occ, xone=rng.standard_normal(synth.ntri(n)),
+                rdm=rng.standard_normal(nact ** 2 * (nact ** 2 + 1) // 2), ffoo=ffoo, fofo=fofo,
+                indn=R.pair_space(occ, nin + nact // 2), lf=lf, C=C)
+
+
+def assembled(m, indn, lam, ab1=False):
+    return api.ab_cas_fofo(m["occ"], m["xone"], indn, m["nact"], m["nin"], t(m["ffoo"]),
+                           t(m["fofo"]), m["rdm"], lam, ab1=ab1)
+
+
+# no inactive, no active, more than one 32-wide chunk of occupied and of all orbitals, sizes
+# around the 8 x 4 row tiles, an inactive occupation below 1 and an active one of exactly 1
+@pytest.mark.parametrize("n,nin,nact,ab1,odd_occ", [(9, 0, 3, False, False), (13, 4, 0, False, False),
+                                                    (40, 33, 2, False, True), (33, 3, 5, True, True),
+                                                    (17, 5, 1, False, False)])
+def test_assembly_tiles(gpu_lib, n, nin, nact, ab1, odd_occ):
+    m = model(n, nin, nact, seed=n)
+    if odd_occ:
+        m["occ"][0], m["occ"][nin] = 0.99, 1.0
+        m["occ"][-1] = 1e-3   # virtual occupations that differ: the general form of every element
+    rng = np.random.default_rng(1)
+    indn = m["indn"][rng.permutation(len(m["indn"]))]
+    rp, rm, re = R.ab_cas_fofo(m["occ"], m["xone"], np.eye(n), indn, nin, nact, m["ffoo"],
+                               m["fofo"], m["rdm"], 0.3, ab1=ab1)
+    gp, gm, ge = assembled(m, indn, 0.3, ab1)
+    assert np.abs(gp.cpu().numpy() - rp).max() < 1e-10 * np.abs(rp).max()
+    assert np.abs(gm.cpu().numpy() - rm).max() < 1e-10 * np.abs(rm).max()
+    assert abs(ge - re) < 1e-9
+
+
+def test_assembly_shows_a_nonfinite_integral_with_zero_weight(gpu_lib):
+    """(01|23) of four inactive orbitals has no weight in A+-B, but stays visible."""
+    m = model(17, 5, 2)
+    m["fofo"][0 + 1 * m["n"], 2 + 3 * m["n"]] = np.nan
+    gp, gm, _ = assembled(m, m["indn"], 0.5)
+    assert not torch.isfinite(gp).all() and not torch.isfinite(gm).all()
