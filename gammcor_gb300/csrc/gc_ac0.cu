@@ -15,7 +15,7 @@
 // and A+-' come out in block order directly (as ABPM0_FOFO assembles them) and
 // every block is a contiguous square. Then:
 //   k_ac0_block_erpa  one CTA per block: ERPASYMM0 in FP64 shared memory (two
-//                     cyclic-Jacobi eigensolves), Y, X and omega of the block;
+//                     Jacobi eigensolves), Y, X and omega of the block;
 //   k_ac0_iv          the (virtual, inactive) pairs: omega = A+(ii,ii), Y = X = 1/sqrt 2;
 //   k_ac0_right       T+ = A+' Xbd, T- = A-' Ybd (block-diagonal right products);
 //   k_ac0_work        work = 2 (Xbd^T T+ - Ybd^T T-) / (omega_i + omega_j);
@@ -32,163 +32,220 @@
 
 namespace {
 
-constexpr int kMaxBlock = 64;  // largest block (threads per block-solve CTA)
+constexpr int kMaxBlock = 64;  // largest block
 constexpr int kRow = kMaxBlock;  // row stride of the block-diagonal factors Yrow / Xrow
 const double kSmall = 1e-6;     // interpa.f:1511
 
-// Cyclic Jacobi (Golub and Van Loan, Alg. 8.5.3) on the symmetric m x m matrix A
-// (row stride ld) in shared memory, one thread per row; V <- eigenvectors (columns),
-// the eigenvalues are left on the diagonal of A. Returns false if 40 sweeps did not
-// bring the off-diagonal norm below 1e-30 of the total (uniform across the block).
-__device__ bool block_jacobi(double *A, double *V, int m, int ld, double *red) {
-  const int l = threadIdx.x;
-  if (l < m)
-    for (int b = 0; b < m; ++b) V[l * ld + b] = l == b ? 1.0 : 0.0;
-  __syncthreads();
+constexpr int kBlkThreads = 256;
+
+// Shared scratch of the block solve.
+struct BlockSh {
+  double red[2 * (kBlkThreads / 32)];
+  double c[kMaxBlock], s[kMaxBlock];  // x_i' = c_i x_i + s_i x_w(i)
+  int w[kMaxBlock];                   // the index that i is rotated with (i itself: none)
+  int p[kMaxBlock / 2];               // pair k: p[k] < q = w[p[k]], or w[p[k]] = p[k]
+};
+
+// FP32 values from FP64 ones scaled by a common power of two (the larger exponent emax goes
+// to 0), and back, by integer operations: conversions share the FP64 pipe.
+__device__ __forceinline__ float to_scaled_f32(double x, int emax) {
+  const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+  const int e = (int)((hi >> 20) & 0x7ff) - emax + 127;
+  if (e < 1) return 0.f;
+  return __uint_as_float((hi & 0x80000000u) | ((unsigned)e << 23) | ((hi & 0xfffffu) << 3) | (lo >> 29));
+}
+__device__ __forceinline__ double f32_to_f64(float x) {  // x normal or zero
+  const unsigned b = __float_as_uint(x);
+  if ((b & 0x7f800000u) == 0) return 0.0;
+  return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + 0x38000000u)), (int)(b << 29));
+}
+
+// Jacobi (Golub and Van Loan, Alg. 8.5.3, and 8.5.6 for the parallel ordering) on the symmetric
+// m x m matrix A (row stride ld >= m) in shared memory; V <- eigenvectors (columns), the
+// eigenvalues are left on the diagonal of A; T is scratch of A's size. Returns false if 40
+// sweeps did not bring the off-diagonal norm below 1e-30 of the total (uniform across the
+// block).
+//
+// A chain of rotations is bound by the latency of each, and a warp's FP64 instruction occupies
+// its quarter of the SM for 64 cycles however few of its lanes are live. So a sweep takes the
+// m (m - 1) / 2 pairs as rounds of m / 2 disjoint pairs (round robin); one thread per pair
+// forms its rotation with eight FP64 instructions; then every element of the upper triangle
+// is one thread's (six instructions, from A into T and back in turn), and so is every pair of
+// elements of V. The tangent is formed in FP32: it decides only how far the pair's element
+// shrinks (to 1e-7 of itself, beside the second-order terms of the other pairs); the rotation
+// itself is orthogonal to FP64 rounding, by a third-order step on the FP32 reciprocal root.
+// Measured for k_ac0_block_erpa with a 15 x 15 block (CAS(6,6), two eigensolves): one rotation
+// at a time 2.67 ms, rounds with FP64 angles and one thread per 2 x 2 block 0.53 ms, this 0.27 ms.
+__device__ bool block_jacobi(double *A, double *V, double *T, int m, int ld, BlockSh &sh) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int M = m + (m & 1), np = M / 2;
+  const int wd = (m & 1) ? m : m + 1;  // folded triangle: row a beside row m - a or m - 1 - a
+  double *src = A, *dst = T;
+  for (int e = tid; e < m * m; e += kBlkThreads) {
+    const int i = e / m, j = e - i * m;
+    V[i * ld + j] = i == j ? 1.0 : 0.0;
+  }
   for (int sweep = 0; sweep < 40; ++sweep) {
-    double off = 0.0, tot = 0.0;
-    if (l < m)
-      for (int b = 0; b < m; ++b) {
-        const double v = A[l * ld + b] * A[l * ld + b];
-        tot += v;
-        if (b != l) off += v;
-      }
-    red[l] = off;
-    red[kMaxBlock + l] = tot;
     __syncthreads();
-    for (int w = kMaxBlock / 2; w > 0; w >>= 1) {
-      if (l < w) {
-        red[l] += red[l + w];
-        red[kMaxBlock + l] += red[kMaxBlock + l + w];
+    double off = 0.0, tot = 0.0;
+    for (int e = tid; e < m * m; e += kBlkThreads) {
+      const int i = e / m, j = e - i * m;
+      const double v = src[i * ld + j] * src[i * ld + j];
+      tot += v;
+      if (i != j) off += v;
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      off += __shfl_down_sync(0xffffffffu, off, o);
+      tot += __shfl_down_sync(0xffffffffu, tot, o);
+    }
+    if (lane == 0) {
+      sh.red[2 * warp] = off;
+      sh.red[2 * warp + 1] = tot;
+    }
+    __syncthreads();
+    off = tot = 0.0;
+    for (int w = 0; w < kBlkThreads / 32; ++w) {
+      off += sh.red[2 * w];
+      tot += sh.red[2 * w + 1];
+    }
+    if (off <= 1e-30 * tot) {  // uniform: every thread added the same values
+      if (src != A) {
+        for (int e = tid; e < m * m; e += kBlkThreads) {
+          const int i = e / m, j = e - i * m;
+          A[i * ld + j] = src[i * ld + j];
+        }
+        __syncthreads();
+      }
+      return true;
+    }
+    for (int k = 0; k < M - 1; ++k) {
+      if (tid < np) {
+        const int x = tid == 0 ? M - 1 : (k + tid) % (M - 1);
+        const int y = tid == 0 ? k : (k - tid + M - 1) % (M - 1);
+        const int p = min(x, y), q = max(x, y);
+        double c = 1.0, sn = 0.0;
+        if (q < m) {
+          const double h = src[p * ld + q], d = src[q * ld + q] - src[p * ld + p];
+          if ((__double_as_longlong(h) << 1) != 0) {
+            // tan = 2h / (d +- sqrt(d^2 + 4 h^2))
+            const int ed = (__double2hiint(d) >> 20) & 0x7ff, eh = (__double2hiint(h) >> 20) & 0x7ff;
+            const int emax = max(ed, eh);
+            const float df = to_scaled_f32(d, emax), hf = 2.f * to_scaled_f32(h, emax);
+            const float r = sqrtf(df * df + hf * hf);
+            const float tf = hf / (df >= 0.f ? df + r : df - r);
+            const double t = f32_to_f64(tf), u = fma(t, t, 1.0);
+            const double y0 = f32_to_f64(rsqrtf(fmaf(tf, tf, 1.f)));
+            const double e = fma(-u, y0 * y0, 1.0);
+            c = fma(e * y0, fma(0.375, e, 0.5), y0);
+            sn = t * c;
+          }
+          sh.w[q] = p;
+          sh.c[q] = c;
+          sh.s[q] = sn;
+        }
+        sh.w[p] = q < m ? q : p;
+        sh.c[p] = c;
+        sh.s[p] = -sn;
+        sh.p[tid] = p;
       }
       __syncthreads();
-    }
-    const bool done = red[0] <= 1e-30 * red[kMaxBlock];
-    __syncthreads();
-    if (done) return true;
-    for (int p = 0; p < m - 1; ++p)
-      for (int q = p + 1; q < m; ++q) {
-        const double apq = A[p * ld + q];
-        if (apq == 0.0) continue;  // uniform: every thread reads the same value
-        const double theta = (A[q * ld + q] - A[p * ld + p]) / (2.0 * apq);
-        const double t = (theta >= 0.0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(theta * theta + 1.0));
-        const double c = 1.0 / sqrt(t * t + 1.0), sn = t * c;
-        __syncthreads();
-        if (l < m) {
-          const double aip = A[l * ld + p], aiq = A[l * ld + q];
-          A[l * ld + p] = c * aip - sn * aiq;
-          A[l * ld + q] = sn * aip + c * aiq;
-        }
-        __syncthreads();
-        if (l < m) {
-          const double api = A[p * ld + l], aqi = A[q * ld + l];
-          A[p * ld + l] = c * api - sn * aqi;
-          A[q * ld + l] = sn * api + c * aqi;
-          const double vip = V[l * ld + p], viq = V[l * ld + q];
-          V[l * ld + p] = c * vip - sn * viq;
-          V[l * ld + q] = sn * vip + c * viq;
-        }
-        __syncthreads();
+      for (int e = tid; e < (m + 1) / 2 * wd; e += kBlkThreads) {
+        const int a = e / wd, b = e - a * wd;
+        const bool first = b < m - a;
+        const int i = first ? a : ((m & 1) ? m - a : m - 1 - a), j = first ? a + b : i + b - (m - a);
+        if (j >= m) continue;
+        const int iw = sh.w[i], jw = sh.w[j];
+        const double ci = sh.c[i], si = sh.s[i], cj = sh.c[j], sj = sh.s[j];
+        const double x = cj * src[i * ld + j] + sj * src[i * ld + jw];
+        const double y = cj * src[iw * ld + j] + sj * src[iw * ld + jw];
+        const double v = ci * x + si * y;
+        dst[i * ld + j] = v;
+        dst[j * ld + i] = v;
       }
+      for (int e = kBlkThreads - 1 - tid; e < m * np; e += kBlkThreads) {
+        const int i = e / np, r = sh.p[e - i * np], u = sh.w[r];
+        if (u == r) continue;
+        const double x = V[i * ld + r], y = V[i * ld + u];
+        V[i * ld + r] = sh.c[r] * x + sh.s[r] * y;
+        V[i * ld + u] = sh.c[u] * y + sh.s[u] * x;
+      }
+      __syncthreads();
+      double *t = src;
+      src = dst;
+      dst = t;
+    }
   }
   return false;
 }
 
-// ERPASYMM0 of every block (one CTA of kMaxBlock threads each): block b covers the
-// block-order positions bstart[b] .. bstart[b] + bsize[b] - 1 of the column-major
-// N x N matrices ap, am (A+-B at lambda = 0). Writes Yrow/Xrow[(s + i) * kRow + c] =
-// Y/X(i, c) of the block and eig[s + c]; a Jacobi that does not converge sets *flag.
-__global__ void __launch_bounds__(kMaxBlock) k_ac0_block_erpa(
+// ERPASYMM0 of every block (one CTA each): block b covers the block-order positions
+// bstart[b] .. bstart[b] + bsize[b] - 1 of the column-major N x N matrices ap, am (A+-B at
+// lambda = 0). Writes Yrow/Xrow[(s + i) * kRow + c] = Y/X(i, c) of the block and eig[s + c]; a
+// Jacobi that does not converge sets *flag. The largest block (active-active pairs) sets
+// the time: its two eigensolves are a chain of rotations.
+__global__ void __launch_bounds__(kBlkThreads) k_ac0_block_erpa(
     int N, const double *__restrict__ ap, const double *__restrict__ am,
-    const int *__restrict__ bstart, const int *__restrict__ bsize, int ld, double *__restrict__ Yrow,
-    double *__restrict__ Xrow, double *__restrict__ eig, int *flag) {
+    const int *__restrict__ bstart, const int *__restrict__ bsize, int rows, int ld,
+    double *__restrict__ Yrow, double *__restrict__ Xrow, double *__restrict__ eig, int *flag) {
   extern __shared__ double sm[];
-  const int s = bstart[blockIdx.x], m = bsize[blockIdx.x];
-  double *A = sm, *B = A + kMaxBlock * ld, *P = B + kMaxBlock * ld, *H = P + kMaxBlock * ld,
-         *V = H + kMaxBlock * ld;
-  __shared__ double red[2 * kMaxBlock];
-  __shared__ double w2[kMaxBlock], sq[kMaxBlock];
-  const int l = threadIdx.x;
+  __shared__ BlockSh sh;
+  __shared__ double w2[kMaxBlock];
+  const int s = bstart[blockIdx.x], m = bsize[blockIdx.x], tid = threadIdx.x;
+  const size_t sz = (size_t)rows * ld;
+  double *A = sm, *B = A + sz, *P = B + sz, *H = P + sz, *V = H + sz;
+  auto each = [&](auto f) {  // f(i, j) over the m x m elements
+    for (int e = tid; e < m * m; e += kBlkThreads) f(e / m, e % m);
+    __syncthreads();
+  };
+  auto dot = [&](const double *x, int sx, const double *y, int sy) {
+    double v = 0.0;
+    for (int k = 0; k < m; ++k) v += x[k * sx] * y[k * sy];
+    return v;
+  };
   // symmetrised blocks (interpa.f:1532-1540)
-  if (l < m)
-    for (int j = 0; j < m; ++j) {
-      const size_t e = (size_t)(s + l) + (size_t)(s + j) * N, t = (size_t)(s + j) + (size_t)(s + l) * N;
-      A[l * ld + j] = 0.5 * (ap[e] + ap[t]);
-      B[l * ld + j] = 0.5 * (am[e] + am[t]);
-    }
-  __syncthreads();
-  if (!block_jacobi(A, V, m, ld, red)) {
-    if (l == 0) atomicOr(flag, 1);
+  each([&](int j, int i) {  // i fastest: consecutive threads read consecutive rows
+    const size_t e = (size_t)(s + i) + (size_t)(s + j) * N, t = (size_t)(s + j) + (size_t)(s + i) * N;
+    A[i * ld + j] = 0.5 * (ap[e] + ap[t]);
+    B[i * ld + j] = 0.5 * (am[e] + am[t]);
+  });
+  if (!block_jacobi(A, V, H, m, ld, sh)) {
+    if (tid == 0) atomicOr(flag, 1);
     return;  // uniform
   }
-  if (l < m) sq[l] = sqrt(fabs(A[l * ld + l]));
+  if (tid < m) w2[tid] = sqrt(fabs(A[tid * ld + tid]));
   __syncthreads();
   // P = V diag(sqrt|e|) V^T = A+^1/2 (interpa.f:1546-1568)
-  if (l < m)
-    for (int j = 0; j < m; ++j) {
-      double v = 0.0;
-      for (int k = 0; k < m; ++k) v += V[l * ld + k] * sq[k] * V[j * ld + k];
-      P[l * ld + j] = v;
-    }
-  __syncthreads();
+  each([&](int i, int j) {
+    double v = 0.0;
+    for (int k = 0; k < m; ++k) v += V[i * ld + k] * w2[k] * V[j * ld + k];
+    P[i * ld + j] = v;
+  });
   // H = A- P, then A <- P H (the symmetrised problem, interpa.f:1578-1581)
-  if (l < m)
-    for (int j = 0; j < m; ++j) {
-      double v = 0.0;
-      for (int k = 0; k < m; ++k) v += B[l * ld + k] * P[k * ld + j];
-      H[l * ld + j] = v;
-    }
-  __syncthreads();
-  if (l < m)
-    for (int j = 0; j < m; ++j) {
-      double v = 0.0;
-      for (int k = 0; k < m; ++k) v += P[l * ld + k] * H[k * ld + j];
-      A[l * ld + j] = v;
-    }
-  __syncthreads();
-  if (l < m)  // the lower triangle, as the eigensolver reads it
-    for (int j = l + 1; j < m; ++j) A[l * ld + j] = A[j * ld + l];
-  __syncthreads();
-  if (!block_jacobi(A, V, m, ld, red)) {
-    if (l == 0) atomicOr(flag, 1);
+  each([&](int i, int j) { H[i * ld + j] = dot(B + i * ld, 1, P + j, ld); });
+  each([&](int i, int j) {  // the lower triangle, as the eigensolver reads it
+    if (i >= j) A[i * ld + j] = A[j * ld + i] = dot(P + i * ld, 1, H + j, ld);
+  });
+  if (!block_jacobi(A, V, H, m, ld, sh)) {
+    if (tid == 0) atomicOr(flag, 1);
     return;
   }
-  if (l < m) w2[l] = A[l * ld + l];
-  __syncthreads();
-  // Y = P Z into H
-  if (l < m)
-    for (int j = 0; j < m; ++j) {
-      double v = 0.0;
-      for (int k = 0; k < m; ++k) v += P[l * ld + k] * V[k * ld + j];
-      H[l * ld + j] = v;
-    }
-  __syncthreads();
-  // thread = mode nu: normalise 2/omega y^T A- y = 1, X = A- y / omega (interpa.f:1598-1648)
-  if (l < m) {
-    const int nu = l;
-    double om = w2[nu];
+  if (tid < m) w2[tid] = A[tid * ld + tid];
+  // Y = P Z into H, A- Y into A
+  each([&](int i, int j) { H[i * ld + j] = dot(P + i * ld, 1, V + j, ld); });
+  each([&](int i, int j) { A[i * ld + j] = dot(B + i * ld, 1, H + j, ld); });
+  // mode nu: normalise 2/omega y^T A- y = 1, X = A- y / omega (interpa.f:1598-1648)
+  if (tid < m) {
+    const int nu = tid;
+    double om = w2[nu], f = 0.0, g = 0.0;
     if (om > kSmall) {
       om = sqrt(om);
-      double sum = 0.0;
-      for (int i = 0; i < m; ++i) {
-        double bi = 0.0;
-        for (int j = 0; j < m; ++j) bi += B[i * ld + j] * H[j * ld + nu];
-        sum += H[i * ld + nu] * bi;
-      }
-      sum *= 2.0 / om;
-      const double f = sum > 0.0 ? 1.0 / sqrt(sum) : 0.0;
-      for (int i = 0; i < m; ++i) H[i * ld + nu] *= f;
-      for (int i = 0; i < m; ++i) {
-        double bi = 0.0;
-        for (int j = 0; j < m; ++j) bi += B[i * ld + j] * H[j * ld + nu];
-        Xrow[(size_t)(s + i) * kRow + nu] = bi / om;
-        Yrow[(size_t)(s + i) * kRow + nu] = H[i * ld + nu];
-      }
-    } else {
-      for (int i = 0; i < m; ++i) {
-        Xrow[(size_t)(s + i) * kRow + nu] = 0.0;
-        Yrow[(size_t)(s + i) * kRow + nu] = 0.0;
-      }
+      const double sum = 2.0 / om * dot(H + nu, ld, A + nu, ld);
+      f = sum > 0.0 ? 1.0 / sqrt(sum) : 0.0;
+      g = f / om;
+    }
+    for (int i = 0; i < m; ++i) {
+      Yrow[(size_t)(s + i) * kRow + nu] = f * H[i * ld + nu];
+      Xrow[(size_t)(s + i) * kRow + nu] = g * A[i * ld + nu];
     }
     eig[s + nu] = om;  // omega, or omega^2 where omega^2 <= Small
   }
@@ -400,11 +457,11 @@ extern "C" int gc_ac0cas_fofo(gc_context *ctx, int nbas, int ninact, int nact, i
   GC_CUDA(ctx, cudaMemsetAsync(flag.p, 0, sizeof(int), ctx->stream));
   if (nblk > 0) {
     const int ld = mmax + 1;
-    const size_t smem = 5 * (size_t)kMaxBlock * ld * sizeof(double);
+    const size_t smem = 5 * (size_t)mmax * ld * sizeof(double);
     GC_CUDA(ctx, cudaFuncSetAttribute(k_ac0_block_erpa, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)smem));
-    k_ac0_block_erpa<<<nblk, kMaxBlock, smem, ctx->stream>>>(N, a0p.p, a0m.p, dbs.p, dbz.p, ld,
-                                                              Yrow.p, Xrow.p, eig.p, flag.p);
+    k_ac0_block_erpa<<<nblk, kBlkThreads, smem, ctx->stream>>>(
+        N, a0p.p, a0m.p, dbs.p, dbz.p, mmax, ld, Yrow.p, Xrow.p, eig.p, flag.p);
     GC_LAUNCHED(ctx);
   }
   if (iv0 < N) {

@@ -63,3 +63,25 @@ def test_assembly_shows_a_nonfinite_integral_with_zero_weight(gpu_lib):
     m["fofo"][0 + 1 * m["n"], 2 + 3 * m["n"]] = np.nan
     gp, gm, _ = assembled(m, m["indn"], 0.5)
     assert not torch.isfinite(gp).all() and not torch.isfinite(gm).all()
+
+
+# AC0 blocks of odd and even size, of one pair, and an active-active block of 55 pairs
+@pytest.mark.parametrize("n,nin,nact", [(12, 2, 1), (14, 1, 2), (21, 2, 5), (30, 0, 11)])
+def test_ac0_block_sizes(gpu_lib, n, nin, nact):
+    from oracle import ac0_ref as A
+    m = model(n, nin, nact, seed=n)
+    # a dominant one-electron diagonal keeps the zeroth-order blocks stable
+    m["xone"] *= 0.05
+    d = np.cumsum(np.arange(1, n + 1)) - 1
+    m["xone"][d] = np.linspace(-30.0, 10.0, n)
+    m["rdm"] = np.zeros_like(m["rdm"])
+    o = m["occ"][nin:nin + nact]
+    e = np.eye(nact)
+    m["rdm"] = synth.pack_rdm2act(2 * np.einsum("p,q,pr,qs->pqrs", o, o, e, e)
+                                  - np.einsum("p,q,ps,qr->pqrs", o, o, e, e))
+    e0, etot = A.ac0cas_fofo(m["occ"], m["xone"], np.eye(n), m["indn"], nin, nact, m["ffoo"],
+                             m["fofo"], m["rdm"])
+    ge, get = api.ac0cas_fofo(m["occ"], m["xone"], m["indn"], nact, nin, t(m["ffoo"]),
+                              t(m["fofo"]), m["rdm"])
+    assert abs(ge - e0) < 1e-9 * max(1.0, abs(e0))
+    assert abs(get - etot) < 1e-9 * max(1.0, abs(etot))
