@@ -642,124 +642,159 @@ __device__ __forceinline__ int exp_of_bits(unsigned long long m) {
 }
 constexpr unsigned long long kInfBits = 0x7ff0000000000000ull;
 
-// Row exponents: e[b][r] = 1 + ilogb(max_k |x[b,r,k]|) (0 for a zero row, kBadExp for a
-// row with a non-finite element), with integer operations on the bit patterns (no FP64
-// pipe): one warp per row (rows whose K elements are contiguous, sk = 1) ...
-__global__ void k_row_exponent(const double *__restrict__ x, int rows, int K, int nb, long long sr,
-                               long long sk, long long sb, int *__restrict__ e) {
-  long long total = (long long)nb * rows;
-  long long wid = (blockIdx.x * (long long)blockDim.x + threadIdx.x) / 32;
-  int lane = threadIdx.x % 32;
-  for (long long t = wid; t < total; t += (long long)gridDim.x * blockDim.x / 32) {
-    int r = (int)(t % rows);
-    long long bb = t / rows;
-    const double *row = x + bb * sb + (long long)r * sr;
-    unsigned long long mx = 0;
-    for (int k = lane; k < K; k += 32) mx = max(mx, abs_bits(row[(long long)k * sk]));
-    for (int off = 16; off > 0; off >>= 1) mx = max(mx, __shfl_down_sync(0xffffffffu, mx, off));
-    if (lane == 0) e[t] = mx >= kInfBits ? kBadExp : (mx ? exp_of_bits(mx) : 0);
-  }
+// e = 1 + ilogb of the row's largest |x| (its bits mx): 0 for a zero row, kBadExp for a row
+// with a non-finite element.
+__device__ __forceinline__ int row_exponent(unsigned long long mx) {
+  return mx >= kInfBits ? kBadExp : (mx ? exp_of_bits(mx) : 0);
 }
 
-// ... or, for consecutive rows contiguous (sr = 1), 32 rows per block with the lanes along
-// the rows (loads coalesced for every k) and 8 warps splitting K.
-__global__ void k_row_exponent_cols(const double *__restrict__ x, int rows, int K,
-                                    long long sk, long long sb, int *__restrict__ e) {
-  __shared__ unsigned long long part[8][32];
-  const int tx = threadIdx.x, ty = threadIdx.y;
-  const int r = blockIdx.x * 32 + tx;
-  const long long bb = blockIdx.y;
-  unsigned long long mx = 0;
-  if (r < rows) {
-    const double *row = x + bb * sb + r;
-    for (int k = ty; k < K; k += 8) mx = max(mx, abs_bits(row[(long long)k * sk]));
-  }
-  part[ty][tx] = mx;
-  __syncthreads();
-  if (ty == 0 && r < rows) {
-    for (int w = 1; w < 8; ++w) mx = max(mx, part[w][tx]);
-    e[bb * rows + r] = mx >= kInfBits ? kBadExp : (mx ? exp_of_bits(mx) : 0);
-  }
-}
-
-// x 2^sh rounded to the nearest integer (ties to even), for |x 2^sh| < 2^62, from the bit
-// pattern of x with integer operations only: the same value as __double2ll_rn(ldexp(x, sh))
-// (the scaling is exact unless the result is below 0.5, which rounds to 0 either way),
-// without the FP64 pipe, which is narrow on GB300.
-__device__ __forceinline__ long long scaled_round(double x, int sh) {
+// Balanced base-128 digits of n = rint(x 2^(7S - e)) (|x| < 2^e, so |n| <= 2^(7S)):
+// n = sum_s a_s 128^(S-1-s), |a_0| <= 128, |a_s| <= 64 otherwise, as FP32 bit patterns whose
+// upper half is the BF16 value. Rounding is to nearest even, as __double2ll_rn(ldexp(x, 7S - e))
+// rounds (that scaling is exact unless the result is below 1/2, which rounds to 0 either way).
+// Integer operations but for one FP32 addition per digit: GB300's FP64 pipe is narrow, and
+// integer-to-float conversions share a quarter-rate pipe. With B = 64 (1 + 128 + ...) added
+// once, the lower digits are plain 7-bit fields minus 64 and the carries are already in place.
+template <int S>
+__device__ __forceinline__ void digits(double x, int e, uint32_t *d) {
   const unsigned long long b = (unsigned long long)__double_as_longlong(x);
   const int E = (int)((b >> 52) & 0x7ff);
-  unsigned long long m = b & 0xfffffffffffffull;
-  int q = -1074;  // x = +-m 2^q
-  if (E != 0) {
-    m |= 1ull << 52;
-    q = E - 1075;
+  const unsigned long long m = (b & 0xfffffffffffffull) | (E ? 1ull << 52 : 0ull);
+  // x = +-m 2^(max(E, 1) - 1075); |x| < 2^e makes the shift at least 53 - 7S > 0, unless the
+  // whole row is subnormal
+  const int sft = e == kBadExp ? 64 : 1075 - max(E, 1) - 7 * S + e;
+  long long n = 0;
+  if (sft < 1)
+    n = (long long)(m << -sft);
+  else if (sft <= 63)
+    n = (long long)((m + ((1ull << (sft - 1)) - 1) + ((m >> sft) & 1)) >> sft);
+  if (b >> 63) n = -n;
+  unsigned long long bias = 0;
+#pragma unroll
+  for (int s = 1; s < S; ++s) bias = bias * 128 + 64;
+  const long long u = n + (long long)bias;
+#pragma unroll
+  for (int s = 1; s < S; ++s) {
+    const int v = (int)(u >> (7 * (S - 1 - s))) & 127;
+    d[s] = __float_as_uint(__int_as_float(0x4B400000 - 64 + v) - 12582912.f);
   }
-  q += sh;
-  unsigned long long n;
-  if (m == 0 || q < -63) {
-    n = 0;  // |x 2^sh| < 2^53 2^-64 < 1/2
-  } else if (q >= 0) {
-    n = m << q;
-  } else {
-    const int sft = -q;  // 1..63
-    const unsigned long long whole = m >> sft, rem = m & ((1ull << sft) - 1),
-                             half = 1ull << (sft - 1);
-    n = whole + ((rem > half || (rem == half && (whole & 1))) ? 1 : 0);
-  }
-  return (b >> 63) ? -(long long)n : (long long)n;
+  d[0] = __float_as_uint(__int_as_float(0x4B400000 + (int)(u >> (7 * (S - 1)))) - 12582912.f);
 }
 
-// Balanced base-128 digits of n = rint(x 2^(7S - e)) (|n| < 2^(7S) since |x| < 2^e):
-// n = sum_s a_s 128^(S-1-s), |a_0| <= 128, |a_s| <= 64 otherwise; plane s gets a_s. All
-// in integer arithmetic.
-__device__ __forceinline__ void store_digits(double x, int e, int S, long long plane, long long o,
-                                             __nv_bfloat16 *__restrict__ planes) {
-  long long n = e == kBadExp ? 0 : scaled_round(x, 7 * S - e);
-  for (int s = S - 1; s > 0; --s) {
-    const long long d = ((n + 64) & 127) - 64;
-    planes[s * plane + o] = __float2bfloat16_rn((float)d);
-    n = (n - d) >> 7;
-  }
-  planes[o] = __float2bfloat16_rn((float)n);
+// Four consecutive elements of one row into their S planes, 8 bytes per plane.
+template <int S>
+__device__ __forceinline__ void store_digits4(const double *x, int e, long long plane, long long o,
+                                              __nv_bfloat16 *__restrict__ planes) {
+  uint32_t d[4][S];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) digits<S>(x[i], e, d[i]);
+#pragma unroll
+  for (int s = 0; s < S; ++s)
+    *reinterpret_cast<uint2 *>(planes + s * plane + o) =
+        make_uint2(__byte_perm(d[0][s], d[1][s], 0x7632), __byte_perm(d[2][s], d[3][s], 0x7632));
 }
 
-// Integer slices: planes[t][b][r][kp] = alpha_t of x[b,r,k] 2^-e[b][r].
-// Rows (b, r) over blockIdx.y, K over the threads: no 64-bit division per element.
-__global__ void k_slice_planes(const double *__restrict__ x, int rows, int K, int Kp, int nb,
-                               long long sr, long long sk, long long sb, int S,
-                               const int *__restrict__ e, __nv_bfloat16 *__restrict__ planes) {
-  const long long plane = (long long)nb * rows * Kp, nrr = (long long)nb * rows;
-  for (long long rr = blockIdx.y; rr < nrr; rr += gridDim.y) {
-    const long long bb = rr / rows;
-    const int r = (int)(rr - bb * rows);
-    const int ex = e[rr];
-    const double *__restrict__ xr = x + bb * sb + (long long)r * sr;
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < Kp; k += gridDim.x * blockDim.x) {
-      const double xv = k < K ? xr[(long long)k * sk] : 0.0;
-      store_digits(xv, ex, S, plane, rr * Kp + k, planes);
+// Row exponents and integer slices, planes[t][b][r][kp] = alpha_t of x[b,r,k] 2^-e[b][r], of an
+// operand whose K elements are contiguous: TPR threads per row, each holding its elements of
+// the row in registers between the maximum and the digits (rows longer than TPR * 4 * kOzHold
+// are read again for the rest). Bound by HBM: 8 bytes read and 2 S written per element. One
+// warp per row up to 1024 elements, so that short rows fill a block; a block per longer row.
+// Measured (5 slices): 3774 x 3774 62 us = 4.1 TB/s, where a pass for the exponents and a pass
+// with 2-byte stores took 155 us.
+constexpr int kOzHold = 8;  // groups of four elements per thread
+template <int S, int TPR>
+__global__ void __launch_bounds__(256) k_oz_rows(const double *__restrict__ x, int rows, int K, int Kp,
+                                                 long long nrr, long long sr, long long sb,
+                                                 int *__restrict__ e,
+                                                 __nv_bfloat16 *__restrict__ planes) {
+  __shared__ unsigned long long part[8];
+  const int t = threadIdx.x % TPR;
+  const long long rr = blockIdx.x * (long long)(256 / TPR) + threadIdx.x / TPR;
+  const bool live = rr < nrr;
+  const long long bb = live ? rr / rows : 0;
+  const double *__restrict__ xr = x + (live ? bb * sb + (rr - bb * rows) * sr : 0);
+  double v[kOzHold][4];
+  unsigned long long mx = 0;
+  const int ng = Kp / 4;
+#pragma unroll
+  for (int g = 0; g < kOzHold; ++g)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int k = (t + g * TPR) * 4 + i;
+      v[g][i] = live && k < K ? xr[k] : 0.0;
     }
+#pragma unroll
+  for (int g = 0; g < kOzHold; ++g)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) mx = max(mx, abs_bits(v[g][i]));
+  if (live)
+    for (int k = TPR * 4 * kOzHold + t; k < K; k += TPR) mx = max(mx, abs_bits(xr[k]));
+  for (int off = 16; off > 0; off >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+  if (TPR > 32) {
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = mx;
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < 8; ++w) mx = max(mx, part[w]);
+  }
+  if (!live) return;
+  const int ex = row_exponent(mx);
+  if (t == 0) e[rr] = ex;
+  const long long plane = nrr * Kp;
+#pragma unroll
+  for (int g = 0; g < kOzHold; ++g)
+    if (t + g * TPR < ng) store_digits4<S>(v[g], ex, plane, rr * Kp + (t + g * TPR) * 4, planes);
+  for (int g = t + kOzHold * TPR; g < ng; g += TPR) {
+    double w[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) w[i] = g * 4 + i < K ? xr[g * 4 + i] : 0.0;
+    store_digits4<S>(w, ex, plane, rr * Kp + g * 4, planes);
   }
 }
 
-// Transposed-read variant (K is the slow index of x).
-__global__ void k_slice_planes_t(const double *__restrict__ x, int rows, int K, int Kp, int nb,
-                                 long long sr, long long sk, long long sb, int S,
-                                 const int *__restrict__ e, __nv_bfloat16 *__restrict__ planes) {
-  __shared__ double tile[32][33];
-  int r0 = blockIdx.x * 32, k0 = blockIdx.y * 32, bb = blockIdx.z;
-  int tx = threadIdx.x, ty = threadIdx.y;
-  for (int i = ty; i < 32; i += 8) {
-    int k = k0 + i, r = r0 + tx;
-    tile[i][tx] = (k < K && r < rows) ? x[bb * sb + (long long)r * sr + (long long)k * sk] : 0.0;
-  }
-  __syncthreads();
-  long long plane = (long long)nb * rows * Kp;
-  for (int i = ty; i < 32; i += 8) {
-    int r = r0 + i, k = k0 + tx;
-    if (r >= rows || k >= Kp) continue;
-    const long long o = ((long long)bb * rows + r) * Kp + k;
-    store_digits(tile[tx][i], e[(long long)bb * rows + r], S, plane, o, planes);
+// The same for any other strides (in use: consecutive rows contiguous, K the slow index). One
+// block takes 32 rows: the maximum with the lanes along the rows, then 64 values of K at a time
+// through shared memory, read along the rows and written along K. The position of k within
+// its 64 is (k / 4) + 16 (k % 4), so that four consecutive k are read without bank conflicts.
+template <int S>
+__global__ void __launch_bounds__(512) k_oz_cols(const double *__restrict__ x, int rows, int K, int Kp,
+                                                 int nb, long long sr, long long sk, long long sb,
+                                                 int *__restrict__ e,
+                                                 __nv_bfloat16 *__restrict__ planes) {
+  __shared__ double tile[32][65];
+  __shared__ unsigned long long part[16][32];
+  __shared__ int es[32];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int r0 = blockIdx.x * 32, r = r0 + tx;
+  const int lr = threadIdx.x >> 4, lk = threadIdx.x & 15;  // row and group of four in the write
+  const long long plane = (long long)nb * rows * Kp;
+  for (int bb = blockIdx.y; bb < nb; bb += gridDim.y) {
+    const double *__restrict__ xr = x + bb * sb + (long long)r * sr;
+    unsigned long long mx = 0;
+    if (r < rows) {
+#pragma unroll 4
+      for (int k = ty; k < K; k += 16) mx = max(mx, abs_bits(xr[(long long)k * sk]));
+    }
+    part[ty][tx] = mx;
+    __syncthreads();
+    if (ty == 0) {
+      for (int w = 1; w < 16; ++w) mx = max(mx, part[w][tx]);
+      es[tx] = row_exponent(mx);
+      if (r < rows) e[(long long)bb * rows + r] = es[tx];
+    }
+    for (int k0 = 0; k0 < Kp; k0 += 64) {
+      __syncthreads();
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int k = ty + 16 * i;
+        tile[tx][(k >> 2) + 16 * (k & 3)] = r < rows && k0 + k < K ? xr[(long long)(k0 + k) * sk] : 0.0;
+      }
+      __syncthreads();
+      if (r0 + lr < rows) {
+        const double v[4] = {tile[lr][lk], tile[lr][lk + 16], tile[lr][lk + 32], tile[lr][lk + 48]};
+        store_digits4<S>(v, es[lr], plane, ((long long)bb * rows + r0 + lr) * Kp + k0 + lk * 4, planes);
+      }
+    }
+    __syncthreads();
   }
 }
 
@@ -961,6 +996,24 @@ int encode_oz_map(gc_context *ctx, OzOperand &op) {
   return GC_OK;
 }
 
+template <int S>
+int slice_operand(gc_context *ctx, OzOperand &op, const double *x, int rows, int K, int nb,
+                  long long sr, long long sk, long long sb) {
+  const long long nrr = (long long)nb * rows;
+  if (sk == 1 && op.Kp <= 128 * kOzHold) {  // one warp holds the row
+    k_oz_rows<S, 32><<<gc::ceil_div(nrr, 8), 256, 0, ctx->stream>>>(x, rows, K, op.Kp, nrr, sr, sb,
+                                                                    op.exps.p, op.buf.p);
+  } else if (sk == 1) {
+    k_oz_rows<S, 256><<<(unsigned)nrr, 256, 0, ctx->stream>>>(x, rows, K, op.Kp, nrr, sr, sb,
+                                                              op.exps.p, op.buf.p);
+  } else {
+    k_oz_cols<S><<<dim3(gc::ceil_div(rows, 32), std::min(nb, 65535)), 512, 0, ctx->stream>>>(
+        x, rows, K, op.Kp, nb, sr, sk, sb, op.exps.p, op.buf.p);
+  }
+  GC_LAUNCHED(ctx);
+  return GC_OK;
+}
+
 int make_oz_operand(gc_context *ctx, OzOperand &op, const double *x, int rows, int K, int nb,
                     long long sr, long long sk, long long sb, int S, int box_rows) {
   op.rows = rows;
@@ -971,27 +1024,11 @@ int make_oz_operand(gc_context *ctx, OzOperand &op, const double *x, int rows, i
   size_t plane = (size_t)nb * rows * op.Kp;
   GC_TRY(op.exps.alloc(ctx, (size_t)nb * rows));
   GC_TRY(op.buf.alloc(ctx, plane * S));
-  if (sr == 1 && sk != 1 && nb <= 65535) {
-    k_row_exponent_cols<<<dim3(gc::ceil_div(rows, 32), nb), dim3(32, 8), 0, ctx->stream>>>(
-        x, rows, K, sk, sb, op.exps.p);
-    GC_LAUNCHED(ctx);
-  } else {
-    size_t warps = (size_t)nb * rows;
-    unsigned grid = std::min<unsigned>(gc::ceil_div(warps * 32, 256), 152u * 64u);
-    k_row_exponent<<<grid, 256, 0, ctx->stream>>>(x, rows, K, nb, sr, sk, sb, op.exps.p);
-    GC_LAUNCHED(ctx);
+  switch (S) {
+    case 4: GC_TRY(slice_operand<4>(ctx, op, x, rows, K, nb, sr, sk, sb)); break;
+    case 5: GC_TRY(slice_operand<5>(ctx, op, x, rows, K, nb, sr, sk, sb)); break;
+    default: GC_TRY(slice_operand<6>(ctx, op, x, rows, K, nb, sr, sk, sb));
   }
-  if (sk == 1) {
-    const dim3 grid(std::min(gc::ceil_div(op.Kp, 256), 4u),
-                    (unsigned)std::min<long long>((long long)nb * rows, 65535));
-    k_slice_planes<<<grid, 256, 0, ctx->stream>>>(x, rows, K, op.Kp, nb, sr, sk, sb, S, op.exps.p,
-                                                   op.buf.p);
-  } else {
-    dim3 grid(gc::ceil_div(rows, 32), gc::ceil_div(op.Kp, 32), nb);
-    k_slice_planes_t<<<grid, dim3(32, 8), 0, ctx->stream>>>(x, rows, K, op.Kp, nb, sr, sk, sb, S,
-                                                             op.exps.p, op.buf.p);
-  }
-  GC_LAUNCHED(ctx);
   op.planes = op.buf.p;
   op.ex = op.exps.p;
   return encode_oz_map(ctx, op);

@@ -85,3 +85,35 @@ def test_ac0_block_sizes(gpu_lib, n, nin, nact):
                               t(m["fofo"]), m["rdm"])
     assert abs(ge - e0) < 1e-9 * max(1.0, abs(e0))
     assert abs(get - etot) < 1e-9 * max(1.0, abs(etot))
+
+
+def sliced_product(A, B, S):
+    """C = A B^T by the balanced base-128 slicing with exact integer sums: the bits that the
+    sliced GEMM has to give (up to 5 slices; every weight's sum fits an int64)."""
+    def cut(X):
+        e = np.where((X != 0).any(1), np.frexp(np.abs(X).max(1))[1], 0)
+        n = np.rint(np.ldexp(X, (7 * S - e)[:, None])).astype(np.int64)
+        d = []
+        for _ in range(S - 1):
+            d.append(((n + 64) & 127) - 64)
+            n = (n - d[-1]) >> 7
+        return e, [n] + d[::-1]
+    ea, a = cut(A)
+    eb, b = cut(B)
+    acc = sum((a[t] @ b[u].T) << (7 * (S - 1 - t - u)) for t in range(S) for u in range(S - t))
+    return np.ldexp(acc.astype(np.float64), ea[:, None] + eb[None, :] - 7 * (S + 1))
+
+
+# rows and K around the 32-row and 64-value tiles of the slicing, zero rows, ties, subnormals
+@pytest.mark.parametrize("S", [4, 5])
+@pytest.mark.parametrize("m,n,k", [(1, 1, 1), (33, 31, 63), (65, 97, 64), (130, 40, 129)])
+def test_sliced_gemm_bits(gpu_lib, S, m, n, k):
+    rng = np.random.default_rng(m * k)
+    A = rng.standard_normal((m, k)) * 2.0 ** rng.integers(-30, 4, (m, k))
+    B = rng.standard_normal((n, k)) * 2.0 ** rng.integers(-30, 4, (n, k))
+    A[::7] = np.round(A[::7] * 2 ** 10) / 2 ** 10     # exact ties among the roundings
+    A[-1] = 0.0
+    if m > 2:
+        A[1] = 3.0 * 2.0 ** -1070 * rng.integers(-5, 6, k)
+    C = api.tc_gemm_nt(t(A), t(B), f"fp64tc{S}").cpu().numpy()
+    assert np.array_equal(C, sliced_product(A, B, S))
