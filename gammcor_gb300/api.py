@@ -138,6 +138,14 @@ def _fortran_cols(t: torch.Tensor) -> torch.Tensor:
     return t.t().contiguous()
 
 
+def _blocks(*blocks: torch.Tensor) -> list[torch.Tensor]:
+    """Column-major FP64 copies of orbital blocks; a tensor given twice is copied once, and the
+    library then sees one block (it uses the symmetry of a pair of equal blocks)."""
+    done = {}
+    return [done.setdefault(id(b), _fortran_cols(b.to(torch.float64))) if id(b) not in done
+            else done[id(b)] for b in blocks]
+
+
 # --------------------------------------------------------------- host helpers
 def gauleg(x1: float, x2: float, n: int):
     """GauLeg (misc.f:828-865)."""
@@ -178,7 +186,7 @@ def tran4_gen(nbas: int, CA: torch.Tensor, CB: torch.Tensor, CC: torch.Tensor, C
     the output file as (nA*nB, nC*nD): row = record ab, column = element cd.
     """
     ctx = ctx or default_context(CA.device.index or 0)
-    cols = [_fortran_cols(c.to(torch.float64)) for c in (CA, CB, CC, CD)]
+    cols = _blocks(CA, CB, CC, CD)
     nA, nB, nC, nD = (c.shape[0] for c in cols)
     if out is None:
         out = torch.empty((nA * nB, nC * nD), dtype=torch.float64, device=CA.device)
@@ -223,18 +231,15 @@ def tran4_factored(nbas: int, lfac: torch.Tensor, CA, CB, CC, CD, precision: str
                    ctx: Context | None = None, out: torch.Tensor | None = None) -> torch.Tensor:
     """tran4_gen's output from the ERI factor; lfac is (ntr, rank) with Fortran meaning."""
     ctx = ctx or default_context(CA.device.index or 0)
-    cols = [_fortran_cols(c.to(torch.float64)) for c in (CA, CB, CC, CD)]
+    cols = _blocks(CA, CB, CC, CD)
     nA, nB, nC, nD = (c.shape[0] for c in cols)
     lcol = _fortran_cols(lfac)
     rank = lfac.shape[1]
     if out is None:
         out = torch.empty((nA * nB, nC * nD), dtype=torch.float64, device=CA.device)
-    same = CA is CC and CB is CD
-    cc = cols[0] if same else cols[2]
-    cd = cols[1] if same else cols[3]
     check(ctx.h, load().gc_tran4_factored(ctx.h, nbas, rank, _ptr(lcol), nA, _ptr(cols[0]), nB,
-                                          _ptr(cols[1]), nC, _ptr(cc), nD, _ptr(cd), _ptr(out),
-                                          PREC[precision]))
+                                          _ptr(cols[1]), nC, _ptr(cols[2]), nD, _ptr(cols[3]),
+                                          _ptr(out), PREC[precision]))
     return out
 
 

@@ -23,6 +23,7 @@
 #include <cuda.h>
 #include <cuda_bf16.h>
 
+#include <memory>
 #include <mutex>
 
 #include "gc_tc_gemm.cuh"
@@ -386,7 +387,8 @@ struct OzPlan {
 };
 
 struct OzEpi {
-  int mode;              // 0 store, 1 dot with r, 2 subtract from the lower triangle of c
+  int mode;              // 0 store, 1 dot with r, 2 subtract from the lower triangle of c,
+                         // 3 store the lower triangle of c and its mirror image
   double *c;
   long long ldn, sb;
   const double *r;
@@ -605,6 +607,11 @@ __global__ void __launch_bounds__(oz_threads(TBN), 1)
             epi.c[o] = cv;
           else if (epi.mode == 2) {
             if (m >= n) epi.c[o] -= cv;
+          } else if (epi.mode == 3) {
+            if (m >= n) {
+              epi.c[o] = cv;
+              epi.c[n + (long long)m * epi.ldn] = cv;  // 32 consecutive per thread
+            }
           } else
             dot += cv * epi.r[o];
         }
@@ -751,6 +758,14 @@ __global__ void __launch_bounds__(256) k_oz_rows(const double *__restrict__ x, i
   }
 }
 
+// Offset c + d n of the packed pair r = c + d (d + 1) / 2, c <= d.
+__device__ __forceinline__ long long tri_offset(int r, int n) {
+  int d = (int)((sqrtf(8.f * (float)r + 1.f) - 1.f) * 0.5f);
+  while ((long long)d * (d + 1) / 2 > r) --d;
+  while ((long long)(d + 1) * (d + 2) / 2 <= r) ++d;
+  return r - (long long)d * (d + 1) / 2 + (long long)d * n;
+}
+
 // The same for any other strides (in use: consecutive rows contiguous, K the slow index). One
 // block takes 32 rows: the maximum with the lanes along the rows, then 64 values of K at a time
 // through shared memory, read along the rows and written along K. The position of k within
@@ -758,7 +773,7 @@ __global__ void __launch_bounds__(256) k_oz_rows(const double *__restrict__ x, i
 template <int S>
 __global__ void __launch_bounds__(512) k_oz_cols(const double *__restrict__ x, int rows, int K, int Kp,
                                                  int nb, long long sr, long long sk, long long sb,
-                                                 int *__restrict__ e,
+                                                 int tri, int *__restrict__ e,
                                                  __nv_bfloat16 *__restrict__ planes) {
   __shared__ double tile[32][65];
   __shared__ unsigned long long part[16][32];
@@ -768,7 +783,8 @@ __global__ void __launch_bounds__(512) k_oz_cols(const double *__restrict__ x, i
   const int lr = threadIdx.x >> 4, lk = threadIdx.x & 15;  // row and group of four in the write
   const long long plane = (long long)nb * rows * Kp;
   for (int bb = blockIdx.y; bb < nb; bb += gridDim.y) {
-    const double *__restrict__ xr = x + bb * sb + (long long)r * sr;
+    // tri > 0: row r is the pair (c, d), c <= d, of a tri x tri matrix (r = c + d (d + 1) / 2)
+    const double *__restrict__ xr = x + bb * sb + (tri > 0 ? tri_offset(r, tri) : r) * sr;
     unsigned long long mx = 0;
     if (r < rows) {
 #pragma unroll 4
@@ -795,6 +811,69 @@ __global__ void __launch_bounds__(512) k_oz_cols(const double *__restrict__ x, i
       }
     }
     __syncthreads();
+  }
+}
+
+// Row exponents and slices of symmetric n x n matrices read from their packed triangles
+// (matrix k at x + k ld, element (p, q), p <= q, at p + q (q + 1) / 2): the operand has a row
+// (k, p) for every p, without the unpacked FP64 matrices ever being written. One block per
+// matrix (blockIdx.y: a share of its rows): the maxima of all rows from one sweep over the
+// triangle (high words only: the exponent is all that is wanted), then one warp per row. A
+// row's elements with q <= p are contiguous in the triangle, the others share their sectors
+// with the rows that the block's other warps hold. Measured for 1494 matrices with n = 249: 0.40
+// ms, where unpacking (0.32), exponents and digits took 1.2 ms.
+template <int S>
+__global__ void __launch_bounds__(256) k_oz_packed(const double *__restrict__ x, long long ld, int n,
+                                                   int Kp, int cnt, int *__restrict__ e,
+                                                   __nv_bfloat16 *__restrict__ planes) {
+  extern __shared__ unsigned rmax[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const double *__restrict__ xk = x + blockIdx.x * ld;
+  for (int p = threadIdx.x; p < n; p += 256) rmax[p] = 0;
+  __syncthreads();
+  for (int q = warp; q < n; q += 8) {
+    const double *__restrict__ c = xk + (long long)q * (q + 1) / 2;
+    unsigned mx = 0;
+    for (int p = lane; p <= q; p += 32) {
+      const unsigned h = (unsigned)__double2hiint(c[p]) & 0x7fffffffu;
+      atomicMax(&rmax[p], h);
+      mx = max(mx, h);
+    }
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    if (lane == 0) atomicMax(&rmax[q], mx);
+  }
+  __syncthreads();
+  const long long row0 = blockIdx.x * (long long)n, plane = (long long)cnt * n * Kp;
+  for (int p = blockIdx.y * 8 + warp; p < n; p += 8 * gridDim.y) {
+    const unsigned h = rmax[p];
+    const int E = (int)(h >> 20);
+    const int ex = E == 0x7ff ? kBadExp : max(E, 1) - 1022;  // a subnormal or zero row: 2^-1021 bounds it
+    if (lane == 0) e[row0 + p] = ex;
+    const double *__restrict__ lo = xk + (long long)p * (p + 1) / 2;
+    for (int k = lane * 4; k < Kp; k += 128) {
+      double v[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int q = k + i;
+        v[i] = q >= n ? 0.0 : (q <= p ? lo[q] : xk[p + (long long)q * (q + 1) / 2]);
+      }
+      store_digits4<S>(v, ex, plane, (row0 + p) * Kp + k, planes);
+    }
+  }
+}
+
+// out[cd + nCD ab] from the product over pairs (row index cd or its packed form, column index
+// ab or its packed form): every element of the pair blocks from the triangles.
+__global__ void k_expand_pairs(const double *__restrict__ cp, long long ldc, int nC, int nD, int symCD,
+                               int nA, int nB, int symAB, double *__restrict__ out) {
+  const int cd = blockIdx.x * blockDim.x + threadIdx.x;
+  if (cd >= nC * nD) return;
+  const int c = cd % nC, d = cd / nC;
+  auto tri = [](int a, int b) { return a <= b ? a + (long long)b * (b + 1) / 2 : b + (long long)a * (a + 1) / 2; };
+  const long long r = symCD ? tri(c, d) : cd;
+  for (int ab = blockIdx.y; ab < nA * nB; ab += gridDim.y) {
+    const long long k = symAB ? tri(ab % nA, ab / nA) : ab;
+    out[cd + (long long)nC * nD * ab] = cp[r + k * ldc];
   }
 }
 
@@ -998,24 +1077,24 @@ int encode_oz_map(gc_context *ctx, OzOperand &op) {
 
 template <int S>
 int slice_operand(gc_context *ctx, OzOperand &op, const double *x, int rows, int K, int nb,
-                  long long sr, long long sk, long long sb) {
+                  long long sr, long long sk, long long sb, int tri) {
   const long long nrr = (long long)nb * rows;
-  if (sk == 1 && op.Kp <= 128 * kOzHold) {  // one warp holds the row
+  if (sk == 1 && !tri && op.Kp <= 128 * kOzHold) {  // one warp holds the row
     k_oz_rows<S, 32><<<gc::ceil_div(nrr, 8), 256, 0, ctx->stream>>>(x, rows, K, op.Kp, nrr, sr, sb,
                                                                     op.exps.p, op.buf.p);
-  } else if (sk == 1) {
+  } else if (sk == 1 && !tri) {
     k_oz_rows<S, 256><<<(unsigned)nrr, 256, 0, ctx->stream>>>(x, rows, K, op.Kp, nrr, sr, sb,
                                                               op.exps.p, op.buf.p);
   } else {
     k_oz_cols<S><<<dim3(gc::ceil_div(rows, 32), std::min(nb, 65535)), 512, 0, ctx->stream>>>(
-        x, rows, K, op.Kp, nb, sr, sk, sb, op.exps.p, op.buf.p);
+        x, rows, K, op.Kp, nb, sr, sk, sb, tri, op.exps.p, op.buf.p);
   }
   GC_LAUNCHED(ctx);
   return GC_OK;
 }
 
 int make_oz_operand(gc_context *ctx, OzOperand &op, const double *x, int rows, int K, int nb,
-                    long long sr, long long sk, long long sb, int S, int box_rows) {
+                    long long sr, long long sk, long long sb, int S, int box_rows, int tri = 0) {
   op.rows = rows;
   op.box_rows = box_rows;
   op.Kp = (K + BK - 1) / BK * BK;
@@ -1025,10 +1104,36 @@ int make_oz_operand(gc_context *ctx, OzOperand &op, const double *x, int rows, i
   GC_TRY(op.exps.alloc(ctx, (size_t)nb * rows));
   GC_TRY(op.buf.alloc(ctx, plane * S));
   switch (S) {
-    case 4: GC_TRY(slice_operand<4>(ctx, op, x, rows, K, nb, sr, sk, sb)); break;
-    case 5: GC_TRY(slice_operand<5>(ctx, op, x, rows, K, nb, sr, sk, sb)); break;
-    default: GC_TRY(slice_operand<6>(ctx, op, x, rows, K, nb, sr, sk, sb));
+    case 4: GC_TRY(slice_operand<4>(ctx, op, x, rows, K, nb, sr, sk, sb, tri)); break;
+    case 5: GC_TRY(slice_operand<5>(ctx, op, x, rows, K, nb, sr, sk, sb, tri)); break;
+    default: GC_TRY(slice_operand<6>(ctx, op, x, rows, K, nb, sr, sk, sb, tri));
   }
+  op.planes = op.buf.p;
+  op.ex = op.exps.p;
+  return encode_oz_map(ctx, op);
+}
+
+// The operand of cnt packed symmetric n x n matrices, one row per (matrix, p).
+int make_oz_packed(gc_context *ctx, OzOperand &op, const double *x, long long ld, int n, int cnt,
+                   int S) {
+  op.rows = cnt * n;
+  op.box_rows = BM;
+  op.Kp = (n + BK - 1) / BK * BK;
+  op.nb = 1;
+  op.S = S;
+  GC_TRY(op.exps.alloc(ctx, (size_t)op.rows));
+  GC_TRY(op.buf.alloc(ctx, (size_t)op.rows * op.Kp * S));
+  // two blocks per SM at least, where a matrix has the rows for it
+  const dim3 grid(cnt, std::max(1u, std::min(gc::ceil_div(304, cnt), gc::ceil_div(n, 8))));
+  const size_t sm = (size_t)n * sizeof(unsigned);
+  if (sm > 48 * 1024) return gc::set_error(ctx, GC_EUNSUPPORTED, "packed operand: n=%d", n);
+  if (S == 4)
+    k_oz_packed<4><<<grid, 256, sm, ctx->stream>>>(x, ld, n, op.Kp, cnt, op.exps.p, op.buf.p);
+  else if (S == 5)
+    k_oz_packed<5><<<grid, 256, sm, ctx->stream>>>(x, ld, n, op.Kp, cnt, op.exps.p, op.buf.p);
+  else
+    k_oz_packed<6><<<grid, 256, sm, ctx->stream>>>(x, ld, n, op.Kp, cnt, op.exps.p, op.buf.p);
+  GC_LAUNCHED(ctx);
   op.planes = op.buf.p;
   op.ex = op.exps.p;
   return encode_oz_map(ctx, op);
@@ -1131,30 +1236,107 @@ int check_flag(gc_context *ctx) {
   return GC_OK;
 }
 
+int tc_half_packed(gc_context *ctx, int precision, int n, int cnt, const double *M, long long ld,
+                   int nhalf, const HalfOut *half) {
+  if (!is_oz(precision))
+    return set_error(ctx, GC_EINVAL, "half_packed: needs a sliced FP64-accurate precision");
+  const OzPlan pl = oz_plan(precision);
+  // The matrices of a chunk have at most 1 GiB of slice planes (and fit the row counts).
+  const long long per = (long long)n * ((n + BK - 1) / BK * BK) * 2 * pl.S;
+  const int cs = (int)std::max<long long>(
+      1, std::min<long long>({(long long)cnt, (1ll << 30) / per, 0x7fffffffll / ((long long)n * n),
+                              65535ll}));
+  struct Side {
+    OzOperand first, second;  // the block contracted first (GEMM B) and the other one
+  };
+  std::vector<std::unique_ptr<Side>> side;
+  for (int h = 0; h < nhalf; ++h) {
+    const HalfOut &o = half[h];
+    side.push_back(std::make_unique<Side>());
+    // M_k is symmetric: the narrower block is contracted first, n x min(nX, nY) instead of
+    // n x nX intermediate columns (FOFO at n = 249, nocc = 28: 5 times fewer products).
+    const bool y1 = o.nY <= o.nX;
+    const int nf = y1 ? o.nY : o.nX;
+    GC_TRY(make_oz_operand(ctx, side[h]->first, y1 ? o.CY : o.CX, nf, n, 1, n, 1, 0, pl.S,
+                           oz_tile(ctx, pl.S, (long long)n * cs, nf, 1)));
+    if (y1)
+      GC_TRY(make_oz_operand(ctx, side[h]->second, o.CX, o.nX, n, 1, n, 1, 0, pl.S, BM));
+    else
+      GC_TRY(make_oz_operand(ctx, side[h]->second, o.CY, o.nY, n, 1, n, 1, 0, pl.S,
+                             oz_tile(ctx, pl.S, o.nX, o.nY, cs)));
+  }
+  for (int k0 = 0; k0 < cnt; k0 += cs) {
+    const int c = std::min(cs, cnt - k0);
+    OzOperand A;
+    GC_TRY(make_oz_packed(ctx, A, M + k0 * ld, ld, n, c, pl.S));
+    for (int h = 0; h < nhalf; ++h) {
+      const HalfOut &o = half[h];
+      const bool y1 = o.nY <= o.nX;
+      const int nf = y1 ? o.nY : o.nX;
+      double *out = o.out + (long long)k0 * o.nX * o.nY;
+      DevBuf<double> T;  // T[(k, p) + f (c n)] = sum_q M_k[p, q] C_first[q, f]
+      GC_TRY(T.alloc(ctx, (size_t)c * n * nf));
+      OzEpi e{0, T.p, (long long)c * n, 0, nullptr, nullptr, nullptr, nullptr, 0, 0};
+      GC_TRY(run_oz(ctx, A, side[h]->first, c * n, nf, 1, pl, e));
+      OzOperand B;
+      if (y1) {
+        // out[x + nX (y + nY k)] = sum_p CX[p, x] T[(k, p), y]: one product, columns (k, y)
+        GC_TRY(make_oz_operand(ctx, B, T.p, nf, n, c, (long long)c * n, 1, n, pl.S,
+                               oz_tile(ctx, pl.S, o.nX, (long long)c * nf, 1)));
+        B.rows = c * nf;
+        B.nb = 1;
+        GC_TRY(encode_oz_map(ctx, B));
+        OzEpi e2{0, out, o.nX, 0, nullptr, nullptr, nullptr, nullptr, 0, 0};
+        GC_TRY(run_oz(ctx, side[h]->second, B, o.nX, c * nf, 1, pl, e2));
+      } else {
+        GC_TRY(make_oz_operand(ctx, B, T.p, nf, n, c, (long long)c * n, 1, n, pl.S, BM));
+        OzEpi e2{0, out, o.nX, (long long)o.nX * o.nY, nullptr, nullptr, nullptr, nullptr, 0, 0};
+        GC_TRY(run_oz(ctx, B, side[h]->second, o.nX, o.nY, c, pl, e2));
+      }
+    }
+  }
+  return GC_OK;  // the device flag is read at the caller's next sync point
+}
+
+int tc_pair_product(gc_context *ctx, int precision, int rank, int nC, int nD, bool symCD,
+                    const double *Z, int nA, int nB, bool symAB, const double *Y, double *out) {
+  if (!is_oz(precision))
+    return set_error(ctx, GC_EINVAL, "pair_product: needs a sliced FP64-accurate precision");
+  const OzPlan pl = oz_plan(precision);
+  const int nCD = nC * nD, nAB = nA * nB;
+  const int R = symCD ? nC * (nC + 1) / 2 : nCD, Q = symAB ? nA * (nA + 1) / 2 : nAB;
+  const bool same = Y == Z && symAB == symCD;
+  DevBuf<double> cp;
+  double *C = out;
+  if (symCD || symAB) {
+    GC_TRY(cp.alloc(ctx, (size_t)R * Q));
+    C = cp.p;
+  }
+  OzOperand a, b;
+  GC_TRY(make_oz_operand(ctx, a, Z, R, rank, 1, 1, nCD, 0, pl.S, BM, symCD ? nC : 0));
+  if (same) {  // symmetric: the lower triangle and its mirror image
+    GC_TRY(alias_oz_operand(ctx, a, b, oz_tile(ctx, pl.S, R, (Q + 1) / 2, 1)));
+    OzEpi e{3, C, R, 0, nullptr, nullptr, nullptr, nullptr, 0, 0, R};
+    GC_TRY(run_oz(ctx, a, b, R, Q, 1, pl, e));
+  } else {
+    GC_TRY(make_oz_operand(ctx, b, Y, Q, rank, 1, 1, nAB, 0, pl.S, oz_tile(ctx, pl.S, R, Q, 1),
+                           symAB ? nA : 0));
+    OzEpi e{0, C, R, 0, nullptr, nullptr, nullptr, nullptr, 0, 0};
+    GC_TRY(run_oz(ctx, a, b, R, Q, 1, pl, e));
+  }
+  if (C != out) {
+    k_expand_pairs<<<dim3(ceil_div(nCD, 256), std::min(nAB, 65535)), 256, 0, ctx->stream>>>(
+        C, R, nC, nD, symCD, nA, nB, symAB, out);
+    GC_LAUNCHED(ctx);
+  }
+  return GC_OK;  // the device flag is read at the caller's next sync point
+}
+
 int tc_two_sided(gc_context *ctx, int precision, int n, int cnt, const double *M, int nX,
                  const double *CX, int nY, const double *CY, double *T1, double *out,
                  long long ostride) {
   if (precision == GC_PREC_FP64)
     return fp64_two_sided(ctx, n, cnt, M, nX, CX, nY, CY, T1, out, ostride);
-  if (is_oz(precision)) {
-    OzPlan pl = oz_plan(precision);
-    {
-      OzOperand A, B;
-      GC_TRY(make_oz_operand(ctx, A, M, n * cnt, n, 1, n, 1, 0, pl.S, BM));
-      GC_TRY(make_oz_operand(ctx, B, CX, nX, n, 1, n, 1, 0, pl.S,
-                             oz_tile(ctx, pl.S, (long long)n * cnt, nX, 1)));
-      OzEpi e{0, T1, (long long)n * cnt, 0, nullptr, nullptr, nullptr, nullptr, 0, 0};
-      GC_TRY(run_oz(ctx, A, B, n * cnt, nX, 1, pl, e));
-    }
-    {
-      OzOperand A, B;
-      GC_TRY(make_oz_operand(ctx, A, T1, nX, n, cnt, (long long)n * cnt, 1, n, pl.S, BM));
-      GC_TRY(make_oz_operand(ctx, B, CY, nY, n, 1, n, 1, 0, pl.S, oz_tile(ctx, pl.S, nX, nY, cnt)));
-      OzEpi e{0, out, nX, ostride, nullptr, nullptr, nullptr, nullptr, 0, 0};
-      GC_TRY(run_oz(ctx, A, B, nX, nY, cnt, pl, e));
-    }
-    return GC_OK;  // the device flag is read at the caller's next sync point
-  }
   int S;
   PassList pl = pass_list(precision, &S);
   // step 1: T1[(k,q), x] = sum_p M_k[p, q] CX[p, x]   (T1 column-major, ld = n*cnt)

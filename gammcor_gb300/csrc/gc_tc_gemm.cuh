@@ -12,7 +12,26 @@ namespace gc {
 // their next synchronisation point.
 int check_flag(gc_context *ctx);
 
-// out_k (nX x nY, column-major, stride ostride) = CX^T M_k CY for cnt
+// Sliced precisions: out_k (nX x nY, column-major, consecutive) = CX^T M_k CY for cnt symmetric
+// n x n matrices given by their packed triangles (M_k at M + k ld, element (p, q), p <= q, at
+// p + q (q + 1) / 2), for one or two pairs of blocks that share the slices of the M_k.
+struct HalfOut {
+  int nX;
+  const double *CX;  // n x nX, column-major
+  int nY;
+  const double *CY;  // n x nY, column-major
+  double *out;       // cnt x (nX x nY)
+};
+int tc_half_packed(gc_context *ctx, int precision, int n, int cnt, const double *M, long long ld,
+                   int nhalf, const HalfOut *half);
+
+// Sliced precisions: out[cd + nCD ab] = sum_P Z[cd + nCD P] Y[ab + nAB P] with cd = c + nC d and
+// ab = a + nA b. symCD / symAB: Z / Y are symmetric in their two indices, and only c <= d /
+// a <= b is computed; Y == Z: only one triangle of the product is.
+int tc_pair_product(gc_context *ctx, int precision, int rank, int nC, int nD, bool symCD,
+                    const double *Z, int nA, int nB, bool symAB, const double *Y, double *out);
+
+// FP64 and split-BF16 precisions: out_k (nX x nY, column-major, stride ostride) = CX^T M_k CY for cnt
 // column-major n x n matrices M_k; T1 is scratch of cnt*n*max(nX) doubles.
 int tc_two_sided(gc_context *ctx, int precision, int n, int cnt, const double *M, int nX,
                  const double *CX, int nY, const double *CY, double *T1, double *out,

@@ -9,6 +9,10 @@
 //
 // gc_tran4_factored produces the same records from the ERI factor L:
 // B_P = CA^T L_P CB for every P, then (ab|cd) = sum_P B_P(ab) B'_P(cd).
+//
+// In the sliced precisions the packed triangles are the operands themselves
+// (tc_half_packed), and a block of orbitals given twice (the same pointer and
+// width) makes its pair index symmetric (tc_pair_product).
 #include "gc_internal.cuh"
 #include "gc_tc_gemm.cuh"
 
@@ -32,6 +36,20 @@ __global__ void unpack_records(const double *__restrict__ G, long long ntr, int 
     long long pq = p <= q ? tri_pack(p, q) : tri_pack(q, p);
     M[t] = G[(rs0 + k) * ntr + pq];
   }
+}
+
+// Mt[c][rs] = H[rs][c0 + c]: columns [c0, c0+cnt) of H (ntr x ncol, column fastest) as packed
+// records.
+__global__ void transpose_columns(const double *__restrict__ H, long long ntr, long long ncol,
+                                  long long c0, int cnt, double *__restrict__ Mt) {
+  __shared__ double tile[32][33];
+  const long long rs0 = (long long)blockIdx.x * 32, cb = (long long)blockIdx.y * 32;
+  const int tx = threadIdx.x, ty = threadIdx.y;  // 32 x 8
+  for (int i = ty; i < 32; i += 8)
+    if (rs0 + i < ntr && cb + tx < cnt) tile[i][tx] = H[(rs0 + i) * ncol + c0 + cb + tx];
+  __syncthreads();
+  for (int j = ty; j < 32; j += 8)
+    if (cb + j < cnt && rs0 + tx < ntr) Mt[(cb + j) * ntr + rs0 + tx] = tile[tx][j];
 }
 
 // Expand columns [c0, c0+cnt) of H (ntr x ncol, row index = packed rs, column
@@ -122,6 +140,21 @@ extern "C" int gc_tran4_gen(gc_context *ctx, int nbas, int nA, const double *CA,
   const long long n2 = (long long)n * n;
   gc::DevBuf<double> H, M, T1;
   GC_TRY(H.alloc(ctx, ntr * nAB));
+  if (gc::is_sliced(precision)) {
+    const gc::HalfOut ab{nA, CA, nB, CB, H.p};
+    GC_TRY(gc::tc_half_packed(ctx, precision, n, (int)ntr, G, ntr, 1, &ab));
+    const int cs = (int)std::max<long long>(1, std::min<long long>(nAB, kChunkBytes / (8 * ntr)));
+    GC_TRY(M.alloc(ctx, (size_t)cs * ntr));
+    for (long long c0 = 0; c0 < nAB; c0 += cs) {
+      const int cnt = (int)std::min<long long>(cs, nAB - c0);
+      transpose_columns<<<dim3(gc::ceil_div(ntr, 32), gc::ceil_div(cnt, 32)), dim3(32, 8), 0,
+                          ctx->stream>>>(H.p, ntr, nAB, c0, cnt, M.p);
+      GC_LAUNCHED(ctx);
+      const gc::HalfOut cd{nC, CC, nD, CD, out + c0 * nCD};
+      GC_TRY(gc::tc_half_packed(ctx, precision, n, cnt, M.p, ntr, 1, &cd));
+    }
+    return gc::check_flag(ctx);
+  }
   int cs = (int)std::max<long long>(1, std::min<long long>(ntr, kChunkBytes / (8 * n2)));
   GC_TRY(M.alloc(ctx, (size_t)cs * n2));
   int tmax = std::max(nA, nC);
@@ -161,6 +194,14 @@ extern "C" int gc_tran4_factored(gc_context *ctx, int nbas, int rank, const doub
   gc::DevBuf<double> Y, Z, M, T1;
   GC_TRY(Y.alloc(ctx, nAB * rank));
   if (!same) GC_TRY(Z.alloc(ctx, nCD * rank));
+  if (gc::is_sliced(precision)) {
+    const gc::HalfOut half[2] = {{nA, CA, nB, CB, Y.p}, {nC, CC, nD, CD, Z.p}};
+    GC_TRY(gc::tc_half_packed(ctx, precision, n, rank, L, ntr, same ? 1 : 2, half));
+    const bool symAB = CA == CB && nA == nB, symCD = CC == CD && nC == nD;
+    GC_TRY(gc::tc_pair_product(ctx, precision, rank, nC, nD, symCD, same ? Y.p : Z.p, nA, nB, symAB,
+                               Y.p, out));
+    return gc::check_flag(ctx);
+  }
   int cs = (int)std::max<long long>(1, std::min<long long>(rank, kChunkBytes / (8 * n2)));
   GC_TRY(M.alloc(ctx, (size_t)cs * n2));
   GC_TRY(T1.alloc(ctx, (size_t)cs * n * std::max(nA, nC)));

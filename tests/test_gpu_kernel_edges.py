@@ -117,3 +117,23 @@ def test_sliced_gemm_bits(gpu_lib, S, m, n, k):
         A[1] = 3.0 * 2.0 ** -1070 * rng.integers(-5, 6, k)
     C = api.tc_gemm_nt(t(A), t(B), f"fp64tc{S}").cpu().numpy()
     assert np.array_equal(C, sliced_product(A, B, S))
+
+
+# widths (nA, nB, nC, nD); -1 repeats the block before it, so that the pair index is symmetric
+@pytest.mark.parametrize("n,widths", [(33, (33, 5, 33, 5)), (33, (5, -1, 33, -1)), (20, (3, 17, 9, -1)),
+                                      (20, (7, -1, 4, 11)), (65, (2, 65, 2, 65)), (5, (1, 1, 5, 2))])
+@pytest.mark.parametrize("entry", ["factored", "gen"])
+def test_transform_block_shapes(gpu_lib, n, widths, entry):
+    rng = np.random.default_rng(n)
+    lf = synth.make_lfac(n, 2 * n + 1, rng) * 0.1
+    C, blocks = np.linalg.qr(rng.standard_normal((n, n)))[0], []
+    for i, w in enumerate(widths):
+        blocks.append(blocks[-1] if w < 0 else t(np.roll(C, i // 2, axis=1)[:, :w]))
+    if widths[:2] == widths[2:]:
+        blocks[2:] = blocks[:2]
+    ref = R.tran4_gen(n, *[b.cpu().numpy() for b in blocks], lf @ lf.T)
+    if entry == "factored":
+        out = api.tran4_factored(n, t(lf), *blocks, precision="fp64tc5")
+    else:
+        out = api.tran4_gen(n, *blocks, t(lf @ lf.T), precision="fp64tc5")
+    assert np.abs(out.cpu().numpy() - ref).max() < 1e-10
