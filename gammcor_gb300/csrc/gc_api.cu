@@ -1,6 +1,8 @@
 // Context management, host-side helpers of the path (GauLeg, prepare_nums,
 // pair builder) and the lambda-quadrature driver ACECORR.
 #include <cmath>
+#include <map>
+#include <mutex>
 
 #include "gc_internal.cuh"
 
@@ -16,6 +18,44 @@ __global__ void k_axpby(size_t count, double a, const double *__restrict__ x, do
 }  // namespace
 
 namespace gc {
+
+namespace {
+struct PoolRef {
+  cudaMemPool_t pool = nullptr;
+  int users = 0;
+};
+std::mutex pool_mu;
+std::map<int, PoolRef> pools;  // by device
+}  // namespace
+
+cudaError_t pool_acquire(int device, cudaMemPool_t *pool) {
+  std::lock_guard<std::mutex> lk(pool_mu);
+  PoolRef &r = pools[device];
+  if (r.users == 0) {
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device;
+    cudaError_t e = cudaMemPoolCreate(&r.pool, &props);
+    if (e != cudaSuccess) return e;
+    unsigned long long keep = kPoolKeep;
+    e = cudaMemPoolSetAttribute(r.pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    if (e != cudaSuccess) {
+      cudaMemPoolDestroy(r.pool);
+      return e;
+    }
+  }
+  r.users++;
+  *pool = r.pool;
+  return cudaSuccess;
+}
+
+void pool_release(int device) {
+  std::lock_guard<std::mutex> lk(pool_mu);
+  PoolRef &r = pools[device];
+  // Buffers that outlive the last context keep their memory until they are freed.
+  if (r.users > 0 && --r.users == 0) cudaMemPoolDestroy(r.pool);
+}
 
 namespace {
 cudaEvent_t phase_event(gc_context *ctx) {
@@ -92,6 +132,10 @@ int gc_create(gc_context **out, int device, void *stream) {
     delete ctx;
     return GC_ECUDA;
   }
+  if ((e = gc::pool_acquire(device, &ctx->pool)) != cudaSuccess) {
+    delete ctx;
+    return e == cudaErrorMemoryAllocation ? GC_ENOMEM : GC_ECUDA;
+  }
   // The caller's stream is used as given (NULL is the legacy default stream),
   // so that work is ordered with whatever produced the inputs on that stream.
   ctx->stream = (cudaStream_t)stream;
@@ -134,6 +178,7 @@ int gc_destroy(gc_context *ctx) {
     cudaEventDestroy(r.b);
   }
   for (cudaEvent_t e : ctx->phase_pool) cudaEventDestroy(e);
+  if (ctx->pool) gc::pool_release(ctx->device);
   delete ctx;
   return GC_OK;
 }

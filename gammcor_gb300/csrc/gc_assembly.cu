@@ -11,10 +11,17 @@
 //     reference accumulates in the same loops.
 // Every coefficient is 1, lambda or (1 - lambda), so A+-B is affine in lambda.
 #include <cmath>
+#include <cstring>
 
 #include "gc_internal.cuh"
 
 namespace {
+
+// h(i, j): a full matrix (column-major), or the packed triangle (hpk).
+__device__ __forceinline__ double one_el(const double *__restrict__ h, int hpk, int n, int i, int j) {
+  if (!hpk) return h[i + (size_t)j * n];
+  return i <= j ? h[i + (size_t)j * (j + 1) / 2] : h[j + (size_t)i * (i + 1) / 2];
+}
 
 struct Geo {
   int n, nin, nact, nocc;
@@ -89,7 +96,8 @@ struct InterWork {  // first warp of each part
 };
 
 __global__ void __launch_bounds__(256)
-    k_intermediates(Geo g, InterWork W, const double *__restrict__ h, const double *__restrict__ occ,
+    k_intermediates(Geo g, InterWork W, const double *__restrict__ h, int hpk,
+                    const double *__restrict__ occ,
                     const int *__restrict__ grp, const double *__restrict__ fofo,
                     const double *__restrict__ ffoo, const double *__restrict__ rv, double lam,
                     Inter I) {
@@ -174,7 +182,7 @@ __global__ void __launch_bounds__(256)
       const int i = (t0 % ch) * 32 + lane, j = t0 / ch;
       if (i >= n) continue;
       const int gi = grp[i], gj = grp[j];
-      const double hv = h[i + (size_t)j * n];
+      const double hv = one_el(h, hpk, n, i, j);
       double corr = 0.0, ai = 0.0, aio = 0.0;
 #pragma unroll 4
       for (int k = 0; k < nocc; ++k) {
@@ -241,7 +249,7 @@ __global__ void __launch_bounds__(256)
       const int e = w - W.wet;
       double v = 0.0;
       for (int i = e * 32 + lane; i < nocc; i += 32 * kEtotWarps)
-        v += 2.0 * occ[i] * h[i + (size_t)i * n];
+        v += 2.0 * occ[i] * one_el(h, hpk, n, i, i);
       const unsigned o2 = (unsigned)nocc * nocc;
       for (unsigned rec = e; rec < o2; rec += kEtotWarps) {  // record (k, l), elements (i, j)
         const int k = rec % nocc, l = rec / nocc;
@@ -420,6 +428,11 @@ __global__ void __launch_bounds__(32 * kAbWarps)
   }
 }
 
+__global__ void k_unpack_h(int n, const double *__restrict__ xone, double *__restrict__ h) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) h[i + (size_t)blockIdx.y * n] = one_el(xone, 1, n, i, blockIdx.y);
+}
+
 // sq_symmetrize (tran.f90:1303-1319): a(i,j) = a(j,i) = (a(i,j) + a(j,i)) / 2.
 __global__ void k_sym_avg(int N, double *__restrict__ a) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -457,6 +470,9 @@ int rotate_h(gc_context *ctx, SysDev &sd, const double *ure_host) {
   DevBuf<double> u, w;
   GC_TRY(u.upload(ctx, ure_host, (size_t)n * n));
   GC_TRY(w.alloc(ctx, (size_t)n * n));
+  GC_TRY(sd.h.alloc(ctx, (size_t)n * n));
+  k_unpack_h<<<dim3(ceil_div(n, 128), n), 128, 0, ctx->stream>>>(n, sd.xone.p, sd.h.p);
+  GC_LAUNCHED(ctx);
   const double one = 1.0, zero = 0.0;
   GC_CUBLAS(ctx, cublasDgemm(ctx->cublas, CUBLAS_OP_N, CUBLAS_OP_N, n, n, n, &one, u.p, n, sd.h.p, n,
                              &zero, w.p, n));
@@ -514,37 +530,17 @@ int sys_upload(gc_context *ctx, SysDev &sd, int nbas, int ninact, int nact, int 
     pp[i] = a;
     pq[i] = b;
   }
-  GC_TRY(sd.occ.upload(ctx, occ, n));
-  GC_TRY(sd.grp.upload(ctx, grp.data(), n));
-  GC_TRY(sd.pair_p.upload(ctx, pp.data(), ndimx));
-  GC_TRY(sd.pair_q.upload(ctx, pq.data(), ndimx));
+  std::vector<double> cpl(ndimx), rpl(ndimx), rmi(ndimx), dnq(ndimx);
   {
-    auto cicoef = [](double o) { return o >= 0.5 ? std::sqrt(o) : -std::sqrt(o); };
-    std::vector<double> cpl(ndimx), cmi(ndimx), rpl(ndimx), rmi(ndimx), dnq(ndimx);
+    std::vector<double> ci(n);
+    for (int i = 0; i < n; ++i) ci[i] = occ[i] >= 0.5 ? std::sqrt(occ[i]) : -std::sqrt(occ[i]);
     for (int i = 0; i < ndimx; ++i) {
-      const double cp = cicoef(occ[pp[i]]), cq = cicoef(occ[pq[i]]);
-      const double op = occ[pp[i]], oq = occ[pq[i]];
+      const double cp = ci[pp[i]], cq = ci[pq[i]], op = occ[pp[i]], oq = occ[pq[i]];
       cpl[i] = cp + cq;
-      cmi[i] = cp - cq;
-      rpl[i] = cpl[i] != 0.0 ? 1.0 / cpl[i] : 0.0;
-      rmi[i] = cmi[i] != 0.0 ? 1.0 / cmi[i] : 0.0;
+      rpl[i] = cp + cq != 0.0 ? 1.0 / (cp + cq) : 0.0;
+      rmi[i] = cp - cq != 0.0 ? 1.0 / (cp - cq) : 0.0;
       dnq[i] = op * (1.0 - oq) + oq * (1.0 - op);
     }
-    GC_TRY(sd.cpl.upload(ctx, cpl.data(), ndimx));
-    GC_TRY(sd.cmi.upload(ctx, cmi.data(), ndimx));
-    GC_TRY(sd.rpl.upload(ctx, rpl.data(), ndimx));
-    GC_TRY(sd.rmi.upload(ctx, rmi.data(), ndimx));
-    GC_TRY(sd.dnq.upload(ctx, dnq.data(), ndimx));
-  }
-  if (xone) {
-    std::vector<double> h((size_t)n * n);
-    size_t t = 0;
-    for (int q = 0; q < n; ++q)
-      for (int p = 0; p <= q; ++p, ++t) {
-        h[p + (size_t)q * n] = xone[t];
-        h[q + (size_t)p * n] = xone[t];
-      }
-    GC_TRY(sd.h.upload(ctx, h.data(), h.size()));
   }
   // Active block of RDM2val(i,j,k,l) = FRDM2(i,k,j,l) (abfofo.f90:84-92, interpa.f:5244-5272);
   // outside it RDM2val is products of occupations, which the kernels form themselves.
@@ -560,7 +556,6 @@ int sys_upload(gc_context *ctx, SysDev &sd, int nbas, int ninact, int nact, int 
             rv[t] = rdm2act[mx * (mx - 1) / 2 + mn - 1];
           }
   }
-  GC_TRY(sd.rv.upload(ctx, rv.data(), rv.size()));
   // Row order of the element kernel: pairs by orbital groups, then tiles of 8 p x 4 q. The
   // pairs are listed per (p, q) cell (head, next) and the cells are walked in that order.
   std::vector<int> slot, head((size_t)n * nocc, -1), next(ndimx);
@@ -578,7 +573,38 @@ int sys_upload(gc_context *ctx, SysDev &sd, int nbas, int ninact, int nact, int 
           for (int q = q0; q < std::min(q0 + 4, qb[gq + 1]); ++q)
             for (int p = p0; p < std::min(p0 + 8, pb[gp + 1]); ++p)
               for (int i = head[p + (size_t)q * n]; i >= 0; i = next[i]) slot.push_back(i);
-  GC_TRY(sd.slot.upload(ctx, slot.data(), ndimx));
+  // One staging buffer, one allocation, one copy: a copy from pageable memory costs some
+  // microseconds whatever its size.
+  struct Part {
+    const void *src;
+    size_t bytes;
+    void **dst;
+  };
+  const size_t N = ndimx, ntr = (size_t)n * (n + 1) / 2;
+  const Part parts[] = {
+      {occ, n * sizeof(double), (void **)&sd.occ.p},
+      {xone, xone ? ntr * sizeof(double) : 0, (void **)&sd.xone.p},
+      {rv.data(), rv.size() * sizeof(double), (void **)&sd.rv.p},
+      {cpl.data(), N * sizeof(double), (void **)&sd.cpl.p},
+      {rpl.data(), N * sizeof(double), (void **)&sd.rpl.p},
+      {rmi.data(), N * sizeof(double), (void **)&sd.rmi.p},
+      {dnq.data(), N * sizeof(double), (void **)&sd.dnq.p},
+      {grp.data(), n * sizeof(int), (void **)&sd.grp.p},
+      {pp.data(), N * sizeof(int), (void **)&sd.pair_p.p},
+      {pq.data(), N * sizeof(int), (void **)&sd.pair_q.p},
+      {slot.data(), N * sizeof(int), (void **)&sd.slot.p},
+  };
+  std::vector<char> stage;
+  for (const Part &p : parts) stage.resize((stage.size() + p.bytes + 15) / 16 * 16);
+  GC_TRY(sd.blob.alloc(ctx, stage.size()));
+  size_t at = 0;
+  for (const Part &p : parts) {
+    if (p.bytes) std::memcpy(stage.data() + at, p.src, p.bytes);
+    *p.dst = sd.blob.p + at;
+    at += (p.bytes + 15) / 16 * 16;
+  }
+  GC_CUDA(ctx, cudaMemcpyAsync(sd.blob.p, stage.data(), stage.size(), cudaMemcpyHostToDevice,
+                               ctx->stream));
   return GC_OK;
 }
 
@@ -614,7 +640,8 @@ int assemble_ab(gc_context *ctx, const SysDev &sd, const double *ffoo, const dou
   const InterWork W{(int)first[0], (int)first[1], (int)first[2], (int)first[3],
                     (int)first[4], (int)first[5], (int)first[6], (int)first[7]};
   k_intermediates<<<std::min<unsigned>(ceil_div((size_t)W.end, 8), 152u * 64u), 256, 0,
-                    ctx->stream>>>(g, W, sd.h.p, sd.occ.p, sd.grp.p, fofo, ffoo, sd.rv.p, alpha, I);
+                    ctx->stream>>>(g, W, sd.h.p ? sd.h.p : sd.xone.p, sd.h.p ? 0 : 1, sd.occ.p, sd.grp.p, fofo,
+                                   ffoo, sd.rv.p, alpha, I);
   GC_LAUNCHED(ctx);
   // Columns per warp: up to 8 share the row part of a warp's work; fewer where 8 would leave
   // the chip with less than 32 warps per SM (N = 570: 30 us with 8, 20 us with 2).

@@ -25,6 +25,7 @@ struct gc_phase_rec {
 struct gc_context {
   int device = 0;
   cudaStream_t stream = nullptr;
+  cudaMemPool_t pool = nullptr;      // the device's workspace pool (gc::pool_acquire)
   cublasHandle_t cublas = nullptr;
   cusolverDnHandle_t cusolver = nullptr;
   int *dev_info = nullptr;           // cuSOLVER info slot
@@ -113,6 +114,15 @@ int set_error(gc_context *ctx, int code, const char *fmt, ...);
                            cudaGetErrorString(e_));                                \
   } while (0)
 
+// The workspace pool of a device, shared by the library's contexts on it and destroyed with
+// the last of them. The driver's default pool gives all free memory back whenever a stream is
+// synchronised, which every call does: mapping 2 GB of workspace anew took 2.4 of the 4.7 ms of
+// a FOFO transform at n = 249. This pool keeps up to kPoolKeep bytes across calls (and
+// gives back what is free beyond that); allocation from it stays stream-ordered.
+constexpr unsigned long long kPoolKeep = 4ull << 30;
+cudaError_t pool_acquire(int device, cudaMemPool_t *pool);
+void pool_release(int device);
+
 // Stream-ordered device buffer owned by a context call.
 template <typename T>
 struct DevBuf {
@@ -133,10 +143,10 @@ struct DevBuf {
     s = ctx->stream;
     n = count;
     if (count == 0) return GC_OK;
-    cudaError_t e = cudaMallocAsync((void **)&p, count * sizeof(T), ctx->stream);
+    cudaError_t e = cudaMallocFromPoolAsync((void **)&p, count * sizeof(T), ctx->pool, ctx->stream);
     if (e != cudaSuccess) {
       p = nullptr;
-      return set_error(ctx, GC_ENOMEM, "cudaMallocAsync(%zu bytes): %s", count * sizeof(T),
+      return set_error(ctx, GC_ENOMEM, "device allocation of %zu bytes: %s", count * sizeof(T),
                        cudaGetErrorString(e));
     }
     return GC_OK;
@@ -158,21 +168,27 @@ inline bool is_sliced(int precision) {
 }
 
 // Per-system description resident on the device ------------------------------
+template <typename T>
+struct DevView {  // an array inside SysDev::blob
+  T *p = nullptr;
+};
 struct SysDev {
   int n = 0, nin = 0, nact = 0, nocc = 0, ndimx = 0;
   int vuni = 0;            // the virtual occupations are all equal
-  DevBuf<double> occ;      // (n)
-  DevBuf<int> grp;         // (n) 0 inactive, 1 active, 2 virtual
-  DevBuf<int> pair_p;      // (ndimx) 0-based p of pair (p > q)
-  DevBuf<int> pair_q;      // (ndimx)
-  DevBuf<double> h;        // (n, n) symmetrised one-electron MO matrix
-  DevBuf<double> rv;       // active block of RDM2val, RV[i + nact*(j + nact*(k + nact*l))]
-  DevBuf<int> slot;        // (ndimx) row order of the element kernel of the assembly
+  DevBuf<char> blob;       // the arrays below: one allocation and one host-to-device copy
+  DevView<double> occ;     // (n)
+  DevView<int> grp;        // (n) 0 inactive, 1 active, 2 virtual
+  DevView<int> pair_p;     // (ndimx) 0-based p of pair (p > q)
+  DevView<int> pair_q;     // (ndimx)
+  DevView<int> slot;       // (ndimx) row order of the element kernel of the assembly
+  DevView<double> xone;    // (n (n + 1) / 2) packed one-electron MO matrix
+  DevView<double> rv;      // active block of RDM2val, RV[i + nact*(j + nact*(k + nact*l))]
   // Per pair i = (p, q), with the CI coefficients C = sign(n - 1/2) sqrt(n) of
-  // ACEneERPA_FOFO / AB_CAS_FOFO: C_p + C_q, C_p - C_q and their reciprocals (0 where
-  // the sum or difference is 0), and n_p (1 - n_q) + n_q (1 - n_p). Computed once on
-  // the host, so that the element kernels spend the narrow FP64 pipe on products only.
-  DevBuf<double> cpl, cmi, rpl, rmi, dnq;  // (ndimx)
+  // ACEneERPA_FOFO / AB_CAS_FOFO: C_p + C_q, the reciprocals of C_p + C_q and C_p - C_q (0 where
+  // that is 0), and n_p (1 - n_q) + n_q (1 - n_p). Computed once on the host, so that the
+  // element kernels spend the narrow FP64 pipe on products only.
+  DevView<double> cpl, rpl, rmi, dnq;  // (ndimx)
+  DevBuf<double> h;        // (n, n) the rotated one-electron matrix, when URe was given
 };
 
 // IndN (2 x N, 1-based) reordered with q outer and p inner: consecutive pairs then
