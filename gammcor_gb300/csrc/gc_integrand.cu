@@ -6,9 +6,12 @@
 //   Kt[pq, rs] = mask * (C_p+C_q)(C_r+C_s) (rs|pq)       (lambda independent)
 //   W = 2 sum_{i,nu} Yk[i,nu] (Kt Yk)[i,nu] - sum_pq mask (n_p(1-n_q)+n_q(1-n_p)) (pq|pq)
 // with Yk = Y restricted to 1e-3 < omega < 1e8. One GEMM and one reduction
-// replace N^2 dot products of length N. On the tensor-core path the diagonal of
+// replace N^2 dot products of length N. On the tensor-core paths the diagonal of
 // Kt is taken out of the product and its term 2 Kt_ii (Yk Yk^T)_ii, which
-// nearly cancels the diagonal correction, is summed in FP64.
+// nearly cancels the diagonal correction, is summed in FP64. The sliced
+// precisions form one triangle of the Gram matrix instead,
+//   W = 2 sum_{i>j} (Kt_ij + Kt_ji)(Yk Yk^T)_ij + sum_i diag_i,
+// half the products, with one operand to slice and Kt itself in FP64.
 #include <cmath>
 
 #include "gc_internal.cuh"
@@ -39,6 +42,60 @@ __global__ void k_kt(int n, int nocc, int N, const int *__restrict__ pp, const i
     diag[i] = same ? 0.0 : -dnq[i] * f;
     kdiag[i] = kv;
   }
+}
+
+// The strict lower triangle of Kt + Kt^T, and per pair the diagonal's two parts: diag, kdiag as
+// in k_kt. One block per 32 x 32 tile of the triangle; the mirror tile is gathered with
+// the same coalescing (lanes along its rows) and turned in shared memory.
+__global__ void __launch_bounds__(256)
+    k_kt_low(int n, int nocc, int N, const int *__restrict__ pp, const int *__restrict__ pq,
+             const double *__restrict__ cpl, const double *__restrict__ dnq,
+             const int *__restrict__ grp, const double *__restrict__ fofo, double *__restrict__ kt,
+             double *__restrict__ diag, double *__restrict__ kdiag) {
+  if (blockIdx.y > blockIdx.x) return;  // tile row x, tile column y
+  __shared__ double tile[32][33];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int i0 = blockIdx.x * 32, j0 = blockIdx.y * 32;
+  const size_t ld = (size_t)n * nocc;
+  auto el = [&](int i, int j) -> double {  // Kt(i, j), without the diagonal's split
+    const int p = pp[i], q = pq[i], r = pp[j], s = pq[j];
+    const bool same = grp[p] == grp[q] && grp[q] == grp[r] && grp[r] == grp[s];
+    const double f = fofo[((size_t)r + (size_t)s * n) * ld + p + (size_t)q * n];  // (rs|pq)
+    if (i == j) diag[i] = same ? 0.0 : -dnq[i] * f;
+    return same ? 0.0 : (cpl[i] * cpl[j]) * f;
+  };
+  for (int k = ty; k < 32; k += 8) {  // mirror tile: rows j0 + tx, columns i0 + k
+    const int i = j0 + tx, j = i0 + k;
+    tile[k][tx] = i < N && j < N && i < j ? el(i, j) : 0.0;
+  }
+  __syncthreads();
+  for (int k = ty; k < 32; k += 8) {
+    const int i = i0 + tx, j = j0 + k;
+    if (i >= N || j > i) continue;
+    const double v = el(i, j);
+    if (i == j)
+      kdiag[i] = v;
+    else
+      kt[i + (size_t)j * N] = v + tile[tx][k];
+  }
+}
+
+// w = 2 sum part + sum_i (diag[i] + 2 kdiag[i] sq[i]): one block, fixed order.
+__global__ void __launch_bounds__(1024)
+    k_w_sum(int np, const double *__restrict__ part, int N, const double *__restrict__ diag,
+            const double *__restrict__ kdiag, const double *__restrict__ sq, double *__restrict__ w) {
+  __shared__ double red[1024];
+  double s = 0.0;
+  for (int i = threadIdx.x; i < np; i += 1024) s += part[i];
+  s *= 2.0;
+  for (int i = threadIdx.x; i < N; i += 1024) s += diag[i] + 2.0 * kdiag[i] * sq[i];
+  red[threadIdx.x] = s;
+  __syncthreads();
+  for (int k = 512; k > 0; k >>= 1) {
+    if (threadIdx.x < k) red[threadIdx.x] += red[threadIdx.x + k];
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) *w = red[0];
 }
 
 // diag[i] += 2 Kt_ii sum_nu Yk[i,nu]^2  (FP64)
@@ -96,6 +153,24 @@ int integrand(gc_context *ctx, const SysDev &sd, const double *Y, const double *
   const size_t NN = (size_t)N * N;
   DevBuf<double> kt, yk, t, diag, kdiag, part;
   GC_TRY(kt.alloc(ctx, NN));
+  if (is_sliced(precision)) {
+    DevBuf<double> buf;
+    GC_TRY(buf.alloc(ctx, 3 * (size_t)N + 1));
+    double *d = buf.p, *kd = d + N, *sq = kd + N, *w = sq + N;
+    const unsigned tiles = ceil_div(N, 32);
+    k_kt_low<<<dim3(tiles, tiles), 256, 0, ctx->stream>>>(sd.n, sd.nocc, N, sd.pair_p.p, sd.pair_q.p,
+                                                          sd.cpl.p, sd.dnq.p, sd.grp.p, fofo, kt.p,
+                                                          d, kd);
+    GC_LAUNCHED(ctx);
+    GC_TRY(tc_gram_dot(ctx, precision, N, Y, eig, kSmallE, kBigE, kt.p, sq, part));
+    k_w_sum<<<1, 1024, 0, ctx->stream>>>((int)part.n, part.p, N, d, kd, sq, w);
+    GC_LAUNCHED(ctx);
+    GC_CUDA(ctx, cudaMemcpyAsync(w_host, w, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+    GC_TRY(check_flag(ctx));  // synchronises
+    if (!std::isfinite(*w_host))
+      return set_error(ctx, GC_ENONFINITE, "integrand: W is not finite (non-finite integrals?)");
+    return GC_OK;
+  }
   GC_TRY(yk.alloc(ctx, NN));
   if (precision == GC_PREC_FP64) GC_TRY(t.alloc(ctx, NN));
   GC_TRY(diag.alloc(ctx, N));

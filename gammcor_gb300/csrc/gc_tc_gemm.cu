@@ -388,7 +388,8 @@ struct OzPlan {
 
 struct OzEpi {
   int mode;              // 0 store, 1 dot with r, 2 subtract from the lower triangle of c,
-                         // 3 store the lower triangle of c and its mirror image
+                         // 3 store the lower triangle of c and its mirror image,
+                         // 4 dot with the strict lower triangle of r
   double *c;
   long long ldn, sb;
   const double *r;
@@ -444,7 +445,11 @@ __global__ void __launch_bounds__(oz_threads(TBN), 1)
   const int nchunks = (kblocks + plan.chunk_kb - 1) / plan.chunk_kb;
   if (epi.tri_period > 0) {  // whole CTA, before any barrier or TMEM is set up
     const int c0 = n0 % epi.tri_period;
-    if (c0 + TBN <= epi.tri_period && c0 >= m0 + BM) return;
+    if (c0 + TBN <= epi.tri_period && c0 >= m0 + BM) {
+      if (epi.mode == 4 && threadIdx.x == 0)
+        epi.partial[blockIdx.x + (long long)gridDim.x * (blockIdx.y + (long long)gridDim.y * blockIdx.z)] = 0.0;
+      return;
+    }
   }
 
   if (threadIdx.x == 0) {
@@ -612,19 +617,20 @@ __global__ void __launch_bounds__(oz_threads(TBN), 1)
               epi.c[o] = cv;
               epi.c[n + (long long)m * epi.ldn] = cv;  // 32 consecutive per thread
             }
-          } else
+          } else if (epi.mode == 1 || m > n) {
             dot += cv * epi.r[o];
+          }
         }
       }
     }
-    if (epi.mode == 1) {
+    if (epi.mode == 1 || epi.mode == 4) {
       for (int off = 16; off > 0; off >>= 1) dot += __shfl_down_sync(0xffffffffu, dot, off);
       if (lane == 0) red[warp - 2] = dot;
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (epi.mode == 1 && threadIdx.x == 0) {
+  if ((epi.mode == 1 || epi.mode == 4) && threadIdx.x == 0) {
     long long cta = blockIdx.x + (long long)gridDim.x * (blockIdx.y + (long long)gridDim.y * blockIdx.z);
     double sum = 0.0;
     for (int w = 0; w < EPI; ++w) sum += red[w];
@@ -766,50 +772,201 @@ __device__ __forceinline__ long long tri_offset(int r, int n) {
   return r - (long long)d * (d + 1) / 2 + (long long)d * n;
 }
 
-// The same for any other strides (in use: consecutive rows contiguous, K the slow index). One
-// block takes 32 rows: the maximum with the lanes along the rows, then 64 values of K at a time
+// What k_oz_cols does beside slicing: columns k of x outside (lo, hi) by eig[k] count as zero,
+// and sq[b][r] = sum_k x[b,r,k]^2 in FP64 (the integrand's dropped modes and its diagonal term).
+// One kernel up to this K: a transform of n = 64 (K = 300) takes 11 us instead of two launches.
+constexpr int kOzShortK = 512;
+struct OzColsOpt {
+  const double *eig = nullptr;
+  double lo = 0.0, hi = 0.0;
+  double *sq = nullptr;
+};
+
+// Element (b, r, k) of an operand with any strides (in use: consecutive rows contiguous, K the
+// slow index), rows by pair index (tri > 0: row r is the pair (c, d), c <= d, of a tri x tri
+// matrix, r = c + d (d + 1) / 2) and columns dropped by opt.eig.
+struct OzColView {
+  const double *x;
+  int rows, K, tri;
+  long long sr, sk, sb;
+  OzColsOpt opt;
+  __device__ __forceinline__ const double *row(long long bb, int r) const {
+    return x + bb * sb + (tri > 0 ? tri_offset(r, tri) : r) * sr;
+  }
+  // lo < eig < hi for 0 < lo < hi, as integers: the FP64 pipe is narrow
+  __device__ __forceinline__ bool kept(int k) const {
+    if (!opt.eig) return true;
+    const long long b = __double_as_longlong(opt.eig[k]);
+    return b > __double_as_longlong(opt.lo) && b < __double_as_longlong(opt.hi);
+  }
+  __device__ __forceinline__ double at(const double *xr, int r, int k) const {
+    double v = r < rows && k < K ? xr[k * sk] : 0.0;
+    if (k < K && !kept(k)) v = 0.0;
+    return v;
+  }
+};
+
+// Such operands in one kernel, for short K (Cholesky panels, small transforms: one launch). A
+// block takes 16 rows: the maximum with the lanes along the rows, then 128 values of K at a time
 // through shared memory, read along the rows and written along K. The position of k within
-// its 64 is (k / 4) + 16 (k % 4), so that four consecutive k are read without bank conflicts.
+// its 128 is (k / 4) + 32 (k % 4), so that four consecutive k are read without bank conflicts.
 template <int S>
-__global__ void __launch_bounds__(512) k_oz_cols(const double *__restrict__ x, int rows, int K, int Kp,
-                                                 int nb, long long sr, long long sk, long long sb,
-                                                 int tri, int *__restrict__ e,
+__global__ void __launch_bounds__(512) k_oz_cols(OzColView X, int Kp, int nb, int *__restrict__ e,
                                                  __nv_bfloat16 *__restrict__ planes) {
-  __shared__ double tile[32][65];
-  __shared__ unsigned long long part[16][32];
-  __shared__ int es[32];
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  const int r0 = blockIdx.x * 32, r = r0 + tx;
-  const int lr = threadIdx.x >> 4, lk = threadIdx.x & 15;  // row and group of four in the write
-  const long long plane = (long long)nb * rows * Kp;
+  constexpr int ROWS = 16, TY = 32;
+  __shared__ double tile[ROWS][129];
+  __shared__ unsigned long long part[TY][ROWS];
+  __shared__ double psq[TY][ROWS];
+  __shared__ int es[ROWS];
+  const int tx = threadIdx.x % ROWS, ty = threadIdx.x / ROWS;
+  const int r0 = blockIdx.x * ROWS, r = r0 + tx;
+  const int lr = threadIdx.x / 32, lk = threadIdx.x % 32;  // row and group of four in the write
+  const long long plane = (long long)nb * X.rows * Kp;
   for (int bb = blockIdx.y; bb < nb; bb += gridDim.y) {
-    // tri > 0: row r is the pair (c, d), c <= d, of a tri x tri matrix (r = c + d (d + 1) / 2)
-    const double *__restrict__ xr = x + bb * sb + (tri > 0 ? tri_offset(r, tri) : r) * sr;
+    const double *xr = X.row(bb, r);
     unsigned long long mx = 0;
-    if (r < rows) {
+    double q = 0.0;
 #pragma unroll 4
-      for (int k = ty; k < K; k += 16) mx = max(mx, abs_bits(xr[(long long)k * sk]));
+    for (int k = ty; k < X.K; k += TY) {
+      const double v = X.at(xr, r, k);
+      mx = max(mx, abs_bits(v));
+      if (X.opt.sq) q += v * v;
     }
     part[ty][tx] = mx;
+    psq[ty][tx] = q;
     __syncthreads();
     if (ty == 0) {
-      for (int w = 1; w < 16; ++w) mx = max(mx, part[w][tx]);
+      for (int w = 1; w < TY; ++w) mx = max(mx, part[w][tx]);
       es[tx] = row_exponent(mx);
-      if (r < rows) e[(long long)bb * rows + r] = es[tx];
+      if (r < X.rows) {
+        e[(long long)bb * X.rows + r] = es[tx];
+        if (X.opt.sq) {
+          for (int w = 1; w < TY; ++w) q += psq[w][tx];
+          X.opt.sq[(long long)bb * X.rows + r] = q;
+        }
+      }
     }
-    for (int k0 = 0; k0 < Kp; k0 += 64) {
+    for (int k0 = 0; k0 < Kp; k0 += 128) {
       __syncthreads();
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        const int k = ty + 16 * i;
-        tile[tx][(k >> 2) + 16 * (k & 3)] = r < rows && k0 + k < K ? xr[(long long)(k0 + k) * sk] : 0.0;
+        const int k = ty + TY * i;
+        tile[tx][(k >> 2) + 32 * (k & 3)] = X.at(xr, r, k0 + k);
       }
       __syncthreads();
-      if (r0 + lr < rows) {
-        const double v[4] = {tile[lr][lk], tile[lr][lk + 16], tile[lr][lk + 32], tile[lr][lk + 48]};
-        store_digits4<S>(v, es[lr], plane, ((long long)bb * rows + r0 + lr) * Kp + k0 + lk * 4, planes);
+      if (r0 + lr < X.rows && k0 + lk * 4 < Kp) {
+        const double v[4] = {tile[lr][lk], tile[lr][lk + 32], tile[lr][lk + 64], tile[lr][lk + 96]};
+        store_digits4<S>(v, es[lr], plane, ((long long)bb * X.rows + r0 + lr) * Kp + k0 + lk * 4, planes);
       }
     }
+    __syncthreads();
+  }
+}
+
+// ... and in two kernels for longer K, so that both passes have blocks enough for the chip:
+// the maxima (and squares) of 64 rows over a share of K, then the digits of 64 x 64 tiles (512
+// contiguous bytes per load). part[share][b][r], psq likewise. Measured (5 slices): 6972 x 1494
+// 19 + 46 us, where one kernel with 16 rows per block took 89 us, with 32 rows 76 us, and a
+// cluster of CTAs sharing the maxima 108 us; 3774 x 3774 with eig and sq 62 + 78 us (one kernel
+// 171 us).
+constexpr int kColW = 64;
+constexpr int kColShare = 1024;  // K per block of k_oz_col_max at most
+__global__ void __launch_bounds__(256) k_oz_col_max(OzColView X, int nb, int share,
+                                                    unsigned long long *__restrict__ part,
+                                                    double *__restrict__ psq) {
+  __shared__ unsigned long long pm[4][kColW];
+  __shared__ double ps[4][kColW];
+  __shared__ unsigned char keep[kColShare];
+  const int tx = threadIdx.x % kColW, ty = threadIdx.x / kColW, r = blockIdx.x * kColW + tx;
+  const int k0 = blockIdx.y * share, k1 = min(X.K, k0 + share);
+  if (X.opt.eig) {
+    for (int k = k0 + threadIdx.x; k < k1; k += 256) keep[k - k0] = X.kept(k);
+    __syncthreads();
+  }
+  for (int bb = blockIdx.z; bb < nb; bb += gridDim.z) {
+    const double *xr = X.row(bb, min(r, X.rows - 1));
+    unsigned long long mx = 0;
+    double q = 0.0;
+    int k = k0 + ty;
+    for (; k + 28 < k1; k += 32) {
+      double v[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] = xr[(k + 4 * i) * X.sk];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        if (X.opt.eig && !keep[k + 4 * i - k0]) v[i] = 0.0;
+        mx = max(mx, abs_bits(v[i]));
+        if (X.opt.sq) q += v[i] * v[i];
+      }
+    }
+    for (; k < k1; k += 4) {
+      const double v = !X.opt.eig || keep[k - k0] ? xr[k * X.sk] : 0.0;
+      mx = max(mx, abs_bits(v));
+      if (X.opt.sq) q += v * v;
+    }
+    pm[ty][tx] = mx;
+    ps[ty][tx] = q;
+    __syncthreads();
+    if (ty == 0 && r < X.rows) {
+      for (int w = 1; w < 4; ++w) {
+        mx = max(mx, pm[w][tx]);
+        q += ps[w][tx];
+      }
+      const size_t o = ((size_t)blockIdx.y * nb + bb) * X.rows + r;
+      part[o] = mx;
+      if (X.opt.sq) psq[o] = q;
+    }
+    __syncthreads();
+  }
+}
+
+template <int S>
+__global__ void __launch_bounds__(256) k_oz_col_digits(OzColView X, int Kp, int nb, int nshare,
+                                                       const unsigned long long *__restrict__ part,
+                                                       const double *__restrict__ psq,
+                                                       int *__restrict__ e,
+                                                       __nv_bfloat16 *__restrict__ planes) {
+  __shared__ double tile[kColW][65];  // k of the 64 at (k / 4) + 16 (k % 4)
+  __shared__ int es[kColW];
+  __shared__ unsigned char keep[64];
+  const int tx = threadIdx.x % kColW, ty = threadIdx.x / kColW;
+  const int r0 = blockIdx.x * kColW, r = r0 + tx, k0 = blockIdx.y * 64;
+  const int lr = threadIdx.x / 16, lk = threadIdx.x % 16;
+  const long long plane = (long long)nb * X.rows * Kp;
+  for (int bb = blockIdx.z; bb < nb; bb += gridDim.z) {
+    const double *xr = X.row(bb, min(r, X.rows - 1));
+    double v[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const int k = k0 + ty + 4 * i;
+      v[i] = r < X.rows && k < X.K ? xr[k * X.sk] : 0.0;
+    }
+    if (threadIdx.x < 64) keep[threadIdx.x] = k0 + threadIdx.x >= X.K || X.kept(k0 + threadIdx.x);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) tile[tx][i + 16 * ty] = v[i];
+    if (ty == 0 && r < X.rows) {
+      unsigned long long mx = 0;
+      double q = 0.0;
+      for (int c = 0; c < nshare; ++c) {
+        const size_t o = ((size_t)c * nb + bb) * X.rows + r;
+        mx = max(mx, part[o]);
+        if (X.opt.sq) q += psq[o];
+      }
+      es[tx] = row_exponent(mx);
+      if (blockIdx.y == 0) {
+        e[(long long)bb * X.rows + r] = es[tx];
+        if (X.opt.sq) X.opt.sq[(long long)bb * X.rows + r] = q;
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int l = lr; l < kColW; l += 16)
+      if (r0 + l < X.rows) {
+        double w[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) w[i] = keep[lk * 4 + i] ? tile[l][lk + 16 * i] : 0.0;
+        store_digits4<S>(w, es[l], plane, ((long long)bb * X.rows + r0 + l) * Kp + k0 + lk * 4, planes);
+      }
     __syncthreads();
   }
 }
@@ -1077,24 +1234,42 @@ int encode_oz_map(gc_context *ctx, OzOperand &op) {
 
 template <int S>
 int slice_operand(gc_context *ctx, OzOperand &op, const double *x, int rows, int K, int nb,
-                  long long sr, long long sk, long long sb, int tri) {
+                  long long sr, long long sk, long long sb, int tri, const OzColsOpt &opt) {
   const long long nrr = (long long)nb * rows;
-  if (sk == 1 && !tri && op.Kp <= 128 * kOzHold) {  // one warp holds the row
+  const bool plain = !tri && !opt.eig && !opt.sq;
+  if (sk == 1 && plain && op.Kp <= 128 * kOzHold) {  // one warp holds the row
     k_oz_rows<S, 32><<<gc::ceil_div(nrr, 8), 256, 0, ctx->stream>>>(x, rows, K, op.Kp, nrr, sr, sb,
                                                                     op.exps.p, op.buf.p);
-  } else if (sk == 1 && !tri) {
+  } else if (sk == 1 && plain) {
     k_oz_rows<S, 256><<<(unsigned)nrr, 256, 0, ctx->stream>>>(x, rows, K, op.Kp, nrr, sr, sb,
                                                               op.exps.p, op.buf.p);
   } else {
-    k_oz_cols<S><<<dim3(gc::ceil_div(rows, 32), std::min(nb, 65535)), 512, 0, ctx->stream>>>(
-        x, rows, K, op.Kp, nb, sr, sk, sb, tri, op.exps.p, op.buf.p);
+    const OzColView X{x, rows, K, tri, sr, sk, sb, opt};
+    if (op.Kp <= kOzShortK) {
+      k_oz_cols<S><<<dim3(gc::ceil_div(rows, 16), std::min(nb, 65535)), 512, 0, ctx->stream>>>(
+          X, op.Kp, nb, op.exps.p, op.buf.p);
+    } else {
+      const int nshare = std::max(std::min(16, (K + 255) / 256), (K + kColShare - 1) / kColShare);
+      const int share = (K + nshare - 1) / nshare;
+      gc::DevBuf<unsigned long long> part;
+      gc::DevBuf<double> psq;
+      GC_TRY(part.alloc(ctx, (size_t)nshare * nrr));
+      if (opt.sq) GC_TRY(psq.alloc(ctx, (size_t)nshare * nrr));
+      const unsigned gz = std::min(nb, 65535);
+      k_oz_col_max<<<dim3(gc::ceil_div(rows, kColW), nshare, gz), 256, 0, ctx->stream>>>(X, nb, share,
+                                                                                      part.p, psq.p);
+      GC_LAUNCHED(ctx);
+      k_oz_col_digits<S><<<dim3(gc::ceil_div(rows, kColW), op.Kp / 64, gz), 256, 0,
+                           ctx->stream>>>(X, op.Kp, nb, nshare, part.p, psq.p, op.exps.p, op.buf.p);
+    }
   }
   GC_LAUNCHED(ctx);
   return GC_OK;
 }
 
 int make_oz_operand(gc_context *ctx, OzOperand &op, const double *x, int rows, int K, int nb,
-                    long long sr, long long sk, long long sb, int S, int box_rows, int tri = 0) {
+                    long long sr, long long sk, long long sb, int S, int box_rows, int tri = 0,
+                    const OzColsOpt &opt = OzColsOpt()) {
   op.rows = rows;
   op.box_rows = box_rows;
   op.Kp = (K + BK - 1) / BK * BK;
@@ -1104,9 +1279,9 @@ int make_oz_operand(gc_context *ctx, OzOperand &op, const double *x, int rows, i
   GC_TRY(op.exps.alloc(ctx, (size_t)nb * rows));
   GC_TRY(op.buf.alloc(ctx, plane * S));
   switch (S) {
-    case 4: GC_TRY(slice_operand<4>(ctx, op, x, rows, K, nb, sr, sk, sb, tri)); break;
-    case 5: GC_TRY(slice_operand<5>(ctx, op, x, rows, K, nb, sr, sk, sb, tri)); break;
-    default: GC_TRY(slice_operand<6>(ctx, op, x, rows, K, nb, sr, sk, sb, tri));
+    case 4: GC_TRY(slice_operand<4>(ctx, op, x, rows, K, nb, sr, sk, sb, tri, opt)); break;
+    case 5: GC_TRY(slice_operand<5>(ctx, op, x, rows, K, nb, sr, sk, sb, tri, opt)); break;
+    default: GC_TRY(slice_operand<6>(ctx, op, x, rows, K, nb, sr, sk, sb, tri, opt));
   }
   op.planes = op.buf.p;
   op.ex = op.exps.p;
@@ -1428,27 +1603,26 @@ int tc_syrk_sub_lower(gc_context *ctx, int precision, int M, int K, const double
   return GC_OK;  // the device flag is read at the caller's next sync point
 }
 
+int tc_gram_dot(gc_context *ctx, int precision, int N, const double *Y, const double *eig, double lo,
+                double hi, const double *Klow, double *sq, DevBuf<double> &part) {
+  if (!is_oz(precision))
+    return set_error(ctx, GC_EINVAL, "gram_dot: needs a sliced FP64-accurate precision");
+  const OzPlan pl = oz_plan(precision);
+  OzOperand a, b;
+  OzColsOpt opt;
+  opt.eig = eig;
+  opt.lo = lo;
+  opt.hi = hi;
+  opt.sq = sq;
+  GC_TRY(make_oz_operand(ctx, a, Y, N, N, 1, 1, N, 0, pl.S, BM, 0, opt));
+  GC_TRY(alias_oz_operand(ctx, a, b, oz_tile(ctx, pl.S, N, (N + 1) / 2, 1)));
+  GC_TRY(part.alloc(ctx, (size_t)ceil_div(N, BM) * ceil_div(N, b.box_rows)));
+  OzEpi e{4, nullptr, N, 0, Klow, part.p, nullptr, nullptr, 0, 0, N};
+  return run_oz(ctx, a, b, N, N, 1, pl, e);
+}
+
 int tc_dot_gemm(gc_context *ctx, int precision, int N, const double *Ksym, const double *Y,
                 double *result) {
-  if (is_oz(precision)) {
-    OzPlan pl = oz_plan(precision);
-    OzOperand a, b;
-    GC_TRY(make_oz_operand(ctx, a, Ksym, N, N, 1, N, 1, 0, pl.S, BM));
-    GC_TRY(make_oz_operand(ctx, b, Y, N, N, 1, N, 1, 0, pl.S, oz_tile(ctx, pl.S, N, N, 1)));
-    size_t ncta = (size_t)ceil_div(N, BM) * ceil_div(N, b.box_rows);
-    DevBuf<double> part;
-    GC_TRY(part.alloc(ctx, ncta));
-    OzEpi e{1, nullptr, N, 0, Y, part.p, nullptr, nullptr, 0, 0};
-    GC_TRY(run_oz(ctx, a, b, N, N, 1, pl, e));
-    std::vector<double> h(ncta);
-    GC_CUDA(ctx, cudaMemcpyAsync(h.data(), part.p, ncta * sizeof(double), cudaMemcpyDeviceToHost,
-                                 ctx->stream));
-    GC_TRY(check_flag(ctx));
-    double sum = 0.0;
-    for (double v : h) sum += v;
-    *result = sum;
-    return GC_OK;
-  }
   int S;
   PassList pl = pass_list(precision, &S);
   Operand a, b;

@@ -41,8 +41,15 @@ int tc_two_sided(gc_context *ctx, int precision, int n, int cnt, const double *M
 int tc_gemm_nt(gc_context *ctx, int precision, int m, int n, int k, const double *A, int lda,
                const double *B, int ldb, double *C, int ldc);
 
-// result = sum_{i,nu} (Ksym Y)[i,nu] * Y[i,nu] for a symmetric N x N Ksym and
-// an N x N Y (both column-major), with the product on tensor cores.
+// Sliced precisions: part (one value per CTA of the product) adds up to
+// sum_{i > j} Klow[i,j] (Yk Yk^T)[i,j], and sq[i] = (Yk Yk^T)[i,i] in FP64, where Yk is the N x N
+// Y (column-major) with the columns outside lo < eig < hi left out. Klow: N x N, strict lower
+// triangle read.
+int tc_gram_dot(gc_context *ctx, int precision, int N, const double *Y, const double *eig, double lo,
+                double hi, const double *Klow, double *sq, DevBuf<double> &part);
+
+// Split-BF16 precisions: result = sum_{i,nu} (Ksym Y)[i,nu] * Y[i,nu] for a symmetric N x N Ksym
+// and an N x N Y (both column-major), with the product on tensor cores.
 int tc_dot_gemm(gc_context *ctx, int precision, int N, const double *Ksym, const double *Y,
                 double *result);
 

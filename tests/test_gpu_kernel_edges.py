@@ -137,3 +137,21 @@ def test_transform_block_shapes(gpu_lib, n, widths, entry):
     else:
         out = api.tran4_gen(n, *blocks, t(lf @ lf.T), precision="fp64tc5")
     assert np.abs(out.cpu().numpy() - ref).max() < 1e-10
+
+
+# pair counts below, at and above the 32-wide tiles and the GEMM's column tiles, dropped modes,
+# and (rs|pq) that differs from (pq|rs): both enter
+@pytest.mark.parametrize("precision", ["fp64tc5", "fp64tc6"])
+@pytest.mark.parametrize("n,nin,nact", [(4, 1, 1), (13, 2, 2), (17, 4, 2), (33, 3, 5)])
+def test_integrand_tiles(gpu_lib, precision, n, nin, nact):
+    m = model(n, nin, nact, seed=n)
+    rng = np.random.default_rng(2)
+    N = len(m["indn"])
+    m["fofo"] = m["fofo"] * (1.0 + 0.1 * rng.standard_normal(m["fofo"].shape))
+    y = np.linalg.qr(rng.standard_normal((N, N)))[0] * 0.7
+    e = rng.uniform(0.1, 20.0, N)
+    e[::5], e[1::7] = -0.1, 2e8
+    ref = R.ac_ene_erpa_fofo(y, e, m["occ"], nin, nact, m["indn"], m["fofo"])
+    w = api.ace_ne_erpa_fofo(t(y.T).t(), t(e), m["occ"], m["indn"], nact, nin, t(m["fofo"]),
+                             precision=precision)
+    assert abs(w - ref) < 5e-9
