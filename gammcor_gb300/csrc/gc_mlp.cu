@@ -4,15 +4,24 @@
 // Layers: in -> H -> H -> H -> out, GELU after every hidden layer. The forward
 // pass reads BF16 copies of the weights and accumulates in FP32; training keeps
 // FP32 master weights and Adam moments and refreshes the BF16 copies after every
-// step. All products go through one tiled shared-memory kernel
+// step.
+//
+// A step of the surrogate's sizes (batches of some hundred rows, 256 units) is bound by launches
+// and by the latency of its chain of layers, not by its 0.2 GFLOP. Layers up to kFusedWidth
+// units therefore take two kernels: k_mlp_rows carries a few rows through all layers forward and,
+// in training, the loss and the data gradient back (everything of a row is local to it, the
+// activations stay in shared memory); k_mlp_dw forms all weight and bias gradients and
+// applies Adam to them. Wider layers, whose weights every block of k_mlp_rows would read
+// again, go through one tiled shared-memory kernel
 //   C[m, n] = sum_k A(m, k) B(n, k)   (A, B with arbitrary strides, B in BF16 or FP32)
-// used for the forward product, the data gradient and the weight gradient.
+// per product.
 //
 // Parameter layout (flattened FP32): W1 (H x in), b1 (H), W2 (H x H), b2,
 // W3 (H x H), b3, W4 (out x H), b4; W row-major (row = output unit).
 #include <cuda_bf16.h>
 
 #include <cmath>
+#include <mutex>
 #include <random>
 
 #include "gc_internal.cuh"
@@ -24,9 +33,10 @@ struct gc_mlp {
   size_t woff[4], boff[4];
   int din[4], dout[4];
   gc::DevBuf<float> master, grad, m1, m2;
-  gc::DevBuf<__nv_bfloat16> wbf;  // BF16 copy of the whole parameter vector
+  gc::DevBuf<__nv_bfloat16> wbf;  // BF16 copy of the whole parameter vector, padded by 16 bytes
   gc::DevBuf<float> act;           // activations / pre-activations for the largest batch seen
   int act_batch = 0;
+  gc::DevBuf<float> lossbuf;       // loss partials of the row blocks, then the loss
   long long step = 0;
 };
 
@@ -132,6 +142,342 @@ __global__ void k_to_bf16(long long n, const float *__restrict__ w, __nv_bfloat1
     o[t] = __float2bfloat16(w[t]);
 }
 
+// Layer table of a network as the fused kernels read it.
+struct Layers {
+  int din[4], dout[4];
+  long long woff[4], boff[4];
+  float *h[4];   // inputs of layers 1..3 kept for the weight gradient (h[l]: output of layer l)
+  float *dz[4];  // dL/dZ of every layer
+};
+
+constexpr int kFusedWidth = 256;   // widest layer of the fused kernels: a warp holds a row of it
+constexpr int kRowThreads = 256, kRowWarps = kRowThreads / 32;
+constexpr int kPer = kFusedWidth / 32;  // inputs per lane
+
+__device__ __forceinline__ float gelu(float v) { return 0.5f * v * (1.f + erff(v * 0.70710678118654752f)); }
+__device__ __forceinline__ float gelu_grad(float z) {
+  return 0.5f * (1.f + erff(z * 0.70710678118654752f)) + z * 0.3989422804014327f * expf(-0.5f * z * z);
+}
+
+// Layer l's weights (BF16, contiguous) into shared memory at dst, 16 bytes per copy from the
+// 16-byte boundary below them; returns the first weight's place. Ends with a barrier.
+__device__ __forceinline__ const __nv_bfloat16 *stage_weights(const __nv_bfloat16 *w, int count,
+                                                              unsigned char *dst) {
+  const uintptr_t a = (uintptr_t)w & ~(uintptr_t)15;
+  const int skip = (int)((uintptr_t)w - a), n16 = (skip + 2 * count + 15) / 16;
+  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+  __syncthreads();  // the buffer's last readers
+  for (int k = threadIdx.x; k < n16; k += kRowThreads)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + 16 * k), "l"(a + 16 * (uintptr_t)k)
+                 : "memory");
+  asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+  return reinterpret_cast<const __nv_bfloat16 *>(dst + skip);
+}
+
+// The kPer weights of row o that this lane holds: inputs 2 lane + 64 j + {0, 1} where the rows
+// are even (4-byte loads), lane + 32 j otherwise; 0 beyond the row.
+template <bool PAIR>
+__device__ __forceinline__ int lane_input(int lane, int k) {
+  return PAIR ? 2 * lane + 64 * (k / 2) + (k & 1) : lane + 32 * k;
+}
+template <bool PAIR>
+__device__ __forceinline__ void lane_weights(const __nv_bfloat16 *w, int o, int din, int lane, float *v) {
+  if (PAIR) {
+    const uint32_t *p = reinterpret_cast<const uint32_t *>(w + (size_t)o * din) + lane;
+#pragma unroll
+    for (int j = 0; j < kPer / 2; ++j) {
+      const uint32_t u = 2 * lane + 64 * j < din ? p[32 * j] : 0u;
+      v[2 * j] = __uint_as_float(u << 16);
+      v[2 * j + 1] = __uint_as_float(u & 0xffff0000u);
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+      const int i = lane + 32 * k;
+      v[k] = i < din ? __bfloat162float(w[(size_t)o * din + i]) : 0.f;
+    }
+  }
+}
+
+// out[r][o] = sum_i in[r][i] W[o, i]: a warp per pair of units, its lanes along the inputs, which
+// they hold in registers for all units.
+template <int R, bool PAIR>
+__device__ __forceinline__ void layer_forward(const float *in, int ld, const __nv_bfloat16 *w, int din,
+                                              int dout, float *out) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float a[R][kPer];
+#pragma unroll
+  for (int k = 0; k < kPer; ++k) {
+    const int i = lane_input<PAIR>(lane, k);
+#pragma unroll
+    for (int r = 0; r < R; ++r) a[r][k] = i < din ? in[r * ld + i] : 0.f;
+  }
+  for (int o = 2 * warp; o < dout; o += 2 * kRowWarps) {
+    float v[2][kPer], acc[2 * R];
+    lane_weights<PAIR>(w, o, din, lane, v[0]);
+    lane_weights<PAIR>(w, min(o + 1, dout - 1), din, lane, v[1]);
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        float s = 0.f;
+#pragma unroll
+        for (int k = 0; k < kPer; ++k) s += a[r][k] * v[u][k];
+        acc[u * R + r] = s;
+      }
+    // the 2 R sums over the lanes at once: each exchange halves the number of sums a lane holds
+    int n = 2 * R, off = 16;
+#pragma unroll
+    for (; n > 1; n /= 2, off /= 2) {
+#pragma unroll
+      for (int k = 0; k < n / 2; ++k) {
+        const bool up = lane & off;
+        const float give = up ? acc[k] : acc[k + n / 2], keep = up ? acc[k + n / 2] : acc[k];
+        acc[k] = keep + __shfl_xor_sync(0xffffffffu, give, off);
+      }
+    }
+    for (; off > 0; off /= 2) acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], off);
+    // the lane's high bits say which sum it holds, highest bit of the index first
+    constexpr int LG = R == 2 ? 2 : 3;
+    const int idx = lane >> (5 - LG);
+    const int u = idx / R, r = idx % R;
+    if ((lane & ((32 >> LG) - 1)) == 0 && o + u < dout) out[r * ld + o + u] = acc[0];
+  }
+}
+
+// out[r][i] = sum_o dz[r][o] W[o, i]: the lanes along i, the units o over the warps, whose sums
+// meet in red [kRowWarps][R][kFusedWidth].
+template <int R, bool PAIR, class F>
+__device__ __forceinline__ void layer_backward(const float *dz, int ld, const __nv_bfloat16 *w, int din,
+                                               int dout, float *red, F put) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float acc[R][kPer] = {};
+  for (int o = warp; o < dout; o += kRowWarps) {
+    float v[kPer];
+    lane_weights<PAIR>(w, o, din, lane, v);
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const float z = dz[r * ld + o];
+#pragma unroll
+      for (int k = 0; k < kPer; ++k) acc[r][k] += z * v[k];
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+#pragma unroll
+    for (int k = 0; k < kPer; ++k)
+      red[(warp * R + r) * kFusedWidth + lane_input<PAIR>(lane, k)] = acc[r][k];
+  __syncthreads();
+  for (int e = threadIdx.x; e < R * din; e += kRowThreads) {
+    const int r = e / din, i = e - r * din;
+    float v = 0.f;
+#pragma unroll
+    for (int k = 0; k < kRowWarps; ++k) v += red[(k * R + r) * kFusedWidth + i];
+    put(i, r, v);
+  }
+}
+
+// R rows through all layers; with t also the loss partial and dL/dZ of every layer. The chain of
+// layers is bound by latency, so each layer's weights come into shared memory with all copies in
+// flight at once, and the arithmetic then reads shared memory and registers only. Measured at 256
+// rows, 256 units: 30 us (81 us while biases and GELU were applied by one lane per unit);
+// a whole training step 222 -> 73 us with this and k_mlp_dw in place of 20 kernels.
+template <int R>
+constexpr size_t rows_smem() {  // weights, two activation buffers, pre-activations, partial sums
+  return 2 * (size_t)kFusedWidth * kFusedWidth + 32 +
+         sizeof(float) * kFusedWidth * R * (2 + 3 + kRowWarps);
+}
+
+template <int R>
+__global__ void __launch_bounds__(kRowThreads)
+    k_mlp_rows(int B, Layers L, const __nv_bfloat16 *__restrict__ W, const float *__restrict__ P,
+               const float *__restrict__ x, const float *__restrict__ t, float inv,
+               float *__restrict__ y, float *__restrict__ part) {
+  extern __shared__ __align__(16) unsigned char sm[];
+  constexpr int LD = kFusedWidth;
+  float *cur = reinterpret_cast<float *>(sm + 2 * (size_t)LD * LD + 32), *nxt = cur + R * LD,
+        *zs = nxt + R * LD, *red = zs + 3 * R * LD;
+  __shared__ float lred[kRowWarps], bias[4 * kFusedWidth];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int b0 = blockIdx.x * R, nr = min(R, B - b0);
+  for (int e = tid; e < R * L.din[0]; e += kRowThreads) {
+    const int r = e / L.din[0], i = e - r * L.din[0];
+    cur[r * LD + i] = r < nr ? x[(long long)(b0 + r) * L.din[0] + i] : 0.f;
+  }
+  for (int l = 0; l < 4; ++l)
+    if (tid < L.dout[l]) bias[l * LD + tid] = P[L.boff[l] + tid];
+  const __nv_bfloat16 *w = nullptr;
+  for (int l = 0; l < 4; ++l) {
+    const int din = L.din[l], dout = L.dout[l];
+    w = stage_weights(W + L.woff[l], din * dout, sm);
+    if ((din & 1) == 0 && ((uintptr_t)w & 3) == 0)
+      layer_forward<R, true>(cur, LD, w, din, dout, nxt);
+    else
+      layer_forward<R, false>(cur, LD, w, din, dout, nxt);
+    __syncthreads();
+    for (int e = tid; e < R * dout; e += kRowThreads) {
+      const int r = e / dout, o = e - r * dout;
+      const float v = nxt[r * LD + o] + bias[l * LD + o];
+      const float h = l == 3 ? v : gelu(v);
+      nxt[r * LD + o] = h;
+      if (l == 3) {
+        if (r < nr && y) y[(long long)(b0 + r) * dout + o] = v;
+      } else if (t) {
+        zs[(l * R + r) * LD + o] = v;
+        if (r < nr) L.h[l][(long long)(b0 + r) * dout + o] = h;
+      }
+    }
+    __syncthreads();
+    float *s = cur;
+    cur = nxt;
+    nxt = s;
+  }
+  if (!t) return;
+  // loss partial and dL/dY
+  const int nout = L.dout[3];
+  float ls = 0.f;
+  for (int e = tid; e < R * nout; e += kRowThreads) {
+    const int r = e / nout, o = e - r * nout;
+    float dv = 0.f;
+    if (r < nr) {
+      const float d = cur[r * LD + o] - t[(long long)(b0 + r) * nout + o];
+      ls += d * d;
+      dv = 2.f * d * inv;
+      L.dz[3][(long long)(b0 + r) * nout + o] = dv;
+    }
+    cur[r * LD + o] = dv;
+  }
+  for (int off = 16; off > 0; off >>= 1) ls += __shfl_down_sync(0xffffffffu, ls, off);
+  if (lane == 0) lred[warp] = ls;
+  __syncthreads();
+  if (tid == 0) {
+    float v = 0.f;
+    for (int k = 0; k < kRowWarps; ++k) v += lred[k];
+    part[blockIdx.x] = v;
+  }
+  // dH = dZ W, dZ of the layer below = dH GELU'(Z); the last layer's weights are in place
+  for (int l = 3; l >= 1; --l) {
+    const int din = L.din[l], dout = L.dout[l];
+    if (l < 3) w = stage_weights(W + L.woff[l], din * dout, sm);
+    auto put = [&](int i, int r, float v) {
+      const float g = v * gelu_grad(zs[((l - 1) * R + r) * LD + i]);
+      nxt[r * LD + i] = g;
+      if (r < nr) L.dz[l - 1][(long long)(b0 + r) * din + i] = g;
+    };
+    if ((din & 1) == 0 && ((uintptr_t)w & 3) == 0)
+      layer_backward<R, true>(cur, LD, w, din, dout, red, put);
+    else
+      layer_backward<R, false>(cur, LD, w, din, dout, red, put);
+    __syncthreads();
+    float *s = cur;
+    cur = nxt;
+    nxt = s;
+  }
+}
+
+struct AdamArgs {
+  int on;  // 0: write the gradients
+  float lr, b1, b2, eps, c1, c2;
+};
+
+__device__ __forceinline__ void adam_one(const AdamArgs &a, long long k, float g, float *w, float *m,
+                                         float *v, __nv_bfloat16 *wbf) {
+  const float mt = a.b1 * m[k] + (1.f - a.b1) * g;
+  const float vt = a.b2 * v[k] + (1.f - a.b2) * g * g;
+  m[k] = mt;
+  v[k] = vt;
+  const float wt = w[k] - a.lr * (mt / a.c1) / (sqrtf(vt / a.c2) + a.eps);
+  w[k] = wt;
+  wbf[k] = __float2bfloat16(wt);
+}
+
+// dW_l[o, i] = sum_b dZ_l[b, o] in_l[b, i] and db_l[o] = sum_b dZ_l[b, o] of every layer, one
+// 32 x 32 tile per block (first[l]: first block of layer l), followed by Adam or stored. Block
+// 0 also turns the loss partials into the loss.
+// Four groups of 256 threads share the rows, so that the latency of a tile's few hundred
+// additions is covered by 32 warps; their sums meet in shared memory in a fixed order (15 us at
+// 256 rows, 256 units; 28 us with one group).
+constexpr int kDwB = 32;      // rows per group and stage
+constexpr int kDwGroups = 4;
+__global__ void __launch_bounds__(256 * kDwGroups)
+    k_mlp_dw(int B, Layers L, int4 first, const float *__restrict__ x, float *__restrict__ grad,
+             float *__restrict__ w, float *__restrict__ m, float *__restrict__ v,
+             __nv_bfloat16 *__restrict__ wbf, AdamArgs ad, int npart, float *__restrict__ lossbuf,
+             double nout) {
+  __shared__ __align__(16) float zt[kDwGroups][kDwB][36];
+  __shared__ float at[kDwGroups][kDwB][33];
+  const int blk = blockIdx.x;
+  const int l = blk >= first.w ? 3 : (blk >= first.z ? 2 : (blk >= first.y ? 1 : 0));
+  const int t0 = blk - (l == 0 ? first.x : (l == 1 ? first.y : (l == 2 ? first.z : first.w)));
+  const int din = L.din[l], dout = L.dout[l], nti = (din + 31) / 32;
+  const int o0 = (t0 / nti) * 32, i0 = (t0 % nti) * 32;
+  const float *dz = L.dz[l], *in = l == 0 ? x : L.h[l - 1];
+  const int gr = threadIdx.x >> 8, tid = threadIdx.x & 255;
+  const int tx = tid & 31, ty = tid >> 5;  // the thread's outputs: i0 + tx; o0 + 4 ty + k
+  float acc[4] = {}, db = 0.f;
+  for (int b = 0; b < B; b += kDwB * kDwGroups) {
+#pragma unroll
+    for (int k = 0; k < kDwB / 8; ++k) {
+      const int r = ty + 8 * k, bb = b + gr * kDwB + r;
+      zt[gr][r][tx] = bb < B && o0 + tx < dout ? dz[(long long)bb * dout + o0 + tx] : 0.f;
+      at[gr][r][tx] = bb < B && i0 + tx < din ? in[(long long)bb * din + i0 + tx] : 0.f;
+    }
+    __syncthreads();
+    float s[4] = {};
+#pragma unroll 8
+    for (int r = 0; r < kDwB; ++r) {
+      const float a = at[gr][r][tx];
+      const float4 z = *reinterpret_cast<const float4 *>(&zt[gr][r][4 * ty]);
+      s[0] += z.x * a;
+      s[1] += z.y * a;
+      s[2] += z.z * a;
+      s[3] += z.w * a;
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) acc[k] += s[k];
+    if (i0 == 0 && ty == 0) {
+      float d = 0.f;
+#pragma unroll 8
+      for (int r = 0; r < kDwB; ++r) d += zt[gr][r][tx];
+      db += d;
+    }
+    __syncthreads();
+  }
+  // the groups' sums: [4 k + ty][tx] per group (zt's storage)
+  float *red = &zt[0][0][0];  // 3 x 32 x 33 floats of the 4 x 32 x 36
+  if (gr > 0) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) red[((gr - 1) * 32 + 4 * ty + k) * 33 + tx] = acc[k];
+    if (ty == 0) at[gr][0][tx] = db;
+  }
+  __syncthreads();
+  if (gr > 0) return;
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+#pragma unroll
+    for (int q = 0; q < kDwGroups - 1; ++q) acc[k] += red[(q * 32 + 4 * ty + k) * 33 + tx];
+  for (int q = 1; q < kDwGroups; ++q) db += at[q][0][tx];
+  auto put = [&](long long k, float g) {
+    if (ad.on)
+      adam_one(ad, k, g, w, m, v, wbf);
+    else
+      grad[k] = g;
+  };
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int o = o0 + 4 * ty + k, i = i0 + tx;
+    if (o < dout && i < din) put(L.woff[l] + (long long)o * din + i, acc[k]);
+  }
+  if (i0 == 0 && ty == 0 && o0 + tx < dout) put(L.boff[l] + o0 + tx, db);
+  if (blk == 0 && ty == 1) {
+    double s = 0.0;
+    for (int k = tx; k < npart; k += 32) s += lossbuf[k];
+    for (int off = 16; off > 0; off >>= 1) s += __shfl_down_sync(0xffffffffu, s, off);
+    if (tx == 0) lossbuf[npart] = (float)(s / nout);
+  }
+}
+
 template <typename TB>
 int prod(gc_context *ctx, int M, int N, int K, const float *A, long long sam, long long sak,
          const TB *B, long long sbn, long long sbk, float *C, long long ldc, const float *bias,
@@ -156,6 +502,74 @@ int ensure_act(gc_context *ctx, gc_mlp *m, int batch) {
   if (batch <= m->act_batch) return GC_OK;
   GC_TRY(m->act.alloc(ctx, layer_floats(m, batch) + 2 * (size_t)batch * max_width(m)));
   m->act_batch = batch;
+  return GC_OK;
+}
+
+bool fused(const gc_mlp *m) { return max_width(m) <= kFusedWidth; }
+
+// The layer table with H_l and dL/dZ_l in the activation workspace.
+int fused_layers(gc_context *ctx, gc_mlp *m, int B, Layers &L) {
+  GC_TRY(ensure_act(ctx, m, B));
+  float *p = m->act.p;
+  for (int l = 0; l < 4; ++l) {
+    L.din[l] = m->din[l];
+    L.dout[l] = m->dout[l];
+    L.woff[l] = (long long)m->woff[l];
+    L.boff[l] = (long long)m->boff[l];
+    L.dz[l] = p;
+    p += (size_t)m->act_batch * m->dout[l];
+    L.h[l] = p;
+    p += (size_t)m->act_batch * m->dout[l];
+  }
+  return GC_OK;
+}
+
+// Rows per block: 2 while that gives one block per SM at most (their shared memory leaves room for
+// one), 4 above.
+int fused_rows_per_block(int B) { return B <= 2 * 152 ? 2 : 4; }
+
+// Forward of x (y), or with t the loss partials and dL/dZ of every layer too.
+template <int R>
+int fused_rows(gc_context *ctx, gc_mlp *m, int B, const Layers &L, const float *x, const float *t,
+               float *y) {
+  static std::once_flag once;
+  static cudaError_t cfg = cudaSuccess;
+  std::call_once(once, [] {
+    cfg = cudaFuncSetAttribute(k_mlp_rows<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)rows_smem<R>());
+  });
+  GC_CUDA(ctx, cfg);
+  k_mlp_rows<R><<<gc::ceil_div(B, R), kRowThreads, rows_smem<R>(), ctx->stream>>>(
+      B, L, m->wbf.p, m->master.p, x, t, 1.f / (float)((long long)B * m->out), y, m->lossbuf.p);
+  GC_LAUNCHED(ctx);
+  return GC_OK;
+}
+int fused_rows(gc_context *ctx, gc_mlp *m, int B, const Layers &L, const float *x, const float *t,
+               float *y) {
+  return fused_rows_per_block(B) == 2 ? fused_rows<2>(ctx, m, B, L, x, t, y)
+                                      : fused_rows<4>(ctx, m, B, L, x, t, y);
+}
+
+// Loss (host, when asked for) and gradient of one batch, stored (ad.on = 0) or applied.
+int fused_step(gc_context *ctx, gc_mlp *m, int B, const float *x, const float *t, float *loss,
+               const AdamArgs &ad) {
+  Layers L;
+  GC_TRY(fused_layers(ctx, m, B, L));
+  const int nblk = gc::ceil_div(B, fused_rows_per_block(B));
+  if (m->lossbuf.n < (size_t)nblk + 1) GC_TRY(m->lossbuf.alloc(ctx, nblk + 1));
+  GC_TRY(fused_rows(ctx, m, B, L, x, t, nullptr));
+  int first[5] = {0};
+  for (int l = 0; l < 4; ++l)
+    first[l + 1] = first[l] + (int)(gc::ceil_div(L.dout[l], 32) * gc::ceil_div(L.din[l], 32));
+  k_mlp_dw<<<first[4], 256 * kDwGroups, 0, ctx->stream>>>(B, L, make_int4(first[0], first[1], first[2], first[3]), x,
+                                              m->grad.p, m->master.p, m->m1.p, m->m2.p, m->wbf.p, ad,
+                                              nblk, m->lossbuf.p, (double)B * m->out);
+  GC_LAUNCHED(ctx);
+  if (loss) {
+    GC_CUDA(ctx, cudaMemcpyAsync(loss, m->lossbuf.p + nblk, sizeof(float), cudaMemcpyDeviceToHost,
+                                 ctx->stream));
+    GC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  }
   return GC_OK;
 }
 
@@ -253,7 +667,7 @@ int gc_mlp_create(gc_context *ctx, int in_dim, int hidden, int out_dim, unsigned
   int r;
   if ((r = m->master.upload(ctx, h.data(), off)) != GC_OK || (r = m->grad.alloc(ctx, off)) != GC_OK ||
       (r = m->m1.alloc(ctx, off)) != GC_OK || (r = m->m2.alloc(ctx, off)) != GC_OK ||
-      (r = m->wbf.alloc(ctx, off)) != GC_OK) {
+      (r = m->wbf.alloc(ctx, off + 8)) != GC_OK) {
     delete m;
     return r;
   }
@@ -291,6 +705,11 @@ int gc_mlp_get_params(gc_context *ctx, gc_mlp *m, float *params_dev) {
 int gc_mlp_forward(gc_context *ctx, gc_mlp *m, int batch, const float *x_dev, float *y_dev) {
   if (!ctx || !m || batch <= 0 || !x_dev || !y_dev) return GC_EINVAL;
   float *Z[4], *H[4];
+  if (fused(m)) {
+    Layers L;
+    GC_TRY(fused_layers(ctx, m, batch, L));
+    return fused_rows(ctx, m, batch, L, x_dev, nullptr, y_dev);
+  }
   GC_TRY(forward(ctx, m, batch, x_dev, Z, H));
   GC_CUDA(ctx, cudaMemcpyAsync(y_dev, H[3], (size_t)batch * m->out * 4, cudaMemcpyDeviceToDevice,
                                ctx->stream));
@@ -300,7 +719,10 @@ int gc_mlp_forward(gc_context *ctx, gc_mlp *m, int batch, const float *x_dev, fl
 int gc_mlp_gradients(gc_context *ctx, gc_mlp *m, int batch, const float *x_dev, const float *t_dev,
                      float *grad_dev, float *loss_host) {
   if (!ctx || !m || batch <= 0 || !x_dev || !t_dev) return GC_EINVAL;
-  GC_TRY(loss_grad(ctx, m, batch, x_dev, t_dev, loss_host));
+  if (fused(m))
+    GC_TRY(fused_step(ctx, m, batch, x_dev, t_dev, loss_host, AdamArgs{}));
+  else
+    GC_TRY(loss_grad(ctx, m, batch, x_dev, t_dev, loss_host));
   if (grad_dev)
     GC_CUDA(ctx, cudaMemcpyAsync(grad_dev, m->grad.p, m->nparam * 4, cudaMemcpyDeviceToDevice,
                                  ctx->stream));
@@ -310,9 +732,16 @@ int gc_mlp_gradients(gc_context *ctx, gc_mlp *m, int batch, const float *x_dev, 
 int gc_mlp_train_step(gc_context *ctx, gc_mlp *m, int batch, const float *x_dev, const float *t_dev,
                       float lr, float *loss_host) {
   if (!ctx || !m || batch <= 0 || !x_dev || !t_dev || !(lr > 0.f)) return GC_EINVAL;
+  const float b1 = 0.9f, b2 = 0.999f;
+  if (fused(m)) {
+    const float s = (float)(m->step + 1);
+    GC_TRY(fused_step(ctx, m, batch, x_dev, t_dev, loss_host,
+                      AdamArgs{1, lr, b1, b2, 1e-8f, 1.f - std::pow(b1, s), 1.f - std::pow(b2, s)}));
+    m->step++;
+    return GC_OK;
+  }
   GC_TRY(loss_grad(ctx, m, batch, x_dev, t_dev, loss_host));
   m->step++;
-  const float b1 = 0.9f, b2 = 0.999f;
   float c1 = 1.f - std::pow(b1, (float)m->step), c2 = 1.f - std::pow(b2, (float)m->step);
   k_adam<<<std::min<unsigned>(gc::ceil_div(m->nparam, 256), 4096u), 256, 0, ctx->stream>>>(
       m->nparam, lr, b1, b2, 1e-8f, c1, c2, m->master.p, m->grad.p, m->m1.p, m->m2.p, m->wbf.p);

@@ -155,3 +155,32 @@ def test_integrand_tiles(gpu_lib, precision, n, nin, nact):
     w = api.ace_ne_erpa_fofo(t(y.T).t(), t(e), m["occ"], m["indn"], nact, nin, t(m["fofo"]),
                              precision=precision)
     assert abs(w - ref) < 5e-9
+
+
+# ragged row blocks, units that are no multiple of 8 or 32, wide outputs, and a layer beyond the
+# fused kernels' width
+@pytest.mark.parametrize("din,hid,dout,B", [(29, 256, 6, 5), (3, 37, 33, 1), (64, 8, 1, 307),
+                                            (5, 258, 3, 9)])
+def test_mlp_sizes(gpu_lib, din, hid, dout, B):
+    from oracle import mlp_ref
+    rng = np.random.default_rng(B)
+    net = api.Mlp(din, hid, dout, seed=2)
+    x = rng.standard_normal((B, din)).astype(np.float32)
+    y = rng.standard_normal((B, dout)).astype(np.float32)
+    p = net.params().cpu().numpy()
+    dims = [din, hid, hid, hid, dout]
+    ref, _, _ = mlp_ref.forward(p, dims, x)
+    assert np.abs(net.forward(x).cpu().numpy() - ref).max() < 1e-4 * np.abs(ref).max()
+    loss_ref, g_ref = mlp_ref.loss_and_grad(p, dims, x, y)
+    loss, g = net.gradients(x, y)
+    assert abs(loss - loss_ref) < 1e-4 * loss_ref
+    g, off = g.cpu().numpy(), 0
+    for l in range(4):
+        for size in (dims[l] * dims[l + 1], dims[l + 1]):
+            a, b = g[off:off + size], g_ref[off:off + size]
+            assert np.abs(a - b).max() < 1e-4 * max(np.abs(b).max(), 1e-12), (l, size)
+            off += size
+    # one Adam step from fresh moments moves every parameter by lr g / (|g| + eps)
+    assert abs(net.train_step(x, y, 1e-3) - loss) < 1e-5 * loss
+    step = p - net.params().cpu().numpy()
+    assert np.abs(step - 1e-3 * g / (np.abs(g) + 1e-8)).max() < 1e-6
