@@ -184,3 +184,29 @@ def test_mlp_sizes(gpu_lib, din, hid, dout, B):
     assert abs(net.train_step(x, y, 1e-3) - loss) < 1e-5 * loss
     step = p - net.params().cpu().numpy()
     assert np.abs(step - 1e-3 * g / (np.abs(g) + 1e-8)).max() < 1e-6
+
+
+# every pair of pair indices at most once (the one-pass road), and one repeated pair far away in
+# the input, beside it in a warp, or mirrored (the exact resolution)
+@pytest.mark.parametrize("fmt", ["pqrs", "dalton8", "dalton16"])
+@pytest.mark.parametrize("repeat", [None, "far", "near", "mirror"])
+@pytest.mark.parametrize("n", [1, 2, 9])
+def test_sort_single_and_repeated_pairs(gpu_lib, fmt, repeat, n):
+    from oracle import sorter_ref as S
+    rng = np.random.default_rng(n)
+    tri = [(a, b) for b in range(1, n + 1) for a in range(1, b + 1)]
+    lab = [(tri[x], tri[y]) for y in range(len(tri)) for x in range(y + 1) if rng.random() < 0.8 or n < 3]
+    if repeat == "far":
+        lab.append(lab[0])
+    elif repeat == "near":
+        lab.insert(1, lab[0])
+    elif repeat == "mirror":
+        lab.append((lab[-1][1], lab[-1][0]))
+    p, q, r, s = (np.array([x[i][j] for x in lab]) for i in (0, 1) for j in (0, 1))
+    lab = {"pqrs": lambda: np.stack([p, q, r, s], 1).ravel(),
+           "dalton8": lambda: p | q << 8 | r << 16 | s << 24,
+           "dalton16": lambda: np.stack([r | s << 16, p | q << 16], 1).ravel()}[fmt]()
+    lab = lab.astype(np.uint32).view(np.int32)
+    vals = rng.standard_normal(len(p))
+    got = api.readtwoint(n, torch.as_tensor(vals, device=DEV), torch.as_tensor(lab, device=DEV), fmt)
+    assert np.array_equal(got.cpu().numpy(), S.readtwoint(n, vals, lab, fmt))
