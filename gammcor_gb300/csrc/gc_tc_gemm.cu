@@ -147,8 +147,8 @@ __device__ __forceinline__ void mma_bf16(uint32_t tmem, uint64_t ad, uint64_t bd
 }
 
 // As mma_bf16, with a use of the A collector buffer: C = 1 reads A from shared memory
-// and keeps it in the buffer, 2 reads the buffer, 3 reads it and releases it, 0
-// discards it (the plain form). The same A descriptor is given with every use.
+// and keeps it in the buffer, 3 reads the buffer and releases it, 0 discards it (the
+// plain form). The same A descriptor is given with both uses.
 template <int C>
 __device__ __forceinline__ void mma_bf16_ca(uint32_t tmem, uint64_t ad, uint64_t bd,
                                             uint32_t idesc, uint32_t accumulate) {
@@ -157,12 +157,6 @@ __device__ __forceinline__ void mma_bf16_ca(uint32_t tmem, uint64_t ad, uint64_t
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::f16.collector::a::fill [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem),
-        "l"(ad), "l"(bd), "r"(idesc), "r"(accumulate));
-  else if constexpr (C == 2)
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16.collector::a::use [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem),
         "l"(ad), "l"(bd), "r"(idesc), "r"(accumulate));
   else if constexpr (C == 3)
     asm volatile(
@@ -401,6 +395,32 @@ struct OzEpi {
                          // tri_period-wide column block (C lower-triangular per block)
 };
 
+// t 2^sc as ldexp((double)t, sc) gives it (t rounded to nearest even), by integer operations:
+// with one FP64 conversion and one FP64 scaling per element the narrow FP64 pipe took 12 us per
+// 128 x 96 tile, as long as the products of K = 256.
+__device__ __forceinline__ double scaled_double(long long t, int sc) {
+  const unsigned long long u = t < 0 ? 0ull - (unsigned long long)t : (unsigned long long)t;
+  if (u == 0) return 0.0;
+  const int e = 63 - __clzll((long long)u);
+  const int E = e + sc + 1023;
+  if (E < 1 || E > 2045) {  // subnormal, overflow or next to it: exact steps, one rounding
+    double x = (double)t;
+    for (; sc < -1000; sc += 1000) x *= 0x1p-1000;
+    for (; sc > 1000; sc -= 1000) x *= 0x1p1000;
+    return x * __longlong_as_double((long long)(sc + 1023) << 52);
+  }
+  unsigned long long m;  // 2^52 <= m <= 2^53
+  if (e <= 52) {
+    m = u << (52 - e);
+  } else {
+    const int sh = e - 52;
+    m = (u + ((1ull << (sh - 1)) - 1) + ((u >> sh) & 1)) >> sh;
+  }
+  // m = 2^53 carries into the exponent
+  const unsigned long long b = ((unsigned long long)E << 52) + (m - (1ull << 52));
+  return __longlong_as_double((long long)(b | (t < 0 ? 1ull << 63 : 0ull)));
+}
+
 template <int S, int TBN>
 __global__ void __launch_bounds__(oz_threads(TBN), 1)
     k_tc_gemm_oz(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
@@ -497,7 +517,6 @@ __global__ void __launch_bounds__(oz_threads(TBN), 1)
       for (int j = (issued > OZ_STAGES ? issued - OZ_STAGES : 0); j < issued; ++j)
         mbar_wait(&full[j % OZ_STAGES], (j / OZ_STAGES) & 1, kDrainNs);
   } else if (warp == 1 && lane == 0) {
-    constexpr uint32_t idesc = instr_desc(TBN);
     bool ok = true;
     for (int g = 0; g < nchunks && ok; ++g) {
       if (g > 0 && !mbar_wait(acce, (g - 1) & 1, wait_ns)) {
@@ -515,29 +534,34 @@ __global__ void __launch_bounds__(oz_threads(TBN), 1)
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t a_base = smem_u32(smem + s * STAGE_BYTES);
         const uint32_t b_base = a_base + S * A_BYTES;
-        // A slice t at K step kk meets the B slices u < S - t back to back, so it is
-        // read from shared memory once and then from the collector buffer. The first
-        // product into weight t+u in the chunk is (0, t+u) at kb0, kk 0.
+        // A slice t meets the B slices u < S - t, which lie one after the other in shared
+        // memory and accumulate into consecutive weights t + u: one product of A slice t with
+        // all of them, (S - t) TBN columns wide (two of equal width above 256). The first
+        // product into every weight of the chunk is t = 0 at kb0, kk 0. With one instruction
+        // per slice product an instruction took about 80 cycles whatever TBN (48 at the tensor
+        // rate for TBN = 96): its A tile alone is 32 cycles of shared-memory reads. At 6290^3
+        // 5.29 -> 4.62 ms (FP64TC5), 4.38 ms with the cheaper epilogue.
 #pragma unroll
-        for (int t = 0; t < S; ++t)
+        for (int t = 0; t < S; ++t) {
+          constexpr int kMaxN = 256;
 #pragma unroll
           for (int kk = 0; kk < OZ_BK / 16; ++kk) {
             const uint64_t ad = smem_desc64(a_base + t * A_BYTES + kk * 32);
             const uint32_t acc_in = (kb == kb0 && t == 0 && kk == 0) ? 0u : 1u;
-            if (t == S - 1) {
-              mma_bf16_ca<0>(tmem + (uint32_t)(t * TBN), ad, smem_desc64(b_base + kk * 32), idesc,
+            const int cols = (S - t) * TBN;
+            if (cols <= kMaxN) {
+              mma_bf16_ca<0>(tmem + (uint32_t)(t * TBN), ad, smem_desc64(b_base + kk * 32),
+                             instr_desc(cols), acc_in);
+            } else {
+              const int half = cols / 2;
+              mma_bf16_ca<1>(tmem + (uint32_t)(t * TBN), ad, smem_desc64(b_base + kk * 32),
+                             instr_desc(half), acc_in);
+              mma_bf16_ca<3>(tmem + (uint32_t)(t * TBN + half), ad,
+                             smem_desc64(b_base + half * (OZ_BK * 2) + kk * 32), instr_desc(half),
                              acc_in);
-              continue;
             }
-            mma_bf16_ca<1>(tmem + (uint32_t)(t * TBN), ad, smem_desc64(b_base + kk * 32), idesc,
-                           acc_in);
-#pragma unroll
-            for (int u = 1; u + t < S - 1; ++u)
-              mma_bf16_ca<2>(tmem + (uint32_t)((t + u) * TBN), ad,
-                             smem_desc64(b_base + u * B_BYTES + kk * 32), idesc, acc_in);
-            mma_bf16_ca<3>(tmem + (uint32_t)((S - 1) * TBN), ad,
-                           smem_desc64(b_base + (S - 1 - t) * B_BYTES + kk * 32), idesc, acc_in);
           }
+        }
         mma_commit(&empty[s]);
       }
       mma_commit(accf);
@@ -549,12 +573,13 @@ __global__ void __launch_bounds__(oz_threads(TBN), 1)
     mma_commit(drainb);
     if (!mbar_wait(drainb, 0, kDrainNs)) atomicExch(&abort_flag, 1);
   } else if (warp >= 2) {
-    // Every chunk's FP32 sums are integers below 2^24, so the weights fold into one
-    // int64 per column by Horner in base 2^7: t = sum_d v_d 2^(7 (SI - 1 - d)) is exact
-    // for the first SI = min(S, 5) weights (|t| < 2^52 per chunk); a sixth weight is
-    // rounded to units of 2^7 first (2^-42 of the scaled product, below FP64 rounding
-    // of the result). The int64 sum over chunks is converted to FP64 once, at the end:
-    // the per-chunk work is integer, not FP64, arithmetic.
+    // Every chunk's FP32 sums v_d are integers below 2^24, so the weights fold into one int64
+    // per column, t = sum_d v_d 2^(7 (SI - 1 - d)), exact for the first SI = min(S, 5) weights
+    // (|t| < 2^52 per chunk); a sixth weight is rounded to units of 2^7 first (2^-42 of the
+    // scaled product, below FP64 rounding of the result). Two weights at a time fit 32 bits
+    // (128 |v_0| + |v_1| and 128 |v_2| + |v_3| are below 2^31: v_0 sums products up to 2^14, v_2
+    // up to 2 2^13 + 2^12, over at most 672 K), and two 32 x 32 + 64 multiply-adds put the pairs
+    // in place: the MMAs of the next chunk wait for this.
     // Four warps per 32 columns (one per TMEM lane quarter, q = warp % 4); warp group
     // h = (warp - 2) / 4 owns columns [32 h, 32 h + 32) of the tile.
     constexpr int SI = S < 5 ? S : 5;
@@ -582,13 +607,21 @@ __global__ void __launch_bounds__(oz_threads(TBN), 1)
         tmem_ld_wait();
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-          long long t = 0;
+          int v[S];
 #pragma unroll
-          for (int d = 0; d < SI; ++d) t = t * 128 + (long long)__float2int_rn(__uint_as_float(r[d][j]));
-#pragma unroll
-          for (int d = SI; d < S; ++d)
-            t += (long long)__float2int_rn(__uint_as_float(r[d][j]) * exp2f(-7.0f * (d - SI + 1)));
-          acc[c0 + j] += t;
+          for (int d = 0; d < SI; ++d) v[d] = __float2int_rn(__uint_as_float(r[d][j]));
+          if (S > SI) v[SI - 1] += __float2int_rn(__uint_as_float(r[S - 1][j]) * 0.0078125f);
+          const int p0 = v[0] * 128 + v[1], p1 = v[2] * 128 + v[3];
+          long long t = acc[c0 + j];
+          if (SI == 5) {
+            t += (long long)p0 * (1 << 21);
+            t += (long long)p1 * 128;
+            t += v[SI - 1];
+          } else {
+            t += (long long)p0 * (1 << 14);
+            t += p1;
+          }
+          acc[c0 + j] = t;
         }
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -606,7 +639,7 @@ __global__ void __launch_bounds__(oz_threads(TBN), 1)
         if (n < N) {
           const int eb = epi.eb[(long long)b * epi.eb_sb + n];
           double cv = (ea == kBadExp || eb == kBadExp) ? __longlong_as_double(0x7ff8000000000000ll)
-                                                       : ldexp((double)acc[j], er + eb);
+                                                       : scaled_double(acc[j], er + eb);
           long long o = (long long)b * epi.sb + m + (long long)n * epi.ldn;
           if (epi.mode == 0)
             epi.c[o] = cv;
@@ -1335,11 +1368,12 @@ static_assert(oz_smem_bytes(4, 128) <= 232448 && oz_smem_bytes(5, 96) <= 232448 
                   oz_smem_bytes(6, 64) <= 232448,
               "sliced GEMM stages exceed the 227 KB of shared memory per CTA");
 
-// Relative time per CTA of each tile width (one CTA per SM at a time), measured at
-// 6290^3 on GB300 (ms per wave of 152 CTAs: FP64TC5 0.227 at 64 and 0.240 at 96;
-// FP64TC4 0.171, 0.183 and 0.201 at 64, 96 and 128). A CTA's time is set by the
-// operand bytes it moves, so a wider tile costs little more per CTA.
-constexpr double kOzTileCost64 = 1.0, kOzTileCost96 = 1.06, kOzTileCost128 = 1.18;
+// Relative time per CTA of the wider tiles (one CTA per SM at a time), measured at 6290^3 on
+// GB300 (ms per wave of 152 CTAs: FP64TC5 0.152 at 64 and 0.199 at 96; FP64TC4 0.124, 0.148 and
+// 0.175 at 64, 96 and 128).
+constexpr double oz_tile_cost(int S, int tbn) {
+  return tbn == 64 ? 1.0 : (tbn == 96 ? (S == 4 ? 1.19 : 1.30) : 1.41);
+}
 
 // Tile width for an M x N x nbatch product: the narrowest width unless a wider one
 // finishes its CTA waves (152 SMs, one CTA each) sooner by the costs above.
@@ -1350,8 +1384,7 @@ int oz_tile(const gc_context *ctx, int S, long long M, long long N, long long nb
   double best_cost = 0.0;
   for (int tbn = 64; tbn <= widest; tbn += 32) {
     const long long ctas = (M + BM - 1) / BM * ((N + tbn - 1) / tbn) * nbatch;
-    const double cost = (double)((ctas + 151) / 152) *
-                        (tbn == 64 ? kOzTileCost64 : (tbn == 96 ? kOzTileCost96 : kOzTileCost128));
+    const double cost = (double)((ctas + 151) / 152) * oz_tile_cost(S, tbn);
     if (tbn == 64 || cost < best_cost) {
       best = tbn;
       best_cost = cost;
