@@ -395,30 +395,27 @@ struct OzEpi {
                          // tri_period-wide column block (C lower-triangular per block)
 };
 
-// t 2^sc as ldexp((double)t, sc) gives it (t rounded to nearest even), by integer operations:
-// with one FP64 conversion and one FP64 scaling per element the narrow FP64 pipe took 12 us per
-// 128 x 96 tile, as long as the products of K = 256.
+// t 2^sc where the result is subnormal, overflows or is next to it: exact steps, one rounding.
+__device__ __noinline__ double scaled_double_edge(long long t, int sc) {
+  double x = (double)t;
+  for (; sc < -1000; sc += 1000) x *= 0x1p-1000;
+  for (; sc > 1000; sc -= 1000) x *= 0x1p1000;
+  return x * __longlong_as_double((long long)(sc + 1023) << 52);
+}
+
+// t 2^sc as ldexp((double)t, sc) gives it (t rounded to nearest even), by integer operations
+// without a branch: with an FP64 conversion and an FP64 scaling per element the narrow FP64
+// pipe took 12 us per 128 x 96 tile, as long as the products of K = 256.
 __device__ __forceinline__ double scaled_double(long long t, int sc) {
   const unsigned long long u = t < 0 ? 0ull - (unsigned long long)t : (unsigned long long)t;
-  if (u == 0) return 0.0;
-  const int e = 63 - __clzll((long long)u);
-  const int E = e + sc + 1023;
-  if (E < 1 || E > 2045) {  // subnormal, overflow or next to it: exact steps, one rounding
-    double x = (double)t;
-    for (; sc < -1000; sc += 1000) x *= 0x1p-1000;
-    for (; sc > 1000; sc -= 1000) x *= 0x1p1000;
-    return x * __longlong_as_double((long long)(sc + 1023) << 52);
-  }
-  unsigned long long m;  // 2^52 <= m <= 2^53
-  if (e <= 52) {
-    m = u << (52 - e);
-  } else {
-    const int sh = e - 52;
-    m = (u + ((1ull << (sh - 1)) - 1) + ((u >> sh) & 1)) >> sh;
-  }
-  // m = 2^53 carries into the exponent
-  const unsigned long long b = ((unsigned long long)E << 52) + (m - (1ull << 52));
-  return __longlong_as_double((long long)(b | (t < 0 ? 1ull << 63 : 0ull)));
+  const int lz = __clzll((long long)u);
+  const int E = 63 - lz + sc + 1023;
+  if (u != 0 && (E < 1 || E > 2045)) return scaled_double_edge(t, sc);
+  const unsigned long long v = u << (lz & 63);  // leading bit at 63 (u != 0)
+  const unsigned long long m = v >> 11;         // 53 bits; rounding may carry into the exponent
+  const unsigned long long up = ((v & 0x7ff) + 0x3ff + (m & 1)) >> 11;
+  const unsigned long long b = ((unsigned long long)E << 52) + (m - (1ull << 52)) + up;
+  return u == 0 ? 0.0 : __longlong_as_double((long long)(b | ((unsigned long long)t & (1ull << 63))));
 }
 
 template <int S, int TBN>
@@ -482,6 +479,16 @@ __global__ void __launch_bounds__(oz_threads(TBN), 1)
     mbar_init(drainb, 1);
     abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  // The exponents of the tile's rows and columns, read while the pipeline starts: read one by
+  // one between the stores of the result (which the compiler cannot move loads across) each
+  // column waits for a load.
+  __shared__ int eb_s[TBN];
+  int ea = 0;
+  if (warp >= 2) {
+    const int t = threadIdx.x - 64, m = m0 + (warp & 3) * 32 + lane;
+    if (t < TBN) eb_s[t] = n0 + t < N ? epi.eb[(long long)b * epi.eb_sb + n0 + t] : 0;
+    if (m < M) ea = epi.ea[(long long)b * epi.ea_sb + m];
   }
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
@@ -631,28 +638,48 @@ __global__ void __launch_bounds__(oz_threads(TBN), 1)
     if (!ok) atomicExch(&abort_flag, 1);
     double dot = 0.0;
     if (ok && m < M) {
-      const int ea = epi.ea[(long long)b * epi.ea_sb + m];
       const int er = ea - 7 * (SI + 1);
+      const long long o0 = (long long)b * epi.sb + m + (long long)(n0 + h * NC) * epi.ldn;
+      // FP64 results first, then one short loop per mode: a tile runs this code once, so its
+      // length counts (this part of a 128 x 64 tile: 6.7 us as one unrolled loop over modes and
+      // edge cases, 4.1 us so).
+      double cv[NC];
 #pragma unroll
       for (int j = 0; j < NC; ++j) {
-        int n = n0 + h * NC + j;
-        if (n < N) {
-          const int eb = epi.eb[(long long)b * epi.eb_sb + n];
-          double cv = (ea == kBadExp || eb == kBadExp) ? __longlong_as_double(0x7ff8000000000000ll)
-                                                       : scaled_double(acc[j], er + eb);
-          long long o = (long long)b * epi.sb + m + (long long)n * epi.ldn;
-          if (epi.mode == 0)
-            epi.c[o] = cv;
-          else if (epi.mode == 2) {
-            if (m >= n) epi.c[o] -= cv;
-          } else if (epi.mode == 3) {
-            if (m >= n) {
-              epi.c[o] = cv;
-              epi.c[n + (long long)m * epi.ldn] = cv;  // 32 consecutive per thread
-            }
-          } else if (epi.mode == 1 || m > n) {
-            dot += cv * epi.r[o];
+        const int eb = eb_s[h * NC + j];
+        const double v = scaled_double(acc[j], eb == kBadExp || ea == kBadExp ? 0 : er + eb);
+        cv[j] = eb == kBadExp || ea == kBadExp ? __longlong_as_double(0x7ff8000000000000ll) : v;
+      }
+      const int n1 = n0 + h * NC, nn = min(NC, N - n1);
+      if (epi.mode == 0) {
+#pragma unroll
+        for (int j = 0; j < NC; ++j)
+          if (j < nn) epi.c[o0 + j * epi.ldn] = cv[j];
+      } else if (epi.mode == 3) {
+        double *mir = epi.c + n1 + (long long)m * epi.ldn;  // 32 consecutive per thread
+#pragma unroll
+        for (int j = 0; j < NC; ++j)
+          if (j < nn && m >= n1 + j) {
+            epi.c[o0 + j * epi.ldn] = cv[j];
+            mir[j] = cv[j];
           }
+      } else {
+        const double *src = epi.mode == 2 ? epi.c : epi.r;
+        // last column of this row: all (1), up to the diagonal (2), below it (4)
+        const int last = epi.mode == 1 ? nn : min(nn, m - n1 + (epi.mode == 2 ? 1 : 0));
+#pragma unroll
+        for (int j0 = 0; j0 < NC; j0 += 8) {  // the loads of a group before its stores
+          double old[8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) old[j] = j0 + j < last ? src[o0 + (j0 + j) * epi.ldn] : 0.0;
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            if (j0 + j < last) {
+              if (epi.mode == 2)
+                epi.c[o0 + (j0 + j) * epi.ldn] = old[j] - cv[j0 + j];
+              else
+                dot += cv[j0 + j] * old[j];
+            }
         }
       }
     }
@@ -1369,10 +1396,10 @@ static_assert(oz_smem_bytes(4, 128) <= 232448 && oz_smem_bytes(5, 96) <= 232448 
               "sliced GEMM stages exceed the 227 KB of shared memory per CTA");
 
 // Relative time per CTA of the wider tiles (one CTA per SM at a time), measured at 6290^3 on
-// GB300 (ms per wave of 152 CTAs: FP64TC5 0.152 at 64 and 0.199 at 96; FP64TC4 0.124, 0.148 and
-// 0.175 at 64, 96 and 128).
+// GB300 (ms per wave of 152 CTAs: FP64TC5 0.149 at 64 and 0.196 at 96; FP64TC4 0.122, 0.145 and
+// 0.174 at 64, 96 and 128).
 constexpr double oz_tile_cost(int S, int tbn) {
-  return tbn == 64 ? 1.0 : (tbn == 96 ? (S == 4 ? 1.19 : 1.30) : 1.41);
+  return tbn == 64 ? 1.0 : (tbn == 96 ? (S == 4 ? 1.19 : 1.31) : 1.43);
 }
 
 // Tile width for an M x N x nbatch product: the narrowest width unless a wider one
