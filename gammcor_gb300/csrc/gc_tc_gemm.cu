@@ -1570,8 +1570,6 @@ int tc_pair_product(gc_context *ctx, int precision, int rank, int nC, int nD, bo
 int tc_two_sided(gc_context *ctx, int precision, int n, int cnt, const double *M, int nX,
                  const double *CX, int nY, const double *CY, double *T1, double *out,
                  long long ostride) {
-  if (precision == GC_PREC_FP64)
-    return fp64_two_sided(ctx, n, cnt, M, nX, CX, nY, CY, T1, out, ostride);
   int S;
   PassList pl = pass_list(precision, &S);
   // step 1: T1[(k,q), x] = sum_p M_k[p, q] CX[p, x]   (T1 column-major, ld = n*cnt)

@@ -31,7 +31,7 @@ int tc_half_packed(gc_context *ctx, int precision, int n, int cnt, const double 
 int tc_pair_product(gc_context *ctx, int precision, int rank, int nC, int nD, bool symCD,
                     const double *Z, int nA, int nB, bool symAB, const double *Y, double *out);
 
-// FP64 and split-BF16 precisions: out_k (nX x nY, column-major, stride ostride) = CX^T M_k CY for cnt
+// Split-BF16 precisions: out_k (nX x nY, column-major, stride ostride) = CX^T M_k CY for cnt
 // column-major n x n matrices M_k; T1 is scratch of cnt*n*max(nX) doubles.
 int tc_two_sided(gc_context *ctx, int precision, int n, int cnt, const double *M, int nX,
                  const double *CX, int nY, const double *CY, double *T1, double *out,
@@ -72,8 +72,5 @@ int tc_gemm_strided_lower(gc_context *ctx, int precision, int M, int N, int K, c
 // b*sb from the base pointers.
 int tc_syrk_sub_lower(gc_context *ctx, int precision, int M, int K, const double *P, long long sm,
                       long long sk, double *C, long long ldc, int nbatch = 1, long long sb = 0);
-
-int fp64_two_sided(gc_context *ctx, int n, int cnt, const double *M, int nX, const double *CX,
-                   int nY, const double *CY, double *T1, double *out, long long ostride);
 
 }  // namespace gc

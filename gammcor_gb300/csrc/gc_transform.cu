@@ -10,13 +10,16 @@
 // gc_tran4_factored produces the same records from the ERI factor L:
 // B_P = CA^T L_P CB for every P, then (ab|cd) = sum_P B_P(ab) B'_P(cd).
 //
-// In the sliced precisions the packed triangles are the operands themselves
-// (tc_half_packed), and a block of orbitals given twice (the same pointer and
-// width) makes its pair index symmetric (tc_pair_product).
+// In FP64 and in the sliced precisions the packed triangles are the operands
+// themselves (half_fp64, tc_half_packed); in the sliced ones a block of orbitals
+// given twice (the same pointer and width) makes its pair index symmetric
+// (tc_pair_product). The split-BF16 precisions expand the triangles.
 #include "gc_internal.cuh"
 #include "gc_tc_gemm.cuh"
 
 namespace {
+
+const size_t kChunkBytes = size_t(1) << 30;  // staging per chunk
 
 __host__ __device__ inline long long tri_pack(int p, int q) {  // p <= q, 0-based
   return (long long)p + (long long)q * (q + 1) / 2;
@@ -99,18 +102,85 @@ __global__ void unpack_factor(const double *__restrict__ L, long long ntr, int n
   }
 }
 
-// Two-sided transform of cnt column-major n x n matrices M_k:
-// out_k (nX x nY, column-major, stride ostride) = CX^T M_k CY.
-int two_sided(gc_context *ctx, int n, int cnt, const double *M, int nX, const double *CX, int nY,
-              const double *CY, double *T1, double *out, long long ostride) {
+// T[p + n (f + nf k)] = sum_q M_k(p, q) C[q + n f] in FP64 for symmetric n x n matrices given by
+// their packed triangles (M_k at M + k ld, element (p, q), p <= q, at p + q (q + 1) / 2). A warp
+// takes 32 rows p and FB columns f of one matrix. Bound by the FP64 pipe (64 cycles per warp
+// instruction and quarter of an SM): the triangle is read in place, element by element, since
+// even its uncoalesced half (q < p: a sector per lane, four q long) hides behind FB FMAs.
+// Measured for the AOTWOSORT transform at n = 64, nocc = 10: 0.21 ms in two launches (85% of the
+// pipe's rate); the whole call 2.28 -> 0.53 ms, of which DGEMM takes 0.30.
+template <int FB>
+__global__ void __launch_bounds__(128) k_half_fp64(int n, int cnt, int nf, int ngf,
+                                                   const double *__restrict__ M, long long ld,
+                                                   const double *__restrict__ C,
+                                                   double *__restrict__ T) {
+  const int lane = threadIdx.x & 31, nch = (n + 31) / 32;
+  const long long items = (long long)cnt * nch * ngf;
+  for (long long w = (blockIdx.x * 128ll + threadIdx.x) >> 5; w < items; w += gridDim.x * 4ll) {
+    const int g = (int)(w % ngf), ch = (int)((w / ngf) % nch);
+    const long long k = w / ((long long)ngf * nch);
+    const int p = ch * 32 + lane, f0 = g * FB;
+    const int pc = min(p, n - 1);  // lanes beyond n repeat the last row
+    const double *__restrict__ m = M + k * ld;
+    const double *__restrict__ row = m + (long long)pc * (pc + 1) / 2;
+    const double *__restrict__ c[FB];
+#pragma unroll
+    for (int f = 0; f < FB; ++f) c[f] = C + (long long)min(f0 + f, nf - 1) * n;
+    double acc[FB] = {};
+#pragma unroll 4
+    for (int q = 0; q < n; ++q) {
+      const double v = q <= pc ? row[q] : m[pc + (long long)q * (q + 1) / 2];
+#pragma unroll
+      for (int f = 0; f < FB; ++f) acc[f] = fma(v, c[f][q], acc[f]);
+    }
+    if (p < n)
+#pragma unroll
+      for (int f = 0; f < FB; ++f)
+        if (f0 + f < nf) T[p + n * (f0 + f + (long long)nf * k)] = acc[f];
+  }
+}
+
+// out_k = CX^T M_k CY (nX x nY, column-major, consecutive) for cnt such matrices in FP64: the
+// narrower block first (k_half_fp64), the other one by one DGEMM over all matrices (batched where
+// the first block is CX).
+int half_fp64(gc_context *ctx, int n, long long cnt, const double *M, int nX, const double *CX,
+              int nY, const double *CY, double *out) {
+  const bool y1 = nY <= nX;
+  const int nf = y1 ? nY : nX;
+  // at most 8 columns per thread, shared out evenly
+  const int ngf = (nf + 7) / 8, fb = (nf + ngf - 1) / ngf;
+  const long long ld = (long long)n * (n + 1) / 2;
+  const int cs = (int)std::max<long long>(
+      1, std::min<long long>({cnt, (long long)kChunkBytes / (8ll * n * nf), 0x7fffffffll / ((long long)n * nf)}));
+  gc::DevBuf<double> T;
+  GC_TRY(T.alloc(ctx, (size_t)cs * n * nf));
   const double one = 1.0, zero = 0.0;
-  // T1 (nX x n*cnt) = CX^T . [M_0 | M_1 | ...]
-  GC_CUBLAS(ctx, cublasDgemm(ctx->cublas, CUBLAS_OP_T, CUBLAS_OP_N, nX, n * cnt, n, &one, CX, n, M,
-                             n, &zero, T1, nX));
-  // out_k = T1_k . CY
-  GC_CUBLAS(ctx, cublasDgemmStridedBatched(ctx->cublas, CUBLAS_OP_N, CUBLAS_OP_N, nX, nY, n, &one,
-                                           T1, nX, (long long)nX * n, CY, n, 0, &zero, out, nX,
-                                           ostride, cnt));
+  for (long long k0 = 0; k0 < cnt; k0 += cs) {
+    const int c = (int)std::min<long long>(cs, cnt - k0);
+    const long long items = (long long)c * ((n + 31) / 32) * ngf;
+    const unsigned grid = (unsigned)std::min<long long>((items + 3) / 4, 152 * 256);
+    const double *Mk = M + k0 * ld, *Cf = y1 ? CY : CX;
+    auto go = [&](auto kern) { kern<<<grid, 128, 0, ctx->stream>>>(n, c, nf, ngf, Mk, ld, Cf, T.p); };
+    switch (fb) {
+      case 1: go(k_half_fp64<1>); break;
+      case 2: go(k_half_fp64<2>); break;
+      case 3: go(k_half_fp64<3>); break;
+      case 4: go(k_half_fp64<4>); break;
+      case 5: go(k_half_fp64<5>); break;
+      case 6: go(k_half_fp64<6>); break;
+      case 7: go(k_half_fp64<7>); break;
+      default: go(k_half_fp64<8>);
+    }
+    GC_LAUNCHED(ctx);
+    double *o = out + k0 * nX * nY;
+    if (y1)
+      GC_CUBLAS(ctx, cublasDgemm(ctx->cublas, CUBLAS_OP_T, CUBLAS_OP_N, nX, c * nY, n, &one, CX, n, T.p,
+                                 n, &zero, o, nX));
+    else
+      GC_CUBLAS(ctx, cublasDgemmStridedBatched(ctx->cublas, CUBLAS_OP_T, CUBLAS_OP_N, nX, nY, n, &one,
+                                               T.p, n, (long long)n * nX, CY, n, 0, &zero, o, nX,
+                                               (long long)nX * nY, c));
+  }
   return GC_OK;
 }
 
@@ -121,8 +191,6 @@ int check_dims(gc_context *ctx, int nbas, int nA, int nB, int nC, int nD) {
                          nbas, nA, nB, nC, nD);
   return GC_OK;
 }
-
-const size_t kChunkBytes = size_t(1) << 30;  // unpacked-matrix staging per chunk
 
 }  // namespace
 
@@ -140,9 +208,15 @@ extern "C" int gc_tran4_gen(gc_context *ctx, int nbas, int nA, const double *CA,
   const long long n2 = (long long)n * n;
   gc::DevBuf<double> H, M, T1;
   GC_TRY(H.alloc(ctx, ntr * nAB));
-  if (gc::is_sliced(precision)) {
-    const gc::HalfOut ab{nA, CA, nB, CB, H.p};
-    GC_TRY(gc::tc_half_packed(ctx, precision, n, (int)ntr, G, ntr, 1, &ab));
+  const bool sliced = gc::is_sliced(precision);
+  if (sliced || precision == GC_PREC_FP64) {
+    auto half = [&](int cnt, const double *packed, int nX, const double *CX, int nY, const double *CY,
+                    double *o) -> int {
+      if (!sliced) return half_fp64(ctx, n, cnt, packed, nX, CX, nY, CY, o);
+      const gc::HalfOut h{nX, CX, nY, CY, o};
+      return gc::tc_half_packed(ctx, precision, n, cnt, packed, ntr, 1, &h);
+    };
+    GC_TRY(half((int)ntr, G, nA, CA, nB, CB, H.p));
     const int cs = (int)std::max<long long>(1, std::min<long long>(nAB, kChunkBytes / (8 * ntr)));
     GC_TRY(M.alloc(ctx, (size_t)cs * ntr));
     for (long long c0 = 0; c0 < nAB; c0 += cs) {
@@ -150,10 +224,9 @@ extern "C" int gc_tran4_gen(gc_context *ctx, int nbas, int nA, const double *CA,
       transpose_columns<<<dim3(gc::ceil_div(ntr, 32), gc::ceil_div(cnt, 32)), dim3(32, 8), 0,
                           ctx->stream>>>(H.p, ntr, nAB, c0, cnt, M.p);
       GC_LAUNCHED(ctx);
-      const gc::HalfOut cd{nC, CC, nD, CD, out + c0 * nCD};
-      GC_TRY(gc::tc_half_packed(ctx, precision, n, cnt, M.p, ntr, 1, &cd));
+      GC_TRY(half(cnt, M.p, nC, CC, nD, CD, out + c0 * nCD));
     }
-    return gc::check_flag(ctx);
+    return sliced ? gc::check_flag(ctx) : GC_OK;
   }
   int cs = (int)std::max<long long>(1, std::min<long long>(ntr, kChunkBytes / (8 * n2)));
   GC_TRY(M.alloc(ctx, (size_t)cs * n2));
@@ -175,7 +248,7 @@ extern "C" int gc_tran4_gen(gc_context *ctx, int nbas, int nA, const double *CA,
     GC_LAUNCHED(ctx);
     GC_TRY(gc::tc_two_sided(ctx, precision, n, cnt, M.p, nC, CC, nD, CD, T1.p, out + c0 * nCD, nCD));
   }
-  return precision == GC_PREC_FP64 ? GC_OK : gc::check_flag(ctx);
+  return gc::check_flag(ctx);
 }
 
 extern "C" int gc_tran4_factored(gc_context *ctx, int nbas, int rank, const double *L, int nA,
@@ -203,9 +276,15 @@ extern "C" int gc_tran4_factored(gc_context *ctx, int nbas, int rank, const doub
     return gc::check_flag(ctx);
   }
   int cs = (int)std::max<long long>(1, std::min<long long>(rank, kChunkBytes / (8 * n2)));
-  GC_TRY(M.alloc(ctx, (size_t)cs * n2));
-  GC_TRY(T1.alloc(ctx, (size_t)cs * n * std::max(nA, nC)));
-  for (int P0 = 0; P0 < rank; P0 += cs) {
+  if (precision == GC_PREC_FP64) {
+    GC_TRY(half_fp64(ctx, n, rank, L, nA, CA, nB, CB, Y.p));
+    if (!same) GC_TRY(half_fp64(ctx, n, rank, L, nC, CC, nD, CD, Z.p));
+    cs = rank;
+  } else {
+    GC_TRY(M.alloc(ctx, (size_t)cs * n2));
+    GC_TRY(T1.alloc(ctx, (size_t)cs * n * std::max(nA, nC)));
+  }
+  for (int P0 = 0; P0 < rank && precision != GC_PREC_FP64; P0 += cs) {
     int cnt = std::min(cs, rank - P0);
     unsigned grid = std::min<unsigned>(gc::ceil_div((size_t)cnt * n2, 256), 152u * 32u);
     unpack_factor<<<grid, 256, 0, ctx->stream>>>(L, ntr, n, P0, cnt, M.p);
@@ -220,14 +299,3 @@ extern "C" int gc_tran4_factored(gc_context *ctx, int nbas, int rank, const doub
                         (int)nCD));
   return precision == GC_PREC_FP64 ? GC_OK : gc::check_flag(ctx);
 }
-
-namespace gc {
-
-// FP64 fallback of the two building blocks; the tensor-core versions live in
-// gc_tc_gemm.cu and are selected by precision.
-int fp64_two_sided(gc_context *ctx, int n, int cnt, const double *M, int nX, const double *CX,
-                   int nY, const double *CY, double *T1, double *out, long long ostride) {
-  return two_sided(ctx, n, cnt, M, nX, CX, nY, CY, T1, out, ostride);
-}
-
-}  // namespace gc

@@ -123,7 +123,8 @@ def test_sliced_gemm_bits(gpu_lib, S, m, n, k):
 @pytest.mark.parametrize("n,widths", [(33, (33, 5, 33, 5)), (33, (5, -1, 33, -1)), (20, (3, 17, 9, -1)),
                                       (20, (7, -1, 4, 11)), (65, (2, 65, 2, 65)), (5, (1, 1, 5, 2))])
 @pytest.mark.parametrize("entry", ["factored", "gen"])
-def test_transform_block_shapes(gpu_lib, n, widths, entry):
+@pytest.mark.parametrize("precision", ["fp64tc5", "fp64"])
+def test_transform_block_shapes(gpu_lib, n, widths, entry, precision):
     rng = np.random.default_rng(n)
     lf = synth.make_lfac(n, 2 * n + 1, rng) * 0.1
     C, blocks = np.linalg.qr(rng.standard_normal((n, n)))[0], []
@@ -133,9 +134,9 @@ def test_transform_block_shapes(gpu_lib, n, widths, entry):
         blocks[2:] = blocks[:2]
     ref = R.tran4_gen(n, *[b.cpu().numpy() for b in blocks], lf @ lf.T)
     if entry == "factored":
-        out = api.tran4_factored(n, t(lf), *blocks, precision="fp64tc5")
+        out = api.tran4_factored(n, t(lf), *blocks, precision=precision)
     else:
-        out = api.tran4_gen(n, *blocks, t(lf @ lf.T), precision="fp64tc5")
+        out = api.tran4_gen(n, *blocks, t(lf @ lf.T), precision=precision)
     assert np.abs(out.cpu().numpy() - ref).max() < 1e-10
 
 
