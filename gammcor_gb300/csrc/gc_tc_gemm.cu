@@ -393,6 +393,7 @@ struct OzEpi {
   long long ea_sb, eb_sb;
   int tri_period;        // > 0: skip tiles wholly above the diagonal of each
                          // tri_period-wide column block (C lower-triangular per block)
+  int tri_upper;         // 1: skip the tiles wholly below the diagonals instead
 };
 
 // t 2^sc where the result is subnormal, overflows or is next to it: exact steps, one rounding.
@@ -462,7 +463,8 @@ __global__ void __launch_bounds__(oz_threads(TBN), 1)
   const int nchunks = (kblocks + plan.chunk_kb - 1) / plan.chunk_kb;
   if (epi.tri_period > 0) {  // whole CTA, before any barrier or TMEM is set up
     const int c0 = n0 % epi.tri_period;
-    if (c0 + TBN <= epi.tri_period && c0 >= m0 + BM) {
+    const bool inside = c0 + TBN <= epi.tri_period;  // all columns in one block
+    if (inside && (epi.tri_upper ? c0 + TBN <= m0 : c0 >= m0 + BM)) {
       if (epi.mode == 4 && threadIdx.x == 0)
         epi.partial[blockIdx.x + (long long)gridDim.x * (blockIdx.y + (long long)gridDim.y * blockIdx.z)] = 0.0;
       return;
@@ -1034,16 +1036,22 @@ __global__ void __launch_bounds__(256) k_oz_col_digits(OzColView X, int Kp, int 
 // Row exponents and slices of symmetric n x n matrices read from their packed triangles
 // (matrix k at x + k ld, element (p, q), p <= q, at p + q (q + 1) / 2): the operand has a row
 // (k, p) for every p, without the unpacked FP64 matrices ever being written. One block per
-// matrix (blockIdx.y: a share of its rows): the maxima of all rows from one sweep over the
-// triangle (high words only: the exponent is all that is wanted), then one warp per row. A
-// row's elements with q <= p are contiguous in the triangle, the others share their sectors
-// with the rows that the block's other warps hold. Measured for 1494 matrices with n = 249: 0.40
-// ms, where unpacking (0.32), exponents and digits took 1.2 ms.
+// matrix (blockIdx.y: a share of its tiles): the maxima of all rows from one sweep over the
+// triangle (high words only: the exponent is all that is wanted), then the triangle again in
+// 64 x 64 tiles through shared memory, each of which gives the digits of its rows and, with their
+// own exponents, of its columns. A tile is loaded along p, contiguous in the triangle.
+// Measured for 1494 matrices with n = 249: 0.37 ms (4.5 TB/s; both sweeps come from HBM), with a
+// warp per row that gathers the elements beyond the diagonal 0.40, with a cluster of four
+// blocks per matrix 0.41, and unpacking, exponents and digits apart 1.2 ms.
 template <int S>
 __global__ void __launch_bounds__(256) k_oz_packed(const double *__restrict__ x, long long ld, int n,
                                                    int Kp, int cnt, int *__restrict__ e,
                                                    __nv_bfloat16 *__restrict__ planes) {
   extern __shared__ unsigned rmax[];
+  // [q][p], row q at (q / 4) + 16 (q % 4): four consecutive q of a column from four rows without
+  // bank conflicts, four consecutive p of a row as two 16-byte reads
+  __shared__ __align__(16) double tile[64][66];
+  auto at = [](int q) { return (q >> 2) + 16 * (q & 3); };
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const double *__restrict__ xk = x + blockIdx.x * ld;
   for (int p = threadIdx.x; p < n; p += 256) rmax[p] = 0;
@@ -1051,6 +1059,7 @@ __global__ void __launch_bounds__(256) k_oz_packed(const double *__restrict__ x,
   for (int q = warp; q < n; q += 8) {
     const double *__restrict__ c = xk + (long long)q * (q + 1) / 2;
     unsigned mx = 0;
+#pragma unroll 4
     for (int p = lane; p <= q; p += 32) {
       const unsigned h = (unsigned)__double2hiint(c[p]) & 0x7fffffffu;
       atomicMax(&rmax[p], h);
@@ -1061,21 +1070,55 @@ __global__ void __launch_bounds__(256) k_oz_packed(const double *__restrict__ x,
   }
   __syncthreads();
   const long long row0 = blockIdx.x * (long long)n, plane = (long long)cnt * n * Kp;
-  for (int p = blockIdx.y * 8 + warp; p < n; p += 8 * gridDim.y) {
-    const unsigned h = rmax[p];
-    const int E = (int)(h >> 20);
-    const int ex = E == 0x7ff ? kBadExp : max(E, 1) - 1022;  // a subnormal or zero row: 2^-1021 bounds it
-    if (lane == 0) e[row0 + p] = ex;
-    const double *__restrict__ lo = xk + (long long)p * (p + 1) / 2;
-    for (int k = lane * 4; k < Kp; k += 128) {
-      double v[4];
+  auto exponent = [&](int p) {
+    const int E = (int)(rmax[p] >> 20);
+    return E == 0x7ff ? kBadExp : max(E, 1) - 1022;  // 2^-1021 bounds a subnormal or zero row
+  };
+  if (blockIdx.y == 0)
+    for (int p = threadIdx.x; p < n; p += 256) e[row0 + p] = exponent(p);
+  const int nt = Kp / 64, tx = threadIdx.x & 63, ty = threadIdx.x >> 6;  // load: p along tx
+  const int lr = threadIdx.x >> 4, lk = threadIdx.x & 15;                // write: row, group of 4
+  for (int t = blockIdx.y; t < nt * (nt + 1) / 2; t += gridDim.y) {
+    int tq = 0;  // tile (tp, tq), tp <= tq
+    while ((tq + 1) * (tq + 2) / 2 <= t) ++tq;
+    const int p0 = (t - tq * (tq + 1) / 2) * 64, q0 = tq * 64;
+    double v[16];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int q = k + i;
-        v[i] = q >= n ? 0.0 : (q <= p ? lo[q] : xk[p + (long long)q * (q + 1) / 2]);
-      }
-      store_digits4<S>(v, ex, plane, (row0 + p) * Kp + k, planes);
+    for (int i = 0; i < 16; ++i) {
+      const int q = q0 + ty + 4 * i, p = p0 + tx;
+      v[i] = q < n && p <= q ? xk[p + (long long)q * (q + 1) / 2] : 0.0;
     }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 16; ++i) tile[at(ty + 4 * i)][tx] = v[i];
+    __syncthreads();
+    if (p0 == q0) {  // the diagonal tile's other half
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const int q = ty + 4 * i;
+        if (tx > q) tile[at(q)][tx] = tile[at(tx)][q];
+      }
+      __syncthreads();
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {  // rows q, K along p
+      const int l = lr + 16 * i;
+      if (q0 + l < n) {
+        const double2 a = *reinterpret_cast<const double2 *>(&tile[at(l)][lk * 4]);
+        const double2 b = *reinterpret_cast<const double2 *>(&tile[at(l)][lk * 4 + 2]);
+        const double w[4] = {a.x, a.y, b.x, b.y};
+        store_digits4<S>(w, exponent(q0 + l), plane, (row0 + q0 + l) * Kp + p0 + lk * 4, planes);
+      }
+    }
+    if (p0 != q0)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {  // rows p, K along q
+        const int l = lr + 16 * i;
+        if (p0 + l < n) {
+          const double w[4] = {tile[lk][l], tile[lk + 16][l], tile[lk + 32][l], tile[lk + 48][l]};
+          store_digits4<S>(w, exponent(p0 + l), plane, (row0 + p0 + l) * Kp + q0 + lk * 4, planes);
+        }
+      }
   }
 }
 
@@ -1358,16 +1401,16 @@ int make_oz_packed(gc_context *ctx, OzOperand &op, const double *x, long long ld
   op.S = S;
   GC_TRY(op.exps.alloc(ctx, (size_t)op.rows));
   GC_TRY(op.buf.alloc(ctx, (size_t)op.rows * op.Kp * S));
-  // two blocks per SM at least, where a matrix has the rows for it
-  const dim3 grid(cnt, std::max(1u, std::min(gc::ceil_div(304, cnt), gc::ceil_div(n, 8))));
+  // two blocks per SM at least, where a matrix has the tiles for it
+  const unsigned nt = op.Kp / 64, tiles = nt * (nt + 1) / 2;
+  const dim3 grid(cnt, std::max(1u, std::min(gc::ceil_div(304, cnt), tiles)));
   const size_t sm = (size_t)n * sizeof(unsigned);
-  if (sm > 48 * 1024) return gc::set_error(ctx, GC_EUNSUPPORTED, "packed operand: n=%d", n);
-  if (S == 4)
-    k_oz_packed<4><<<grid, 256, sm, ctx->stream>>>(x, ld, n, op.Kp, cnt, op.exps.p, op.buf.p);
-  else if (S == 5)
-    k_oz_packed<5><<<grid, 256, sm, ctx->stream>>>(x, ld, n, op.Kp, cnt, op.exps.p, op.buf.p);
-  else
-    k_oz_packed<6><<<grid, 256, sm, ctx->stream>>>(x, ld, n, op.Kp, cnt, op.exps.p, op.buf.p);
+  constexpr size_t kMaxSm = 128 * 1024;
+  if (sm > kMaxSm) return gc::set_error(ctx, GC_EUNSUPPORTED, "packed operand: n=%d", n);
+  auto kern = S == 4 ? k_oz_packed<4> : (S == 5 ? k_oz_packed<5> : k_oz_packed<6>);
+  if (sm > 8 * 1024)
+    GC_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSm));
+  kern<<<grid, 256, sm, ctx->stream>>>(x, ld, n, op.Kp, cnt, op.exps.p, op.buf.p);
   GC_LAUNCHED(ctx);
   op.planes = op.buf.p;
   op.ex = op.exps.p;
@@ -1403,15 +1446,23 @@ constexpr double oz_tile_cost(int S, int tbn) {
 }
 
 // Tile width for an M x N x nbatch product: the narrowest width unless a wider one
-// finishes its CTA waves (152 SMs, one CTA each) sooner by the costs above.
-int oz_tile(const gc_context *ctx, int S, long long M, long long N, long long nbatch) {
+// finishes its CTA waves (152 SMs, one CTA each) sooner by the costs above. tri: only the
+// tiles that reach the lower triangle of an M x M product are computed (N = M); at 3774 that
+// is 4.1 waves of 96-wide tiles, 5 in effect, and 64-wide ones finish sooner.
+int oz_tile(const gc_context *ctx, int S, long long M, long long N, long long nbatch,
+            bool tri = false) {
   const int widest = oz_max_tile(S);
   if (ctx->oz_tile > 0) return std::min(ctx->oz_tile, widest);
   int best = 64;
   double best_cost = 0.0;
   for (int tbn = 64; tbn <= widest; tbn += 32) {
-    const long long ctas = (M + BM - 1) / BM * ((N + tbn - 1) / tbn) * nbatch;
-    const double cost = (double)((ctas + 151) / 152) * oz_tile_cost(S, tbn);
+    const long long ntm = (M + BM - 1) / BM, ntn = (N + tbn - 1) / tbn;
+    long long ctas = ntm * ntn;
+    if (tri) {
+      ctas = 0;
+      for (long long i = 0; i < ntm; ++i) ctas += std::min(ntn, (std::min((i + 1) * BM, M) + tbn - 1) / tbn);
+    }
+    const double cost = (double)((ctas * nbatch + 151) / 152) * oz_tile_cost(S, tbn);
     if (tbn == 64 || cost < best_cost) {
       best = tbn;
       best_cost = cost;
@@ -1521,7 +1572,9 @@ int tc_half_packed(gc_context *ctx, int precision, int n, int cnt, const double 
         B.rows = c * nf;
         B.nb = 1;
         GC_TRY(encode_oz_map(ctx, B));
-        OzEpi e2{0, out, o.nX, 0, nullptr, nullptr, nullptr, nullptr, 0, 0};
+        // a block with itself: x <= y is all that tc_pair_product reads
+        const bool sym = o.sym;
+        OzEpi e2{0, out, o.nX, 0, nullptr, nullptr, nullptr, nullptr, 0, 0, sym ? nf : 0, sym ? 1 : 0};
         GC_TRY(run_oz(ctx, side[h]->second, B, o.nX, c * nf, 1, pl, e2));
       } else {
         GC_TRY(make_oz_operand(ctx, B, T.p, nf, n, c, (long long)c * n, 1, n, pl.S, BM));
@@ -1550,7 +1603,7 @@ int tc_pair_product(gc_context *ctx, int precision, int rank, int nC, int nD, bo
   OzOperand a, b;
   GC_TRY(make_oz_operand(ctx, a, Z, R, rank, 1, 1, nCD, 0, pl.S, BM, symCD ? nC : 0));
   if (same) {  // symmetric: the lower triangle and its mirror image
-    GC_TRY(alias_oz_operand(ctx, a, b, oz_tile(ctx, pl.S, R, (Q + 1) / 2, 1)));
+    GC_TRY(alias_oz_operand(ctx, a, b, oz_tile(ctx, pl.S, R, Q, 1, true)));
     OzEpi e{3, C, R, 0, nullptr, nullptr, nullptr, nullptr, 0, 0, R};
     GC_TRY(run_oz(ctx, a, b, R, Q, 1, pl, e));
   } else {
@@ -1655,7 +1708,7 @@ int tc_syrk_sub_lower(gc_context *ctx, int precision, int M, int K, const double
   OzPlan pl = oz_plan(precision);
   OzOperand a, b;
   GC_TRY(make_oz_operand(ctx, a, P, M, K, nbatch, sm, sk, sb, pl.S, BM));
-  GC_TRY(alias_oz_operand(ctx, a, b, oz_tile(ctx, pl.S, M, M, nbatch)));
+  GC_TRY(alias_oz_operand(ctx, a, b, oz_tile(ctx, pl.S, M, M, nbatch, true)));
   OzEpi e{2, C, ldc, nbatch > 1 ? sb : 0, nullptr, nullptr, nullptr, nullptr, 0, 0, M};
   GC_TRY(run_oz(ctx, a, b, M, M, nbatch, pl, e));
   return GC_OK;  // the device flag is read at the caller's next sync point
@@ -1673,7 +1726,7 @@ int tc_gram_dot(gc_context *ctx, int precision, int N, const double *Y, const do
   opt.hi = hi;
   opt.sq = sq;
   GC_TRY(make_oz_operand(ctx, a, Y, N, N, 1, 1, N, 0, pl.S, BM, 0, opt));
-  GC_TRY(alias_oz_operand(ctx, a, b, oz_tile(ctx, pl.S, N, (N + 1) / 2, 1)));
+  GC_TRY(alias_oz_operand(ctx, a, b, oz_tile(ctx, pl.S, N, N, 1, true)));
   GC_TRY(part.alloc(ctx, (size_t)ceil_div(N, BM) * ceil_div(N, b.box_rows)));
   OzEpi e{4, nullptr, N, 0, Klow, part.p, nullptr, nullptr, 0, 0, N};
   return run_oz(ctx, a, b, N, N, 1, pl, e);

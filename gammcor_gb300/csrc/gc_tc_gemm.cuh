@@ -14,13 +14,15 @@ int check_flag(gc_context *ctx);
 
 // Sliced precisions: out_k (nX x nY, column-major, consecutive) = CX^T M_k CY for cnt symmetric
 // n x n matrices given by their packed triangles (M_k at M + k ld, element (p, q), p <= q, at
-// p + q (q + 1) / 2), for one or two pairs of blocks that share the slices of the M_k.
+// p + q (q + 1) / 2), for one or two pairs of blocks that share the slices of the M_k. With
+// sym (CX == CY, nX == nY) out_k(x, y) may be left out for x > y.
 struct HalfOut {
   int nX;
   const double *CX;  // n x nX, column-major
   int nY;
   const double *CY;  // n x nY, column-major
   double *out;       // cnt x (nX x nY)
+  bool sym = false;
 };
 int tc_half_packed(gc_context *ctx, int precision, int n, int cnt, const double *M, long long ld,
                    int nhalf, const HalfOut *half);

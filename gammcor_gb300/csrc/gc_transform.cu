@@ -268,9 +268,9 @@ extern "C" int gc_tran4_factored(gc_context *ctx, int nbas, int rank, const doub
   GC_TRY(Y.alloc(ctx, nAB * rank));
   if (!same) GC_TRY(Z.alloc(ctx, nCD * rank));
   if (gc::is_sliced(precision)) {
-    const gc::HalfOut half[2] = {{nA, CA, nB, CB, Y.p}, {nC, CC, nD, CD, Z.p}};
-    GC_TRY(gc::tc_half_packed(ctx, precision, n, rank, L, ntr, same ? 1 : 2, half));
     const bool symAB = CA == CB && nA == nB, symCD = CC == CD && nC == nD;
+    const gc::HalfOut half[2] = {{nA, CA, nB, CB, Y.p, symAB}, {nC, CC, nD, CD, Z.p, symCD}};
+    GC_TRY(gc::tc_half_packed(ctx, precision, n, rank, L, ntr, same ? 1 : 2, half));
     GC_TRY(gc::tc_pair_product(ctx, precision, rank, nC, nD, symCD, same ? Y.p : Z.p, nA, nB, symAB,
                                Y.p, out));
     return gc::check_flag(ctx);

@@ -121,7 +121,8 @@ def test_sliced_gemm_bits(gpu_lib, S, m, n, k):
 
 # widths (nA, nB, nC, nD); -1 repeats the block before it, so that the pair index is symmetric
 @pytest.mark.parametrize("n,widths", [(33, (33, 5, 33, 5)), (33, (5, -1, 33, -1)), (20, (3, 17, 9, -1)),
-                                      (20, (7, -1, 4, 11)), (65, (2, 65, 2, 65)), (5, (1, 1, 5, 2))])
+                                      (20, (7, -1, 4, 11)), (65, (2, 65, 2, 65)), (5, (1, 1, 5, 2)),
+                                      (130, (3, -1, 130, -1))])
 @pytest.mark.parametrize("entry", ["factored", "gen"])
 @pytest.mark.parametrize("precision", ["fp64tc5", "fp64"])
 def test_transform_block_shapes(gpu_lib, n, widths, entry, precision):
