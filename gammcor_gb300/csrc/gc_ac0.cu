@@ -17,11 +17,10 @@
 //   k_ac0_block_erpa  one CTA per block: ERPASYMM0 in FP64 shared memory (two
 //                     Jacobi eigensolves), Y, X and omega of the block;
 //   k_ac0_iv          the (virtual, inactive) pairs: omega = A+(ii,ii), Y = X = 1/sqrt 2;
-//   k_ac0_right       T+ = A+' Xbd, T- = A-' Ybd (block-diagonal right products);
-//   k_ac0_work        work = 2 (Xbd^T T+ - Ybd^T T-) / (omega_i + omega_j);
-//   k_ac0_back_right  U = work Ybd^T;
-//   k_ac0_energy      C = Ybd U contracted with the masked, CI-weighted FOFO
-//                     integrals on the fly, one partial sum per CTA.
+//   k_ac0_right       T+ = A+' Xbd, T- = A-' Ybd, TK = K Ybd (block-diagonal right products; K:
+//                     the masked, CI-weighted FOFO integrals, gathered);
+//   k_ac0_work        the energy sum_{r<=c} of 2 (Xbd^T T+ - Ybd^T T-) / (omega_r + omega_c) times
+//                     Ybd^T TK, one partial sum per block.
 // Every pass is O(N^2 m) for blocks of size m (at most nact(nact-1)/2): there is
 // no O(N^3) step, unlike the ERPA solves of the lambda quadrature.
 #include <algorithm>
@@ -263,85 +262,69 @@ __global__ void k_ac0_iv(int N, int iv0, const double *__restrict__ ap, double *
   Xrow[(size_t)i * kRow] = fac;
 }
 
-// T+[r, c] = sum_k A+'[r, k] Xbd[k, c], T-[r, c] = sum_k A-'[r, k] Ybd[k, c], the sum over
-// k in the block of c (bs[c] .. bs[c] + bz[c] - 1). Threads along r: coalesced columns.
-__global__ void k_ac0_right(int N, const double *__restrict__ a1p, const double *__restrict__ a1m,
-                            const int *__restrict__ bs, const int *__restrict__ bz,
-                            const double *__restrict__ Xrow, const double *__restrict__ Yrow,
-                            double *__restrict__ tp, double *__restrict__ tm) {
+// T+ = A+' Xbd, T- = A-' Ybd and TK = K Ybd with the block-diagonal Xbd, Ybd (the sum over k in
+// the block of c, positions bs[c] .. bs[c] + bz[c] - 1) and the energy's weights
+// K[r, k] = (C_p + C_q)(C_r' + C_s') (r's'|pq) for pairs r = (p, q), k = (r', s') not in one
+// orbital group, gathered here. The rows up to the end of c's block are all that k_ac0_work
+// reads. Threads along r: coalesced columns.
+__global__ void k_ac0_right(int N, int n, int nocc, const double *__restrict__ a1p,
+                            const double *__restrict__ a1m, const int *__restrict__ bs,
+                            const int *__restrict__ bz, const double *__restrict__ Xrow,
+                            const double *__restrict__ Yrow, const int *__restrict__ pp,
+                            const int *__restrict__ pq, const double *__restrict__ cpl,
+                            const int *__restrict__ grp, const double *__restrict__ fofo,
+                            double *__restrict__ tp, double *__restrict__ tm,
+                            double *__restrict__ tk) {
   const int r = blockIdx.x * blockDim.x + threadIdx.x, c = blockIdx.y;
-  if (r >= N) return;
   const int s = bs[c], m = bz[c], cc = c - s;
-  double vp = 0.0, vm = 0.0;
+  if (r >= s + m) return;
+  const int p = pp[r], q = pq[r], g = grp[p], gg = grp[q];
+  const size_t ld = (size_t)n * nocc;
+  double vp = 0.0, vm = 0.0, vk = 0.0;
   for (int b = 0; b < m; ++b) {
-    const size_t e = (size_t)r + (size_t)(s + b) * N;
-    vp += a1p[e] * Xrow[(size_t)(s + b) * kRow + cc];
-    vm += a1m[e] * Yrow[(size_t)(s + b) * kRow + cc];
+    const int k = s + b, rr = pp[k], ss = pq[k];
+    const size_t e = (size_t)r + (size_t)k * N;
+    const double y = Yrow[(size_t)k * kRow + cc];
+    vp += a1p[e] * Xrow[(size_t)k * kRow + cc];
+    vm += a1m[e] * y;
+    if (!(g == gg && gg == grp[rr] && grp[rr] == grp[ss]))
+      vk += cpl[k] * fofo[((size_t)rr + (size_t)ss * n) * ld + p + (size_t)q * n] * y;
   }
-  tp[(size_t)r + (size_t)c * N] = vp;
-  tm[(size_t)r + (size_t)c * N] = vm;
+  const size_t o = (size_t)r + (size_t)c * N;
+  tp[o] = vp;
+  tm[o] = vm;
+  tk[o] = cpl[r] * vk;
 }
 
+// The energy sum_{r,c} work[r, c] (Ybd^T K Ybd)[r, c] with
 // work[r, c] = 2 ((Xbd^T T+)[r, c] - (Ybd^T T-)[r, c]) / (omega_r + omega_c) where both
-// omegas are nonzero, else 0 (AC0CAS_FOFO, abfofo.f90:1625-1633).
-__global__ void k_ac0_work(int N, const double *__restrict__ tp, const double *__restrict__ tm,
-                           const int *__restrict__ bs, const int *__restrict__ bz,
-                           const double *__restrict__ Xrow, const double *__restrict__ Yrow,
-                           const double *__restrict__ eig, double *__restrict__ work) {
-  const int r = blockIdx.x * blockDim.x + threadIdx.x, c = blockIdx.y;
-  if (r >= N) return;
-  const double er = eig[r], ec = eig[c];
-  double v = 0.0;
-  if (er != 0.0 && ec != 0.0) {
-    const int s = bs[r], m = bz[r], rr = r - s;
-    double xp = 0.0, ym = 0.0;
-    for (int b = 0; b < m; ++b) {
-      const size_t e = (size_t)(s + b) + (size_t)c * N;
-      xp += Xrow[(size_t)(s + b) * kRow + rr] * tp[e];
-      ym += Yrow[(size_t)(s + b) * kRow + rr] * tm[e];
-    }
-    v = 2.0 * (xp - ym) / (er + ec);
-  }
-  work[(size_t)r + (size_t)c * N] = v;
-}
-
-// U[r, c] = sum_k work[r, k] Ybd[c, k], k in the block of c (ABPM_BACKTRAN, right factor).
-__global__ void k_ac0_back_right(int N, const double *__restrict__ work, const int *__restrict__ bs,
-                                 const int *__restrict__ bz, const double *__restrict__ Yrow,
-                                 double *__restrict__ u) {
-  const int r = blockIdx.x * blockDim.x + threadIdx.x, c = blockIdx.y;
-  if (r >= N) return;
-  const int s = bs[c], m = bz[c];
-  double v = 0.0;
-  for (int b = 0; b < m; ++b)
-    v += work[(size_t)r + (size_t)(s + b) * N] * Yrow[(size_t)c * kRow + b];
-  u[(size_t)r + (size_t)c * N] = v;
-}
-
-// C[r, c] = sum_k Ybd[r, k] U[k, c] (k in the block of r), contracted on the fly with
-// (C_p + C_q)(C_r' + C_s') (r's'|pq) for pairs r = (p, q), c = (r', s') not in one orbital
-// group (the energy loop of AC0CAS_FOFO, abfofo.f90:1676-1720); one partial per CTA.
-__global__ void k_ac0_energy(int n, int nocc, int N, const double *__restrict__ u,
-                             const int *__restrict__ bs, const int *__restrict__ bz,
-                             const double *__restrict__ Yrow, const int *__restrict__ pp,
-                             const int *__restrict__ pq, const double *__restrict__ cpl,
-                             const int *__restrict__ grp, const double *__restrict__ fofo,
-                             double *__restrict__ part) {
+// omegas are nonzero, else 0 (AC0CAS_FOFO, abfofo.f90:1625-1720, with the back-transform Ybd work
+// Ybd^T moved to the symmetric weights). Both factors are symmetric: r <= c, the others counted
+// twice. One partial sum per block. Measured at NDimX 1832 (n = 120, CAS(6,6)) with k_ac0_right:
+// 161 us, where the products, the back-transform and the energy loop over all r, c took 280.
+__global__ void __launch_bounds__(256)
+    k_ac0_work(int N, const double *__restrict__ tp, const double *__restrict__ tm,
+               const double *__restrict__ tk, const int *__restrict__ bs, const int *__restrict__ bz,
+               const double *__restrict__ Xrow, const double *__restrict__ Yrow,
+               const double *__restrict__ eig, double *__restrict__ part) {
   __shared__ double red[256];
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   double e = 0.0;
   if (r < N) {
-    const int p = pp[r], q = pq[r], s = bs[r], m = bz[r];
-    const double cpq = cpl[r];  // C_p + C_q
-    const size_t ld = (size_t)n * nocc;
+    const double er = eig[r];
+    const int s = bs[r], m = bz[r], rr = r - s;
     for (int c = blockIdx.y; c < N; c += gridDim.y) {
-      const int rr = pp[c], ss = pq[c];
-      if (grp[p] == grp[q] && grp[q] == grp[rr] && grp[rr] == grp[ss]) continue;
-      double cv = 0.0;
-      for (int b = 0; b < m; ++b)
-        cv += Yrow[(size_t)r * kRow + b] * u[(size_t)(s + b) + (size_t)c * N];
-      const double f = fofo[((size_t)rr + (size_t)ss * n) * ld + p + (size_t)q * n];  // (r's'|pq)
-      e += cpq * cpl[c] * cv * f;
+      const double ec = eig[c];
+      if (c < r || er == 0.0 || ec == 0.0) continue;
+      double xp = 0.0, ym = 0.0, yk = 0.0;
+      for (int b = 0; b < m; ++b) {
+        const size_t t = (size_t)(s + b) + (size_t)c * N;
+        const double y = Yrow[(size_t)(s + b) * kRow + rr];
+        xp += Xrow[(size_t)(s + b) * kRow + rr] * tp[t];
+        ym += y * tm[t];
+        yk += y * tk[t];
+      }
+      e += (r == c ? 2.0 : 4.0) * (xp - ym) * yk / (er + ec);
     }
   }
   red[threadIdx.x] = e;
@@ -438,8 +421,7 @@ extern "C" int gc_ac0cas_fofo(gc_context *ctx, int nbas, int ninact, int nact, i
   GC_TRY(a0m.alloc(ctx, NN));
   GC_TRY(a1p.alloc(ctx, NN));
   GC_TRY(a1m.alloc(ctx, NN));
-  GC_TRY(gc::assemble_ab(ctx, sd, ffoo, fofo, 0.0, a0p.p, a0m.p, etot, 0));
-  GC_TRY(gc::assemble_ab(ctx, sd, ffoo, fofo, 1.0, a1p.p, a1m.p, nullptr, 1));
+  GC_TRY(gc::assemble_ab_pair(ctx, sd, ffoo, fofo, {{0.0, 0, a0p.p, a0m.p}, {1.0, 1, a1p.p, a1m.p}}, etot));
   GC_TRY(Yrow.alloc(ctx, (size_t)N * kRow));
   GC_TRY(Xrow.alloc(ctx, (size_t)N * kRow));
   GC_TRY(eig.alloc(ctx, N));
@@ -469,25 +451,19 @@ extern "C" int gc_ac0cas_fofo(gc_context *ctx, int nbas, int ninact, int nact, i
                                                                  eig.p);
     GC_LAUNCHED(ctx);
   }
-  // Products with the block-diagonal factors. Buffers are reused in stream order:
-  // T+ -> a0p, T- -> a0m, work -> a1p, U -> a0p.
-  const dim3 blk(256), grid(gc::ceil_div(N, 256), N);
-  k_ac0_right<<<grid, blk, 0, ctx->stream>>>(N, a1p.p, a1m.p, pbs.p, pbz.p, Xrow.p, Yrow.p, a0p.p,
-                                             a0m.p);
+  // Products with the block-diagonal factors; T+ and T- go into a0p and a0m.
+  gc::DevBuf<double> tk, part, res;
+  GC_TRY(tk.alloc(ctx, NN));
+  k_ac0_right<<<dim3(gc::ceil_div(N, 256), N), 256, 0, ctx->stream>>>(
+      N, n, nocc, a1p.p, a1m.p, pbs.p, pbz.p, Xrow.p, Yrow.p, sd.pair_p.p, sd.pair_q.p, sd.cpl.p,
+      sd.grp.p, fofo, a0p.p, a0m.p, tk.p);
   GC_LAUNCHED(ctx);
-  k_ac0_work<<<grid, blk, 0, ctx->stream>>>(N, a0p.p, a0m.p, pbs.p, pbz.p, Xrow.p, Yrow.p, eig.p,
-                                            a1p.p);
-  GC_LAUNCHED(ctx);
-  k_ac0_back_right<<<grid, blk, 0, ctx->stream>>>(N, a1p.p, pbs.p, pbz.p, Yrow.p, a0p.p);
-  GC_LAUNCHED(ctx);
-  const unsigned gy = (unsigned)std::min(N, 1024);
+  const unsigned gy = (unsigned)std::min(N, 256);
   const size_t npart = (size_t)gc::ceil_div(N, 256) * gy;
-  gc::DevBuf<double> part, res;
   GC_TRY(part.alloc(ctx, npart));
   GC_TRY(res.alloc(ctx, 1));
-  k_ac0_energy<<<dim3(gc::ceil_div(N, 256), gy), 256, 0, ctx->stream>>>(
-      n, nocc, N, a0p.p, pbs.p, pbz.p, Yrow.p, sd.pair_p.p, sd.pair_q.p, sd.cpl.p, sd.grp.p, fofo,
-      part.p);
+  k_ac0_work<<<dim3(gc::ceil_div(N, 256), gy), 256, 0, ctx->stream>>>(
+      N, a0p.p, a0m.p, tk.p, pbs.p, pbz.p, Xrow.p, Yrow.p, eig.p, part.p);
   GC_LAUNCHED(ctx);
   k_sum<<<1, 1024, 0, ctx->stream>>>(npart, part.p, res.p);
   GC_LAUNCHED(ctx);

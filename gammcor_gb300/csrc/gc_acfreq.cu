@@ -260,8 +260,7 @@ extern "C" int gc_ac_freq_fofo(gc_context *ctx, int nbas, int ninact, int nact, 
   for (auto *b : {&a0p, &a0m, &a1p, &a1m, &L, &U}) GC_TRY(b->alloc(ctx, NN));
   GC_TRY(w.alloc(ctx, N));
   // A+-B at lambda = 0 and 1; the slope A+-1 = A+-B(1) - A+-B(0) (ac_fofo.f90:41-52)
-  GC_TRY(gc::assemble_ab(ctx, sd, ffoo, fofo, 0.0, a0p.p, a0m.p, etot));
-  GC_TRY(gc::assemble_ab(ctx, sd, ffoo, fofo, 1.0, a1p.p, a1m.p, nullptr));
+  GC_TRY(gc::assemble_ab_pair(ctx, sd, ffoo, fofo, {{0.0, 0, a0p.p, a0m.p}, {1.0, 0, a1p.p, a1m.p}}, etot));
   GC_TRY(gc::axpby_into(ctx, NN, 1.0, a1p.p, -1.0, a0p.p, a1p.p));
   GC_TRY(gc::axpby_into(ctx, NN, 1.0, a1m.p, -1.0, a0m.p, a1m.p));
   // A+0 = L L^T, L^T A-0 L = U W U^T; without a Cholesky factor (A+B(0) not positive

@@ -324,8 +324,7 @@ int gc_acecorr(gc_context *ctx, int nbas, int ninact, int nact, int ndimx, const
     GC_TRY(a0m.alloc(ctx, NN));
     GC_TRY(a1p.alloc(ctx, NN));
     GC_TRY(a1m.alloc(ctx, NN));
-    GC_TRY(gc::assemble_ab(ctx, sd, ffoo, fofo, 0.0, a0p.p, a0m.p, &e0));
-    GC_TRY(gc::assemble_ab(ctx, sd, ffoo, fofo, 1.0, a1p.p, a1m.p, nullptr));
+    GC_TRY(gc::assemble_ab_pair(ctx, sd, ffoo, fofo, {{0.0, 0, a0p.p, a0m.p}, {1.0, 0, a1p.p, a1m.p}}, &e0));
   }
   double acc = 0.0;
   for (int i = 0; i < ngrid; ++i) {

@@ -12,6 +12,7 @@
 // Every coefficient is 1, lambda or (1 - lambda), so A+-B is affine in lambda.
 #include <cmath>
 #include <cstring>
+#include <memory>
 
 #include "gc_internal.cuh"
 
@@ -25,12 +26,24 @@ __device__ __forceinline__ double one_el(const double *__restrict__ h, int hpk, 
 
 struct Geo {
   int n, nin, nact, nocc;
-  // AB1 = .false.: AuxCoeff = 1 for four equal groups, HNO kept inside a group with the
-  // (1 - lambda) inactive/active correction. AB1 = .true. (the lambda derivative,
-  // abfofo.f90:109-156 and HNOCoef, abfofo.f90:167-171, 4494-4500): AuxCoeff = 0 there,
-  // HNO zeroed inside a group and the correction taken with coefficient -1.
-  double same = 1.0;   // AuxCoeff of four equal groups
-  int ab1 = 0;
+};
+
+// One pair A+-B of an assembly: what depends on lambda and the AB1 switch.
+// AB1 = .false.: AuxCoeff = 1 for four equal groups, HNO kept inside a group with the
+// (1 - lambda) inactive/active correction. AB1 = .true. (the lambda derivative,
+// abfofo.f90:109-156 and HNOCoef, abfofo.f90:167-171, 4494-4500): AuxCoeff = 0 there,
+// HNO zeroed inside a group and the correction taken with coefficient -1.
+struct Setting {
+  double lam;
+  double same;   // AuxCoeff of four equal groups
+  int ab1;
+  double2 *ct;                        // ct[q + nocc s], see k_ab (nocc x nocc)
+  double *hno, *auxi, *auxio, *wmat;  // n x n, column-major
+  double *abp, *abm;
+};
+constexpr int kMaxSet = 2;
+struct Settings {
+  Setting s[kMaxSet];
 };
 
 __device__ __forceinline__ double Fofo(const double *__restrict__ f, const Geo &g, int a, int b,
@@ -43,9 +56,9 @@ __device__ __forceinline__ double Ffoo(const double *__restrict__ f, const Geo &
   size_t ld = (size_t)g.n * g.n;
   return f[(size_t)(c + (size_t)d * g.nocc) * ld + a + (size_t)b * g.n];
 }
-// AuxCoeff(g1,g2,g3,g4): g.same if the four orbital groups are equal, else lambda.
-__device__ __forceinline__ double AC(const Geo &g, int a, int b, int c, int d, double lam) {
-  return (a == b && b == c && c == d) ? g.same : lam;
+// AuxCoeff(g1,g2,g3,g4): st.same if the four orbital groups are equal, else lambda.
+__device__ __forceinline__ double AC(const Setting &st, int a, int b, int c, int d) {
+  return (a == b && b == c && c == d) ? st.same : st.lam;
 }
 // AuxInd(g1,g2) of AB_CAS_FOFO: 1 for inactive/active combinations other than
 // active-active, 2 for active-active, 0 otherwise.
@@ -76,9 +89,7 @@ __device__ __forceinline__ double RVa(const double *__restrict__ rv, int na, int
 //   Z13[q,s,p,r] = sum (Tq|sU) RV[t,p,u,r]
 struct Inter {
   double2 *za, *zb, *zc, *zd;
-  double2 *ct;                        // ct[q + nocc s], see k_ab (nocc x nocc)
-  double *hno, *auxi, *auxio, *wmat;  // n x n, column-major
-  double *part;                       // kEtotWarps partial sums of E_CAS
+  double *part;  // kEtotWarps partial sums of E_CAS
 };
 
 constexpr int kEtotWarps = 256;
@@ -97,10 +108,9 @@ struct InterWork {  // first warp of each part
 
 __global__ void __launch_bounds__(256)
     k_intermediates(Geo g, InterWork W, const double *__restrict__ h, int hpk,
-                    const double *__restrict__ occ,
-                    const int *__restrict__ grp, const double *__restrict__ fofo,
-                    const double *__restrict__ ffoo, const double *__restrict__ rv, double lam,
-                    Inter I) {
+                    const double *__restrict__ occ, const int *__restrict__ grp,
+                    const double *__restrict__ fofo, const double *__restrict__ ffoo,
+                    const double *__restrict__ rv, const __grid_constant__ Settings sets, Inter I) {
   const int lane = threadIdx.x & 31;
   const int n = g.n, nin = g.nin, na = g.nact, nocc = g.nocc, nv = n - nin;
   const size_t ldo = (size_t)n * nocc, ldf = (size_t)n * n;
@@ -178,7 +188,8 @@ __global__ void __launch_bounds__(256)
       I.zd[q + (size_t)nocc * (s + (size_t)nocc * (p + na * r))] = make_double2(x, y);
     } else if (w < W.wwm) {  // HNO, AuxI, AuxIO at (i, j)
       const int ch = (n + 31) / 32;
-      const int t0 = w - W.wone;
+      const Setting &st = sets.s[(w - W.wone) / (ch * n)];
+      const int t0 = (w - W.wone) % (ch * n);
       const int i = (t0 % ch) * 32 + lane, j = t0 / ch;
       if (i >= n) continue;
       const int gi = grp[i], gj = grp[j];
@@ -191,21 +202,22 @@ __global__ void __launch_bounds__(256)
         const double jv = Ffoo(ffoo, g, i, j, k, k);  // (ij|kk)
         const double kv = Fofo(fofo, g, j, k, i, k);  // (jk|ik)
         if (gi == gj && gk != gi) corr += ok * (2.0 * jv - kv);
-        const double t = ok * (2.0 * AC(g, gi, gj, gk, gk, lam) * jv - AC(g, gi, gi, gj, gk, lam) * kv);
+        const double t = ok * (2.0 * AC(st, gi, gj, gk, gk) * jv - AC(st, gi, gi, gj, gk) * kv);
         ai += t;
         if (k < nin) aio += t;
       }
       const size_t o = i + (size_t)j * n;
-      I.hno[o] = (gi != gj) ? lam * hv : (g.ab1 ? -corr : hv + (1.0 - lam) * corr);
-      I.auxi[o] = ai;
-      I.auxio[o] = aio;
+      st.hno[o] = (gi != gj) ? st.lam * hv : (st.ab1 ? -corr : hv + (1.0 - st.lam) * corr);
+      st.auxi[o] = ai;
+      st.auxio[o] = aio;
     } else if (w < W.wct) {
       // WMAT(k, r) = sum_{i,j,l < nocc} AuxCoeff(k,l,i,j) (ij|kl) RDM2val(i,j,r,l), 0 for
       // r >= nocc. RDM2val(i,j,r,l) is 2 n_i n_r delta_ij delta_rl - n_i n_r delta_il delta_rj
       // unless i and r are both active (and only where one of n_i, n_r is 1), and the active
       // 2-RDM for four active orbitals: 2 nocc + nact^3 terms instead of nocc^3.
       const int ch = (n + 31) / 32;
-      const int t0 = w - W.wwm;
+      const Setting &st = sets.s[(w - W.wwm) / (ch * n)];
+      const int t0 = (w - W.wwm) % (ch * n);
       const int k = (t0 % ch) * 32 + lane, r = t0 / ch;
       if (k >= n) continue;
       double v = 0.0;
@@ -217,11 +229,11 @@ __global__ void __launch_bounds__(256)
           const double ni = occ[i];
           const int gi = grp[i];
           const double c = ((i >= nin && r >= nin) || !(ni == 1.0 || nr == 1.0)) ? 0.0 : ni * nr;
-          v += c * (2.0 * AC(g, gk, gr, gi, gi, lam) * Fofo(fofo, g, i, i, k, r) -
-                    AC(g, gk, gi, gi, gr, lam) * Fofo(fofo, g, i, r, k, i));
+          v += c * (2.0 * AC(st, gk, gr, gi, gi) * Fofo(fofo, g, i, i, k, r) -
+                    AC(st, gk, gi, gi, gr) * Fofo(fofo, g, i, r, k, i));
         }
         if (r >= nin) {
-          const double c = AC(g, gk, 1, 1, 1, lam);
+          const double c = AC(st, gk, 1, 1, 1);
           double a = 0.0;
 #pragma unroll 8
           for (int t = 0; t < na * na * na; ++t) {  // flat: eight loads in flight
@@ -231,17 +243,19 @@ __global__ void __launch_bounds__(256)
           v += c * a;
         }
       }
-      I.wmat[k + (size_t)r * n] = v;
+      st.wmat[k + (size_t)r * n] = v;
     } else if (w < W.wet) {
-      const int t = (w - W.wct) * 32 + lane;
+      const int chc = (nocc * nocc + 31) / 32;
+      const Setting &st = sets.s[(w - W.wct) / chc];
+      const int t = (w - W.wct) % chc * 32 + lane;
       if (t >= nocc * nocc) continue;
       const int q = t % nocc, s = t / nocc;
       // C = sign(n - 1/2) sqrt(n); a sum or difference of 0 is not divided by
       auto ci = [&](int a) { return occ[a] >= 0.5 ? sqrt(occ[a]) : -sqrt(occ[a]); };
       const double cv = ci(n - 1), cq = ci(q), cs = ci(s);
       const double dp = (cv + cq) * (cv + cs), dm = (cv - cq) * (cv - cs);
-      const double x = grp[q] + grp[s] <= 1 ? lam * (occ[q] * occ[s]) : 0.0;
-      I.ct[t] = make_double2(dp != 0.0 ? x / dp : x, dm != 0.0 ? x / dm : x);
+      const double x = grp[q] + grp[s] <= 1 ? st.lam * (occ[q] * occ[s]) : 0.0;
+      st.ct[t] = make_double2(dp != 0.0 ? x / dp : x, dm != 0.0 ? x / dm : x);
     } else {
       // E_CAS = 2 sum_i n_i h_ii + sum RDM2val(i,j,k,l) (ij|kl), kEtotWarps partial sums in a
       // fixed order. Every integral is read, also those with a zero RDM2val, so that a
@@ -304,9 +318,10 @@ __device__ __forceinline__ bool nonfinite(double x) {
 __global__ void __launch_bounds__(32 * kAbWarps)
     k_ab(Geo g, int N, int cols, const int *__restrict__ slot, const int *__restrict__ pp,
          const int *__restrict__ pq, const double *__restrict__ occ, const int *__restrict__ grp,
-         const double *__restrict__ fofo, const double *__restrict__ ffoo, Inter I, double lam,
-         int vuni, const double *__restrict__ rpl, const double *__restrict__ rmi, double *__restrict__ abp,
-         double *__restrict__ abm) {
+         const double *__restrict__ fofo, const double *__restrict__ ffoo, Inter I,
+         const __grid_constant__ Setting st, int vuni, const double *__restrict__ rpl,
+         const double *__restrict__ rmi) {
+  double *__restrict__ abp = st.abp, *__restrict__ abm = st.abm;
   const int sl = (blockIdx.x * kAbWarps + (threadIdx.x >> 5)) * 32 + (threadIdx.x & 31);
   if (sl >= N) return;
   const int i = slot[sl];
@@ -335,8 +350,8 @@ __global__ void __launch_bounds__(32 * kAbWarps)
   }
   auto aux = [&](int ga, int gb, int x, int y) -> double {
     const int a = AuxInd(ga, gb);
-    if (a == 1) return I.auxi[x + (size_t)y * n];
-    if (a == 2) return I.auxio[x + (size_t)y * n];
+    if (a == 1) return st.auxi[x + (size_t)y * n];
+    if (a == 2) return st.auxio[x + (size_t)y * n];
     return 0.0;
   };
   const bool vrow = vuni && gp == 2;
@@ -348,16 +363,16 @@ __global__ void __launch_bounds__(32 * kAbWarps)
     const double rj_p = rpl[j], rj_m = rmi[j];
     const size_t o = i + (size_t)j * N;
     if (vrow && gr == 2 && !(qa && sa)) {
-      const double2 k = I.ct[q + nocc * s];
+      const double2 k = st.ct[q + nocc * s];
       const double v1 = f1[((size_t)r + (size_t)s * n) * ldo], v2 = f2[(size_t)r * ldo + (size_t)s * n],
                    v3 = f3[(size_t)s * nocc * ldf + (size_t)r * n];
       double vp = k.x * (v2 - v3), vm = k.y * fma(4.0, v1, -(v2 + v3));
       if (p == r || q == s) {  // the one-body part (q = r and p = s cannot be)
         double ob = 0.0;
         if (p == r)
-          ob = (op - os) * I.hno[q + (size_t)s * n] - I.wmat[q + (size_t)s * n] + op * aux(gp, gr, q, s);
+          ob = (op - os) * st.hno[q + (size_t)s * n] - st.wmat[q + (size_t)s * n] + op * aux(gp, gr, q, s);
         if (q == s)
-          ob += (oq - orr) * I.hno[p + (size_t)r * n] - I.wmat[p + (size_t)r * n] + oq * aux(gq, gs, p, r);
+          ob += (oq - orr) * st.hno[p + (size_t)r * n] - st.wmat[p + (size_t)r * n] + oq * aux(gq, gs, p, r);
         vp += (zi_p && nonzero(rj_p)) ? ob * (ri_p * rj_p) : ob;
         vm += (zi_m && nonzero(rj_m)) ? ob * (ri_m * rj_m) : ob;
       }
@@ -375,7 +390,7 @@ __global__ void __launch_bounds__(32 * kAbWarps)
       if (gq + gs <= 1) x1 = fma(oq, os, x1);
       if (gq + gr <= 1) x1 = fma(-oq, orr, x1);
       if (gp + gs <= 1) x1 = fma(-op, os, x1);
-      const double t = AC(g, gp, gq, gr, gs, lam) * x1;
+      const double t = AC(st, gp, gq, gr, gs) * x1;
       // A- += 4 t (rs|pq); anti: t (ps|rq), read as (rq|ps); sym: -t (pr|qs)
       Mo = 4.0 * t * f1[((size_t)r + (size_t)s * n) * ldo];
       A = t * f2[(size_t)r * ldo + (size_t)s * n];
@@ -383,40 +398,40 @@ __global__ void __launch_bounds__(32 * kAbWarps)
     }
     if (ra && qa && p >= nin) {  // FOFO T1 (p -> q), FFOO T2 (p -> q) and T5
       const double2 z = I.za[(p - nin) + (size_t)nv * (s + (size_t)nocc * (qA + na * (r - nin)))];
-      const double c = AC(g, gp, gs, 1, 1, lam);
+      const double c = AC(st, gp, gs, 1, 1);
       S = fma(c, z.x, S);
       A = fma(c, z.y, A);
     }
     if (sa && r >= nin) {
       if (pa) {  // FOFO T3, T4 (p -> q) and T6
         const double2 z = I.zb[(r - nin) + (size_t)nv * (q + (size_t)nocc * (pA + na * (s - nin)))];
-        const double c = AC(g, gq, gr, 1, 1, lam);
+        const double c = AC(st, gq, gr, 1, 1);
         S = fma(c, z.x, S);
         A = fma(c, z.y, A);
       }
       if (qa && p >= nin) {  // FOFO T4 and T6 (p -> q), FFOO T3
         const double2 z = I.zc[(p - nin) + (size_t)nv * ((r - nin) + (size_t)nv * (qA + na * (s - nin)))];
-        const double c = AC(g, gp, gr, 1, 1, lam);
+        const double c = AC(st, gp, gr, 1, 1);
         S = fma(c, z.x, S);
         A = fma(c, z.y, A);
       }
     }
     if (ra && pa) {  // FFOO T1, T2 and T5 (p -> q)
       const double2 z = I.zd[q + (size_t)nocc * (s + (size_t)nocc * (pA + na * (r - nin)))];
-      const double c = AC(g, gq, gs, 1, 1, lam);
+      const double c = AC(st, gq, gs, 1, 1);
       S = fma(c, z.x, S);
       A = fma(c, z.y, A);
     }
     // one-body part (final loop of AB_CAS_FOFO): sym (p = r, q = s) and anti (q = r, p = s)
     if (p == r || q == s || q == r || p == s) {
       if (p == r)
-        S += (op - os) * I.hno[q + (size_t)s * n] - I.wmat[q + (size_t)s * n] + op * aux(gp, gr, q, s);
+        S += (op - os) * st.hno[q + (size_t)s * n] - st.wmat[q + (size_t)s * n] + op * aux(gp, gr, q, s);
       if (q == s)
-        S += (oq - orr) * I.hno[p + (size_t)r * n] - I.wmat[p + (size_t)r * n] + oq * aux(gq, gs, p, r);
+        S += (oq - orr) * st.hno[p + (size_t)r * n] - st.wmat[p + (size_t)r * n] + oq * aux(gq, gs, p, r);
       if (q == r)
-        A += (oq - os) * I.hno[p + (size_t)s * n] - I.wmat[p + (size_t)s * n] + oq * aux(gq, gr, p, s);
+        A += (oq - os) * st.hno[p + (size_t)s * n] - st.wmat[p + (size_t)s * n] + oq * aux(gq, gr, p, s);
       if (p == s)
-        A += (op - orr) * I.hno[q + (size_t)r * n] - I.wmat[q + (size_t)r * n] + op * aux(gp, gs, q, r);
+        A += (op - orr) * st.hno[q + (size_t)r * n] - st.wmat[q + (size_t)r * n] + op * aux(gp, gs, q, r);
     }
     double vp = S + A, vm = S - A + Mo;
     // divide by (C_p + C_q)(C_r + C_s) and (C_p - C_q)(C_r - C_s) where they are not 0,
@@ -608,31 +623,32 @@ int sys_upload(gc_context *ctx, SysDev &sd, int nbas, int ninact, int nact, int 
   return GC_OK;
 }
 
-int assemble_ab(gc_context *ctx, const SysDev &sd, const double *ffoo, const double *fofo,
-                double alpha, double *abplus, double *abmin, double *etot_host, int ab1) {
-  PhaseScope ph(ctx, GC_PHASE_ASSEMBLY);
-  Geo g{sd.n, sd.nin, sd.nact, sd.nocc, ab1 ? 0.0 : 1.0, ab1 ? 1 : 0};
+int assemble(gc_context *ctx, const SysDev &sd, const double *ffoo, const double *fofo, int ns,
+             const AbSpec *spec, double *etot_host) {
+  auto ph = std::make_unique<PhaseScope>(ctx, GC_PHASE_ASSEMBLY);  // of the first pair
+  Geo g{sd.n, sd.nin, sd.nact, sd.nocc};
   const int n = sd.n, N = sd.ndimx, nocc = sd.nocc, nv = n - sd.nin;
   const size_t na2 = (size_t)sd.nact * sd.nact, n2 = (size_t)n * n;
   const size_t sab = (size_t)nv * nocc * na2, sc = (size_t)nv * nv * na2,
                o2 = (size_t)nocc * nocc, sdd = o2 * na2;
   DevBuf<double> buf;
-  GC_TRY(buf.alloc(ctx, 2 * (2 * sab + sc + sdd + o2) + 4 * n2 + kEtotWarps));
+  GC_TRY(buf.alloc(ctx, 2 * (2 * sab + sc + sdd + ns * o2) + 4 * ns * n2 + kEtotWarps));
   Inter I;
   I.za = reinterpret_cast<double2 *>(buf.p);
   I.zb = I.za + sab;
   I.zc = I.zb + sab;
   I.zd = I.zc + sc;
-  I.ct = I.zd + sdd;
-  I.hno = reinterpret_cast<double *>(I.ct + o2);
-  I.auxi = I.hno + n2;
-  I.auxio = I.auxi + n2;
-  I.wmat = I.auxio + n2;
-  I.part = I.wmat + n2;
+  double2 *ct = I.zd + sdd;
+  double *d = reinterpret_cast<double *>(ct + ns * o2);
+  Settings sets{};
+  for (int e = 0; e < ns; ++e, d += 4 * n2)
+    sets.s[e] = Setting{spec[e].alpha, spec[e].ab1 ? 0.0 : 1.0, spec[e].ab1, ct + e * o2,
+                        d, d + n2, d + 2 * n2, d + 3 * n2, spec[e].abplus, spec[e].abmin};
+  I.part = d;
   const long long chv = ceil_div(nv, 32), chn = ceil_div(n, 32), cho = ceil_div(nocc, 32);
   const long long cnt[7] = {chv * nv * (long long)na2, chv * nocc * (long long)na2,
-                            cho * nocc * (long long)na2, chn * n, chn * n, ceil_div(o2, 32),
-                            etot_host ? kEtotWarps : 0};
+                            cho * nocc * (long long)na2, ns * chn * n, ns * chn * n,
+                            (long long)ns * ceil_div(o2, 32), etot_host ? kEtotWarps : 0};
   long long first[8] = {0};
   for (int k = 0; k < 7; ++k) first[k + 1] = first[k] + cnt[k];
   if (first[7] > 0x7fffffffll - (1 << 24))
@@ -640,8 +656,8 @@ int assemble_ab(gc_context *ctx, const SysDev &sd, const double *ffoo, const dou
   const InterWork W{(int)first[0], (int)first[1], (int)first[2], (int)first[3],
                     (int)first[4], (int)first[5], (int)first[6], (int)first[7]};
   k_intermediates<<<std::min<unsigned>(ceil_div((size_t)W.end, 8), 152u * 64u), 256, 0,
-                    ctx->stream>>>(g, W, sd.h.p ? sd.h.p : sd.xone.p, sd.h.p ? 0 : 1, sd.occ.p, sd.grp.p, fofo,
-                                   ffoo, sd.rv.p, alpha, I);
+                    ctx->stream>>>(g, W, sd.h.p ? sd.h.p : sd.xone.p, sd.h.p ? 0 : 1, sd.occ.p,
+                                   sd.grp.p, fofo, ffoo, sd.rv.p, sets, I);
   GC_LAUNCHED(ctx);
   // Columns per warp: up to 8 share the row part of a warp's work; fewer where 8 would leave
   // the chip with less than 32 warps per SM (N = 570: 30 us with 8, 20 us with 2).
@@ -649,16 +665,19 @@ int assemble_ab(gc_context *ctx, const SysDev &sd, const double *ffoo, const dou
   const dim3 g3(ceil_div(N, 32 * kAbWarps), ceil_div(N, cols));
   if (g3.y > 65535)
     return set_error(ctx, GC_EUNSUPPORTED, "assembly: ndimx=%d too large", N);
-  k_ab<<<g3, 32 * kAbWarps, 0, ctx->stream>>>(g, N, cols, sd.slot.p, sd.pair_p.p, sd.pair_q.p, sd.occ.p,
-                                              sd.grp.p, fofo, ffoo, I, alpha, sd.vuni, sd.rpl.p, sd.rmi.p,
-                                              abplus, abmin);
-  GC_LAUNCHED(ctx);
-  if (ab1) {  // AB_CAS_FOFO symmetrises the AB1 matrices (sq_symmetrize, abfofo.f90:260-263)
-    dim3 bs(32, 8), gs(ceil_div(N, 32), ceil_div(N, 8));
-    k_sym_avg<<<gs, bs, 0, ctx->stream>>>(N, abplus);
+  for (int e = 0; e < ns; ++e) {
+    if (e > 0) ph = nullptr, ph = std::make_unique<PhaseScope>(ctx, GC_PHASE_ASSEMBLY);
+    k_ab<<<g3, 32 * kAbWarps, 0, ctx->stream>>>(g, N, cols, sd.slot.p, sd.pair_p.p, sd.pair_q.p,
+                                                sd.occ.p, sd.grp.p, fofo, ffoo, I, sets.s[e], sd.vuni,
+                                                sd.rpl.p, sd.rmi.p);
     GC_LAUNCHED(ctx);
-    k_sym_avg<<<gs, bs, 0, ctx->stream>>>(N, abmin);
-    GC_LAUNCHED(ctx);
+    if (spec[e].ab1) {  // AB_CAS_FOFO symmetrises the AB1 matrices (sq_symmetrize, abfofo.f90:260-263)
+      dim3 bs(32, 8), gs(ceil_div(N, 32), ceil_div(N, 8));
+      k_sym_avg<<<gs, bs, 0, ctx->stream>>>(N, spec[e].abplus);
+      GC_LAUNCHED(ctx);
+      k_sym_avg<<<gs, bs, 0, ctx->stream>>>(N, spec[e].abmin);
+      GC_LAUNCHED(ctx);
+    }
   }
   if (etot_host) {
     double hpart[kEtotWarps];
@@ -669,6 +688,17 @@ int assemble_ab(gc_context *ctx, const SysDev &sd, const double *ffoo, const dou
     *etot_host = e;
   }
   return GC_OK;
+}
+
+int assemble_ab(gc_context *ctx, const SysDev &sd, const double *ffoo, const double *fofo,
+                double alpha, double *abplus, double *abmin, double *etot_host, int ab1) {
+  const AbSpec spec{alpha, ab1, abplus, abmin};
+  return assemble(ctx, sd, ffoo, fofo, 1, &spec, etot_host);
+}
+
+int assemble_ab_pair(gc_context *ctx, const SysDev &sd, const double *ffoo, const double *fofo,
+                     const AbSpec (&spec)[2], double *etot_host) {
+  return assemble(ctx, sd, ffoo, fofo, 2, spec, etot_host);
 }
 
 }  // namespace gc

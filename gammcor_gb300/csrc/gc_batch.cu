@@ -83,8 +83,8 @@ int build_state(gc_context *ctx, const gc_system &s, const gc_ac_params &par, Sy
     GC_TRY(st.a0m.alloc(ctx, NN));
     GC_TRY(st.a1p.alloc(ctx, NN));
     GC_TRY(st.a1m.alloc(ctx, NN));
-    GC_TRY(gc::assemble_ab(ctx, st.sd, st.ffoo.p, st.fofo.p, 0.0, st.a0p.p, st.a0m.p, &st.e0));
-    GC_TRY(gc::assemble_ab(ctx, st.sd, st.ffoo.p, st.fofo.p, 1.0, st.a1p.p, st.a1m.p, nullptr));
+    GC_TRY(gc::assemble_ab_pair(ctx, st.sd, st.ffoo.p, st.fofo.p,
+                                {{0.0, 0, st.a0p.p, st.a0m.p}, {1.0, 0, st.a1p.p, st.a1m.p}}, &st.e0));
   }
   st.built = 1;
   return GC_OK;

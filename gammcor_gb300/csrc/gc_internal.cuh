@@ -203,6 +203,15 @@ int sys_upload(gc_context *ctx, SysDev &sd, int nbas, int ninact, int nact, int 
 
 // Assembly (gc_assembly.cu).
 // ab1 = 1: the AB1 form of AB_CAS_FOFO (the lambda derivative, symmetrised).
+struct AbSpec {
+  double alpha;
+  int ab1;
+  double *abplus, *abmin;
+};
+// Two pairs A+-B from one set of 2-RDM intermediates (lambda = 0 and 1 of the affine form, or 0
+// and the derivative); E_CAS in *etot_host when given.
+int assemble_ab_pair(gc_context *ctx, const SysDev &sd, const double *ffoo, const double *fofo,
+                     const AbSpec (&spec)[2], double *etot_host);
 int assemble_ab(gc_context *ctx, const SysDev &sd, const double *ffoo, const double *fofo,
                 double alpha, double *abplus, double *abmin, double *etot_host, int ab1 = 0);
 // One-electron matrix of sd rotated in place: h <- URe h URe^T, symmetrised.
