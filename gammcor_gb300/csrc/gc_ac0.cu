@@ -177,11 +177,36 @@ __device__ bool block_jacobi(double *A, double *V, double *T, int m, int ld, Blo
   return false;
 }
 
+// A = L L^T (lower, zero above) of the symmetric m x m matrix A, in place, right-looking; false,
+// with A half done, at the first pivot that is not positive (uniform across the block).
+__device__ bool block_cholesky(double *A, int m, int ld) {
+  for (int k = 0; k < m; ++k) {
+    const double d = A[k * ld + k];  // every thread reads the same pivot
+    if (!(d > 0.0)) return false;
+    const double r = rsqrt(d);
+    __syncthreads();
+    for (int i = k + threadIdx.x; i < m; i += kBlkThreads) A[i * ld + k] *= r;
+    __syncthreads();
+    const int w = m - k - 1;
+    for (int e = threadIdx.x; e < w * w; e += kBlkThreads) {
+      const int i = k + 1 + e / w, j = k + 1 + e % w;
+      if (j <= i) A[i * ld + j] -= A[i * ld + k] * A[j * ld + k];
+    }
+    __syncthreads();
+  }
+  for (int e = threadIdx.x; e < m * m; e += kBlkThreads)
+    if (e % m > e / m) A[(e / m) * ld + e % m] = 0.0;
+  __syncthreads();
+  return true;
+}
+
 // ERPASYMM0 of every block (one CTA each): block b covers the block-order positions
 // bstart[b] .. bstart[b] + bsize[b] - 1 of the column-major N x N matrices ap, am (A+-B at
 // lambda = 0). Writes Yrow/Xrow[(s + i) * kRow + c] = Y/X(i, c) of the block and eig[s + c]; a
 // Jacobi that does not converge sets *flag. The largest block (active-active pairs) sets
-// the time: its two eigensolves are a chain of rotations.
+// the time: its eigensolves are a chain of rotations. A positive definite A+ is factored, L
+// takes the place of A+^1/2 (L^T A- L has the eigenvalues of A+^1/2 A- A+^1/2, and L u is the
+// same mode), and one of the two eigensolves falls away: 149 us for CAS(6,6), 270 with two.
 __global__ void __launch_bounds__(kBlkThreads) k_ac0_block_erpa(
     int N, const double *__restrict__ ap, const double *__restrict__ am,
     const int *__restrict__ bstart, const int *__restrict__ bsize, int rows, int ld,
@@ -207,22 +232,25 @@ __global__ void __launch_bounds__(kBlkThreads) k_ac0_block_erpa(
     A[i * ld + j] = 0.5 * (ap[e] + ap[t]);
     B[i * ld + j] = 0.5 * (am[e] + am[t]);
   });
-  if (!block_jacobi(A, V, H, m, ld, sh)) {
-    if (tid == 0) atomicOr(flag, 1);
-    return;  // uniform
+  each([&](int i, int j) { P[i * ld + j] = A[i * ld + j]; });
+  if (!block_cholesky(P, m, ld)) {
+    if (!block_jacobi(A, V, H, m, ld, sh)) {
+      if (tid == 0) atomicOr(flag, 1);
+      return;  // uniform
+    }
+    if (tid < m) w2[tid] = sqrt(fabs(A[tid * ld + tid]));
+    __syncthreads();
+    // P = V diag(sqrt|e|) V^T = A+^1/2 (interpa.f:1546-1568)
+    each([&](int i, int j) {
+      double v = 0.0;
+      for (int k = 0; k < m; ++k) v += V[i * ld + k] * w2[k] * V[j * ld + k];
+      P[i * ld + j] = v;
+    });
   }
-  if (tid < m) w2[tid] = sqrt(fabs(A[tid * ld + tid]));
-  __syncthreads();
-  // P = V diag(sqrt|e|) V^T = A+^1/2 (interpa.f:1546-1568)
-  each([&](int i, int j) {
-    double v = 0.0;
-    for (int k = 0; k < m; ++k) v += V[i * ld + k] * w2[k] * V[j * ld + k];
-    P[i * ld + j] = v;
-  });
-  // H = A- P, then A <- P H (the symmetrised problem, interpa.f:1578-1581)
+  // H = A- P, then A <- P^T H (the symmetrised problem, interpa.f:1578-1581)
   each([&](int i, int j) { H[i * ld + j] = dot(B + i * ld, 1, P + j, ld); });
   each([&](int i, int j) {  // the lower triangle, as the eigensolver reads it
-    if (i >= j) A[i * ld + j] = A[j * ld + i] = dot(P + i * ld, 1, H + j, ld);
+    if (i >= j) A[i * ld + j] = A[j * ld + i] = dot(P + i, ld, H + j, ld);
   });
   if (!block_jacobi(A, V, H, m, ld, sh)) {
     if (tid == 0) atomicOr(flag, 1);

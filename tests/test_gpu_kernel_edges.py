@@ -65,15 +65,19 @@ def test_assembly_shows_a_nonfinite_integral_with_zero_weight(gpu_lib):
     assert not torch.isfinite(gp).all() and not torch.isfinite(gm).all()
 
 
-# AC0 blocks of odd and even size, of one pair, and an active-active block of 55 pairs
-@pytest.mark.parametrize("n,nin,nact", [(12, 2, 1), (14, 1, 2), (21, 2, 5), (30, 0, 11)])
-def test_ac0_block_sizes(gpu_lib, n, nin, nact):
+# AC0 blocks of odd and even size, of one pair, and an active-active block of 55 pairs; with a
+# one-electron part whose order is turned, A+ of some blocks is not positive definite
+@pytest.mark.parametrize("n,nin,nact,turn", [(12, 2, 1, 0), (14, 1, 2, 0), (21, 2, 5, 0), (30, 0, 11, 0),
+                                             (21, 2, 5, 1), (18, 3, 4, 1)])
+def test_ac0_block_sizes(gpu_lib, n, nin, nact, turn):
     from oracle import ac0_ref as A
     m = model(n, nin, nact, seed=n)
     # a dominant one-electron diagonal keeps the zeroth-order blocks stable
     m["xone"] *= 0.05
     d = np.cumsum(np.arange(1, n + 1)) - 1
     m["xone"][d] = np.linspace(-30.0, 10.0, n)
+    if turn:
+        m["xone"][d[nin:nin + nact]] = m["xone"][d[nin:nin + nact]][::-1]
     m["rdm"] = np.zeros_like(m["rdm"])
     o = m["occ"][nin:nin + nact]
     e = np.eye(nact)
