@@ -357,7 +357,15 @@ __global__ void __launch_bounds__(192, 1)
 // one gives more CTAs to a small product. oz_tile() picks one per GEMM; every
 // width gives the same result bits (each element's integer sums are the same).
 constexpr int OZ_BK = 32;      // K per stage: 32 BF16 = one 64-byte swizzled row
-constexpr int OZ_STAGES = 3;   // each stage holds every slice of A and of B
+// Each stage holds every slice of A and of B. The 32-wide tile (products with at most 32 columns:
+// the occupied block of a transform) takes two, so that two CTAs share an SM and one's
+// epilogue runs beside the other's products (372006 x 28 x 249: 185 us, with the 64-wide tile
+// 283 us).
+__host__ __device__ constexpr int oz_stages(int tbn) { return tbn == 32 ? 2 : 3; }
+// TMEM columns allocated: a power of two that holds the S weight accumulators.
+__host__ __device__ constexpr int oz_tmem_cols(int S, int tbn) {
+  return S * tbn <= 128 ? 128 : (S * tbn <= 256 ? 256 : 512);
+}
 constexpr int OZ_MAXS = 6;
 // Row exponent of a row holding a NaN or an infinity: its slices are zero and
 // every product element of the row comes out NaN, so non-finite inputs stay
@@ -420,7 +428,7 @@ __device__ __forceinline__ double scaled_double(long long t, int sc) {
 }
 
 template <int S, int TBN>
-__global__ void __launch_bounds__(oz_threads(TBN), 1)
+__global__ void __launch_bounds__(oz_threads(TBN), TBN == 32 ? 2 : 1)
     k_tc_gemm_oz(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
                  int M, int N, int kblocks, int a_batched, int b_batched, OzPlan plan, OzEpi epi,
                  int *err_flag, unsigned long long wait_ns) {
@@ -428,14 +436,15 @@ __global__ void __launch_bounds__(oz_threads(TBN), 1)
   // and of the B tile (TBN rows): every slice product t+u < S of the block is
   // issued from it, so each slice tile crosses L2 -> shared memory once per block.
   static_assert(S * TBN <= 512 && TBN % 32 == 0, "S weight accumulators exceed TMEM");
-  constexpr int EPI = oz_epi_warps(TBN);
+  constexpr int EPI = oz_epi_warps(TBN), STG = oz_stages(TBN);
+  constexpr uint32_t TCOLS = oz_tmem_cols(S, TBN);
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   constexpr uint32_t A_BYTES = BM * OZ_BK * 2, B_BYTES = TBN * OZ_BK * 2;
   constexpr uint32_t STAGE_BYTES = S * (A_BYTES + B_BYTES);
-  uint64_t *full = (uint64_t *)(smem + OZ_STAGES * STAGE_BYTES);
-  uint64_t *empty = full + OZ_STAGES;
-  uint64_t *accf = empty + OZ_STAGES;
+  uint64_t *full = (uint64_t *)(smem + STG * STAGE_BYTES);
+  uint64_t *empty = full + STG;
+  uint64_t *accf = empty + STG;
   uint64_t *acce = accf + 1;
   uint64_t *drainb = acce + 1;  // abort path: completion of the MMAs already issued
   uint32_t *tmem_slot = (uint32_t *)(drainb + 1);
@@ -472,7 +481,7 @@ __global__ void __launch_bounds__(oz_threads(TBN), 1)
   }
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < OZ_STAGES; ++s) {
+    for (int s = 0; s < STG; ++s) {
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], 1);
     }
@@ -495,7 +504,7 @@ __global__ void __launch_bounds__(oz_threads(TBN), 1)
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                      smem_u32(tmem_slot)),
-                 "r"(512u));
+                 "r"(TCOLS));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -506,8 +515,8 @@ __global__ void __launch_bounds__(oz_threads(TBN), 1)
   if (warp == 0 && lane == 0) {
     int issued = 0;
     for (int kb = 0; kb < kblocks && !*abort_v; ++kb) {
-      const int s = kb % OZ_STAGES;
-      if (!mbar_wait(&empty[s], ((kb / OZ_STAGES) & 1) ^ 1, wait_ns)) {
+      const int s = kb % STG;
+      if (!mbar_wait(&empty[s], ((kb / STG) & 1) ^ 1, wait_ns)) {
         atomicExch(&abort_flag, 1);
         break;
       }
@@ -522,9 +531,9 @@ __global__ void __launch_bounds__(oz_threads(TBN), 1)
                     b_batched ? b : 0, u);
       issued = kb + 1;
     }
-    if (*abort_v)  // only the last OZ_STAGES loads can still be in flight
-      for (int j = (issued > OZ_STAGES ? issued - OZ_STAGES : 0); j < issued; ++j)
-        mbar_wait(&full[j % OZ_STAGES], (j / OZ_STAGES) & 1, kDrainNs);
+    if (*abort_v)  // only the last STG loads can still be in flight
+      for (int j = (issued > STG ? issued - STG : 0); j < issued; ++j)
+        mbar_wait(&full[j % STG], (j / STG) & 1, kDrainNs);
   } else if (warp == 1 && lane == 0) {
     bool ok = true;
     for (int g = 0; g < nchunks && ok; ++g) {
@@ -535,8 +544,8 @@ __global__ void __launch_bounds__(oz_threads(TBN), 1)
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const int kb0 = g * plan.chunk_kb, kb1 = min(kblocks, kb0 + plan.chunk_kb);
       for (int kb = kb0; kb < kb1; ++kb) {
-        const int s = kb % OZ_STAGES;
-        if (!mbar_wait(&full[s], (kb / OZ_STAGES) & 1, wait_ns) || *abort_v) {
+        const int s = kb % STG;
+        if (!mbar_wait(&full[s], (kb / STG) & 1, wait_ns) || *abort_v) {
           ok = false;
           break;
         }
@@ -639,7 +648,7 @@ __global__ void __launch_bounds__(oz_threads(TBN), 1)
     }
     if (!ok) atomicExch(&abort_flag, 1);
     double dot = 0.0;
-    if (ok && m < M) {
+    if (ok) {
       const int er = ea - 7 * (SI + 1);
       const long long o0 = (long long)b * epi.sb + m + (long long)(n0 + h * NC) * epi.ldn;
       // FP64 results first, then one short loop per mode: a tile runs this code once, so its
@@ -652,19 +661,26 @@ __global__ void __launch_bounds__(oz_threads(TBN), 1)
         const double v = scaled_double(acc[j], eb == kBadExp || ea == kBadExp ? 0 : er + eb);
         cv[j] = eb == kBadExp || ea == kBadExp ? __longlong_as_double(0x7ff8000000000000ll) : v;
       }
-      const int n1 = n0 + h * NC, nn = min(NC, N - n1);
+      const int n1 = n0 + h * NC, nn = m < M ? min(NC, N - n1) : 0;
       if (epi.mode == 0) {
 #pragma unroll
         for (int j = 0; j < NC; ++j)
           if (j < nn) epi.c[o0 + j * epi.ldn] = cv[j];
       } else if (epi.mode == 3) {
-        double *mir = epi.c + n1 + (long long)m * epi.ldn;  // 32 consecutive per thread
 #pragma unroll
         for (int j = 0; j < NC; ++j)
-          if (j < nn && m >= n1 + j) {
-            epi.c[o0 + j * epi.ldn] = cv[j];
-            mir[j] = cv[j];
-          }
+          if (j < nn && m >= n1 + j) epi.c[o0 + j * epi.ldn] = cv[j];
+        // the mirror image, turned in shared memory (the stages are free: every load was
+        // consumed by a product that has completed): stores of 32 consecutive elements
+        double *tr = reinterpret_cast<double *>(smem) + (warp - 2) * (32 * 33);
+#pragma unroll
+        for (int j = 0; j < NC; ++j) tr[j * 33 + lane] = cv[j];
+        __syncwarp();
+        const int n = n1 + lane, mb = m0 + q * 32;
+        for (int i = 0; i < 32; ++i) {
+          const int mm = mb + i;
+          if (mm < M && n < N && mm >= n) epi.c[n + (long long)mm * epi.ldn] = tr[lane * 33 + i];
+        }
       } else {
         const double *src = epi.mode == 2 ? epi.c : epi.r;
         // last column of this row: all (1), up to the diagonal (2), below it (4)
@@ -701,7 +717,7 @@ __global__ void __launch_bounds__(oz_threads(TBN), 1)
   if (threadIdx.x == 0 && abort_flag) atomicExch(err_flag, 1);
   if (warp == 1) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u));
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TCOLS));
   }
 }
 
@@ -771,13 +787,12 @@ __device__ __forceinline__ void store_digits4(const double *x, int e, long long 
 
 // Row exponents and integer slices, planes[t][b][r][kp] = alpha_t of x[b,r,k] 2^-e[b][r], of an
 // operand whose K elements are contiguous: TPR threads per row, each holding its elements of
-// the row in registers between the maximum and the digits (rows longer than TPR * 4 * kOzHold
-// are read again for the rest). Bound by HBM: 8 bytes read and 2 S written per element. One
+// the row in registers between the maximum and the digits (kOzHold groups of four; rows longer
+// than TPR * 4 * kOzHold are read again for the rest). Bound by HBM: 8 bytes read and 2 S written per element. One
 // warp per row up to 1024 elements, so that short rows fill a block; a block per longer row.
 // Measured (5 slices): 3774 x 3774 62 us = 4.1 TB/s, where a pass for the exponents and a pass
 // with 2-byte stores took 155 us.
-constexpr int kOzHold = 8;  // groups of four elements per thread
-template <int S, int TPR>
+template <int S, int TPR, int kOzHold>
 __global__ void __launch_bounds__(256) k_oz_rows(const double *__restrict__ x, int rows, int K, int Kp,
                                                  long long nrr, long long sr, long long sb,
                                                  int *__restrict__ e,
@@ -1340,11 +1355,13 @@ int slice_operand(gc_context *ctx, OzOperand &op, const double *x, int rows, int
                   long long sr, long long sk, long long sb, int tri, const OzColsOpt &opt) {
   const long long nrr = (long long)nb * rows;
   const bool plain = !tri && !opt.eig && !opt.sq;
-  if (sk == 1 && plain && op.Kp <= 128 * kOzHold) {  // one warp holds the row
-    k_oz_rows<S, 32><<<gc::ceil_div(nrr, 8), 256, 0, ctx->stream>>>(x, rows, K, op.Kp, nrr, sr, sb,
-                                                                    op.exps.p, op.buf.p);
+  if (sk == 1 && plain && op.Kp <= 1024) {
+    // one warp holds the row; up to K = 256 with half the registers (140454 x 153: 182 -> 115 us)
+    auto kern = op.Kp <= 256 ? k_oz_rows<S, 32, 2> : k_oz_rows<S, 32, 8>;
+    kern<<<gc::ceil_div(nrr, 8), 256, 0, ctx->stream>>>(x, rows, K, op.Kp, nrr, sr, sb, op.exps.p,
+                                                        op.buf.p);
   } else if (sk == 1 && plain) {
-    k_oz_rows<S, 256><<<(unsigned)nrr, 256, 0, ctx->stream>>>(x, rows, K, op.Kp, nrr, sr, sb,
+    k_oz_rows<S, 256, 8><<<(unsigned)nrr, 256, 0, ctx->stream>>>(x, rows, K, op.Kp, nrr, sr, sb,
                                                               op.exps.p, op.buf.p);
   } else {
     const OzColView X{x, rows, K, tri, sr, sk, sb, opt};
@@ -1431,8 +1448,8 @@ int alias_oz_operand(gc_context *ctx, const OzOperand &src, OzOperand &op, int b
 
 // alignment pad, stages, 2 * stages + 3 barriers, TMEM slot
 constexpr size_t oz_smem_bytes(int S, int tbn) {
-  return 1024 + OZ_STAGES * (size_t)S * (BM * OZ_BK * 2 + tbn * OZ_BK * 2) +
-         (2 * OZ_STAGES + 3) * 8 + 16;
+  return 1024 + oz_stages(tbn) * (size_t)S * (BM * OZ_BK * 2 + tbn * OZ_BK * 2) +
+         (2 * oz_stages(tbn) + 3) * 8 + 16;
 }
 static_assert(oz_smem_bytes(4, 128) <= 232448 && oz_smem_bytes(5, 96) <= 232448 &&
                   oz_smem_bytes(6, 64) <= 232448,
@@ -1453,6 +1470,7 @@ int oz_tile(const gc_context *ctx, int S, long long M, long long N, long long nb
             bool tri = false) {
   const int widest = oz_max_tile(S);
   if (ctx->oz_tile > 0) return std::min(ctx->oz_tile, widest);
+  if (N <= 32 && !tri) return 32;
   int best = 64;
   double best_cost = 0.0;
   for (int tbn = 64; tbn <= widest; tbn += 32) {
@@ -1498,6 +1516,9 @@ int run_oz(gc_context *ctx, const OzOperand &A, const OzOperand &B, int M, int N
   epi.ea_sb = A.nb > 1 ? A.rows : 0;
   epi.eb_sb = B.nb > 1 ? B.rows : 0;
   const int w = B.box_rows;
+  if (pl.S == 6 && w == 32) return launch_oz<6, 32>(ctx, A, B, M, N, nbatch, pl, epi);
+  if (pl.S == 5 && w == 32) return launch_oz<5, 32>(ctx, A, B, M, N, nbatch, pl, epi);
+  if (pl.S == 4 && w == 32) return launch_oz<4, 32>(ctx, A, B, M, N, nbatch, pl, epi);
   if (pl.S == 6 && w == 64) return launch_oz<6, 64>(ctx, A, B, M, N, nbatch, pl, epi);
   if (pl.S == 5 && w == 64) return launch_oz<5, 64>(ctx, A, B, M, N, nbatch, pl, epi);
   if (pl.S == 5 && w == 96) return launch_oz<5, 96>(ctx, A, B, M, N, nbatch, pl, epi);
