@@ -260,8 +260,11 @@ __device__ __forceinline__ bool joined(const double *lam, const double *colm, in
   return fabs(lam[k + 1] - lam[k]) <= fmax(colm[k], colm[k + 1]) / kTau;
 }
 
+// list[0] counts the clusters of two or more (zeroed by the caller), list[1..] holds their starts
+// in no particular order: the block kernels walk it instead of looking at every index.
 __global__ void k_clusters(int N, const double *__restrict__ lam, const double *__restrict__ colm,
-                           int *__restrict__ cstart, int *__restrict__ csize, int *flag) {
+                           int *__restrict__ cstart, int *__restrict__ csize, int *flag,
+                           int *__restrict__ list) {
   int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= N) return;
   int s = k;
@@ -273,52 +276,55 @@ __global__ void k_clusters(int N, const double *__restrict__ lam, const double *
   if (too_long) atomicOr(flag, 1);
   cstart[k] = s;
   csize[k] = e - s;
+  if (s == k && e - s > 1) list[1 + atomicAdd(list, 1)] = k;
 }
 
 constexpr int kLd = kMaxCluster + 1;  // padded row of the shared blocks
 constexpr size_t kClusterSmem = 3 * (size_t)kMaxCluster * kLd * sizeof(double);
 constexpr size_t kBlkSmem = 2 * (size_t)kMaxCluster * kLd * sizeof(double);
 
-// One block of kMaxCluster threads per cluster of size >= 2 (block k where
-// cstart[k] == k): V_C with V_C^T G_CC V_C = I and V_C^T S_CC V_C diagonal, stored
+// One block of kMaxCluster threads per cluster of size >= 2 (`list` of k_clusters, starting
+// at k): V_C with V_C^T G_CC V_C = I and V_C^T S_CC V_C diagonal, stored
 // as rows k..k+m-1 of Vbuf (N x kMaxCluster, row-major). Failures set bit 2 of *flag.
 __global__ void __launch_bounds__(kMaxCluster) k_cluster_eig(
-    int N, const double *__restrict__ G, const double *__restrict__ S, const int *__restrict__ cstart,
+    int N, const double *__restrict__ G, const double *__restrict__ S, const int *__restrict__ list,
     const int *__restrict__ csize, double *__restrict__ Vbuf, int *flag, int *maxc) {
-  const int k = blockIdx.x;
-  const int m = csize[k];
-  if (cstart[k] != k || m < 2) return;
   extern __shared__ double sm[];
   double *A = sm, *C = sm + kMaxCluster * kLd, *V = sm + 2 * kMaxCluster * kLd;
   __shared__ double red[2][kMaxCluster];
+  __shared__ int perm[kMaxCluster];
   const int l = threadIdx.x;
-  if (l < m)
-    for (int b = 0; b < m; ++b) {
-      size_t e = (size_t)(k + l) + (size_t)(k + b) * N;
-      A[l * kLd + b] = S[e];
-      C[l * kLd + b] = G[e];
-      V[l * kLd + b] = l == b ? 1.0 : 0.0;
-    }
-  __syncthreads();
-  // G_CC = C C^T (lower, left-looking)
-  for (int j = 0; j < m; ++j) {
-    if (l == 0) {
-      double d = C[j * kLd + j];
-      for (int q = 0; q < j; ++q) d -= C[j * kLd + q] * C[j * kLd + q];
-      C[j * kLd + j] = d > 0.0 ? sqrt(d) : -1.0;
-    }
+  for (int ci = blockIdx.x; ci < list[0]; ci += gridDim.x) {
+    const int k = list[1 + ci];
+    const int m = csize[k];
+    __syncthreads();  // the shared blocks of the last cluster
+    if (l < m)
+      for (int b = 0; b < m; ++b) {
+        size_t e = (size_t)(k + l) + (size_t)(k + b) * N;
+        A[l * kLd + b] = S[e];
+        C[l * kLd + b] = G[e];
+        V[l * kLd + b] = l == b ? 1.0 : 0.0;
+      }
     __syncthreads();
-    const double cjj = C[j * kLd + j];
-    if (!(cjj > 0.0)) {
-      if (l == 0) atomicOr(flag, 2);
-      return;  // uniform: every thread read the same cjj
-    }
-    if (l > j && l < m) {
-      double v = C[l * kLd + j];
-      for (int q = 0; q < j; ++q) v -= C[l * kLd + q] * C[j * kLd + q];
-      C[l * kLd + j] = v / cjj;
-    }
-    __syncthreads();
+    // G_CC = C C^T (lower, left-looking)
+    for (int j = 0; j < m; ++j) {
+      if (l == 0) {
+        double d = C[j * kLd + j];
+        for (int q = 0; q < j; ++q) d -= C[j * kLd + q] * C[j * kLd + q];
+        C[j * kLd + j] = d > 0.0 ? sqrt(d) : -1.0;
+      }
+      __syncthreads();
+      const double cjj = C[j * kLd + j];
+      if (!(cjj > 0.0)) {
+        if (l == 0) atomicOr(flag, 2);
+        return;  // uniform: every thread read the same cjj
+      }
+      if (l > j && l < m) {
+        double v = C[l * kLd + j];
+        for (int q = 0; q < j; ++q) v -= C[l * kLd + q] * C[j * kLd + q];
+        C[l * kLd + j] = v / cjj;
+      }
+      __syncthreads();
   }
   // A <- C^-1 A (thread = column), then A <- A C^-T (thread = row), symmetrise
   if (l < m)
@@ -397,7 +403,6 @@ __global__ void __launch_bounds__(kMaxCluster) k_cluster_eig(
   // Order the block's eigenpairs by eigenvalue (Jacobi leaves them unordered): the
   // next iteration groups clusters from neighbouring indices, which must then hold
   // neighbouring eigenvalues.
-  __shared__ int perm[kMaxCluster];
   if (l == 0) {
     for (int b = 0; b < m; ++b) perm[b] = b;
     for (int b = 1; b < m; ++b) {  // insertion sort on the diagonal of A
@@ -429,57 +434,62 @@ __global__ void __launch_bounds__(kMaxCluster) k_cluster_eig(
   if (l < m)
     for (int b = 0; b < m; ++b) Vbuf[(size_t)(k + l) * kMaxCluster + b] = V[l * kLd + b];
   if (l == 0) atomicMax(maxc, m);
+  }
 }
 
 // X[:, C] <- X[:, C] V_C for every cluster C, rows 0..nrows-1 (kMaxCluster rows
 // per block; the block of X and V_C staged in shared memory).
 __global__ void __launch_bounds__(kMaxCluster) k_blk_right(
-    int nrows, double *__restrict__ X, long long ld, const int *__restrict__ cstart,
+    int nrows, double *__restrict__ X, long long ld, const int *__restrict__ list,
     const int *__restrict__ csize, const double *__restrict__ Vbuf) {
-  const int k = blockIdx.y;
-  const int m = csize[k];
-  if (cstart[k] != k || m < 2) return;
   extern __shared__ double sm[];
   double *Vs = sm, *Xs = sm + kMaxCluster * kLd;
   const int t = threadIdx.x;
-  for (int b = 0; b < m; ++b)
-    if (t < m) Vs[b * kLd + t] = Vbuf[(size_t)(k + b) * kMaxCluster + t];
-  const int i = blockIdx.x * kMaxCluster + t;
-  if (i < nrows)
-    for (int b = 0; b < m; ++b) Xs[t * kLd + b] = X[i + (size_t)(k + b) * ld];
-  __syncthreads();
-  if (i >= nrows) return;
-  for (int j = 0; j < m; ++j) {
-    double v = 0.0;
-    for (int b = 0; b < m; ++b) v += Xs[t * kLd + b] * Vs[b * kLd + j];
-    X[i + (size_t)(k + j) * ld] = v;
+  for (int ci = blockIdx.y; ci < list[0]; ci += gridDim.y) {
+    const int k = list[1 + ci];
+    const int m = csize[k];
+    __syncthreads();  // Vs and Xs of the last cluster
+    for (int b = 0; b < m; ++b)
+      if (t < m) Vs[b * kLd + t] = Vbuf[(size_t)(k + b) * kMaxCluster + t];
+    const int i = blockIdx.x * kMaxCluster + t;
+    if (i < nrows)
+      for (int b = 0; b < m; ++b) Xs[t * kLd + b] = X[i + (size_t)(k + b) * ld];
+    __syncthreads();
+    if (i < nrows)
+      for (int j = 0; j < m; ++j) {
+        double v = 0.0;
+        for (int b = 0; b < m; ++b) v += Xs[t * kLd + b] * Vs[b * kLd + j];
+        X[i + (size_t)(k + j) * ld] = v;
+      }
   }
 }
 
 // X[C, :] <- V_C^T X[C, :] (trans = 1) or V_C X[C, :] (trans = 0), columns 0..ncols-1.
 __global__ void __launch_bounds__(kMaxCluster) k_blk_left(
-    int ncols, double *__restrict__ X, long long ld, int trans, const int *__restrict__ cstart,
+    int ncols, double *__restrict__ X, long long ld, int trans, const int *__restrict__ list,
     const int *__restrict__ csize, const double *__restrict__ Vbuf) {
-  const int k = blockIdx.y;
-  const int m = csize[k];
-  if (cstart[k] != k || m < 2) return;
   extern __shared__ double sm[];
   double *Vs = sm, *Xs = sm + kMaxCluster * kLd;
   const int t = threadIdx.x;
-  // Vs[a][b] = (trans ? V^T : V)[a][b]
-  for (int a = 0; a < m; ++a)
-    if (t < m)
-      Vs[a * kLd + t] = trans ? Vbuf[(size_t)(k + t) * kMaxCluster + a]
-                              : Vbuf[(size_t)(k + a) * kMaxCluster + t];
-  const int c = blockIdx.x * kMaxCluster + t;
-  if (c < ncols)
-    for (int b = 0; b < m; ++b) Xs[t * kLd + b] = X[(size_t)(k + b) + (size_t)c * ld];
-  __syncthreads();
-  if (c >= ncols) return;
-  for (int a = 0; a < m; ++a) {
-    double v = 0.0;
-    for (int b = 0; b < m; ++b) v += Vs[a * kLd + b] * Xs[t * kLd + b];
-    X[(size_t)(k + a) + (size_t)c * ld] = v;
+  for (int ci = blockIdx.y; ci < list[0]; ci += gridDim.y) {
+    const int k = list[1 + ci];
+    const int m = csize[k];
+    __syncthreads();  // Vs and Xs of the last cluster
+    // Vs[a][b] = (trans ? V^T : V)[a][b]
+    for (int a = 0; a < m; ++a)
+      if (t < m)
+        Vs[a * kLd + t] = trans ? Vbuf[(size_t)(k + t) * kMaxCluster + a]
+                                : Vbuf[(size_t)(k + a) * kMaxCluster + t];
+    const int c = blockIdx.x * kMaxCluster + t;
+    if (c < ncols)
+      for (int b = 0; b < m; ++b) Xs[t * kLd + b] = X[(size_t)(k + b) + (size_t)c * ld];
+    __syncthreads();
+    if (c < ncols)
+      for (int a = 0; a < m; ++a) {
+        double v = 0.0;
+        for (int b = 0; b < m; ++b) v += Vs[a * kLd + b] * Xs[t * kLd + b];
+        X[(size_t)(k + a) + (size_t)c * ld] = v;
+      }
   }
 }
 
@@ -605,7 +615,7 @@ int refine_from_fp32(gc_context *ctx, int N, int prec, const double *M, const fl
   *fallback = false;
   const size_t NN = (size_t)N * N;
   gc::DevBuf<double> U0, U1, vbuf, dS, dG;
-  gc::DevBuf<int> cst, csz, flag;
+  gc::DevBuf<int> cst, csz, flag, list;
   gc::DevBuf<double> colm;
   GC_TRY(U0.alloc(ctx, 2 * NN));
   GC_TRY(U1.alloc(ctx, 2 * NN));
@@ -614,6 +624,7 @@ int refine_from_fp32(gc_context *ctx, int N, int prec, const double *M, const fl
   GC_TRY(dG.alloc(ctx, N));
   GC_TRY(cst.alloc(ctx, N));
   GC_TRY(csz.alloc(ctx, N));
+  GC_TRY(list.alloc(ctx, N + 1));
   GC_TRY(flag.alloc(ctx, 2));
   GC_TRY(colm.alloc(ctx, N));
   GC_CUDA(ctx, cudaFuncSetAttribute(k_cluster_eig, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -652,17 +663,22 @@ int refine_from_fp32(gc_context *ctx, int N, int prec, const double *M, const fl
     GC_LAUNCHED(ctx);
     k_col_coupling<<<N, 256, 0, ctx->stream>>>(N, G, S, lam, colm.p);
     GC_LAUNCHED(ctx);
-    k_clusters<<<gN, 256, 0, ctx->stream>>>(N, lam, colm.p, cst.p, csz.p, flag.p);
+    GC_CUDA(ctx, cudaMemsetAsync(list.p, 0, sizeof(int), ctx->stream));
+    k_clusters<<<gN, 256, 0, ctx->stream>>>(N, lam, colm.p, cst.p, csz.p, flag.p, list.p);
     GC_LAUNCHED(ctx);
-    k_cluster_eig<<<N, kMaxCluster, kClusterSmem, ctx->stream>>>(N, G, S, cst.p, csz.p, vbuf.p,
-                                                                 flag.p, flag.p + 1);
+    // Blocks for a few dozen clusters at once (a spectrum has tens, not N): with a block per
+    // index that left at once unless a cluster began there, the seven launches of two
+    // iterations took 310 us at N = 1390.
+    const unsigned nc = std::min(N, 64);
+    k_cluster_eig<<<nc, kMaxCluster, kClusterSmem, ctx->stream>>>(N, G, S, list.p, csz.p, vbuf.p,
+                                                                  flag.p, flag.p + 1);
     GC_LAUNCHED(ctx);
-    const dim3 gr(gc::ceil_div(N, kMaxCluster), N), gl2(gc::ceil_div(2 * (size_t)N, kMaxCluster), N);
-    k_blk_right<<<gr, kMaxCluster, kBlkSmem, ctx->stream>>>(N, G, N, cst.p, csz.p, vbuf.p);
+    const dim3 gr(gc::ceil_div(N, kMaxCluster), nc), gl2(gc::ceil_div(2 * (size_t)N, kMaxCluster), nc);
+    k_blk_right<<<gr, kMaxCluster, kBlkSmem, ctx->stream>>>(N, G, N, list.p, csz.p, vbuf.p);
     GC_LAUNCHED(ctx);
-    k_blk_right<<<gr, kMaxCluster, kBlkSmem, ctx->stream>>>(N, S, N, cst.p, csz.p, vbuf.p);
+    k_blk_right<<<gr, kMaxCluster, kBlkSmem, ctx->stream>>>(N, S, N, list.p, csz.p, vbuf.p);
     GC_LAUNCHED(ctx);
-    k_blk_left<<<gl2, kMaxCluster, kBlkSmem, ctx->stream>>>(2 * N, G, N, 1, cst.p, csz.p, vbuf.p);
+    k_blk_left<<<gl2, kMaxCluster, kBlkSmem, ctx->stream>>>(2 * N, G, N, 1, list.p, csz.p, vbuf.p);
     GC_LAUNCHED(ctx);
     k_rayleigh<<<gN, 256, 0, ctx->stream>>>(N, G, S, lam, dS.p, dG.p);
     GC_LAUNCHED(ctx);
@@ -680,7 +696,7 @@ int refine_from_fp32(gc_context *ctx, int N, int prec, const double *M, const fl
     }
     k_second_order<<<ew, 256, 0, ctx->stream>>>(NN, N, P, S);
     GC_LAUNCHED(ctx);
-    k_blk_left<<<gr, kMaxCluster, kBlkSmem, ctx->stream>>>(N, P, N, 0, cst.p, csz.p, vbuf.p);
+    k_blk_left<<<gr, kMaxCluster, kBlkSmem, ctx->stream>>>(N, P, N, 0, list.p, csz.p, vbuf.p);
     GC_LAUNCHED(ctx);
     GC_TRY(product(ctx, prec, false, N, N, N, X, N, P, N, G, N));        // X' = X (V (I + E))
     std::swap(cur, nxt);
@@ -729,16 +745,34 @@ int chol_plain(gc_context *ctx, int N, double *A, int *minor) {
 constexpr int kCholNb = 64;
 constexpr int kCholLd = kCholNb + 1;  // padded column stride of the shared block
 
+// 1 / d for d > 0 to about an ulp: FP32 reciprocal of the mantissa, one third-order step. A
+// library square root and division are a chain of some 25 FP64 instructions, each of which
+// holds its quarter of the SM for 64 cycles; the conversions are integer work for that reason.
+__device__ __forceinline__ double reciprocal(double d) {
+  const unsigned hi = (unsigned)__double2hiint(d), lo = (unsigned)__double2loint(d);
+  const int e = (int)(hi >> 20) - 1023;  // d > 0
+  if (e < -1000 || e > 1000) return 1.0 / d;
+  const double m = __hiloint2double((int)((hi & 0xfffffu) | 0x3ff00000u), (int)lo);  // [1, 2)
+  const float mf = __uint_as_float(0x3f800000u | ((hi & 0xfffffu) << 3) | (lo >> 29));
+  const unsigned yb = __float_as_uint(__fdividef(1.f, mf));  // (1/2, 1]
+  const double y = __hiloint2double((int)((yb >> 3) + 0x38000000u), (int)(yb << 29));
+  const double r = fma(-m, y, 1.0);
+  const double z = fma(y, fma(r, r, r), y);
+  return __hiloint2double((int)((unsigned)__double2hiint(z) - ((unsigned)e << 20)), __double2loint(z));
+}
+
 // Right-looking Cholesky of the kb x kb (kb <= 64) diagonal block A (leading
 // dimension lda) in shared memory; L's lower triangle is written back. The update of
 // step k uses the unscaled column k and the pivot's reciprocal, a_ij -= a_ik a_jk / d_k,
 // and the columns are scaled by 1/sqrt(d_k) at the end, so a step needs one barrier.
-// Thread 0 updates the next diagonal element and forms that pivot's factors (one FP64
-// square root and one division) while warps 1-7 update the rest of the trailing
-// triangle: the pivot's latency, not the FP64 work of one SM, set the time of a step.
-// A pivot that is not positive (or not finite) records its global order k0 + k + 1 in
-// *info, unless an earlier block already did, and is replaced by 1 so that the rest
-// stays finite.
+// Panels of 16 columns: a step updates the rest of its panel only (thread 0 the next diagonal
+// element and its pivot, the others one element per lane), and the columns to the right take the
+// panel's 16 updates at once, 16 FMAs per element: with the whole trailing triangle updated in
+// every step the half-empty warps of that one SM's FP64 pipe set the time (85 us per block;
+// 59 us so). A pivot that is not positive (or not finite) records its global order
+// k0 + k + 1 in *info, unless an earlier block already did, and is replaced by 1 so that the
+// rest stays finite.
+constexpr int kPanel = 16;
 __global__ void __launch_bounds__(256) k_potrf_block(int kb, double *__restrict__ A, long long lda,
                                                      int k0, int *__restrict__ info,
                                                      long long sb) {
@@ -746,9 +780,10 @@ __global__ void __launch_bounds__(256) k_potrf_block(int kb, double *__restrict_
   A += blockIdx.x * sb;
   info += blockIdx.x;
   __shared__ double s[kCholNb * kCholLd];
-  __shared__ double rk[kCholNb], sq[kCholNb], isq[kCholNb];  // 1/d, sqrt(d), 1/sqrt(d)
+  __shared__ double u[kPanel * kCholLd];                     // a panel's columns over their pivots
+  __shared__ double dk[kCholNb], rk[kCholNb], sq[kCholNb], isq[kCholNb];  // d, 1/d, roots
   __shared__ int bad;
-  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int t = threadIdx.x;
   for (int e = t; e < kb * kb; e += blockDim.x) {
     const int i = e % kb, j = e / kb;
     s[i + j * kCholLd] = i >= j ? A[i + j * lda] : 0.0;
@@ -759,10 +794,8 @@ __global__ void __launch_bounds__(256) k_potrf_block(int kb, double *__restrict_
       if (!bad) bad = k + 1;
       d = 1.0;
     }
-    const double is = 1.0 / sqrt(d);
-    isq[k] = is;
-    sq[k] = d * is;
-    rk[k] = is * is;
+    dk[k] = d;
+    rk[k] = reciprocal(d);
   };
   __syncthreads();
   if (t == 0) {
@@ -770,22 +803,51 @@ __global__ void __launch_bounds__(256) k_potrf_block(int kb, double *__restrict_
     pivot(0);
   }
   __syncthreads();
-  for (int k = 0; k + 1 < kb; ++k) {
-    const double r = rk[k];
-    if (t == 0) {  // the next diagonal element, then its pivot
-      const double akk = s[(k + 1) + k * kCholLd];
-      s[(k + 1) + (k + 1) * kCholLd] -= akk * (akk * r);
-      pivot(k + 1);
-    } else if (warp > 0) {
-      // the rest of the trailing lower triangle: warps 1-7 over columns j, lanes along them
-      for (int j = k + warp; j < kb; j += 7) {
-        const double tj = s[j + k * kCholLd] * r;
-        for (int i = j + lane; i < kb; i += 32)
-          if (i != k + 1) s[i + j * kCholLd] -= s[i + k * kCholLd] * tj;
+  for (int p0 = 0; p0 < kb; p0 += kPanel) {
+    const int p1 = min(p0 + kPanel, kb);
+    for (int k = p0; k + 1 < p1; ++k) {
+      const double r = rk[k];
+      const int rows = kb - k - 1, cnt = rows * (p1 - k - 1);
+      if (t == 0) {  // the next diagonal element, then its pivot
+        const double akk = s[(k + 1) + k * kCholLd];
+        s[(k + 1) + (k + 1) * kCholLd] -= akk * (akk * r);
+        pivot(k + 1);
+      } else if (t >= 32) {
+        for (int e = t - 32; e < cnt; e += 224) {
+          const int j = k + 1 + e / rows, i = k + 1 + e % rows;
+          if (i >= j && i + j != 2 * (k + 1))
+            s[i + j * kCholLd] -= s[i + k * kCholLd] * (s[j + k * kCholLd] * r);
+        }
       }
+      __syncthreads();
     }
-    __syncthreads();
+    const int w = kb - p1;  // the columns to the right of the panel
+    if (w > 0) {
+      for (int e = t; e < w * kPanel; e += 256) {  // a panel before another one is full
+        const int j = p1 + e % w, k = e / w;
+        u[j + k * kCholLd] = s[j + (p0 + k) * kCholLd] * rk[p0 + k];
+      }
+      __syncthreads();
+      for (int e = t; e < w * w; e += 256) {
+        const int j = p1 + e / w, i = p1 + e % w;
+        if (i < j) continue;
+        double v = s[i + j * kCholLd];
+#pragma unroll
+        for (int k = 0; k < kPanel; ++k)
+          v = fma(-s[i + (p0 + k) * kCholLd], u[j + k * kCholLd], v);
+        s[i + j * kCholLd] = v;
+      }
+      __syncthreads();
+      if (t == 0) pivot(p1);
+      __syncthreads();
+    }
   }
+  if (t < kb) {  // the roots, off the chain of pivots
+    const double is = 1.0 / sqrt(dk[t]);
+    isq[t] = is;
+    sq[t] = dk[t] * is;
+  }
+  __syncthreads();
   for (int e = t; e < kb * kb; e += blockDim.x) {
     const int i = e % kb, j = e / kb;
     if (i > j)
@@ -797,19 +859,22 @@ __global__ void __launch_bounds__(256) k_potrf_block(int kb, double *__restrict_
 }
 
 // Panel solve X L11^T = P for the m x 64 panel P below a factored 64-wide diagonal
-// block L11 (both in the matrix, leading dimension lda), X overwriting P. Four lanes
-// share a row, each holding the columns j = q (mod 4) of it in registers; column j is
-// finished by its owner lane, broadcast to the other three by a shuffle and eliminated
-// from their later columns (right-looking). A warp then holds 8 rows, so the FP64 work
-// of a panel is spread over four times as many warps as with one row per thread (GB300's
-// FP64 pipe is narrow and shared by the warps of an SM). L11 sits in shared memory with
-// a padded row stride, read by the four lanes of a row from four banks.
-constexpr int kTrsmRowsPerWarp = 8;
+// block L11 (both in the matrix, leading dimension lda), X overwriting P. LPR lanes
+// share a row, each holding the columns j = q (mod LPR) of it in registers; column j is
+// finished by its owner lane, broadcast to the others by a shuffle and eliminated
+// from their later columns (right-looking). L11 sits in shared memory with
+// a padded row stride, read by the lanes of a row from different banks. A warp's FP64
+// instructions set the time (64 cycles each on its quarter of an SM): 576 of them with 4 lanes
+// per row and 8 rows per warp, 224 with 16 lanes and 2 rows. Few rows (one matrix of order
+// 1390: 42 blocks of 4 warps) take 16 lanes, 33 -> 18 us; many take 4, which is less work
+// in all.
 constexpr int kTrsmWarps = 4;
+template <int LPR>
 __global__ void __launch_bounds__(32 * kTrsmWarps) k_trsm_rows(int m, const double *__restrict__ L11,
                                                               long long lda,
                                                               double *__restrict__ P,
                                                               long long sb) {
+  constexpr int NT = kCholNb / LPR;
   L11 += blockIdx.y * sb;  // matrix blockIdx.y of a batch
   P += blockIdx.y * sb;
   __shared__ double Ls[kCholNb * kCholLd];  // Ls[i * kCholLd + j] = L(i, j), j <= i
@@ -819,28 +884,28 @@ __global__ void __launch_bounds__(32 * kTrsmWarps) k_trsm_rows(int m, const doub
     Ls[i * kCholLd + j] = j <= i ? L11[i + j * lda] : 0.0;
   }
   for (int j = threadIdx.x; j < kCholNb; j += blockDim.x) rd[j] = 1.0 / L11[j + j * lda];
-  __syncthreads();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, q = lane & 3;
-  const long long r = ((long long)blockIdx.x * kTrsmWarps + warp) * kTrsmRowsPerWarp + (lane >> 2);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, q = lane % LPR;
+  const long long r = ((long long)blockIdx.x * kTrsmWarps + warp) * (32 / LPR) + lane / LPR;
   const bool live = r < m;
-  double acc[kCholNb / 4];
+  double acc[NT];
 #pragma unroll
-  for (int t = 0; t < kCholNb / 4; ++t) acc[t] = live ? P[r + (4 * t + q) * lda] : 0.0;
+  for (int t = 0; t < NT; ++t) acc[t] = live ? P[r + (LPR * t + q) * lda] : 0.0;
+  __syncthreads();
 #pragma unroll
   for (int j = 0; j < kCholNb; ++j) {
-    const int t0 = j >> 2, q0 = j & 3;
+    const int t0 = j / LPR, q0 = j % LPR;
     double xj = acc[t0] * rd[j];  // the owner lane's value is the one broadcast
-    xj = __shfl_sync(0xffffffffu, xj, (lane & ~3) | q0);
+    xj = __shfl_sync(0xffffffffu, xj, (lane & ~(LPR - 1)) | q0);
     if (q == q0) acc[t0] = xj;
 #pragma unroll
-    for (int t = t0; t < kCholNb / 4; ++t) {
-      const int i = 4 * t + q;
+    for (int t = t0; t < NT; ++t) {
+      const int i = LPR * t + q;
       if (i > j) acc[t] = fma(-xj, Ls[i * kCholLd + j], acc[t]);
     }
   }
   if (live)
 #pragma unroll
-    for (int t = 0; t < kCholNb / 4; ++t) P[r + (4 * t + q) * lda] = acc[t];
+    for (int t = 0; t < NT; ++t) P[r + (LPR * t + q) * lda] = acc[t];
 }
 
 // Cholesky A = L L^T of the lower triangles of nmat N x N matrices (column-major, matrix
@@ -863,8 +928,13 @@ int chol_blocked_batch(gc_context *ctx, int N, int nmat, double *A, long long sb
     GC_LAUNCHED(ctx);
     if (m == 0) break;
     double *P = A11 + kb;  // rows k0+kb.., columns k0..k0+kb
-    k_trsm_rows<<<dim3(gc::ceil_div(m, kTrsmWarps * kTrsmRowsPerWarp), nmat), 32 * kTrsmWarps, 0,
-                  ctx->stream>>>(m, A11, lda, P, sb);
+    // 16 lanes per row while that is two waves of warps (152 SMs, four at a time) or less
+    if ((long long)m * nmat <= 4 * 608)
+      k_trsm_rows<16><<<dim3(gc::ceil_div(m, kTrsmWarps * 2), nmat), 32 * kTrsmWarps, 0, ctx->stream>>>(
+          m, A11, lda, P, sb);
+    else
+      k_trsm_rows<4><<<dim3(gc::ceil_div(m, kTrsmWarps * 8), nmat), 32 * kTrsmWarps, 0, ctx->stream>>>(
+          m, A11, lda, P, sb);
     GC_LAUNCHED(ctx);
     GC_TRY(gc::tc_syrk_sub_lower(ctx, prec, m, kb, P, 1, lda, P + (size_t)kb * lda, lda, nmat, sb));
   }
