@@ -1355,14 +1355,18 @@ int slice_operand(gc_context *ctx, OzOperand &op, const double *x, int rows, int
                   long long sr, long long sk, long long sb, int tri, const OzColsOpt &opt) {
   const long long nrr = (long long)nb * rows;
   const bool plain = !tri && !opt.eig && !opt.sq;
-  if (sk == 1 && plain && op.Kp <= 1024) {
-    // one warp holds the row; up to K = 256 with half the registers (140454 x 153: 182 -> 115 us)
-    auto kern = op.Kp <= 256 ? k_oz_rows<S, 32, 2> : k_oz_rows<S, 32, 8>;
-    kern<<<gc::ceil_div(nrr, 8), 256, 0, ctx->stream>>>(x, rows, K, op.Kp, nrr, sr, sb, op.exps.p,
-                                                        op.buf.p);
-  } else if (sk == 1 && plain) {
-    k_oz_rows<S, 256, 8><<<(unsigned)nrr, 256, 0, ctx->stream>>>(x, rows, K, op.Kp, nrr, sr, sb,
-                                                              op.exps.p, op.buf.p);
+  if (sk == 1 && plain) {
+    // One warp holds a row up to K = 256 (140454 x 153: 182 -> 115 us against the instance for
+    // 1024, which has twice the registers) and, for rows enough to fill the chip, up to 1024;
+    // else a block holds it, with the registers for its length (1390 x 1390: 12 us, with the registers for K = 8192 20 us).
+    const bool warp_row = op.Kp <= 256 || (op.Kp <= 1024 && nrr >= 152 * 16);
+    auto kern = op.Kp <= 256 ? k_oz_rows<S, 32, 2>
+                             : (warp_row ? k_oz_rows<S, 32, 8>
+                                         : (op.Kp <= 1024 ? k_oz_rows<S, 256, 1>
+                                                          : (op.Kp <= 2048 ? k_oz_rows<S, 256, 2>
+                                                                           : k_oz_rows<S, 256, 8>)));
+    kern<<<warp_row ? gc::ceil_div(nrr, 8) : (unsigned)nrr, 256, 0, ctx->stream>>>(
+        x, rows, K, op.Kp, nrr, sr, sb, op.exps.p, op.buf.p);
   } else {
     const OzColView X{x, rows, K, tri, sr, sk, sb, opt};
     if (op.Kp <= kOzShortK) {
