@@ -33,7 +33,7 @@ struct gc_mlp {
   size_t woff[4], boff[4];
   int din[4], dout[4];
   gc::DevBuf<float> master, grad, m1, m2;
-  gc::DevBuf<__nv_bfloat16> wbf;  // BF16 copy of the whole parameter vector, padded by 16 bytes
+  gc::DevBuf<__nv_bfloat16> wbf;  // BF16 copy of the whole parameter vector
   gc::DevBuf<float> act;           // activations / pre-activations for the largest batch seen
   int act_batch = 0;
   gc::DevBuf<float> lossbuf;       // loss partials of the row blocks, then the loss
@@ -150,143 +150,119 @@ struct Layers {
   float *dz[4];  // dL/dZ of every layer
 };
 
-constexpr int kFusedWidth = 256;   // widest layer of the fused kernels: a warp holds a row of it
+constexpr int kFusedWidth = 256;   // widest layer of the fused kernels: one unit per thread
 constexpr int kRowThreads = 256, kRowWarps = kRowThreads / 32;
-constexpr int kPer = kFusedWidth / 32;  // inputs per lane
 
 __device__ __forceinline__ float gelu(float v) { return 0.5f * v * (1.f + erff(v * 0.70710678118654752f)); }
 __device__ __forceinline__ float gelu_grad(float z) {
   return 0.5f * (1.f + erff(z * 0.70710678118654752f)) + z * 0.3989422804014327f * expf(-0.5f * z * z);
 }
 
-// Layer l's weights (BF16, contiguous) into shared memory at dst, 16 bytes per copy from the
-// 16-byte boundary below them; returns the first weight's place. Ends with a barrier.
-__device__ __forceinline__ const __nv_bfloat16 *stage_weights(const __nv_bfloat16 *w, int count,
-                                                              unsigned char *dst) {
-  const uintptr_t a = (uintptr_t)w & ~(uintptr_t)15;
-  const int skip = (int)((uintptr_t)w - a), n16 = (skip + 2 * count + 15) / 16;
-  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+// Layer weights in shared memory: row o (BF16) at w + o * ld. Rows of a multiple of 8 weights on
+// 16-byte boundaries are copied 16 bytes at a time with all copies in flight, and padded by
+// 16 bytes, so that a thread per row reads 16 bytes without bank conflicts (vec).
+struct Staged {
+  const __nv_bfloat16 *w;
+  int ld;
+  bool vec;
+};
+__device__ __forceinline__ Staged stage_weights(const __nv_bfloat16 *w, int din, int dout,
+                                                unsigned char *dst) {
+  const bool vec = (din & 7) == 0 && ((uintptr_t)w & 15) == 0;
+  const int ld = vec ? din + 8 : din;
   __syncthreads();  // the buffer's last readers
-  for (int k = threadIdx.x; k < n16; k += kRowThreads)
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + 16 * k), "l"(a + 16 * (uintptr_t)k)
-                 : "memory");
-  asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
-  __syncthreads();
-  return reinterpret_cast<const __nv_bfloat16 *>(dst + skip);
-}
-
-// The kPer weights of row o that this lane holds: inputs 2 lane + 64 j + {0, 1} where the rows
-// are even (4-byte loads), lane + 32 j otherwise; 0 beyond the row.
-template <bool PAIR>
-__device__ __forceinline__ int lane_input(int lane, int k) {
-  return PAIR ? 2 * lane + 64 * (k / 2) + (k & 1) : lane + 32 * k;
-}
-template <bool PAIR>
-__device__ __forceinline__ void lane_weights(const __nv_bfloat16 *w, int o, int din, int lane, float *v) {
-  if (PAIR) {
-    const uint32_t *p = reinterpret_cast<const uint32_t *>(w + (size_t)o * din) + lane;
-#pragma unroll
-    for (int j = 0; j < kPer / 2; ++j) {
-      const uint32_t u = 2 * lane + 64 * j < din ? p[32 * j] : 0u;
-      v[2 * j] = __uint_as_float(u << 16);
-      v[2 * j + 1] = __uint_as_float(u & 0xffff0000u);
+  if (vec) {
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    const int n16 = din / 8;
+    for (int c = threadIdx.x; c < dout * n16; c += kRowThreads) {
+      const int o = c / n16, k = c - o * n16;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + 2 * (o * ld + 8 * k)),
+                   "l"(w + (size_t)o * din + 8 * k)
+                   : "memory");
     }
+    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
   } else {
-#pragma unroll
-    for (int k = 0; k < kPer; ++k) {
-      const int i = lane + 32 * k;
-      v[k] = i < din ? __bfloat162float(w[(size_t)o * din + i]) : 0.f;
-    }
+    __nv_bfloat16 *p = reinterpret_cast<__nv_bfloat16 *>(dst);
+#pragma unroll 4
+    for (int c = threadIdx.x; c < dout * din; c += kRowThreads) p[c] = w[c];
   }
+  __syncthreads();
+  return {reinterpret_cast<const __nv_bfloat16 *>(dst), ld, vec};
 }
 
-// out[r][o] = sum_i in[r][i] W[o, i]: a warp per pair of units, its lanes along the inputs, which
-// they hold in registers for all units.
-template <int R, bool PAIR>
-__device__ __forceinline__ void layer_forward(const float *in, int ld, const __nv_bfloat16 *w, int din,
+// out[r][o] = sum_i in[r][i] W[o, i]: a thread per unit, the sum in one chain in the order of i
+// (as the tiled kernel of wider layers adds it).
+template <int R>
+__device__ __forceinline__ void layer_forward(const float *in, int ld, const Staged &w, int din,
                                               int dout, float *out) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  float a[R][kPer];
-#pragma unroll
-  for (int k = 0; k < kPer; ++k) {
-    const int i = lane_input<PAIR>(lane, k);
-#pragma unroll
-    for (int r = 0; r < R; ++r) a[r][k] = i < din ? in[r * ld + i] : 0.f;
-  }
-  for (int o = 2 * warp; o < dout; o += 2 * kRowWarps) {
-    float v[2][kPer], acc[2 * R];
-    lane_weights<PAIR>(w, o, din, lane, v[0]);
-    lane_weights<PAIR>(w, min(o + 1, dout - 1), din, lane, v[1]);
-#pragma unroll
-    for (int u = 0; u < 2; ++u)
+  const int o = threadIdx.x;
+  if (o >= dout) return;
+  const __nv_bfloat16 *wo = w.w + o * w.ld;
+  float acc[R] = {};
+  if (w.vec) {
+#pragma unroll 4
+    for (int i = 0; i < din; i += 8) {
+      const uint4 q = *reinterpret_cast<const uint4 *>(wo + i);
+      const uint32_t u[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
       for (int r = 0; r < R; ++r) {
-        float s = 0.f;
+        const float4 a = *reinterpret_cast<const float4 *>(in + r * ld + i);
+        const float4 b = *reinterpret_cast<const float4 *>(in + r * ld + i + 4);
+        const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
 #pragma unroll
-        for (int k = 0; k < kPer; ++k) s += a[r][k] * v[u][k];
-        acc[u * R + r] = s;
-      }
-    // the 2 R sums over the lanes at once: each exchange halves the number of sums a lane holds
-    int n = 2 * R, off = 16;
-#pragma unroll
-    for (; n > 1; n /= 2, off /= 2) {
-#pragma unroll
-      for (int k = 0; k < n / 2; ++k) {
-        const bool up = lane & off;
-        const float give = up ? acc[k] : acc[k + n / 2], keep = up ? acc[k + n / 2] : acc[k];
-        acc[k] = keep + __shfl_xor_sync(0xffffffffu, give, off);
+        for (int k = 0; k < 8; ++k)
+          acc[r] += v[k] * __uint_as_float((k & 1) ? u[k / 2] & 0xffff0000u : u[k / 2] << 16);
       }
     }
-    for (; off > 0; off /= 2) acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], off);
-    // the lane's high bits say which sum it holds, highest bit of the index first
-    constexpr int LG = R == 2 ? 2 : 3;
-    const int idx = lane >> (5 - LG);
-    const int u = idx / R, r = idx % R;
-    if ((lane & ((32 >> LG) - 1)) == 0 && o + u < dout) out[r * ld + o + u] = acc[0];
+  } else {
+#pragma unroll 4
+    for (int i = 0; i < din; ++i) {
+      const float wv = __bfloat162float(wo[i]);
+#pragma unroll
+      for (int r = 0; r < R; ++r) acc[r] += in[r * ld + i] * wv;
+    }
   }
+#pragma unroll
+  for (int r = 0; r < R; ++r) out[r * ld + o] = acc[r];
 }
 
-// out[r][i] = sum_o dz[r][o] W[o, i]: the lanes along i, the units o over the warps, whose sums
-// meet in red [kRowWarps][R][kFusedWidth].
-template <int R, bool PAIR, class F>
-__device__ __forceinline__ void layer_backward(const float *dz, int ld, const __nv_bfloat16 *w, int din,
-                                               int dout, float *red, F put) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  float acc[R][kPer] = {};
-  for (int o = warp; o < dout; o += kRowWarps) {
-    float v[kPer];
-    lane_weights<PAIR>(w, o, din, lane, v);
+// put(i, r, sum_o dz[r][o] W[o, i]): a thread per input, the sum in one chain in the order of o.
+template <int R, class F>
+__device__ __forceinline__ void layer_backward(const float *dz, int ld, const Staged &w, int din,
+                                               int dout, F put) {
+  const int i = threadIdx.x;
+  if (i >= din) return;
+  float acc[R] = {};
+  int o = 0;
+#pragma unroll 2
+  for (; o + 4 <= dout; o += 4) {
+    float wv[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) wv[k] = __bfloat162float(w.w[(o + k) * w.ld + i]);
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-      const float z = dz[r * ld + o];
-#pragma unroll
-      for (int k = 0; k < kPer; ++k) acc[r][k] += z * v[k];
+      const float4 z = *reinterpret_cast<const float4 *>(dz + r * ld + o);
+      acc[r] += z.x * wv[0];
+      acc[r] += z.y * wv[1];
+      acc[r] += z.z * wv[2];
+      acc[r] += z.w * wv[3];
     }
   }
+  for (; o < dout; ++o)
 #pragma unroll
-  for (int r = 0; r < R; ++r)
+    for (int r = 0; r < R; ++r) acc[r] += dz[r * ld + o] * __bfloat162float(w.w[o * w.ld + i]);
 #pragma unroll
-    for (int k = 0; k < kPer; ++k)
-      red[(warp * R + r) * kFusedWidth + lane_input<PAIR>(lane, k)] = acc[r][k];
-  __syncthreads();
-  for (int e = threadIdx.x; e < R * din; e += kRowThreads) {
-    const int r = e / din, i = e - r * din;
-    float v = 0.f;
-#pragma unroll
-    for (int k = 0; k < kRowWarps; ++k) v += red[(k * R + r) * kFusedWidth + i];
-    put(i, r, v);
-  }
+  for (int r = 0; r < R; ++r) put(i, r, acc[r]);
 }
 
 // R rows through all layers; with t also the loss partial and dL/dZ of every layer. The chain of
 // layers is bound by latency, so each layer's weights come into shared memory with all copies in
 // flight at once, and the arithmetic then reads shared memory and registers only. Measured at 256
-// rows, 256 units: 30 us (81 us while biases and GELU were applied by one lane per unit);
-// a whole training step 222 -> 73 us with this and k_mlp_dw in place of 20 kernels.
+// rows, 256 units: 33 us; a whole training step 221 -> 76 us with this and k_mlp_dw in
+// place of 20 kernels.
 template <int R>
-constexpr size_t rows_smem() {  // weights, two activation buffers, pre-activations, partial sums
-  return 2 * (size_t)kFusedWidth * kFusedWidth + 32 +
-         sizeof(float) * kFusedWidth * R * (2 + 3 + kRowWarps);
+constexpr size_t rows_smem() {  // weights, two activation buffers, pre-activations
+  return 2 * (size_t)kFusedWidth * (kFusedWidth + 8) + sizeof(float) * kFusedWidth * R * (2 + 3);
 }
 
 template <int R>
@@ -296,8 +272,8 @@ __global__ void __launch_bounds__(kRowThreads)
                float *__restrict__ y, float *__restrict__ part) {
   extern __shared__ __align__(16) unsigned char sm[];
   constexpr int LD = kFusedWidth;
-  float *cur = reinterpret_cast<float *>(sm + 2 * (size_t)LD * LD + 32), *nxt = cur + R * LD,
-        *zs = nxt + R * LD, *red = zs + 3 * R * LD;
+  float *cur = reinterpret_cast<float *>(sm + 2 * (size_t)LD * (LD + 8)), *nxt = cur + R * LD,
+        *zs = nxt + R * LD;
   __shared__ float lred[kRowWarps], bias[4 * kFusedWidth];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int b0 = blockIdx.x * R, nr = min(R, B - b0);
@@ -307,14 +283,11 @@ __global__ void __launch_bounds__(kRowThreads)
   }
   for (int l = 0; l < 4; ++l)
     if (tid < L.dout[l]) bias[l * LD + tid] = P[L.boff[l] + tid];
-  const __nv_bfloat16 *w = nullptr;
+  Staged w{};
   for (int l = 0; l < 4; ++l) {
     const int din = L.din[l], dout = L.dout[l];
-    w = stage_weights(W + L.woff[l], din * dout, sm);
-    if ((din & 1) == 0 && ((uintptr_t)w & 3) == 0)
-      layer_forward<R, true>(cur, LD, w, din, dout, nxt);
-    else
-      layer_forward<R, false>(cur, LD, w, din, dout, nxt);
+    w = stage_weights(W + L.woff[l], din, dout, sm);
+    layer_forward<R>(cur, LD, w, din, dout, nxt);
     __syncthreads();
     for (int e = tid; e < R * dout; e += kRowThreads) {
       const int r = e / dout, o = e - r * dout;
@@ -359,16 +332,13 @@ __global__ void __launch_bounds__(kRowThreads)
   // dH = dZ W, dZ of the layer below = dH GELU'(Z); the last layer's weights are in place
   for (int l = 3; l >= 1; --l) {
     const int din = L.din[l], dout = L.dout[l];
-    if (l < 3) w = stage_weights(W + L.woff[l], din * dout, sm);
+    if (l < 3) w = stage_weights(W + L.woff[l], din, dout, sm);
     auto put = [&](int i, int r, float v) {
       const float g = v * gelu_grad(zs[((l - 1) * R + r) * LD + i]);
       nxt[r * LD + i] = g;
       if (r < nr) L.dz[l - 1][(long long)(b0 + r) * din + i] = g;
     };
-    if ((din & 1) == 0 && ((uintptr_t)w & 3) == 0)
-      layer_backward<R, true>(cur, LD, w, din, dout, red, put);
-    else
-      layer_backward<R, false>(cur, LD, w, din, dout, red, put);
+    layer_backward<R>(cur, LD, w, din, dout, put);
     __syncthreads();
     float *s = cur;
     cur = nxt;
@@ -395,69 +365,48 @@ __device__ __forceinline__ void adam_one(const AdamArgs &a, long long k, float g
 // dW_l[o, i] = sum_b dZ_l[b, o] in_l[b, i] and db_l[o] = sum_b dZ_l[b, o] of every layer, one
 // 32 x 32 tile per block (first[l]: first block of layer l), followed by Adam or stored. Block
 // 0 also turns the loss partials into the loss.
-// Four groups of 256 threads share the rows, so that the latency of a tile's few hundred
-// additions is covered by 32 warps; their sums meet in shared memory in a fixed order (15 us at
-// 256 rows, 256 units; 28 us with one group).
-constexpr int kDwB = 32;      // rows per group and stage
-constexpr int kDwGroups = 4;
-__global__ void __launch_bounds__(256 * kDwGroups)
+// All rows of a chunk are read at once, then each output is one chain of additions in the order
+// of the rows (15 us at 256 rows, 256 units).
+constexpr int kDwB = 256;  // rows per chunk
+constexpr size_t kDwSmem = sizeof(float) * kDwB * (36 + 33);
+__global__ void __launch_bounds__(256)
     k_mlp_dw(int B, Layers L, int4 first, const float *__restrict__ x, float *__restrict__ grad,
              float *__restrict__ w, float *__restrict__ m, float *__restrict__ v,
              __nv_bfloat16 *__restrict__ wbf, AdamArgs ad, int npart, float *__restrict__ lossbuf,
              double nout) {
-  __shared__ __align__(16) float zt[kDwGroups][kDwB][36];
-  __shared__ float at[kDwGroups][kDwB][33];
+  extern __shared__ __align__(16) float dws[];
+  float *zt = dws, *at = dws + kDwB * 36;  // [row][36], [row][33]
   const int blk = blockIdx.x;
   const int l = blk >= first.w ? 3 : (blk >= first.z ? 2 : (blk >= first.y ? 1 : 0));
   const int t0 = blk - (l == 0 ? first.x : (l == 1 ? first.y : (l == 2 ? first.z : first.w)));
   const int din = L.din[l], dout = L.dout[l], nti = (din + 31) / 32;
   const int o0 = (t0 / nti) * 32, i0 = (t0 % nti) * 32;
   const float *dz = L.dz[l], *in = l == 0 ? x : L.h[l - 1];
-  const int gr = threadIdx.x >> 8, tid = threadIdx.x & 255;
+  const int tid = threadIdx.x;
   const int tx = tid & 31, ty = tid >> 5;  // the thread's outputs: i0 + tx; o0 + 4 ty + k
   float acc[4] = {}, db = 0.f;
-  for (int b = 0; b < B; b += kDwB * kDwGroups) {
-#pragma unroll
-    for (int k = 0; k < kDwB / 8; ++k) {
-      const int r = ty + 8 * k, bb = b + gr * kDwB + r;
-      zt[gr][r][tx] = bb < B && o0 + tx < dout ? dz[(long long)bb * dout + o0 + tx] : 0.f;
-      at[gr][r][tx] = bb < B && i0 + tx < din ? in[(long long)bb * din + i0 + tx] : 0.f;
+  for (int b = 0; b < B; b += kDwB) {
+    const int nb = min(kDwB, B - b);
+#pragma unroll 16
+    for (int r = ty; r < nb; r += 8) {
+      zt[r * 36 + tx] = o0 + tx < dout ? dz[(long long)(b + r) * dout + o0 + tx] : 0.f;
+      at[r * 33 + tx] = i0 + tx < din ? in[(long long)(b + r) * din + i0 + tx] : 0.f;
     }
     __syncthreads();
-    float s[4] = {};
 #pragma unroll 8
-    for (int r = 0; r < kDwB; ++r) {
-      const float a = at[gr][r][tx];
-      const float4 z = *reinterpret_cast<const float4 *>(&zt[gr][r][4 * ty]);
-      s[0] += z.x * a;
-      s[1] += z.y * a;
-      s[2] += z.z * a;
-      s[3] += z.w * a;
+    for (int r = 0; r < nb; ++r) {
+      const float a = at[r * 33 + tx];
+      const float4 z = *reinterpret_cast<const float4 *>(zt + r * 36 + 4 * ty);
+      acc[0] += z.x * a;
+      acc[1] += z.y * a;
+      acc[2] += z.z * a;
+      acc[3] += z.w * a;
     }
-#pragma unroll
-    for (int k = 0; k < 4; ++k) acc[k] += s[k];
-    if (i0 == 0 && ty == 0) {
-      float d = 0.f;
+    if (i0 == 0 && ty == 0)
 #pragma unroll 8
-      for (int r = 0; r < kDwB; ++r) d += zt[gr][r][tx];
-      db += d;
-    }
+      for (int r = 0; r < nb; ++r) db += zt[r * 36 + tx];
     __syncthreads();
   }
-  // the groups' sums: [4 k + ty][tx] per group (zt's storage)
-  float *red = &zt[0][0][0];  // 3 x 32 x 33 floats of the 4 x 32 x 36
-  if (gr > 0) {
-#pragma unroll
-    for (int k = 0; k < 4; ++k) red[((gr - 1) * 32 + 4 * ty + k) * 33 + tx] = acc[k];
-    if (ty == 0) at[gr][0][tx] = db;
-  }
-  __syncthreads();
-  if (gr > 0) return;
-#pragma unroll
-  for (int k = 0; k < 4; ++k)
-#pragma unroll
-    for (int q = 0; q < kDwGroups - 1; ++q) acc[k] += red[(q * 32 + 4 * ty + k) * 33 + tx];
-  for (int q = 1; q < kDwGroups; ++q) db += at[q][0][tx];
   auto put = [&](long long k, float g) {
     if (ad.on)
       adam_one(ad, k, g, w, m, v, wbf);
@@ -561,7 +510,13 @@ int fused_step(gc_context *ctx, gc_mlp *m, int B, const float *x, const float *t
   int first[5] = {0};
   for (int l = 0; l < 4; ++l)
     first[l + 1] = first[l] + (int)(gc::ceil_div(L.dout[l], 32) * gc::ceil_div(L.din[l], 32));
-  k_mlp_dw<<<first[4], 256 * kDwGroups, 0, ctx->stream>>>(B, L, make_int4(first[0], first[1], first[2], first[3]), x,
+  static std::once_flag once;
+  static cudaError_t cfg = cudaSuccess;
+  std::call_once(once, [] {
+    cfg = cudaFuncSetAttribute(k_mlp_dw, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDwSmem);
+  });
+  GC_CUDA(ctx, cfg);
+  k_mlp_dw<<<first[4], 256, kDwSmem, ctx->stream>>>(B, L, make_int4(first[0], first[1], first[2], first[3]), x,
                                               m->grad.p, m->master.p, m->m1.p, m->m2.p, m->wbf.p, ad,
                                               nblk, m->lossbuf.p, (double)B * m->out);
   GC_LAUNCHED(ctx);
@@ -667,7 +622,7 @@ int gc_mlp_create(gc_context *ctx, int in_dim, int hidden, int out_dim, unsigned
   int r;
   if ((r = m->master.upload(ctx, h.data(), off)) != GC_OK || (r = m->grad.alloc(ctx, off)) != GC_OK ||
       (r = m->m1.alloc(ctx, off)) != GC_OK || (r = m->m2.alloc(ctx, off)) != GC_OK ||
-      (r = m->wbf.alloc(ctx, off + 8)) != GC_OK) {
+      (r = m->wbf.alloc(ctx, off)) != GC_OK) {
     delete m;
     return r;
   }
