@@ -303,25 +303,27 @@ __global__ void k_ac0_right(int N, int n, int nocc, const double *__restrict__ a
                             const int *__restrict__ grp, const double *__restrict__ fofo,
                             double *__restrict__ tp, double *__restrict__ tm,
                             double *__restrict__ tk) {
-  const int r = blockIdx.x * blockDim.x + threadIdx.x, c = blockIdx.y;
-  const int s = bs[c], m = bz[c], cc = c - s;
-  if (r >= s + m) return;
-  const int p = pp[r], q = pq[r], g = grp[p], gg = grp[q];
-  const size_t ld = (size_t)n * nocc;
-  double vp = 0.0, vm = 0.0, vk = 0.0;
-  for (int b = 0; b < m; ++b) {
-    const int k = s + b, rr = pp[k], ss = pq[k];
-    const size_t e = (size_t)r + (size_t)k * N;
-    const double y = Yrow[(size_t)k * kRow + cc];
-    vp += a1p[e] * Xrow[(size_t)k * kRow + cc];
-    vm += a1m[e] * y;
-    if (!(g == gg && gg == grp[rr] && grp[rr] == grp[ss]))
-      vk += cpl[k] * fofo[((size_t)rr + (size_t)ss * n) * ld + p + (size_t)q * n] * y;
+  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  for (int c = blockIdx.y; c < N; c += gridDim.y) {
+    const int s = bs[c], m = bz[c], cc = c - s;
+    if (r >= s + m) continue;
+    const int p = pp[r], q = pq[r], g = grp[p], gg = grp[q];
+    const size_t ld = (size_t)n * nocc;
+    double vp = 0.0, vm = 0.0, vk = 0.0;
+    for (int b = 0; b < m; ++b) {
+      const int k = s + b, rr = pp[k], ss = pq[k];
+      const size_t e = (size_t)r + (size_t)k * N;
+      const double y = Yrow[(size_t)k * kRow + cc];
+      vp += a1p[e] * Xrow[(size_t)k * kRow + cc];
+      vm += a1m[e] * y;
+      if (!(g == gg && gg == grp[rr] && grp[rr] == grp[ss]))
+        vk += cpl[k] * fofo[((size_t)rr + (size_t)ss * n) * ld + p + (size_t)q * n] * y;
+    }
+    const size_t o = (size_t)r + (size_t)c * N;
+    tp[o] = vp;
+    tm[o] = vm;
+    tk[o] = cpl[r] * vk;
   }
-  const size_t o = (size_t)r + (size_t)c * N;
-  tp[o] = vp;
-  tm[o] = vm;
-  tk[o] = cpl[r] * vk;
 }
 
 // The energy sum_{r,c} work[r, c] (Ybd^T K Ybd)[r, c] with
@@ -482,7 +484,7 @@ extern "C" int gc_ac0cas_fofo(gc_context *ctx, int nbas, int ninact, int nact, i
   // Products with the block-diagonal factors; T+ and T- go into a0p and a0m.
   gc::DevBuf<double> tk, part, res;
   GC_TRY(tk.alloc(ctx, NN));
-  k_ac0_right<<<dim3(gc::ceil_div(N, 256), N), 256, 0, ctx->stream>>>(
+  k_ac0_right<<<dim3(gc::ceil_div(N, 256), std::min(N, 65535)), 256, 0, ctx->stream>>>(
       N, n, nocc, a1p.p, a1m.p, pbs.p, pbz.p, Xrow.p, Yrow.p, sd.pair_p.p, sd.pair_q.p, sd.cpl.p,
       sd.grp.p, fofo, a0p.p, a0m.p, tk.p);
   GC_LAUNCHED(ctx);

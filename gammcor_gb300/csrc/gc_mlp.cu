@@ -21,7 +21,6 @@
 #include <cuda_bf16.h>
 
 #include <cmath>
-#include <mutex>
 #include <random>
 
 #include "gc_internal.cuh"
@@ -481,13 +480,9 @@ int fused_rows_per_block(int B) { return B <= 2 * 152 ? 2 : 4; }
 template <int R>
 int fused_rows(gc_context *ctx, gc_mlp *m, int B, const Layers &L, const float *x, const float *t,
                float *y) {
-  static std::once_flag once;
-  static cudaError_t cfg = cudaSuccess;
-  std::call_once(once, [] {
-    cfg = cudaFuncSetAttribute(k_mlp_rows<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)rows_smem<R>());
-  });
-  GC_CUDA(ctx, cfg);
+  // on every call: the setting holds for one device
+  GC_CUDA(ctx, cudaFuncSetAttribute(k_mlp_rows<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)rows_smem<R>()));
   k_mlp_rows<R><<<gc::ceil_div(B, R), kRowThreads, rows_smem<R>(), ctx->stream>>>(
       B, L, m->wbf.p, m->master.p, x, t, 1.f / (float)((long long)B * m->out), y, m->lossbuf.p);
   GC_LAUNCHED(ctx);
@@ -510,12 +505,8 @@ int fused_step(gc_context *ctx, gc_mlp *m, int B, const float *x, const float *t
   int first[5] = {0};
   for (int l = 0; l < 4; ++l)
     first[l + 1] = first[l] + (int)(gc::ceil_div(L.dout[l], 32) * gc::ceil_div(L.din[l], 32));
-  static std::once_flag once;
-  static cudaError_t cfg = cudaSuccess;
-  std::call_once(once, [] {
-    cfg = cudaFuncSetAttribute(k_mlp_dw, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDwSmem);
-  });
-  GC_CUDA(ctx, cfg);
+  GC_CUDA(ctx, cudaFuncSetAttribute(k_mlp_dw, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)kDwSmem));
   k_mlp_dw<<<first[4], 256, kDwSmem, ctx->stream>>>(B, L, make_int4(first[0], first[1], first[2], first[3]), x,
                                               m->grad.p, m->master.p, m->m1.p, m->m2.p, m->wbf.p, ad,
                                               nblk, m->lossbuf.p, (double)B * m->out);

@@ -1426,7 +1426,7 @@ int make_oz_packed(gc_context *ctx, OzOperand &op, const double *x, long long ld
   const unsigned nt = op.Kp / 64, tiles = nt * (nt + 1) / 2;
   const dim3 grid(cnt, std::max(1u, std::min(gc::ceil_div(304, cnt), tiles)));
   const size_t sm = (size_t)n * sizeof(unsigned);
-  constexpr size_t kMaxSm = 128 * 1024;
+  constexpr size_t kMaxSm = 188 * 1024;  // n <= 48128, beyond the 46340 whose n^2 fits an int
   if (sm > kMaxSm) return gc::set_error(ctx, GC_EUNSUPPORTED, "packed operand: n=%d", n);
   auto kern = S == 4 ? k_oz_packed<4> : (S == 5 ? k_oz_packed<5> : k_oz_packed<6>);
   if (sm > 8 * 1024)
