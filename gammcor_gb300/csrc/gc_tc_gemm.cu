@@ -198,6 +198,12 @@ __device__ __forceinline__ void tmem_ld8_issue(uint32_t taddr, uint32_t *r) {
                : "r"(taddr));
 }
 
+__device__ __forceinline__ void tmem_ld4_issue(uint32_t taddr, uint32_t *r) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(taddr));
+}
+
 __device__ __forceinline__ void tmem_ld_wait() {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
@@ -352,16 +358,16 @@ __global__ void __launch_bounds__(192, 1)
 // chunks short enough that every FP32 partial sum is an integer below 2^24, so
 // each chunk is exact, and the epilogue adds the chunks in FP64 registers.
 // Column tile (TBN rows of B): the S weight accumulators take S * TBN of the 512 TMEM
-// columns, so TBN = 128 for S = 4, 96 for S = 5 and 64 for S = 6 at most. A wider
+// columns, so TBN = 128 for S = 4, 96 for S = 5 and 64 for S = 6 at most (half of them where two
+// CTAs share an SM: 48 for S <= 5, 32). A wider
 // tile reads fewer operand bytes per product (shared memory and L2); a narrower
 // one gives more CTAs to a small product. oz_tile() picks one per GEMM; every
 // width gives the same result bits (each element's integer sums are the same).
 constexpr int OZ_BK = 32;      // K per stage: 32 BF16 = one 64-byte swizzled row
-// Each stage holds every slice of A and of B. The 32-wide tile (products with at most 32 columns:
-// the occupied block of a transform) takes two, so that two CTAs share an SM and one's
-// epilogue runs beside the other's products (372006 x 28 x 249: 185 us, with the 64-wide tile
-// 283 us).
-__host__ __device__ constexpr int oz_stages(int tbn) { return tbn == 32 ? 2 : 3; }
+// Each stage holds every slice of A and of B. The 32- and 48-wide tiles (the occupied block of a
+// transform; products with a short K) take two, so that two CTAs share an SM and one's epilogue
+// runs beside the other's products (372006 x 28 x 249: 185 us, with the 64-wide tile 270 us).
+__host__ __device__ constexpr int oz_stages(int tbn) { return tbn < 64 ? 2 : 3; }
 // TMEM columns allocated: a power of two that holds the S weight accumulators.
 __host__ __device__ constexpr int oz_tmem_cols(int S, int tbn) {
   return S * tbn <= 128 ? 128 : (S * tbn <= 256 ? 256 : 512);
@@ -373,8 +379,13 @@ constexpr int OZ_MAXS = 6;
 constexpr int kBadExp = 0x7fffffff;
 
 constexpr int OZ_GROUP_M = 8;  // row tiles per raster group
-// Epilogue: four warps (one per TMEM lane quarter) per 32 columns of the tile.
-__host__ __device__ constexpr int oz_epi_warps(int tbn) { return 4 * (tbn / 32); }
+// Epilogue: four warps (one per TMEM lane quarter) per 16 columns of the tile. It is a chain of
+// integer operations per column, bound by latency, so more warps with fewer columns each
+// shorten it: with 32 columns per warp 140454 x 153 x 64 took 219 us instead of 197 (64-wide), with
+// 48 columns 191 us instead of 141 (48-wide). From 96 columns on 16 would leave too few registers
+// (or more than 1024 threads), and gained nothing.
+__host__ __device__ constexpr int oz_epi_cols(int tbn) { return tbn >= 96 ? 32 : 16; }
+__host__ __device__ constexpr int oz_epi_warps(int tbn) { return 4 * (tbn / oz_epi_cols(tbn)); }
 __host__ __device__ constexpr int oz_threads(int tbn) {  // TMA warp, MMA warp, epilogue
   return 64 + 32 * oz_epi_warps(tbn);
 }
@@ -428,14 +439,14 @@ __device__ __forceinline__ double scaled_double(long long t, int sc) {
 }
 
 template <int S, int TBN>
-__global__ void __launch_bounds__(oz_threads(TBN), TBN == 32 ? 2 : 1)
+__global__ void __launch_bounds__(oz_threads(TBN), TBN < 64 ? 2 : 1)
     k_tc_gemm_oz(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
                  int M, int N, int kblocks, int a_batched, int b_batched, OzPlan plan, OzEpi epi,
                  int *err_flag, unsigned long long wait_ns) {
   // One stage = the K block [kb*32, kb*32+32) of all S slices of the A tile (128 rows)
   // and of the B tile (TBN rows): every slice product t+u < S of the block is
   // issued from it, so each slice tile crosses L2 -> shared memory once per block.
-  static_assert(S * TBN <= 512 && TBN % 32 == 0, "S weight accumulators exceed TMEM");
+  static_assert(S * TBN <= (TBN < 64 ? 256 : 512) && TBN % 16 == 0, "S weight accumulators exceed TMEM");
   constexpr int EPI = oz_epi_warps(TBN), STG = oz_stages(TBN);
   constexpr uint32_t TCOLS = oz_tmem_cols(S, TBN);
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -598,10 +609,10 @@ __global__ void __launch_bounds__(oz_threads(TBN), TBN == 32 ? 2 : 1)
     // (128 |v_0| + |v_1| and 128 |v_2| + |v_3| are below 2^31: v_0 sums products up to 2^14, v_2
     // up to 2 2^13 + 2^12, over at most 672 K), and two 32 x 32 + 64 multiply-adds put the pairs
     // in place: the MMAs of the next chunk wait for this.
-    // Four warps per 32 columns (one per TMEM lane quarter, q = warp % 4); warp group
-    // h = (warp - 2) / 4 owns columns [32 h, 32 h + 32) of the tile.
+    // Four warps per NC columns (one per TMEM lane quarter, q = warp % 4); warp group
+    // h = (warp - 2) / 4 owns columns [NC h, NC h + NC) of the tile.
     constexpr int SI = S < 5 ? S : 5;
-    constexpr int NC = 32;
+    constexpr int NC = oz_epi_cols(TBN), LW = NC == 16 ? 4 : 8;
     const int q = warp & 3;
     const int h = (warp - 2) / 4;
     const int m = m0 + q * 32 + lane;
@@ -616,15 +627,19 @@ __global__ void __launch_bounds__(oz_threads(TBN), TBN == 32 ? 2 : 1)
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
-      for (int c0 = 0; c0 < NC; c0 += 8) {
-        uint32_t r[S][8];
+      for (int c0 = 0; c0 < NC; c0 += LW) {
+        uint32_t r[S][LW];
 #pragma unroll
-        for (int d = 0; d < S; ++d)
-          tmem_ld8_issue(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(d * TBN + h * NC + c0),
-                         r[d]);
+        for (int d = 0; d < S; ++d) {
+          const uint32_t a = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(d * TBN + h * NC + c0);
+          if constexpr (LW == 8)
+            tmem_ld8_issue(a, r[d]);
+          else
+            tmem_ld4_issue(a, r[d]);
+        }
         tmem_ld_wait();
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
+        for (int j = 0; j < LW; ++j) {
           int v[S];
 #pragma unroll
           for (int d = 0; d < SI; ++d) v[d] = __float2int_rn(__uint_as_float(r[d][j]));
@@ -671,15 +686,16 @@ __global__ void __launch_bounds__(oz_threads(TBN), TBN == 32 ? 2 : 1)
         for (int j = 0; j < NC; ++j)
           if (j < nn && m >= n1 + j) epi.c[o0 + j * epi.ldn] = cv[j];
         // the mirror image, turned in shared memory (the stages are free: every load was
-        // consumed by a product that has completed): stores of 32 consecutive elements
-        double *tr = reinterpret_cast<double *>(smem) + (warp - 2) * (32 * 33);
+        // consumed by a product that has completed): stores of NC consecutive elements
+        double *tr = reinterpret_cast<double *>(smem) + (warp - 2) * (NC * 33);
 #pragma unroll
         for (int j = 0; j < NC; ++j) tr[j * 33 + lane] = cv[j];
         __syncwarp();
-        const int n = n1 + lane, mb = m0 + q * 32;
-        for (int i = 0; i < 32; ++i) {
-          const int mm = mb + i;
-          if (mm < M && n < N && mm >= n) epi.c[n + (long long)mm * epi.ldn] = tr[lane * 33 + i];
+        const int n = n1 + lane % NC, mb = m0 + q * 32 + lane / NC;
+        for (int i = 0; i < NC; ++i) {
+          const int k = i * (32 / NC), mm = mb + k;
+          if (mm < M && n < N && mm >= n)
+            epi.c[n + (long long)mm * epi.ldn] = tr[(lane % NC) * 33 + k + lane / NC];
         }
       } else {
         const double *src = epi.mode == 2 ? epi.c : epi.r;
@@ -1459,35 +1475,48 @@ static_assert(oz_smem_bytes(4, 128) <= 232448 && oz_smem_bytes(5, 96) <= 232448 
                   oz_smem_bytes(6, 64) <= 232448,
               "sliced GEMM stages exceed the 227 KB of shared memory per CTA");
 
-// Relative time per CTA of the wider tiles (one CTA per SM at a time), measured at 6290^3 on
-// GB300 (ms per wave of 152 CTAs: FP64TC5 0.149 at 64 and 0.196 at 96; FP64TC4 0.122, 0.145 and
-// 0.174 at 64, 96 and 128).
-constexpr double oz_tile_cost(int S, int tbn) {
-  return tbn == 64 ? 1.0 : (tbn == 96 ? (S == 4 ? 1.19 : 1.31) : 1.43);
+// Time in us of one wave of tiles (152 CTAs, 304 of the 48-wide tile) for K = 64 kb: the
+// pipeline's start and the epilogue, and the products. Measured on GB300 at 140454 x 153 for
+// K = 64..1024; at 6290^3 the waves so come out within 2%. The 48-wide tile's two CTAs per SM run
+// one's epilogue beside the other's products: the best of the widths up to K of about 500
+// (K = 64: 141 us against 183 with 96 columns and 197 with 64; K = 249: 236, 263, 285), where the
+// epilogue is longer than the products.
+double oz_wave_us(int S, int tbn, double kb) {
+  const bool s4 = S == 4;
+  switch (tbn) {
+    case 48: return s4 ? 7.0 + 1.68 * kb : 7.3 + 2.12 * kb;
+    case 64: return s4 ? 7.2 + 1.08 * kb : 7.5 + 1.42 * kb;
+    case 96: return s4 ? 9.6 + 1.43 * kb : 10.3 + 1.93 * kb;
+    default: return 12.3 + 1.61 * kb;
+  }
 }
 
-// Tile width for an M x N x nbatch product: the narrowest width unless a wider one
-// finishes its CTA waves (152 SMs, one CTA each) sooner by the costs above. tri: only the
-// tiles that reach the lower triangle of an M x M product are computed (N = M); at 3774 that
-// is 4.1 waves of 96-wide tiles, 5 in effect, and 64-wide ones finish sooner.
-int oz_tile(const gc_context *ctx, int S, long long M, long long N, long long nbatch,
+// Tile width for an M x N x K x nbatch product: the one whose waves of CTAs finish first by the
+// times above. tri: only the tiles that reach the lower triangle of an M x M product are
+// computed (N = M). Six slices take 64 columns (two CTAs of 48 would not fit TMEM), products of
+// at most 32 columns the 32-wide tile.
+int oz_tile(const gc_context *ctx, int S, long long M, long long N, long long K, long long nbatch,
             bool tri = false) {
   const int widest = oz_max_tile(S);
   if (ctx->oz_tile > 0) return std::min(ctx->oz_tile, widest);
   if (N <= 32 && !tri) return 32;
-  int best = 64;
-  double best_cost = 0.0;
-  for (int tbn = 64; tbn <= widest; tbn += 32) {
+  if (widest == 64) return 64;
+  int best = 0;
+  double best_us = 0.0;
+  for (int tbn : {64, 48, 96, 128}) {
+    if (tbn > widest) continue;
     const long long ntm = (M + BM - 1) / BM, ntn = (N + tbn - 1) / tbn;
     long long ctas = ntm * ntn;
     if (tri) {
       ctas = 0;
       for (long long i = 0; i < ntm; ++i) ctas += std::min(ntn, (std::min((i + 1) * BM, M) + tbn - 1) / tbn);
     }
-    const double cost = (double)((ctas * nbatch + 151) / 152) * oz_tile_cost(S, tbn);
-    if (tbn == 64 || cost < best_cost) {
+    const int per_wave = tbn == 48 ? 304 : 152;
+    const double us = (double)((ctas * nbatch + per_wave - 1) / per_wave) *
+                      oz_wave_us(S, tbn, (double)((K + BK - 1) / BK));
+    if (best == 0 || us < best_us) {
       best = tbn;
-      best_cost = cost;
+      best_us = us;
     }
   }
   return best;
@@ -1523,6 +1552,10 @@ int run_oz(gc_context *ctx, const OzOperand &A, const OzOperand &B, int M, int N
   if (pl.S == 6 && w == 32) return launch_oz<6, 32>(ctx, A, B, M, N, nbatch, pl, epi);
   if (pl.S == 5 && w == 32) return launch_oz<5, 32>(ctx, A, B, M, N, nbatch, pl, epi);
   if (pl.S == 4 && w == 32) return launch_oz<4, 32>(ctx, A, B, M, N, nbatch, pl, epi);
+  if (w == 48) {
+    if (pl.S == 5) return launch_oz<5, 48>(ctx, A, B, M, N, nbatch, pl, epi);
+    if (pl.S == 4) return launch_oz<4, 48>(ctx, A, B, M, N, nbatch, pl, epi);
+  }
   if (pl.S == 6 && w == 64) return launch_oz<6, 64>(ctx, A, B, M, N, nbatch, pl, epi);
   if (pl.S == 5 && w == 64) return launch_oz<5, 64>(ctx, A, B, M, N, nbatch, pl, epi);
   if (pl.S == 5 && w == 96) return launch_oz<5, 96>(ctx, A, B, M, N, nbatch, pl, epi);
@@ -1569,12 +1602,12 @@ int tc_half_packed(gc_context *ctx, int precision, int n, int cnt, const double 
     const bool y1 = o.nY <= o.nX;
     const int nf = y1 ? o.nY : o.nX;
     GC_TRY(make_oz_operand(ctx, side[h]->first, y1 ? o.CY : o.CX, nf, n, 1, n, 1, 0, pl.S,
-                           oz_tile(ctx, pl.S, (long long)n * cs, nf, 1)));
+                           oz_tile(ctx, pl.S, (long long)n * cs, nf, n, 1)));
     if (y1)
       GC_TRY(make_oz_operand(ctx, side[h]->second, o.CX, o.nX, n, 1, n, 1, 0, pl.S, BM));
     else
       GC_TRY(make_oz_operand(ctx, side[h]->second, o.CY, o.nY, n, 1, n, 1, 0, pl.S,
-                             oz_tile(ctx, pl.S, o.nX, o.nY, cs)));
+                             oz_tile(ctx, pl.S, o.nX, o.nY, n, cs)));
   }
   for (int k0 = 0; k0 < cnt; k0 += cs) {
     const int c = std::min(cs, cnt - k0);
@@ -1593,7 +1626,7 @@ int tc_half_packed(gc_context *ctx, int precision, int n, int cnt, const double 
       if (y1) {
         // out[x + nX (y + nY k)] = sum_p CX[p, x] T[(k, p), y]: one product, columns (k, y)
         GC_TRY(make_oz_operand(ctx, B, T.p, nf, n, c, (long long)c * n, 1, n, pl.S,
-                               oz_tile(ctx, pl.S, o.nX, (long long)c * nf, 1)));
+                               oz_tile(ctx, pl.S, o.nX, (long long)c * nf, n, 1)));
         B.rows = c * nf;
         B.nb = 1;
         GC_TRY(encode_oz_map(ctx, B));
@@ -1628,11 +1661,11 @@ int tc_pair_product(gc_context *ctx, int precision, int rank, int nC, int nD, bo
   OzOperand a, b;
   GC_TRY(make_oz_operand(ctx, a, Z, R, rank, 1, 1, nCD, 0, pl.S, BM, symCD ? nC : 0));
   if (same) {  // symmetric: the lower triangle and its mirror image
-    GC_TRY(alias_oz_operand(ctx, a, b, oz_tile(ctx, pl.S, R, Q, 1, true)));
+    GC_TRY(alias_oz_operand(ctx, a, b, oz_tile(ctx, pl.S, R, Q, rank, 1, true)));
     OzEpi e{3, C, R, 0, nullptr, nullptr, nullptr, nullptr, 0, 0, R};
     GC_TRY(run_oz(ctx, a, b, R, Q, 1, pl, e));
   } else {
-    GC_TRY(make_oz_operand(ctx, b, Y, Q, rank, 1, 1, nAB, 0, pl.S, oz_tile(ctx, pl.S, R, Q, 1),
+    GC_TRY(make_oz_operand(ctx, b, Y, Q, rank, 1, 1, nAB, 0, pl.S, oz_tile(ctx, pl.S, R, Q, rank, 1),
                            symAB ? nA : 0));
     OzEpi e{0, C, R, 0, nullptr, nullptr, nullptr, nullptr, 0, 0};
     GC_TRY(run_oz(ctx, a, b, R, Q, 1, pl, e));
@@ -1682,7 +1715,7 @@ int tc_gemm_nt(gc_context *ctx, int precision, int m, int n, int k, const double
     OzPlan pl = oz_plan(precision);
     OzOperand a, b;
     GC_TRY(make_oz_operand(ctx, a, A, m, k, 1, 1, lda, 0, pl.S, BM));
-    GC_TRY(make_oz_operand(ctx, b, B, n, k, 1, 1, ldb, 0, pl.S, oz_tile(ctx, pl.S, m, n, 1)));
+    GC_TRY(make_oz_operand(ctx, b, B, n, k, 1, 1, ldb, 0, pl.S, oz_tile(ctx, pl.S, m, n, k, 1)));
     OzEpi e{0, C, ldc, 0, nullptr, nullptr, nullptr, nullptr, 0, 0};
     GC_TRY(run_oz(ctx, a, b, m, n, 1, pl, e));
     return GC_OK;  // the device flag is read at the caller's next sync point
@@ -1706,7 +1739,7 @@ int tc_gemm_strided(gc_context *ctx, int precision, int M, int N, int K, const d
   OzPlan pl = oz_plan(precision);
   OzOperand a, b;
   GC_TRY(make_oz_operand(ctx, a, A, M, K, 1, sam, sak, 0, pl.S, BM));
-  GC_TRY(make_oz_operand(ctx, b, B, N, K, 1, sbn, sbk, 0, pl.S, oz_tile(ctx, pl.S, M, N, 1)));
+  GC_TRY(make_oz_operand(ctx, b, B, N, K, 1, sbn, sbk, 0, pl.S, oz_tile(ctx, pl.S, M, N, K, 1)));
   OzEpi e{0, C, ldc, 0, nullptr, nullptr, nullptr, nullptr, 0, 0};
   GC_TRY(run_oz(ctx, a, b, M, N, 1, pl, e));
   return GC_OK;  // the device flag is read at the caller's next sync point
@@ -1720,7 +1753,7 @@ int tc_gemm_strided_lower(gc_context *ctx, int precision, int M, int N, int K, c
   OzPlan pl = oz_plan(precision);
   OzOperand a, b;
   GC_TRY(make_oz_operand(ctx, a, A, M, K, 1, sam, sak, 0, pl.S, BM));
-  GC_TRY(make_oz_operand(ctx, b, B, N, K, 1, sbn, sbk, 0, pl.S, oz_tile(ctx, pl.S, M, N, 1)));
+  GC_TRY(make_oz_operand(ctx, b, B, N, K, 1, sbn, sbk, 0, pl.S, oz_tile(ctx, pl.S, M, N, K, 1)));
   OzEpi e{0, C, ldc, 0, nullptr, nullptr, nullptr, nullptr, 0, 0, period};
   GC_TRY(run_oz(ctx, a, b, M, N, 1, pl, e));
   return GC_OK;  // the device flag is read at the caller's next sync point
@@ -1733,7 +1766,7 @@ int tc_syrk_sub_lower(gc_context *ctx, int precision, int M, int K, const double
   OzPlan pl = oz_plan(precision);
   OzOperand a, b;
   GC_TRY(make_oz_operand(ctx, a, P, M, K, nbatch, sm, sk, sb, pl.S, BM));
-  GC_TRY(alias_oz_operand(ctx, a, b, oz_tile(ctx, pl.S, M, M, nbatch, true)));
+  GC_TRY(alias_oz_operand(ctx, a, b, oz_tile(ctx, pl.S, M, M, K, nbatch, true)));
   OzEpi e{2, C, ldc, nbatch > 1 ? sb : 0, nullptr, nullptr, nullptr, nullptr, 0, 0, M};
   GC_TRY(run_oz(ctx, a, b, M, M, nbatch, pl, e));
   return GC_OK;  // the device flag is read at the caller's next sync point
@@ -1751,7 +1784,7 @@ int tc_gram_dot(gc_context *ctx, int precision, int N, const double *Y, const do
   opt.hi = hi;
   opt.sq = sq;
   GC_TRY(make_oz_operand(ctx, a, Y, N, N, 1, 1, N, 0, pl.S, BM, 0, opt));
-  GC_TRY(alias_oz_operand(ctx, a, b, oz_tile(ctx, pl.S, N, N, 1, true)));
+  GC_TRY(alias_oz_operand(ctx, a, b, oz_tile(ctx, pl.S, N, N, N, 1, true)));
   GC_TRY(part.alloc(ctx, (size_t)ceil_div(N, BM) * ceil_div(N, b.box_rows)));
   OzEpi e{4, nullptr, N, 0, Klow, part.p, nullptr, nullptr, 0, 0, N};
   return run_oz(ctx, a, b, N, N, 1, pl, e);
@@ -1837,7 +1870,7 @@ extern "C" int gc_tc_gemm_time(gc_context *ctx, int precision, int m, int n, int
     OzPlan pl = oz_plan(precision);
     OzOperand A, B;
     GC_TRY(make_oz_operand(ctx, A, a.p, m, k, 1, k, 1, 0, pl.S, BM));
-    GC_TRY(make_oz_operand(ctx, B, b.p, n, k, 1, k, 1, 0, pl.S, oz_tile(ctx, pl.S, m, n, 1)));
+    GC_TRY(make_oz_operand(ctx, B, b.p, n, k, 1, k, 1, 0, pl.S, oz_tile(ctx, pl.S, m, n, k, 1)));
     OzEpi e{0, c.p, m, 0, nullptr, nullptr, nullptr, nullptr, 0, 0};
     GC_TRY(run_oz(ctx, A, B, m, n, 1, pl, e));  // warm-up
     GC_CUDA(ctx, cudaEventRecord(ev.a, ctx->stream));

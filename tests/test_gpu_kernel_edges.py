@@ -123,6 +123,39 @@ def test_sliced_gemm_bits(gpu_lib, S, m, n, k):
     assert np.array_equal(C, sliced_product(A, B, S))
 
 
+# Products whose waves of tiles make the default another width than the forced one, with ragged
+# rows, columns and K: plain, symmetric (FOFO with one pair of blocks) and reduced (integrand)
+@pytest.mark.parametrize("S", [4, 5])
+def test_sliced_gemm_tile_choice(gpu_lib, S):
+    g = torch.Generator(device=DEV).manual_seed(S)
+    rnd = lambda *s: torch.randn(*s, dtype=torch.float64, device=DEV, generator=g)
+    n, nin, nact, prec = 76, 28, 4, f"fp64tc{S}"
+    occ = np.r_[np.ones(nin), 0.9, 0.7, 0.2, 0.1, np.zeros(n - nin - nact)]
+    indn = R.pair_space(occ, nin + 2)
+    N, nocc = len(indn), nin + nact
+    A, B, L = rnd(19401, 33), rnd(141, 33), rnd(64, 101 * 100 // 2).t()
+    C = torch.linalg.qr(rnd(100, 100))[0]
+    Co = C[:, :30].contiguous()
+    Y, fofo = torch.linalg.qr(rnd(N, N))[0], rnd(n * nocc, n * nocc)
+    eig = torch.linspace(0.1, 9.0, N, dtype=torch.float64, device=DEV)
+    eig[::5] = -0.1  # dropped modes: Y Y^T is no unit matrix
+    got = []
+    for width in (0, 64):
+        ctx = api.Context(0)
+        try:
+            ctx.set_gemm_tile(width)
+            got.append((api.tc_gemm_nt(A, B, prec, ctx=ctx),
+                        api.tran4_factored(100, L, C, Co, C, Co, precision=prec, ctx=ctx),
+                        api.ace_ne_erpa_fofo(Y, eig, occ, indn, nact, nin, fofo, precision=prec,
+                                             ctx=ctx)))
+        finally:
+            ctx.close()
+    assert torch.equal(got[0][0], got[1][0])
+    assert torch.equal(got[0][1], got[1][1])
+    # N^2 terms, each within 2^-52 of itself, added in another grouping
+    assert abs(got[0][2] - got[1][2]) <= 1e-12 * N * fofo.abs().max().item()
+
+
 # widths (nA, nB, nC, nD); -1 repeats the block before it, so that the pair index is symmetric
 @pytest.mark.parametrize("n,widths", [(33, (33, 5, 33, 5)), (33, (5, -1, 33, -1)), (20, (3, 17, 9, -1)),
                                       (20, (7, -1, 4, 11)), (65, (2, 65, 2, 65)), (5, (1, 1, 5, 2)),
