@@ -366,7 +366,7 @@ __global__ void __launch_bounds__(192, 1)
 constexpr int OZ_BK = 32;      // K per stage: 32 BF16 = one 64-byte swizzled row
 // Each stage holds every slice of A and of B. The 32- and 48-wide tiles (the occupied block of a
 // transform; products with a short K) take two, so that two CTAs share an SM and one's epilogue
-// runs beside the other's products (372006 x 28 x 249: 185 us, with the 64-wide tile 270 us).
+// runs beside the other's products (372006 x 28 x 249: 170 us, with the 64-wide tile 270 us).
 __host__ __device__ constexpr int oz_stages(int tbn) { return tbn < 64 ? 2 : 3; }
 // TMEM columns allocated: a power of two that holds the S weight accumulators.
 __host__ __device__ constexpr int oz_tmem_cols(int S, int tbn) {
