@@ -147,8 +147,8 @@ __device__ __forceinline__ void mma_bf16(uint32_t tmem, uint64_t ad, uint64_t bd
 }
 
 // As mma_bf16, with a use of the A collector buffer: C = 1 reads A from shared memory
-// and keeps it in the buffer, 3 reads the buffer and releases it, 0 discards it (the
-// plain form). The same A descriptor is given with both uses.
+// and keeps it in the buffer, 2 reads the buffer, 3 reads it and releases it, 0 discards it (the
+// plain form). The same A descriptor is given with every use.
 template <int C>
 __device__ __forceinline__ void mma_bf16_ca(uint32_t tmem, uint64_t ad, uint64_t bd,
                                             uint32_t idesc, uint32_t accumulate) {
@@ -157,6 +157,12 @@ __device__ __forceinline__ void mma_bf16_ca(uint32_t tmem, uint64_t ad, uint64_t
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::f16.collector::a::fill [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem),
+        "l"(ad), "l"(bd), "r"(idesc), "r"(accumulate));
+  else if constexpr (C == 2)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16.collector::a::use [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem),
         "l"(ad), "l"(bd), "r"(idesc), "r"(accumulate));
   else if constexpr (C == 3)
     asm volatile(
@@ -206,6 +212,14 @@ __device__ __forceinline__ void tmem_ld4_issue(uint32_t taddr, uint32_t *r) {
 
 __device__ __forceinline__ void tmem_ld_wait() {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+// One lane of a converged warp, the same one every time.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t ok;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+               : "=r"(ok));
+  return ok != 0;
 }
 
 // ------------------------------------------------------------------- kernel
@@ -464,6 +478,7 @@ __global__ void __launch_bounds__(oz_threads(TBN), TBN < 64 ? 2 : 1)
   __shared__ double red[EPI];
 
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  const int role = __shfl_sync(0xffffffffu, warp, 0);  // warp, uniform for the compiler too
   // Grouped raster: CTAs are scheduled roughly in linear order, so consecutive ones
   // take OZ_GROUP_M row tiles before moving to the next column tile. A wave of CTAs
   // then shares a few A and B panels in L2 instead of sweeping every A panel
@@ -545,7 +560,7 @@ __global__ void __launch_bounds__(oz_threads(TBN), TBN < 64 ? 2 : 1)
     if (*abort_v)  // only the last STG loads can still be in flight
       for (int j = (issued > STG ? issued - STG : 0); j < issued; ++j)
         mbar_wait(&full[j % STG], (j / STG) & 1, kDrainNs);
-  } else if (warp == 1 && lane == 0) {
+  } else if (role == 1 && elect_one()) {
     bool ok = true;
     for (int g = 0; g < nchunks && ok; ++g) {
       if (g > 0 && !mbar_wait(acce, (g - 1) & 1, wait_ns)) {
@@ -563,34 +578,36 @@ __global__ void __launch_bounds__(oz_threads(TBN), TBN < 64 ? 2 : 1)
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t a_base = smem_u32(smem + s * STAGE_BYTES);
         const uint32_t b_base = a_base + S * A_BYTES;
-        // A slice t meets the B slices u < S - t, which lie one after the other in shared
-        // memory and accumulate into consecutive weights t + u: one product of A slice t with
-        // all of them, (S - t) TBN columns wide (two of equal width above 256). The first
-        // product into every weight of the chunk is t = 0 at kb0, kk 0. With one instruction
-        // per slice product an instruction took about 80 cycles whatever TBN (48 at the tensor
-        // rate for TBN = 96): its A tile alone is 32 cycles of shared-memory reads. At 6290^3
-        // 5.29 -> 4.62 ms (FP64TC5), 4.38 ms with the cheaper epilogue.
+        // One product per pair of slices, weight t + u always in its own TBN columns: the order in
+        // which MMAs take effect is only guaranteed between those of one accumulator and one
+        // shape. A slice t meets its B slices back to back, so that it is read from shared memory
+        // once and then from the collector buffer (a product without it takes 1.15 times as long
+        // at 96 columns, 1.3 at 64). The first product into every weight of the chunk is t = 0 at
+        // kb0, kk 0. The issuing thread is elected and its descriptors are an addition to a
+        // warp-uniform base: with lane 0 of a divided warp and descriptors put together
+        // per product, issuing took longer than the product (6290^3 FP64TC5: 5.58 ms, so 4.23).
+        const uint64_t da = smem_desc64(a_base), db = smem_desc64(b_base);
 #pragma unroll
-        for (int t = 0; t < S; ++t) {
-          constexpr int kMaxN = 256;
+        for (int t = 0; t < S; ++t)
 #pragma unroll
           for (int kk = 0; kk < OZ_BK / 16; ++kk) {
-            const uint64_t ad = smem_desc64(a_base + t * A_BYTES + kk * 32);
+            const uint64_t ad = da + (uint64_t)((t * A_BYTES + kk * 32) >> 4);
             const uint32_t acc_in = (kb == kb0 && t == 0 && kk == 0) ? 0u : 1u;
-            const int cols = (S - t) * TBN;
-            if (cols <= kMaxN) {
-              mma_bf16_ca<0>(tmem + (uint32_t)(t * TBN), ad, smem_desc64(b_base + kk * 32),
-                             instr_desc(cols), acc_in);
-            } else {
-              const int half = cols / 2;
-              mma_bf16_ca<1>(tmem + (uint32_t)(t * TBN), ad, smem_desc64(b_base + kk * 32),
-                             instr_desc(half), acc_in);
-              mma_bf16_ca<3>(tmem + (uint32_t)(t * TBN + half), ad,
-                             smem_desc64(b_base + half * (OZ_BK * 2) + kk * 32), instr_desc(half),
-                             acc_in);
+            constexpr uint32_t idesc = instr_desc(TBN);
+#pragma unroll
+            for (int u = 0; u + t < S; ++u) {
+              const uint64_t bd = db + (uint64_t)((u * B_BYTES + kk * 32) >> 4);
+              const uint32_t d = tmem + (uint32_t)((t + u) * TBN);
+              if (t == S - 1)
+                mma_bf16_ca<0>(d, ad, bd, idesc, acc_in);
+              else if (u == 0)
+                mma_bf16_ca<1>(d, ad, bd, idesc, acc_in);
+              else if (u + t < S - 1)
+                mma_bf16_ca<2>(d, ad, bd, idesc, acc_in);
+              else
+                mma_bf16_ca<3>(d, ad, bd, idesc, acc_in);
             }
           }
-        }
         mma_commit(&empty[s]);
       }
       mma_commit(accf);
@@ -1477,14 +1494,14 @@ static_assert(oz_smem_bytes(4, 128) <= 232448 && oz_smem_bytes(5, 96) <= 232448 
 
 // Time in us of one wave of tiles (152 CTAs, 304 of the 48-wide tile) for K = 64 kb: the
 // pipeline's start and the epilogue, and the products. Measured on GB300 at 140454 x 153 for
-// K = 64..1024; at 6290^3 the waves so come out within 2%. The 48-wide tile's two CTAs per SM run
-// one's epilogue beside the other's products: the best of the widths up to K of about 500
-// (K = 64: 141 us against 183 with 96 columns and 197 with 64; K = 249: 236, 263, 285), where the
-// epilogue is longer than the products.
+// K = 64..2048, where the waves so come out within 9%. The 48-wide tile's two CTAs per SM run
+// one's epilogue beside the other's products: the best of the widths up to K of about 300 with 5
+// slices and 500 with 4 (5 slices, K = 64: 137 us against 183 with 96 columns and 197 with 64;
+// K = 256: 254, 260, 284; K = 512: 407, 356, 398), where the epilogue is longer than the products.
 double oz_wave_us(int S, int tbn, double kb) {
   const bool s4 = S == 4;
   switch (tbn) {
-    case 48: return s4 ? 7.0 + 1.68 * kb : 7.3 + 2.12 * kb;
+    case 48: return s4 ? 7.0 + 1.68 * kb : 6.6 + 2.57 * kb;
     case 64: return s4 ? 7.2 + 1.08 * kb : 7.5 + 1.42 * kb;
     case 96: return s4 ? 9.6 + 1.43 * kb : 10.3 + 1.93 * kb;
     default: return 12.3 + 1.61 * kb;
