@@ -1318,13 +1318,9 @@ size_t smem_bytes(int bn) {
 int run_gemm(gc_context *ctx, const Operand &A, const Operand &B, int M, int N, int nbatch,
              const PassList &pl, const Epi &epi) {
   if (A.Kp != B.Kp) return gc::set_error(ctx, GC_EINVAL, "tc_gemm: K mismatch");
-  static std::once_flag once;
-  static cudaError_t cfg = cudaSuccess;
-  std::call_once(once, [] {
-    cfg = cudaFuncSetAttribute(k_tc_gemm<BN_T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)smem_bytes(BN_T));
-  });
-  GC_CUDA(ctx, cfg);
+  // on every call: the setting holds for one device
+  GC_CUDA(ctx, cudaFuncSetAttribute(k_tc_gemm<BN_T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)smem_bytes(BN_T)));
   dim3 grid(gc::ceil_div(M, BM), gc::ceil_div(N, BN_T), nbatch);
   k_tc_gemm<BN_T><<<grid, 192, smem_bytes(BN_T), ctx->stream>>>(
       A.map, B.map, M, N, A.Kp / BK, A.nb > 1 ? 1 : 0, B.nb > 1 ? 1 : 0, pl, epi, ctx->dev_flag,
@@ -1542,13 +1538,9 @@ int oz_tile(const gc_context *ctx, int S, long long M, long long N, long long K,
 template <int S, int TBN>
 int launch_oz(gc_context *ctx, const OzOperand &A, const OzOperand &B, int M, int N, int nbatch,
               const OzPlan &pl, const OzEpi &epi) {
-  static std::once_flag once;
-  static cudaError_t cfg = cudaSuccess;
-  std::call_once(once, [] {
-    cfg = cudaFuncSetAttribute(k_tc_gemm_oz<S, TBN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)oz_smem_bytes(S, TBN));
-  });
-  GC_CUDA(ctx, cfg);
+  // on every call: the setting holds for one device
+  GC_CUDA(ctx, cudaFuncSetAttribute(k_tc_gemm_oz<S, TBN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)oz_smem_bytes(S, TBN)));
   dim3 grid(gc::ceil_div(M, BM), gc::ceil_div(N, TBN), nbatch);
   k_tc_gemm_oz<S, TBN><<<grid, oz_threads(TBN), oz_smem_bytes(S, TBN), ctx->stream>>>(
       A.map, B.map, M, N, A.Kp / OZ_BK, A.nb > 1 ? 1 : 0, B.nb > 1 ? 1 : 0, pl, epi, ctx->dev_flag,
