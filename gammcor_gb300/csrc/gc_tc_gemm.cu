@@ -378,10 +378,14 @@ __global__ void __launch_bounds__(192, 1)
 // one gives more CTAs to a small product. oz_tile() picks one per GEMM; every
 // width gives the same result bits (each element's integer sums are the same).
 constexpr int OZ_BK = 32;      // K per stage: 32 BF16 = one 64-byte swizzled row
-// Each stage holds every slice of A and of B. The 32- and 48-wide tiles (the occupied block of a
-// transform; products with a short K) take two, so that two CTAs share an SM and one's epilogue
-// runs beside the other's products (372006 x 28 x 249: 170 us, with the 64-wide tile 270 us).
-__host__ __device__ constexpr int oz_stages(int tbn) { return tbn < 64 ? 2 : 3; }
+// Each stage holds every slice of A and of B. The 32- and 48-wide tiles of 4 and 5 slices (the
+// occupied block of a transform; products with a short K) take two, so that two CTAs share an SM and
+// one's epilogue runs beside the other's products (372006 x 28 x 249, 5 slices: 177 us, with the
+// 64-wide tile 268). Two CTAs of six slices do not fit an SM's shared memory, so they take
+// three stages (372006 x 28 x 249: 255 us, with two 266, with the 64-wide tile 308; x 512: 416, 561,
+// 499).
+__host__ __device__ constexpr int oz_ctas(int S, int tbn) { return S < 6 && tbn < 64 ? 2 : 1; }
+__host__ __device__ constexpr int oz_stages(int S, int tbn) { return oz_ctas(S, tbn) == 2 ? 2 : 3; }
 // TMEM columns allocated: a power of two that holds the S weight accumulators.
 __host__ __device__ constexpr int oz_tmem_cols(int S, int tbn) {
   return S * tbn <= 128 ? 128 : (S * tbn <= 256 ? 256 : 512);
@@ -453,15 +457,15 @@ __device__ __forceinline__ double scaled_double(long long t, int sc) {
 }
 
 template <int S, int TBN>
-__global__ void __launch_bounds__(oz_threads(TBN), TBN < 64 ? 2 : 1)
+__global__ void __launch_bounds__(oz_threads(TBN), oz_ctas(S, TBN))
     k_tc_gemm_oz(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
                  int M, int N, int kblocks, int a_batched, int b_batched, OzPlan plan, OzEpi epi,
                  int *err_flag, unsigned long long wait_ns) {
   // One stage = the K block [kb*32, kb*32+32) of all S slices of the A tile (128 rows)
   // and of the B tile (TBN rows): every slice product t+u < S of the block is
   // issued from it, so each slice tile crosses L2 -> shared memory once per block.
-  static_assert(S * TBN <= (TBN < 64 ? 256 : 512) && TBN % 16 == 0, "S weight accumulators exceed TMEM");
-  constexpr int EPI = oz_epi_warps(TBN), STG = oz_stages(TBN);
+  static_assert(S * TBN <= 512 / oz_ctas(S, TBN) && TBN % 16 == 0, "S weight accumulators exceed TMEM");
+  constexpr int EPI = oz_epi_warps(TBN), STG = oz_stages(S, TBN);
   constexpr uint32_t TCOLS = oz_tmem_cols(S, TBN);
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -1481,12 +1485,15 @@ int alias_oz_operand(gc_context *ctx, const OzOperand &src, OzOperand &op, int b
 
 // alignment pad, stages, 2 * stages + 3 barriers, TMEM slot
 constexpr size_t oz_smem_bytes(int S, int tbn) {
-  return 1024 + oz_stages(tbn) * (size_t)S * (BM * OZ_BK * 2 + tbn * OZ_BK * 2) +
-         (2 * oz_stages(tbn) + 3) * 8 + 16;
+  return 1024 + oz_stages(S, tbn) * (size_t)S * (BM * OZ_BK * 2 + tbn * OZ_BK * 2) +
+         (2 * oz_stages(S, tbn) + 3) * 8 + 16;
 }
 static_assert(oz_smem_bytes(4, 128) <= 232448 && oz_smem_bytes(5, 96) <= 232448 &&
                   oz_smem_bytes(6, 64) <= 232448,
               "sliced GEMM stages exceed the 227 KB of shared memory per CTA");
+// 228 KB per SM, 1 KB of it reserved per CTA, and less than 1 KB of static shared memory each
+static_assert(2 * (oz_smem_bytes(5, 48) + 2048) <= 233472 && 2 * (oz_smem_bytes(5, 32) + 2048) <= 233472,
+              "the narrow tiles' two CTAs do not fit the shared memory of an SM");
 
 // Time in us of one wave of tiles (152 CTAs, 304 of the 48-wide tile) for K = 64 kb: the
 // pipeline's start and the epilogue, and the products. Measured on GB300 at 140454 x 153 for
@@ -1506,8 +1513,10 @@ double oz_wave_us(int S, int tbn, double kb) {
 
 // Tile width for an M x N x K x nbatch product: the one whose waves of CTAs finish first by the
 // times above. tri: only the tiles that reach the lower triangle of an M x M product are
-// computed (N = M). Six slices take 64 columns (two CTAs of 48 would not fit TMEM), products of
-// at most 32 columns the 32-wide tile.
+// computed (N = M). Products of at most 32 columns take the 32-wide tile, and six slices 64 columns
+// otherwise: two CTAs of 48 would not fit TMEM, and 32 columns are slower unless the product leaves most
+// SMs idle (140454 x 153 x 256: 334 us with 64, 388 with 32; 6290 x 6290 x 249: 511, 700; but
+// 512^3: 25 and 19).
 int oz_tile(const gc_context *ctx, int S, long long M, long long N, long long K, long long nbatch,
             bool tri = false) {
   const int widest = oz_max_tile(S);

@@ -65,3 +65,10 @@ def test_bits_over_several_chunks(gpu_lib, S, m, n, k, width):
             assert torch.equal(api.tc_gemm_nt(A, B, f"fp64tc{S}", ctx=ctx), ref)
     finally:
         ctx.close()
+
+
+# The 32-wide tile of six slices (three stages of 32 K): fewer K blocks than stages, as many, more
+@pytest.mark.parametrize("k", [1, 33, 96, 129, 250])
+def test_six_slices_in_the_narrow_tile(gpu_lib, k):
+    A, B = operands(300, 17, k, k)
+    assert torch.equal(api.tc_gemm_nt(A, B, "fp64tc6"), sliced_product(A, B, 6))
