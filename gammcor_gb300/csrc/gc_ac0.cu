@@ -17,8 +17,8 @@
 //   k_ac0_block_erpa  one CTA per block: ERPASYMM0 in FP64 shared memory (two
 //                     Jacobi eigensolves), Y, X and omega of the block;
 //   k_ac0_iv          the (virtual, inactive) pairs: omega = A+(ii,ii), Y = X = 1/sqrt 2;
-//   k_ac0_right       T+ = A+' Xbd, T- = A-' Ybd, TK = K Ybd (block-diagonal right products; K:
-//                     the masked, CI-weighted FOFO integrals, gathered);
+//   k_ac0_right       T+ = A+' Xbd, T- = A-' Ybd (block-diagonal right products);
+//   k_ac0_right_k     TK = K Ybd (K: the masked, CI-weighted FOFO integrals, gathered);
 //   k_ac0_work        the energy sum_{r<=c} of 2 (Xbd^T T+ - Ybd^T T-) / (omega_r + omega_c) times
 //                     Ybd^T TK, one partial sum per block.
 // Every pass is O(N^2 m) for blocks of size m (at most nact(nact-1)/2): there is
@@ -290,39 +290,52 @@ __global__ void k_ac0_iv(int N, int iv0, const double *__restrict__ ap, double *
   Xrow[(size_t)i * kRow] = fac;
 }
 
-// T+ = A+' Xbd, T- = A-' Ybd and TK = K Ybd with the block-diagonal Xbd, Ybd (the sum over k in
-// the block of c, positions bs[c] .. bs[c] + bz[c] - 1) and the energy's weights
+// T+ = A+' Xbd and T- = A-' Ybd with the block-diagonal Xbd, Ybd (the sum over k in the block of
+// c, positions bs[c] .. bs[c] + bz[c] - 1). The rows up to the end of c's block are all that
+// k_ac0_work reads. Threads along r: coalesced columns.
+__global__ void k_ac0_right(int N, const double *__restrict__ a1p, const double *__restrict__ a1m,
+                            const int *__restrict__ bs, const int *__restrict__ bz,
+                            const double *__restrict__ Xrow, const double *__restrict__ Yrow,
+                            double *__restrict__ tp, double *__restrict__ tm) {
+  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  for (int c = blockIdx.y; c < N; c += gridDim.y) {
+    const int s = bs[c], m = bz[c], cc = c - s;
+    if (r >= s + m) continue;
+    double vp = 0.0, vm = 0.0;
+    for (int b = 0; b < m; ++b) {
+      const size_t e = (size_t)r + (size_t)(s + b) * N;
+      vp += a1p[e] * Xrow[(size_t)(s + b) * kRow + cc];
+      vm += a1m[e] * Yrow[(size_t)(s + b) * kRow + cc];
+    }
+    const size_t o = (size_t)r + (size_t)c * N;
+    tp[o] = vp;
+    tm[o] = vm;
+  }
+}
+
+// TK = K Ybd, the same rows, with the energy's weights
 // K[r, k] = (C_p + C_q)(C_r' + C_s') (r's'|pq) for pairs r = (p, q), k = (r', s') not in one
-// orbital group, gathered here. The rows up to the end of c's block are all that k_ac0_work
-// reads. Threads along r: coalesced columns.
-__global__ void k_ac0_right(int N, int n, int nocc, const double *__restrict__ a1p,
-                            const double *__restrict__ a1m, const int *__restrict__ bs,
-                            const int *__restrict__ bz, const double *__restrict__ Xrow,
-                            const double *__restrict__ Yrow, const int *__restrict__ pp,
-                            const int *__restrict__ pq, const double *__restrict__ cpl,
-                            const int *__restrict__ grp, const double *__restrict__ fofo,
-                            double *__restrict__ tp, double *__restrict__ tm,
-                            double *__restrict__ tk) {
+// orbital group, gathered here. A launch of its own, after k_ac0_right: TK then takes the place
+// of A+', and four N x N matrices are held instead of five.
+__global__ void k_ac0_right_k(int N, int n, int nocc, const int *__restrict__ bs,
+                              const int *__restrict__ bz, const double *__restrict__ Yrow,
+                              const int *__restrict__ pp, const int *__restrict__ pq,
+                              const double *__restrict__ cpl, const int *__restrict__ grp,
+                              const double *__restrict__ fofo, double *__restrict__ tk) {
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   for (int c = blockIdx.y; c < N; c += gridDim.y) {
     const int s = bs[c], m = bz[c], cc = c - s;
     if (r >= s + m) continue;
     const int p = pp[r], q = pq[r], g = grp[p], gg = grp[q];
     const size_t ld = (size_t)n * nocc;
-    double vp = 0.0, vm = 0.0, vk = 0.0;
+    double vk = 0.0;
     for (int b = 0; b < m; ++b) {
       const int k = s + b, rr = pp[k], ss = pq[k];
-      const size_t e = (size_t)r + (size_t)k * N;
-      const double y = Yrow[(size_t)k * kRow + cc];
-      vp += a1p[e] * Xrow[(size_t)k * kRow + cc];
-      vm += a1m[e] * y;
       if (!(g == gg && gg == grp[rr] && grp[rr] == grp[ss]))
-        vk += cpl[k] * fofo[((size_t)rr + (size_t)ss * n) * ld + p + (size_t)q * n] * y;
+        vk += cpl[k] * fofo[((size_t)rr + (size_t)ss * n) * ld + p + (size_t)q * n] *
+              Yrow[(size_t)k * kRow + cc];
     }
-    const size_t o = (size_t)r + (size_t)c * N;
-    tp[o] = vp;
-    tm[o] = vm;
-    tk[o] = cpl[r] * vk;
+    tk[(size_t)r + (size_t)c * N] = cpl[r] * vk;
   }
 }
 
@@ -481,19 +494,21 @@ extern "C" int gc_ac0cas_fofo(gc_context *ctx, int nbas, int ninact, int nact, i
                                                                  eig.p);
     GC_LAUNCHED(ctx);
   }
-  // Products with the block-diagonal factors; T+ and T- go into a0p and a0m.
-  gc::DevBuf<double> tk, part, res;
-  GC_TRY(tk.alloc(ctx, NN));
-  k_ac0_right<<<dim3(gc::ceil_div(N, 256), std::min(N, 65535)), 256, 0, ctx->stream>>>(
-      N, n, nocc, a1p.p, a1m.p, pbs.p, pbz.p, Xrow.p, Yrow.p, sd.pair_p.p, sd.pair_q.p, sd.cpl.p,
-      sd.grp.p, fofo, a0p.p, a0m.p, tk.p);
+  // Products with the block-diagonal factors; T+ and T- go into a0p and a0m, then TK into a1p.
+  gc::DevBuf<double> part, res;
+  const dim3 gr(gc::ceil_div(N, 256), std::min(N, 65535));
+  k_ac0_right<<<gr, 256, 0, ctx->stream>>>(N, a1p.p, a1m.p, pbs.p, pbz.p, Xrow.p, Yrow.p, a0p.p, a0m.p);
+  GC_LAUNCHED(ctx);
+  double *tk = a1p.p;
+  k_ac0_right_k<<<gr, 256, 0, ctx->stream>>>(N, n, nocc, pbs.p, pbz.p, Yrow.p, sd.pair_p.p, sd.pair_q.p,
+                                             sd.cpl.p, sd.grp.p, fofo, tk);
   GC_LAUNCHED(ctx);
   const unsigned gy = (unsigned)std::min(N, 256);
   const size_t npart = (size_t)gc::ceil_div(N, 256) * gy;
   GC_TRY(part.alloc(ctx, npart));
   GC_TRY(res.alloc(ctx, 1));
   k_ac0_work<<<dim3(gc::ceil_div(N, 256), gy), 256, 0, ctx->stream>>>(
-      N, a0p.p, a0m.p, tk.p, pbs.p, pbz.p, Xrow.p, Yrow.p, eig.p, part.p);
+      N, a0p.p, a0m.p, tk, pbs.p, pbz.p, Xrow.p, Yrow.p, eig.p, part.p);
   GC_LAUNCHED(ctx);
   k_sum<<<1, 1024, 0, ctx->stream>>>(npart, part.p, res.p);
   GC_LAUNCHED(ctx);
