@@ -18,7 +18,8 @@
 //                     Jacobi eigensolves), Y, X and omega of the block;
 //   k_ac0_iv          the (virtual, inactive) pairs: omega = A+(ii,ii), Y = X = 1/sqrt 2;
 //   k_ac0_right       T+ = A+' Xbd, T- = A-' Ybd (block-diagonal right products);
-//   k_ac0_right_k     TK = K Ybd (K: the masked, CI-weighted FOFO integrals, gathered);
+//   k_ac0_weights     K: the masked, CI-weighted FOFO integrals, symmetrised;
+//   k_ac0_right_k     TK = K Ybd;
 //   k_ac0_work        the energy sum_{r<=c} of 2 (Xbd^T T+ - Ybd^T T-) / (omega_r + omega_c) times
 //                     Ybd^T TK, one partial sum per block.
 // Every pass is O(N^2 m) for blocks of size m (at most nact(nact-1)/2): there is
@@ -313,29 +314,61 @@ __global__ void k_ac0_right(int N, const double *__restrict__ a1p, const double 
   }
 }
 
-// TK = K Ybd, the same rows, with the energy's weights
-// K[r, k] = (C_p + C_q)(C_r' + C_s') (r's'|pq) for pairs r = (p, q), k = (r', s') not in one
-// orbital group, gathered here. A launch of its own, after k_ac0_right: TK then takes the place
-// of A+', and four N x N matrices are held instead of five.
-__global__ void k_ac0_right_k(int N, int n, int nocc, const int *__restrict__ bs,
+// K = (K0 + K0^T) / 2 of the energy's weights K0[r, k] = (C_p + C_q)(C_r' + C_s') (r's'|pq) for
+// pairs r = (p, q), k = (r', s') not in one orbital group: the energy sums over all r, k with a
+// symmetric factor, so both of (r's'|pq) and (pq|r's') enter, which may differ (FOFO blocks are
+// symmetric to the rounding of their transform). One block per 32 x 32 tile of the lower triangle; its
+// mirror tile is gathered with the same coalescing and turned in shared memory, and both are
+// stored. K is formed once, where it was gathered again for every column of a block, and takes the
+// place of A+', as TK then takes that of A-': four N x N matrices are held.
+__global__ void __launch_bounds__(256)
+    k_ac0_weights(int N, int n, int nocc, const int *__restrict__ pp, const int *__restrict__ pq,
+                  const double *__restrict__ cpl, const int *__restrict__ grp,
+                  const double *__restrict__ fofo, double *__restrict__ kw) {
+  __shared__ double mirror[32][33], turned[32][33];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const size_t ld = (size_t)n * nocc;
+  auto el = [&](int i, int j) -> double {
+    const int p = pp[i], q = pq[i], r = pp[j], s = pq[j];
+    if (grp[p] == grp[q] && grp[q] == grp[r] && grp[r] == grp[s]) return 0.0;
+    return cpl[i] * cpl[j] * fofo[((size_t)r + (size_t)s * n) * ld + p + (size_t)q * n];
+  };
+  const int nt = (N + 31) / 32, i0 = blockIdx.x * 32;
+  for (int tj = blockIdx.y; tj <= (int)blockIdx.x && tj < nt; tj += gridDim.y) {
+    const int j0 = tj * 32;
+    __syncthreads();  // the tiles of the last turn
+    for (int k = ty; k < 32; k += 8) {
+      const int i = j0 + tx, j = i0 + k;
+      mirror[k][tx] = i < N && j < N ? el(i, j) : 0.0;
+    }
+    __syncthreads();
+    for (int k = ty; k < 32; k += 8) {
+      const int i = i0 + tx, j = j0 + k;
+      const double v = i < N && j < N ? 0.5 * (el(i, j) + mirror[tx][k]) : 0.0;
+      if (i < N && j < N) kw[i + (size_t)j * N] = v;
+      turned[k][tx] = v;
+    }
+    __syncthreads();
+    if (i0 != j0)
+      for (int k = ty; k < 32; k += 8) {
+        const int i = j0 + tx, j = i0 + k;
+        if (i < N && j < N) kw[i + (size_t)j * N] = turned[tx][k];
+      }
+  }
+}
+
+// TK = K Ybd, the rows of k_ac0_right.
+__global__ void k_ac0_right_k(int N, const double *__restrict__ kw, const int *__restrict__ bs,
                               const int *__restrict__ bz, const double *__restrict__ Yrow,
-                              const int *__restrict__ pp, const int *__restrict__ pq,
-                              const double *__restrict__ cpl, const int *__restrict__ grp,
-                              const double *__restrict__ fofo, double *__restrict__ tk) {
+                              double *__restrict__ tk) {
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   for (int c = blockIdx.y; c < N; c += gridDim.y) {
     const int s = bs[c], m = bz[c], cc = c - s;
     if (r >= s + m) continue;
-    const int p = pp[r], q = pq[r], g = grp[p], gg = grp[q];
-    const size_t ld = (size_t)n * nocc;
-    double vk = 0.0;
-    for (int b = 0; b < m; ++b) {
-      const int k = s + b, rr = pp[k], ss = pq[k];
-      if (!(g == gg && gg == grp[rr] && grp[rr] == grp[ss]))
-        vk += cpl[k] * fofo[((size_t)rr + (size_t)ss * n) * ld + p + (size_t)q * n] *
-              Yrow[(size_t)k * kRow + cc];
-    }
-    tk[(size_t)r + (size_t)c * N] = cpl[r] * vk;
+    double v = 0.0;
+    for (int b = 0; b < m; ++b)
+      v += kw[(size_t)r + (size_t)(s + b) * N] * Yrow[(size_t)(s + b) * kRow + cc];
+    tk[(size_t)r + (size_t)c * N] = v;
   }
 }
 
@@ -343,8 +376,7 @@ __global__ void k_ac0_right_k(int N, int n, int nocc, const int *__restrict__ bs
 // work[r, c] = 2 ((Xbd^T T+)[r, c] - (Ybd^T T-)[r, c]) / (omega_r + omega_c) where both
 // omegas are nonzero, else 0 (AC0CAS_FOFO, abfofo.f90:1625-1720, with the back-transform Ybd work
 // Ybd^T moved to the symmetric weights). Both factors are symmetric: r <= c, the others counted
-// twice. One partial sum per block. Measured at NDimX 1832 (n = 120, CAS(6,6)) with k_ac0_right:
-// 161 us, where the products, the back-transform and the energy loop over all r, c took 280.
+// twice. One partial sum per block.
 __global__ void __launch_bounds__(256)
     k_ac0_work(int N, const double *__restrict__ tp, const double *__restrict__ tm,
                const double *__restrict__ tk, const int *__restrict__ bs, const int *__restrict__ bz,
@@ -494,14 +526,18 @@ extern "C" int gc_ac0cas_fofo(gc_context *ctx, int nbas, int ninact, int nact, i
                                                                  eig.p);
     GC_LAUNCHED(ctx);
   }
-  // Products with the block-diagonal factors; T+ and T- go into a0p and a0m, then TK into a1p.
+  // Products with the block-diagonal factors; T+ and T- go into a0p and a0m, then K into a1p and TK
+  // into a1m.
   gc::DevBuf<double> part, res;
   const dim3 gr(gc::ceil_div(N, 256), std::min(N, 65535));
   k_ac0_right<<<gr, 256, 0, ctx->stream>>>(N, a1p.p, a1m.p, pbs.p, pbz.p, Xrow.p, Yrow.p, a0p.p, a0m.p);
   GC_LAUNCHED(ctx);
-  double *tk = a1p.p;
-  k_ac0_right_k<<<gr, 256, 0, ctx->stream>>>(N, n, nocc, pbs.p, pbz.p, Yrow.p, sd.pair_p.p, sd.pair_q.p,
-                                             sd.cpl.p, sd.grp.p, fofo, tk);
+  double *kw = a1p.p, *tk = a1m.p;
+  const unsigned nt = gc::ceil_div(N, 32);
+  k_ac0_weights<<<dim3(nt, std::min(nt, 65535u)), 256, 0, ctx->stream>>>(
+      N, n, nocc, sd.pair_p.p, sd.pair_q.p, sd.cpl.p, sd.grp.p, fofo, kw);
+  GC_LAUNCHED(ctx);
+  k_ac0_right_k<<<gr, 256, 0, ctx->stream>>>(N, kw, pbs.p, pbz.p, Yrow.p, tk);
   GC_LAUNCHED(ctx);
   const unsigned gy = (unsigned)std::min(N, 256);
   const size_t npart = (size_t)gc::ceil_div(N, 256) * gy;
