@@ -515,8 +515,10 @@ extern "C" int gc_ac0cas_fofo(gc_context *ctx, int nbas, int ninact, int nact, i
   if (nblk > 0) {
     const int ld = mmax + 1;
     const size_t smem = 5 * (size_t)mmax * ld * sizeof(double);
+    // always the largest block's: a smaller limit could come between this and another thread's launch
+    constexpr int kMaxSmem = 5 * kMaxBlock * (kMaxBlock + 1) * (int)sizeof(double);
     GC_CUDA(ctx, cudaFuncSetAttribute(k_ac0_block_erpa, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)smem));
+                                      kMaxSmem));
     k_ac0_block_erpa<<<nblk, kBlkThreads, smem, ctx->stream>>>(
         N, a0p.p, a0m.p, dbs.p, dbz.p, mmax, ld, Yrow.p, Xrow.p, eig.p, flag.p);
     GC_LAUNCHED(ctx);

@@ -2,6 +2,7 @@
 several threads."""
 import subprocess
 import sys
+from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
 import numpy as np
@@ -87,3 +88,17 @@ def test_ac0_takes_both_of_rs_pq_and_pq_rs(gpu_lib, n, nin, nact):
     assert abs(ref - A.ac0cas_fofo(occ, xone, np.eye(n), indn, nin, nact, ffoo, fofo, rdm)[0]) < 1e-12
     assert abs(energy(s, fofo) - ref) < 1e-9
     assert abs(energy(s, odd) - ref) < 1e-9
+
+
+def test_ac0_from_threads_with_blocks_of_different_size(gpu_lib):
+    """Blocks of 45 pairs and of one pair at the same time: no call may take its shared-memory limit
+    from the other's."""
+    def repeat(s):
+        ctx = api.Context(0, torch.cuda.Stream())
+        try:
+            return {round(energy(s, s[6], ctx), 9) for _ in range(600)}
+        finally:
+            ctx.close()
+    with ThreadPoolExecutor(2) as ex:
+        for got in ex.map(repeat, [system(14, 0, 10), system(9, 2, 2)]):
+            assert len(got) == 1
