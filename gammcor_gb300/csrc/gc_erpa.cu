@@ -325,115 +325,115 @@ __global__ void __launch_bounds__(kMaxCluster) k_cluster_eig(
         C[l * kLd + j] = v / cjj;
       }
       __syncthreads();
-  }
-  // A <- C^-1 A (thread = column), then A <- A C^-T (thread = row), symmetrise
-  if (l < m)
-    for (int i = 0; i < m; ++i) {
-      double v = A[i * kLd + l];
-      for (int q = 0; q < i; ++q) v -= C[i * kLd + q] * A[q * kLd + l];
-      A[i * kLd + l] = v / C[i * kLd + i];
     }
-  __syncthreads();
-  if (l < m)
-    for (int b = 0; b < m; ++b) {
-      double v = A[l * kLd + b];
-      for (int q = 0; q < b; ++q) v -= A[l * kLd + q] * C[b * kLd + q];
-      A[l * kLd + b] = v / C[b * kLd + b];
-    }
-  __syncthreads();
-  if (l < m)
-    for (int b = l + 1; b < m; ++b) {
-      double v = 0.5 * (A[l * kLd + b] + A[b * kLd + l]);
-      A[l * kLd + b] = v;
-      A[b * kLd + l] = v;
-    }
-  __syncthreads();
-  // cyclic Jacobi (Golub and Van Loan, Alg. 8.5.3), at most 40 sweeps
-  bool converged = false;
-  for (int sweep = 0; sweep < 40; ++sweep) {
-    double off = 0.0, tot = 0.0;
+    // A <- C^-1 A (thread = column), then A <- A C^-T (thread = row), symmetrise
+    if (l < m)
+      for (int i = 0; i < m; ++i) {
+        double v = A[i * kLd + l];
+        for (int q = 0; q < i; ++q) v -= C[i * kLd + q] * A[q * kLd + l];
+        A[i * kLd + l] = v / C[i * kLd + i];
+      }
+    __syncthreads();
     if (l < m)
       for (int b = 0; b < m; ++b) {
-        double v = A[l * kLd + b] * A[l * kLd + b];
-        tot += v;
-        if (b != l) off += v;
+        double v = A[l * kLd + b];
+        for (int q = 0; q < b; ++q) v -= A[l * kLd + q] * C[b * kLd + q];
+        A[l * kLd + b] = v / C[b * kLd + b];
       }
-    red[0][l] = off;
-    red[1][l] = tot;
     __syncthreads();
-    for (int w = kMaxCluster / 2; w > 0; w >>= 1) {
-      if (l < w) {
-        red[0][l] += red[0][l + w];
-        red[1][l] += red[1][l + w];
+    if (l < m)
+      for (int b = l + 1; b < m; ++b) {
+        double v = 0.5 * (A[l * kLd + b] + A[b * kLd + l]);
+        A[l * kLd + b] = v;
+        A[b * kLd + l] = v;
       }
+    __syncthreads();
+    // cyclic Jacobi (Golub and Van Loan, Alg. 8.5.3), at most 40 sweeps
+    bool converged = false;
+    for (int sweep = 0; sweep < 40; ++sweep) {
+      double off = 0.0, tot = 0.0;
+      if (l < m)
+        for (int b = 0; b < m; ++b) {
+          double v = A[l * kLd + b] * A[l * kLd + b];
+          tot += v;
+          if (b != l) off += v;
+        }
+      red[0][l] = off;
+      red[1][l] = tot;
       __syncthreads();
+      for (int w = kMaxCluster / 2; w > 0; w >>= 1) {
+        if (l < w) {
+          red[0][l] += red[0][l + w];
+          red[1][l] += red[1][l + w];
+        }
+        __syncthreads();
+      }
+      converged = red[0][0] <= 1e-30 * red[1][0];
+      __syncthreads();
+      if (converged) break;
+      for (int p = 0; p < m - 1; ++p)
+        for (int q = p + 1; q < m; ++q) {
+          const double apq = A[p * kLd + q];
+          if (apq == 0.0) continue;  // uniform: all threads read the same value
+          const double theta = (A[q * kLd + q] - A[p * kLd + p]) / (2.0 * apq);
+          const double t = (theta >= 0.0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(theta * theta + 1.0));
+          const double c = 1.0 / sqrt(t * t + 1.0), sn = t * c;
+          __syncthreads();
+          if (l < m) {
+            double aip = A[l * kLd + p], aiq = A[l * kLd + q];
+            A[l * kLd + p] = c * aip - sn * aiq;
+            A[l * kLd + q] = sn * aip + c * aiq;
+          }
+          __syncthreads();
+          if (l < m) {
+            double api = A[p * kLd + l], aqi = A[q * kLd + l];
+            A[p * kLd + l] = c * api - sn * aqi;
+            A[q * kLd + l] = sn * api + c * aqi;
+            double vip = V[l * kLd + p], viq = V[l * kLd + q];
+            V[l * kLd + p] = c * vip - sn * viq;
+            V[l * kLd + q] = sn * vip + c * viq;
+          }
+          __syncthreads();
+        }
     }
-    converged = red[0][0] <= 1e-30 * red[1][0];
+    if (!converged) {
+      if (l == 0) atomicOr(flag, 2);
+      return;
+    }
+    // Order the block's eigenpairs by eigenvalue (Jacobi leaves them unordered): the
+    // next iteration groups clusters from neighbouring indices, which must then hold
+    // neighbouring eigenvalues.
+    if (l == 0) {
+      for (int b = 0; b < m; ++b) perm[b] = b;
+      for (int b = 1; b < m; ++b) {  // insertion sort on the diagonal of A
+        const int pb = perm[b];
+        const double v = A[pb * kLd + pb];
+        int q = b - 1;
+        while (q >= 0 && A[perm[q] * kLd + perm[q]] > v) {
+          perm[q + 1] = perm[q];
+          --q;
+        }
+        perm[q + 1] = pb;
+      }
+    }
     __syncthreads();
-    if (converged) break;
-    for (int p = 0; p < m - 1; ++p)
-      for (int q = p + 1; q < m; ++q) {
-        const double apq = A[p * kLd + q];
-        if (apq == 0.0) continue;  // uniform: all threads read the same value
-        const double theta = (A[q * kLd + q] - A[p * kLd + p]) / (2.0 * apq);
-        const double t = (theta >= 0.0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(theta * theta + 1.0));
-        const double c = 1.0 / sqrt(t * t + 1.0), sn = t * c;
-        __syncthreads();
-        if (l < m) {
-          double aip = A[l * kLd + p], aiq = A[l * kLd + q];
-          A[l * kLd + p] = c * aip - sn * aiq;
-          A[l * kLd + q] = sn * aip + c * aiq;
-        }
-        __syncthreads();
-        if (l < m) {
-          double api = A[p * kLd + l], aqi = A[q * kLd + l];
-          A[p * kLd + l] = c * api - sn * aqi;
-          A[q * kLd + l] = sn * api + c * aqi;
-          double vip = V[l * kLd + p], viq = V[l * kLd + q];
-          V[l * kLd + p] = c * vip - sn * viq;
-          V[l * kLd + q] = sn * vip + c * viq;
-        }
-        __syncthreads();
+    if (l < m)
+      for (int b = 0; b < m; ++b) A[l * kLd + b] = V[l * kLd + perm[b]];
+    __syncthreads();
+    if (l < m)
+      for (int b = 0; b < m; ++b) V[l * kLd + b] = A[l * kLd + b];
+    __syncthreads();
+    // V_C = C^-T V (thread = column, backward substitution)
+    if (l < m)
+      for (int i = m - 1; i >= 0; --i) {
+        double v = V[i * kLd + l];
+        for (int q = i + 1; q < m; ++q) v -= C[q * kLd + i] * V[q * kLd + l];
+        V[i * kLd + l] = v / C[i * kLd + i];
       }
-  }
-  if (!converged) {
-    if (l == 0) atomicOr(flag, 2);
-    return;
-  }
-  // Order the block's eigenpairs by eigenvalue (Jacobi leaves them unordered): the
-  // next iteration groups clusters from neighbouring indices, which must then hold
-  // neighbouring eigenvalues.
-  if (l == 0) {
-    for (int b = 0; b < m; ++b) perm[b] = b;
-    for (int b = 1; b < m; ++b) {  // insertion sort on the diagonal of A
-      const int pb = perm[b];
-      const double v = A[pb * kLd + pb];
-      int q = b - 1;
-      while (q >= 0 && A[perm[q] * kLd + perm[q]] > v) {
-        perm[q + 1] = perm[q];
-        --q;
-      }
-      perm[q + 1] = pb;
-    }
-  }
-  __syncthreads();
-  if (l < m)
-    for (int b = 0; b < m; ++b) A[l * kLd + b] = V[l * kLd + perm[b]];
-  __syncthreads();
-  if (l < m)
-    for (int b = 0; b < m; ++b) V[l * kLd + b] = A[l * kLd + b];
-  __syncthreads();
-  // V_C = C^-T V (thread = column, backward substitution)
-  if (l < m)
-    for (int i = m - 1; i >= 0; --i) {
-      double v = V[i * kLd + l];
-      for (int q = i + 1; q < m; ++q) v -= C[q * kLd + i] * V[q * kLd + l];
-      V[i * kLd + l] = v / C[i * kLd + i];
-    }
-  __syncthreads();
-  if (l < m)
-    for (int b = 0; b < m; ++b) Vbuf[(size_t)(k + l) * kMaxCluster + b] = V[l * kLd + b];
-  if (l == 0) atomicMax(maxc, m);
+    __syncthreads();
+    if (l < m)
+      for (int b = 0; b < m; ++b) Vbuf[(size_t)(k + l) * kMaxCluster + b] = V[l * kLd + b];
+    if (l == 0) atomicMax(maxc, m);
   }
 }
 
