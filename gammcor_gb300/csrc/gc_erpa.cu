@@ -666,11 +666,12 @@ int refine_from_fp32(gc_context *ctx, int N, int prec, const double *M, const fl
     GC_CUDA(ctx, cudaMemsetAsync(list.p, 0, sizeof(int), ctx->stream));
     k_clusters<<<gN, 256, 0, ctx->stream>>>(N, lam, colm.p, cst.p, csz.p, flag.p, list.p);
     GC_LAUNCHED(ctx);
-    // Blocks for a few dozen clusters at once (a spectrum has tens, not N): with a block per
+    // The kernels walk the list of clusters: two block solves per SM at most (their shared memory), and
+    // 64 rows of blocks in the products, whose other grid dimension fills the chip. With a block per
     // index that left at once unless a cluster began there, the seven launches of two
     // iterations took 310 us at N = 1390.
-    const unsigned nc = std::min(N, 64);
-    k_cluster_eig<<<nc, kMaxCluster, kClusterSmem, ctx->stream>>>(N, G, S, list.p, csz.p, vbuf.p,
+    const unsigned ns = std::min(N, 304), nc = std::min(N, 64);
+    k_cluster_eig<<<ns, kMaxCluster, kClusterSmem, ctx->stream>>>(N, G, S, list.p, csz.p, vbuf.p,
                                                                   flag.p, flag.p + 1);
     GC_LAUNCHED(ctx);
     const dim3 gr(gc::ceil_div(N, kMaxCluster), nc), gl2(gc::ceil_div(2 * (size_t)N, kMaxCluster), nc);
