@@ -29,6 +29,7 @@
 #include <vector>
 
 #include "gc_internal.cuh"
+#include "gc_math.cuh"
 
 namespace {
 
@@ -46,20 +47,6 @@ struct BlockSh {
   int p[kMaxBlock / 2];               // pair k: p[k] < q = w[p[k]], or w[p[k]] = p[k]
 };
 
-// FP32 values from FP64 ones scaled by a common power of two (the larger exponent emax goes
-// to 0), and back, by integer operations: conversions share the FP64 pipe.
-__device__ __forceinline__ float to_scaled_f32(double x, int emax) {
-  const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
-  const int e = (int)((hi >> 20) & 0x7ff) - emax + 127;
-  if (e < 1) return 0.f;
-  return __uint_as_float((hi & 0x80000000u) | ((unsigned)e << 23) | ((hi & 0xfffffu) << 3) | (lo >> 29));
-}
-__device__ __forceinline__ double f32_to_f64(float x) {  // x normal or zero
-  const unsigned b = __float_as_uint(x);
-  if ((b & 0x7f800000u) == 0) return 0.0;
-  return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + 0x38000000u)), (int)(b << 29));
-}
-
 // Jacobi (Golub and Van Loan, Alg. 8.5.3, and 8.5.6 for the parallel ordering) on the symmetric
 // m x m matrix A (row stride ld >= m) in shared memory; V <- eigenvectors (columns), the
 // eigenvalues are left on the diagonal of A; T is scratch of A's size. Returns false if 40
@@ -71,9 +58,8 @@ __device__ __forceinline__ double f32_to_f64(float x) {  // x normal or zero
 // m (m - 1) / 2 pairs as rounds of m / 2 disjoint pairs (round robin); one thread per pair
 // forms its rotation with eight FP64 instructions; then every element of the upper triangle
 // is one thread's (six instructions, from A into T and back in turn), and so is every pair of
-// elements of V. The tangent is formed in FP32: it decides only how far the pair's element
-// shrinks (to 1e-7 of itself, beside the second-order terms of the other pairs); the rotation
-// itself is orthogonal to FP64 rounding, by a third-order step on the FP32 reciprocal root.
+// elements of V. A pair's element shrinks by the FP32 tangent's error only, which the second-order
+// terms of the other pairs exceed.
 // Measured for k_ac0_block_erpa with a 15 x 15 block (CAS(6,6), two eigensolves): one rotation
 // at a time 2.67 ms, rounds with FP64 angles and one thread per 2 x 2 block 0.53 ms, this 0.27 ms.
 __device__ bool block_jacobi(double *A, double *V, double *T, int m, int ld, BlockSh &sh) {
@@ -126,19 +112,7 @@ __device__ bool block_jacobi(double *A, double *V, double *T, int m, int ld, Blo
         double c = 1.0, sn = 0.0;
         if (q < m) {
           const double h = src[p * ld + q], d = src[q * ld + q] - src[p * ld + p];
-          if ((__double_as_longlong(h) << 1) != 0) {
-            // tan = 2h / (d +- sqrt(d^2 + 4 h^2))
-            const int ed = (__double2hiint(d) >> 20) & 0x7ff, eh = (__double2hiint(h) >> 20) & 0x7ff;
-            const int emax = max(ed, eh);
-            const float df = to_scaled_f32(d, emax), hf = 2.f * to_scaled_f32(h, emax);
-            const float r = sqrtf(df * df + hf * hf);
-            const float tf = hf / (df >= 0.f ? df + r : df - r);
-            const double t = f32_to_f64(tf), u = fma(t, t, 1.0);
-            const double y0 = f32_to_f64(rsqrtf(fmaf(tf, tf, 1.f)));
-            const double e = fma(-u, y0 * y0, 1.0);
-            c = fma(e * y0, fma(0.375, e, 0.5), y0);
-            sn = t * c;
-          }
+          if ((__double_as_longlong(h) << 1) != 0) gc::jacobi_rotation(h, d, &c, &sn);
           sh.w[q] = p;
           sh.c[q] = c;
           sh.s[q] = sn;

@@ -11,6 +11,7 @@
 #include <functional>
 
 #include "gc_internal.cuh"
+#include "gc_math.cuh"
 #include "gc_tc_gemm.cuh"
 
 namespace {
@@ -746,22 +747,6 @@ int chol_plain(gc_context *ctx, int N, double *A, int *minor) {
 constexpr int kCholNb = 64;
 constexpr int kCholLd = kCholNb + 1;  // padded column stride of the shared block
 
-// 1 / d for d > 0 to about an ulp: FP32 reciprocal of the mantissa, one third-order step. A
-// library square root and division are a chain of some 25 FP64 instructions, each of which
-// holds its quarter of the SM for 64 cycles; the conversions are integer work for that reason.
-__device__ __forceinline__ double reciprocal(double d) {
-  const unsigned hi = (unsigned)__double2hiint(d), lo = (unsigned)__double2loint(d);
-  const int e = (int)(hi >> 20) - 1023;  // d > 0
-  if (e < -1000 || e > 1000) return 1.0 / d;
-  const double m = __hiloint2double((int)((hi & 0xfffffu) | 0x3ff00000u), (int)lo);  // [1, 2)
-  const float mf = __uint_as_float(0x3f800000u | ((hi & 0xfffffu) << 3) | (lo >> 29));
-  const unsigned yb = __float_as_uint(__fdividef(1.f, mf));  // (1/2, 1]
-  const double y = __hiloint2double((int)((yb >> 3) + 0x38000000u), (int)(yb << 29));
-  const double r = fma(-m, y, 1.0);
-  const double z = fma(y, fma(r, r, r), y);
-  return __hiloint2double((int)((unsigned)__double2hiint(z) - ((unsigned)e << 20)), __double2loint(z));
-}
-
 // Right-looking Cholesky of the kb x kb (kb <= 64) diagonal block A (leading
 // dimension lda) in shared memory; L's lower triangle is written back. The update of
 // step k uses the unscaled column k and the pivot's reciprocal, a_ij -= a_ik a_jk / d_k,
@@ -796,7 +781,7 @@ __global__ void __launch_bounds__(256) k_potrf_block(int kb, double *__restrict_
       d = 1.0;
     }
     dk[k] = d;
-    rk[k] = reciprocal(d);
+    rk[k] = gc::reciprocal(d);
   };
   __syncthreads();
   if (t == 0) {
