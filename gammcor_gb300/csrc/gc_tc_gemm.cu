@@ -390,7 +390,6 @@ __host__ __device__ constexpr int oz_stages(int S, int tbn) { return oz_ctas(S, 
 __host__ __device__ constexpr int oz_tmem_cols(int S, int tbn) {
   return S * tbn <= 128 ? 128 : (S * tbn <= 256 ? 256 : 512);
 }
-constexpr int OZ_MAXS = 6;
 // Row exponent of a row holding a NaN or an infinity: its slices are zero and
 // every product element of the row comes out NaN, so non-finite inputs stay
 // visible in the result (the integer slices cannot carry them).
@@ -411,16 +410,13 @@ __host__ __device__ constexpr int oz_max_tile(int S) { return S <= 4 ? 128 : (S 
 
 struct OzPlan {
   int S;          // slices per operand
-  int npass;      // S(S+1)/2
   int chunk_kb;   // OZ_BK-wide K blocks per exact chunk
-  int pa[OZ_MAXS * (OZ_MAXS + 1) / 2], pb[OZ_MAXS * (OZ_MAXS + 1) / 2],
-      pd[OZ_MAXS * (OZ_MAXS + 1) / 2];
 };
 
 struct OzEpi {
-  int mode;              // 0 store, 1 dot with r, 2 subtract from the lower triangle of c,
-                         // 3 store the lower triangle of c and its mirror image,
-                         // 4 dot with the strict lower triangle of r
+  int mode;              // 0 store, 1 dot with the strict lower triangle of r,
+                         // 2 subtract from the lower triangle of c,
+                         // 3 store the lower triangle of c and its mirror image
   double *c;
   long long ldn, sb;
   const double *r;
@@ -504,7 +500,7 @@ __global__ void __launch_bounds__(oz_threads(TBN), oz_ctas(S, TBN))
     const int c0 = n0 % epi.tri_period;
     const bool inside = c0 + TBN <= epi.tri_period;  // all columns in one block
     if (inside && (epi.tri_upper ? c0 + TBN <= m0 : c0 >= m0 + BM)) {
-      if (epi.mode == 4 && threadIdx.x == 0)
+      if (epi.mode == 1 && threadIdx.x == 0)
         epi.partial[blockIdx.x + (long long)gridDim.x * (blockIdx.y + (long long)gridDim.y * blockIdx.z)] = 0.0;
       return;
     }
@@ -720,8 +716,8 @@ __global__ void __launch_bounds__(oz_threads(TBN), oz_ctas(S, TBN))
         }
       } else {
         const double *src = epi.mode == 2 ? epi.c : epi.r;
-        // last column of this row: all (1), up to the diagonal (2), below it (4)
-        const int last = epi.mode == 1 ? nn : min(nn, m - n1 + (epi.mode == 2 ? 1 : 0));
+        // last column of this row: below the diagonal (1), up to it (2)
+        const int last = min(nn, m - n1 + (epi.mode == 2 ? 1 : 0));
 #pragma unroll
         for (int j0 = 0; j0 < NC; j0 += 8) {  // the loads of a group before its stores
           double old[8];
@@ -738,14 +734,14 @@ __global__ void __launch_bounds__(oz_threads(TBN), oz_ctas(S, TBN))
         }
       }
     }
-    if (epi.mode == 1 || epi.mode == 4) {
+    if (epi.mode == 1) {
       for (int off = 16; off > 0; off >>= 1) dot += __shfl_down_sync(0xffffffffu, dot, off);
       if (lane == 0) red[warp - 2] = dot;
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if ((epi.mode == 1 || epi.mode == 4) && threadIdx.x == 0) {
+  if (epi.mode == 1 && threadIdx.x == 0) {
     long long cta = blockIdx.x + (long long)gridDim.x * (blockIdx.y + (long long)gridDim.y * blockIdx.z);
     double sum = 0.0;
     for (int w = 0; w < EPI; ++w) sum += red[w];
@@ -1350,15 +1346,6 @@ bool is_oz(int precision) { return gc::is_sliced(precision); }
 OzPlan oz_plan(int precision) {
   OzPlan p{};
   p.S = precision == GC_PREC_FP64TC6 ? 6 : (precision == GC_PREC_FP64TC4 ? 4 : 5);
-  int n = 0;
-  for (int d = 0; d < p.S; ++d)
-    for (int t = 0; t <= d; ++t) {
-      p.pa[n] = t;
-      p.pb[n] = d - t;
-      p.pd[n] = d;
-      ++n;
-    }
-  p.npass = n;
   // exact FP32 partial sums: (S+2) 2^12 c < 2^24 and 2^14 c < 2^24
   int c = (4096 / (p.S + 2)) / OZ_BK * OZ_BK;
   if ((long long)(p.S + 2) * 4096 * c >= (1ll << 24)) c -= OZ_BK;
@@ -1804,7 +1791,7 @@ int tc_gram_dot(gc_context *ctx, int precision, int N, const double *Y, const do
   GC_TRY(make_oz_operand(ctx, a, Y, N, N, 1, 1, N, 0, pl.S, BM, 0, opt));
   GC_TRY(alias_oz_operand(ctx, a, b, oz_tile(ctx, pl.S, N, N, N, 1, true)));
   GC_TRY(part.alloc(ctx, (size_t)ceil_div(N, BM) * ceil_div(N, b.box_rows)));
-  OzEpi e{4, nullptr, N, 0, Klow, part.p, nullptr, nullptr, 0, 0, N};
+  OzEpi e{1, nullptr, N, 0, Klow, part.p, nullptr, nullptr, 0, 0, N};
   return run_oz(ctx, a, b, N, N, 1, pl, e);
 }
 
