@@ -386,9 +386,9 @@ constexpr int OZ_BK = 32;      // K per stage: 32 BF16 = one 64-byte swizzled ro
 // 499).
 __host__ __device__ constexpr int oz_ctas(int S, int tbn) { return S < 6 && tbn < 64 ? 2 : 1; }
 __host__ __device__ constexpr int oz_stages(int S, int tbn) { return oz_ctas(S, tbn) == 2 ? 2 : 3; }
-// TMEM columns allocated: a power of two that holds the S weight accumulators.
-__host__ __device__ constexpr int oz_tmem_cols(int S, int tbn) {
-  return S * tbn <= 128 ? 128 : (S * tbn <= 256 ? 256 : 512);
+// TMEM columns allocated: a power of two that holds the weight accumulators.
+__host__ __device__ constexpr int oz_tmem_cols(int weights, int tbn) {
+  return weights * tbn <= 128 ? 128 : (weights * tbn <= 256 ? 256 : 512);
 }
 // Row exponent of a row holding a NaN or an infinity: its slices are zero and
 // every product element of the row comes out NaN, so non-finite inputs stay
@@ -414,7 +414,7 @@ struct OzPlan {
 };
 
 struct OzEpi {
-  int mode;              // 0 store, 1 dot with the strict lower triangle of r,
+  int mode;              // 0 store, 1 dot with the strict lower triangle of r (GRAM instances),
                          // 2 subtract from the lower triangle of c,
                          // 3 store the lower triangle of c and its mirror image
   double *c;
@@ -452,7 +452,11 @@ __device__ __forceinline__ double scaled_double(long long t, int sc) {
   return u == 0 ? 0.0 : __longlong_as_double((long long)(b | ((unsigned long long)t & (1ull << 63))));
 }
 
-template <int S, int TBN>
+// GRAM: the integrand's product (mode 1). It keeps one weight more, the products with t + u = S:
+// dotted with integrals, the dropped ones made up most of the error of W, which was 2 to 10 times that
+// of the form with Kt Yk (CPU emulation and batch systems of 600 to 1000 pairs); with them it is that
+// form's or less, as the digits alone then limit it.
+template <int S, int TBN, bool GRAM = false>
 __global__ void __launch_bounds__(oz_threads(TBN), oz_ctas(S, TBN))
     k_tc_gemm_oz(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
                  int M, int N, int kblocks, int a_batched, int b_batched, OzPlan plan, OzEpi epi,
@@ -460,9 +464,10 @@ __global__ void __launch_bounds__(oz_threads(TBN), oz_ctas(S, TBN))
   // One stage = the K block [kb*32, kb*32+32) of all S slices of the A tile (128 rows)
   // and of the B tile (TBN rows): every slice product t+u < S of the block is
   // issued from it, so each slice tile crosses L2 -> shared memory once per block.
-  static_assert(S * TBN <= 512 / oz_ctas(S, TBN) && TBN % 16 == 0, "S weight accumulators exceed TMEM");
+  constexpr int NW = GRAM ? S + 1 : S;  // weights
+  static_assert(NW * TBN <= 512 / oz_ctas(S, TBN) && TBN % 16 == 0, "weight accumulators exceed TMEM");
   constexpr int EPI = oz_epi_warps(TBN), STG = oz_stages(S, TBN);
-  constexpr uint32_t TCOLS = oz_tmem_cols(S, TBN);
+  constexpr uint32_t TCOLS = oz_tmem_cols(NW, TBN);
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   constexpr uint32_t A_BYTES = BM * OZ_BK * 2, B_BYTES = TBN * OZ_BK * 2;
@@ -500,7 +505,7 @@ __global__ void __launch_bounds__(oz_threads(TBN), oz_ctas(S, TBN))
     const int c0 = n0 % epi.tri_period;
     const bool inside = c0 + TBN <= epi.tri_period;  // all columns in one block
     if (inside && (epi.tri_upper ? c0 + TBN <= m0 : c0 >= m0 + BM)) {
-      if (epi.mode == 1 && threadIdx.x == 0)
+      if (GRAM && threadIdx.x == 0)
         epi.partial[blockIdx.x + (long long)gridDim.x * (blockIdx.y + (long long)gridDim.y * blockIdx.z)] = 0.0;
       return;
     }
@@ -582,9 +587,9 @@ __global__ void __launch_bounds__(oz_threads(TBN), oz_ctas(S, TBN))
         // which MMAs take effect is only guaranteed between those of one accumulator and one
         // shape. A slice t meets its B slices back to back, so that it is read from shared memory
         // once and then from the collector buffer (a product without it takes 1.15 times as long
-        // at 96 columns, 1.3 at 64). The first product into every weight of the chunk is t = 0 at
-        // kb0, kk 0. The issuing thread is elected and its descriptors are an addition to a
-        // warp-uniform base: with lane 0 of a divided warp and descriptors put together
+        // at 96 columns, 1.3 at 64). The first product into a weight of the chunk is t = 0 (t = 1 for
+        // weight S) at kb0, kk 0. The issuing thread is elected and its descriptors are an addition
+        // to a warp-uniform base: with lane 0 of a divided warp and descriptors put together
         // per product, issuing took longer than the product (6290^3 FP64TC5: 5.58 ms, so 4.23).
         const uint64_t da = smem_desc64(a_base), db = smem_desc64(b_base);
 #pragma unroll
@@ -592,17 +597,19 @@ __global__ void __launch_bounds__(oz_threads(TBN), oz_ctas(S, TBN))
 #pragma unroll
           for (int kk = 0; kk < OZ_BK / 16; ++kk) {
             const uint64_t ad = da + (uint64_t)((t * A_BYTES + kk * 32) >> 4);
-            const uint32_t acc_in = (kb == kb0 && t == 0 && kk == 0) ? 0u : 1u;
             constexpr uint32_t idesc = instr_desc(TBN);
+            const int last = S < NW - t ? S - 1 : NW - 1 - t;
 #pragma unroll
-            for (int u = 0; u + t < S; ++u) {
+            for (int u = 0; u <= last; ++u) {
               const uint64_t bd = db + (uint64_t)((u * B_BYTES + kk * 32) >> 4);
               const uint32_t d = tmem + (uint32_t)((t + u) * TBN);
-              if (t == S - 1)
+              const bool first = t == 0 || (t == 1 && u == S - 1);
+              const uint32_t acc_in = (kb == kb0 && first && kk == 0) ? 0u : 1u;
+              if (last == 0)
                 mma_bf16_ca<0>(d, ad, bd, idesc, acc_in);
               else if (u == 0)
                 mma_bf16_ca<1>(d, ad, bd, idesc, acc_in);
-              else if (u + t < S - 1)
+              else if (u < last)
                 mma_bf16_ca<2>(d, ad, bd, idesc, acc_in);
               else
                 mma_bf16_ca<3>(d, ad, bd, idesc, acc_in);
@@ -620,15 +627,15 @@ __global__ void __launch_bounds__(oz_threads(TBN), oz_ctas(S, TBN))
     if (!mbar_wait(drainb, 0, kDrainNs)) atomicExch(&abort_flag, 1);
   } else if (warp >= 2) {
     // Every chunk's FP32 sums v_d are integers below 2^24, so the weights fold into one int64
-    // per column, t = sum_d v_d 2^(7 (SI - 1 - d)), exact for the first SI = min(S, 5) weights
-    // (|t| < 2^52 per chunk); a sixth weight is rounded to units of 2^7 first (2^-42 of the
-    // scaled product, below FP64 rounding of the result). Two weights at a time fit 32 bits
+    // per column, t = sum_d v_d 2^(7 (SI - 1 - d)), exact for the first SI = min(NW, 5) weights
+    // (|t| < 2^52 per chunk); what comes after is rounded to units of the fifth first (2^-42 of the
+    // scaled product per chunk, beside six slices cut at 2^-42 each). Two weights at a time fit 32 bits
     // (128 |v_0| + |v_1| and 128 |v_2| + |v_3| are below 2^31: v_0 sums products up to 2^14, v_2
     // up to 2 2^13 + 2^12, over at most 672 K), and two 32 x 32 + 64 multiply-adds put the pairs
     // in place: the MMAs of the next chunk wait for this.
     // Four warps per NC columns (one per TMEM lane quarter, q = warp % 4); warp group
     // h = (warp - 2) / 4 owns columns [NC h, NC h + NC) of the tile.
-    constexpr int SI = S < 5 ? S : 5;
+    constexpr int SI = NW < 5 ? NW : 5;
     constexpr int NC = oz_epi_cols(TBN), LW = NC == 16 ? 4 : 8;
     const int q = warp & 3;
     const int h = (warp - 2) / 4;
@@ -645,9 +652,9 @@ __global__ void __launch_bounds__(oz_threads(TBN), oz_ctas(S, TBN))
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
       for (int c0 = 0; c0 < NC; c0 += LW) {
-        uint32_t r[S][LW];
+        uint32_t r[NW][LW];
 #pragma unroll
-        for (int d = 0; d < S; ++d) {
+        for (int d = 0; d < NW; ++d) {
           const uint32_t a = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(d * TBN + h * NC + c0);
           if constexpr (LW == 8)
             tmem_ld8_issue(a, r[d]);
@@ -657,10 +664,13 @@ __global__ void __launch_bounds__(oz_threads(TBN), oz_ctas(S, TBN))
         tmem_ld_wait();
 #pragma unroll
         for (int j = 0; j < LW; ++j) {
-          int v[S];
+          int v[SI];
 #pragma unroll
           for (int d = 0; d < SI; ++d) v[d] = __float2int_rn(__uint_as_float(r[d][j]));
-          if (S > SI) v[SI - 1] += __float2int_rn(__uint_as_float(r[S - 1][j]) * 0.0078125f);
+          if (NW == SI + 1) v[SI - 1] += __float2int_rn(__uint_as_float(r[SI][j]) * 0.0078125f);
+          if (NW == SI + 2)
+            v[SI - 1] += __float2int_rn((__uint_as_float(r[SI + 1][j]) * 0.0078125f +
+                                         __uint_as_float(r[SI][j])) * 0.0078125f);
           const int p0 = v[0] * 128 + v[1], p1 = v[2] * 128 + v[3];
           long long t = acc[c0 + j];
           if (SI == 5) {
@@ -694,7 +704,12 @@ __global__ void __launch_bounds__(oz_threads(TBN), oz_ctas(S, TBN))
         cv[j] = eb == kBadExp || ea == kBadExp ? __longlong_as_double(0x7ff8000000000000ll) : v;
       }
       const int n1 = n0 + h * NC, nn = m < M ? min(NC, N - n1) : 0;
-      if (epi.mode == 0) {
+      if constexpr (GRAM) {
+        const int last = min(nn, m - n1);  // columns below the diagonal
+#pragma unroll
+        for (int j = 0; j < NC; ++j)
+          if (j < last) dot += cv[j] * epi.r[o0 + j * epi.ldn];
+      } else if (epi.mode == 0) {
 #pragma unroll
         for (int j = 0; j < NC; ++j)
           if (j < nn) epi.c[o0 + j * epi.ldn] = cv[j];
@@ -715,33 +730,26 @@ __global__ void __launch_bounds__(oz_threads(TBN), oz_ctas(S, TBN))
             epi.c[n + (long long)mm * epi.ldn] = tr[(lane % NC) * 33 + k + lane / NC];
         }
       } else {
-        const double *src = epi.mode == 2 ? epi.c : epi.r;
-        // last column of this row: below the diagonal (1), up to it (2)
-        const int last = min(nn, m - n1 + (epi.mode == 2 ? 1 : 0));
+        const int last = min(nn, m - n1 + 1);  // columns up to the diagonal
 #pragma unroll
         for (int j0 = 0; j0 < NC; j0 += 8) {  // the loads of a group before its stores
           double old[8];
 #pragma unroll
-          for (int j = 0; j < 8; ++j) old[j] = j0 + j < last ? src[o0 + (j0 + j) * epi.ldn] : 0.0;
+          for (int j = 0; j < 8; ++j) old[j] = j0 + j < last ? epi.c[o0 + (j0 + j) * epi.ldn] : 0.0;
 #pragma unroll
           for (int j = 0; j < 8; ++j)
-            if (j0 + j < last) {
-              if (epi.mode == 2)
-                epi.c[o0 + (j0 + j) * epi.ldn] = old[j] - cv[j0 + j];
-              else
-                dot += cv[j0 + j] * old[j];
-            }
+            if (j0 + j < last) epi.c[o0 + (j0 + j) * epi.ldn] = old[j] - cv[j0 + j];
         }
       }
     }
-    if (epi.mode == 1) {
+    if (GRAM) {
       for (int off = 16; off > 0; off >>= 1) dot += __shfl_down_sync(0xffffffffu, dot, off);
       if (lane == 0) red[warp - 2] = dot;
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (epi.mode == 1 && threadIdx.x == 0) {
+  if (GRAM && threadIdx.x == 0) {
     long long cta = blockIdx.x + (long long)gridDim.x * (blockIdx.y + (long long)gridDim.y * blockIdx.z);
     double sum = 0.0;
     for (int w = 0; w < EPI; ++w) sum += red[w];
@@ -1531,19 +1539,22 @@ int oz_tile(const gc_context *ctx, int S, long long M, long long N, long long K,
   return best;
 }
 
-template <int S, int TBN>
+template <int S, int TBN, bool GRAM = false>
 int launch_oz(gc_context *ctx, const OzOperand &A, const OzOperand &B, int M, int N, int nbatch,
               const OzPlan &pl, const OzEpi &epi) {
   // on every call: the setting holds for one device
-  GC_CUDA(ctx, cudaFuncSetAttribute(k_tc_gemm_oz<S, TBN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  GC_CUDA(ctx, cudaFuncSetAttribute(k_tc_gemm_oz<S, TBN, GRAM>,
+                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)oz_smem_bytes(S, TBN)));
   dim3 grid(gc::ceil_div(M, BM), gc::ceil_div(N, TBN), nbatch);
-  k_tc_gemm_oz<S, TBN><<<grid, oz_threads(TBN), oz_smem_bytes(S, TBN), ctx->stream>>>(
+  k_tc_gemm_oz<S, TBN, GRAM><<<grid, oz_threads(TBN), oz_smem_bytes(S, TBN), ctx->stream>>>(
       A.map, B.map, M, N, A.Kp / OZ_BK, A.nb > 1 ? 1 : 0, B.nb > 1 ? 1 : 0, pl, epi, ctx->dev_flag,
       ctx->wait_ns);
   GC_LAUNCHED(ctx);
   return GC_OK;
 }
+
+constexpr int kGramTile = 64;
 
 // The B operand's TMA box height is the column tile width of the launch.
 int run_oz(gc_context *ctx, const OzOperand &A, const OzOperand &B, int M, int N, int nbatch,
@@ -1554,6 +1565,11 @@ int run_oz(gc_context *ctx, const OzOperand &A, const OzOperand &B, int M, int N
   epi.ea_sb = A.nb > 1 ? A.rows : 0;
   epi.eb_sb = B.nb > 1 ? B.rows : 0;
   const int w = B.box_rows;
+  if (epi.mode == 1) {  // one width: S + 1 accumulators of 96 columns would not fit TMEM for S = 5
+    if (pl.S == 6) return launch_oz<6, kGramTile, true>(ctx, A, B, M, N, nbatch, pl, epi);
+    if (pl.S == 5) return launch_oz<5, kGramTile, true>(ctx, A, B, M, N, nbatch, pl, epi);
+    return launch_oz<4, kGramTile, true>(ctx, A, B, M, N, nbatch, pl, epi);
+  }
   if (pl.S == 6 && w == 32) return launch_oz<6, 32>(ctx, A, B, M, N, nbatch, pl, epi);
   if (pl.S == 5 && w == 32) return launch_oz<5, 32>(ctx, A, B, M, N, nbatch, pl, epi);
   if (pl.S == 4 && w == 32) return launch_oz<4, 32>(ctx, A, B, M, N, nbatch, pl, epi);
@@ -1789,7 +1805,7 @@ int tc_gram_dot(gc_context *ctx, int precision, int N, const double *Y, const do
   opt.hi = hi;
   opt.sq = sq;
   GC_TRY(make_oz_operand(ctx, a, Y, N, N, 1, 1, N, 0, pl.S, BM, 0, opt));
-  GC_TRY(alias_oz_operand(ctx, a, b, oz_tile(ctx, pl.S, N, N, N, 1, true)));
+  GC_TRY(alias_oz_operand(ctx, a, b, kGramTile));
   GC_TRY(part.alloc(ctx, (size_t)ceil_div(N, BM) * ceil_div(N, b.box_rows)));
   OzEpi e{1, nullptr, N, 0, Klow, part.p, nullptr, nullptr, 0, 0, N};
   return run_oz(ctx, a, b, N, N, 1, pl, e);
