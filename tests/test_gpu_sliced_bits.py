@@ -72,3 +72,26 @@ def test_bits_over_several_chunks(gpu_lib, S, m, n, k, width):
 def test_six_slices_in_the_narrow_tile(gpu_lib, k):
     A, B = operands(300, 17, k, k)
     assert torch.equal(api.tc_gemm_nt(A, B, "fp64tc6"), sliced_product(A, B, 6))
+
+
+def test_narrow_tiles_of_several_kernels_share_sms(gpu_lib):
+    """32- and 48-wide tiles and the split-BF16 GEMM from four threads at once: CTAs of different
+    kernels on one SM, each with its own slices in the collector buffer, leave each other's bits alone."""
+    from concurrent.futures import ThreadPoolExecutor
+    jobs = [("fp64tc5", *operands(20000, 30, 700, 1)), ("fp64tc4", *operands(20000, 31, 700, 2)),
+            ("fp64tc5", *operands(38900, 47, 300, 3)), ("bf16x6", *operands(3000, 700, 700, 4))]
+    torch.cuda.synchronize()
+
+    def repeat(job):
+        prec, A, B = job
+        stream = torch.cuda.Stream()
+        ctx = api.Context(0, stream)
+        try:
+            with torch.cuda.stream(stream):
+                ref = api.tc_gemm_nt(A, B, prec, ctx=ctx)
+                same = all(torch.equal(api.tc_gemm_nt(A, B, prec, ctx=ctx), ref) for _ in range(40))
+                return same and (prec == "bf16x6" or torch.equal(ref, sliced_product(A, B, int(prec[-1]))))
+        finally:
+            ctx.close()
+    with ThreadPoolExecutor(4) as ex:
+        assert all(ex.map(repeat, jobs))
