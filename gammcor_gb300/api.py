@@ -98,7 +98,8 @@ class Context:
 
     def set_gemm_tile(self, width: int):
         """Column tile of the sliced FP64-accurate GEMMs: 0 picks per product,
-        64/96/128 forces it (capped by the slice count); results are identical."""
+        64/96/128 forces it (capped by the slice count; the integrand's has 64); results are
+        identical."""
         check(self.h, load().gc_set_gemm_tile(self.h, int(width)))
 
     def eig_refine_stats(self) -> dict:

@@ -11,7 +11,8 @@
 // nearly cancels the diagonal correction, is summed in FP64. The sliced
 // precisions form one triangle of the Gram matrix instead,
 //   W = 2 sum_{i>j} (Kt_ij + Kt_ji)(Yk Yk^T)_ij + sum_i diag_i,
-// half the products, with one operand to slice and Kt itself in FP64.
+// on half the matrix, with one operand to slice and Kt itself in FP64 (NDimX 3774, FP64TC5: 1.16 ms, with
+// Kt Yk 3.1 ms; the error of W is that of the digits of Y alone).
 #include <cmath>
 
 #include "gc_internal.cuh"

@@ -370,7 +370,7 @@ __global__ void __launch_bounds__(192, 1)
 // C[r,c] = 2^(e_r+f_c) sum_{t+u<S} 2^-7(t+u+2) sum_k alpha_t[r,k] beta_u[c,k].
 // The products of one weight d = t+u share a TMEM accumulator; K is cut into
 // chunks short enough that every FP32 partial sum is an integer below 2^24, so
-// each chunk is exact, and the epilogue adds the chunks in FP64 registers.
+// each chunk is exact, and the epilogue adds the chunks in int64 registers.
 // Column tile (TBN rows of B): the S weight accumulators take S * TBN of the 512 TMEM
 // columns, so TBN = 128 for S = 4, 96 for S = 5 and 64 for S = 6 at most (half of them where two
 // CTAs share an SM: 48 for S <= 5, 32). A wider

@@ -46,7 +46,7 @@ int tc_gemm_nt(gc_context *ctx, int precision, int m, int n, int k, const double
 // Sliced precisions: part (one value per CTA of the product) adds up to
 // sum_{i > j} Klow[i,j] (Yk Yk^T)[i,j], and sq[i] = (Yk Yk^T)[i,i] in FP64, where Yk is the N x N
 // Y (column-major) with the columns outside lo < eig < hi left out. Klow: N x N, strict lower
-// triangle read.
+// triangle read. The product keeps one weight of the slices more than the others do.
 int tc_gram_dot(gc_context *ctx, int precision, int N, const double *Y, const double *eig, double lo,
                 double hi, const double *Klow, double *sq, DevBuf<double> &part);
 

@@ -120,8 +120,9 @@ int gc_set_chol_blocked(gc_context *ctx, int on);
 int gc_set_pipeline_wait(gc_context *ctx, unsigned long long ns);
 /* Column tile width of the FP64-accurate sliced GEMMs (GC_PREC_FP64TC4/5/6): 0
  * (the default) picks one per product from its shape, 64, 96 or 128 forces it
- * (capped at 128 for FP64TC4, 96 for FP64TC5, 64 for FP64TC6). Every width gives
- * the same result bits; only the speed differs. No counterpart in the reference. */
+ * (capped at 128 for FP64TC4, 96 for FP64TC5, 64 for FP64TC6; the integrand's
+ * product has 64 columns always). Every width gives the same result bits; only the
+ * speed differs. No counterpart in the reference. */
 int gc_set_gemm_tile(gc_context *ctx, int width);
 /* on = 1 (default): the batched AC calls (gc_ac_energy_batched, sessions) solve the FP32
  * eigenproblems of all lambda points of a system in one batched cuSOLVER call
